@@ -115,6 +115,25 @@ struct Ctx {
     int listState = 0;
     double listErrTol = 0.0;
     int64_t listEntries = 0;
+    // tile walks (idw_tile.cu): node order (per volume), term geometry (per
+    // surface definition); scales, lists and weight digits, valid for the current
+    // den0, tileErrTol and law (tileState 1; -1 when some node has no scale);
+    // motion records per surface
+    double volLo[3] = {0, 0, 0}, volHi[3] = {0, 0, 0};
+    int areaExp = 0;  // scales the largest node area to near one
+    bool tileOrderValid = false;
+    DevBuf<int> tileOrder;
+    DevBuf<float> tileScale;
+    DevBuf<float4> tileGeo, tileSums;
+    DevBuf<uint4> tileMot, tileDig, tileDig3;
+    DevBuf<unsigned> tileWord;  // 12 column maxima, the walk's counter, the bad flag
+    DevBuf<int64_t> tileOffs;
+    DevBuf<int> tileTerm;
+    DevBuf<unsigned> tileMask;
+    DevBuf<unsigned long long> tileCnt;
+    int tileState = 0, tileListState = 0;  // tileListState: 1 lists, 2 lists and digits, -1 too large, 0 not made
+    int64_t tileListEntries = 0;
+    double tileErrTol = 0.0, tileLdefFact = 0.0, tileAlphaToB = 0.0;
     // adjoint
     DevBuf<double> ptAdj, nodeAdj, xub, dxs;
     bool haveDxs = false;
@@ -288,14 +307,15 @@ int validate_options(Ctx *c, const idw_options *o) {
     return IDW_OK;
 }
 
-// Per-warp nodal properties and cluster aggregates of the current surface.
-int refresh_nodal(Ctx *c) {
+// Per-warp nodal properties and cluster aggregates of the current surface;
+// gated = 1 adds the FP32 motion arrays of the gated walks (mixed precision).
+int refresh_nodal(Ctx *c, int gated) {
     SurfaceDev s = surf_dev(c);
     launch_gather_xu(c->nUnique, c->xuInd.p, c->xs.p, c->xu.p, c->stream);
     launch_nodal(s, c->xu.p, c->ptXA.p, c->normals0.p, c->tmpAi.p, c->isCorner.p, c->opt.useRotations, c->ptMB.p,
                  c->stream);
     launch_set_data(tree_dev(c), c->ptMB.p, c->nodeMB.p, setdata_scratch(c), c->stream);
-    if (c->opt.precision == IDW_PREC_MIXED) {
+    if (gated && c->opt.precision == IDW_PREC_MIXED) {
         launch_mixed_nodal(c->nUnique, tree_dev(c), c->nodeMB.p, c->ptXA.p, c->ptMB.p, c->ptDM.p, c->ptDMl.p,
                            c->stream);
         launch_mixed_nodes(tree_dev(c), c->nodeMB.p, c->ptMB.p, c->nodeDC.p, c->nodeDCl.p, c->nodeDn.p, c->refDB.p,
@@ -314,6 +334,7 @@ int finish_den0(Ctx *c) {
     c->gdenValid = false;
     c->denPValid = false;
     c->listState = 0;
+    c->tileListState = c->tileState = 0;
     c->den0Valid = true;
     return IDW_OK;
 }
@@ -470,6 +491,10 @@ int idw_create_common_grid(void *ctx, const double *volnodes, int64_t nvol, int 
         if (volume_bbox(nvol, c->xv0.p, lo, hi, &nonFinite, c->stream))
             return fail(c, IDW_ERR_CUDA, "volume bounding box failed");
         if (nonFinite) return fail(c, IDW_ERR_NONFINITE, "non-finite volume coordinates");
+        for (int q = 0; q < 3; ++q) {
+            c->volLo[q] = lo[q];
+            c->volHi[q] = hi[q];
+        }
         DevBuf<unsigned long long> codes, codesAlt;
         DevBuf<int> idx;
         CKA(codes.alloc(nvol));
@@ -482,9 +507,11 @@ int idw_create_common_grid(void *ctx, const double *volnodes, int64_t nvol, int 
         if (e) return e;
     }
     c->haveVolume = true;
+    c->tileOrderValid = false;
     // a new volume needs a new initialize (records and estimates are per node)
     c->haveTree = false;
     c->listState = 0;
+    c->tileListState = c->tileState = 0;
     c->den0Valid = false;
     c->haveWarp = false;
     c->haveDxs = false;
@@ -753,6 +780,10 @@ int idw_initialize_warping(void *ctx, const double *pts, int32_t npts, const dou
     c->gdenValid = false;
     c->denPValid = false;
     c->listState = 0;
+    c->tileListState = c->tileState = 0;
+    double maxA = 0.0;
+    for (int i = 0; i < n; ++i) maxA = std::max(maxA, std::fabs(ai[i]));
+    c->areaExp = maxA > 0.0 && std::isfinite(maxA) ? -std::ilogb(maxA) : 0;
     c->den0Valid = false;
     CK(cudaStreamSynchronize(st));
     c->haveTree = true;
@@ -866,6 +897,151 @@ static int ensure_gate_den(Ctx *c, const TreeDevF &tf, const PointsDevF &pf, con
     return IDW_OK;
 }
 
+// The tile walks serve the fast mixed walk at the default exponents and the
+// default precision gate (or a looser one: their error is below the gate's).
+// A tighter gate asks for terms in double-float, which the gated walks have.
+// The FP32 reverse product (IDW_ADJ_FAST) divides by the gated walk's
+// denominators, so its forward walk stays the gated one, and so do the
+// diagnostics.  Three symmetry planes (8 mirror images) bound the scratch, and
+// kTileMost node images the weight digits (about 2.5 kB each); both limits
+// apply with the lists on and off, so the results agree.
+constexpr int64_t kTileMost = int64_t(1) << 25;
+
+static bool tile_applies(const Ctx *c, const EvalConsts &k) {
+    return c->opt.precision == IDW_PREC_MIXED && c->opt.evalMode == IDW_EVAL_FAST &&
+           c->opt.adjointPrecision == IDW_ADJ_PRECISE && c->opt.mixedGate >= 2e-3 && k.law.isInt && k.law.ia == 3 &&
+           k.law.ib == 5 && !k.slotStats && c->sym.nLoop <= 8 && c->nVol > 0 && c->nVol * c->sym.nLoop <= kTileMost;
+}
+
+static TileDev tile_dev(Ctx *c) {
+    TileDev td;
+    td.order = c->tileOrder.p;
+    td.scale = c->tileScale.p;
+    td.geo = c->tileGeo.p;
+    td.mot = c->tileMot.p;
+    td.colMax = c->tileWord.p;
+    td.counter = c->tileWord.p + 12;
+    td.areaExp = c->areaExp;
+    return td;
+}
+
+// Half of the free device memory holds `bytes` more.
+static int fits_half(Ctx *c, double bytes, bool &yes) {
+    size_t freeB = 0, totalB = 0;
+    CK(cudaMemGetInfo(&freeB, &totalB));
+    yes = bytes <= 0.5 * double(freeB);
+    return IDW_OK;
+}
+
+// What a tile walk needs besides the motions: node order, term geometry, node
+// scales, and (unless off) the lists and the weight digits, each when it fits.
+// use = false when the walk does not apply or some node has no scale.
+static int ensure_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalConsts &k, TileLists &lists,
+                       bool &use) {
+    lists = TileLists{};
+    use = tile_applies(c, k);
+    if (!use) return IDW_OK;
+    const bool off = c->opt.walkLists == IDW_WALK_LISTS_OFF;
+    if (c->tileErrTol != c->opt.errTol) c->tileState = c->tileListState = 0;
+    if (c->tileLdefFact != c->opt.LdefFact || c->tileAlphaToB != k.law.alphaToBexp) c->tileState = 0;  // the lists stay
+    if (c->tileState == 0 || (c->tileState == 1 && !off && c->tileListState == 0)) {
+        const size_t nTerms = size_t(c->nUnique) + size_t(c->nNodes);
+        const int64_t units = walk_list_warps(c->nVol) * c->sym.nLoop;
+        const bool newLists = !off && c->tileListState == 0;
+        c->tileState = 0;
+        if (newLists) {
+            c->tileTerm.release();
+            c->tileMask.release();
+            c->tileDig.release();
+            c->tileDig3.release();
+            CKA(c->tileOffs.alloc(size_t(units) + 1));
+        }
+        CKA(c->tileGeo.alloc(2 * nTerms));
+        CKA(c->tileMot.alloc(8 * nTerms));
+        CKA(c->tileWord.alloc(14));
+        CKA(c->tileScale.alloc(size_t(c->nVol)));
+        CKA(c->tileSums.alloc(2 * size_t(c->sym.nLoop) * size_t(c->nVol)));
+        CKA(c->tileOrder.alloc(size_t(c->nVol)));
+        if (!c->tileOrderValid) {
+            const int rc = tile_order(vol_dev(c), c->volLo, c->volHi, c->tileOrder.p, c->stream);
+            if (rc) return fail(c, rc == -2 ? IDW_ERR_NOMEM : IDW_ERR_CUDA, "node order of the tile walks failed");
+            c->tileOrderValid = true;
+        }
+        launch_tile_geo(tree_dev(c), c->nUnique, c->ptXA.p, c->areaExp, c->tileGeo.p, c->stream);
+        int *bad = reinterpret_cast<int *>(c->tileWord.p + 13);
+        const int64_t total = count_tile_lists(tree_dev(c), tf, vol_dev(c), rec, k, tile_dev(c),
+                                               newLists ? c->tileOffs.p : nullptr, c->tileScale.p, bad, c->stream);
+        if (total < 0) return fail(c, IDW_ERR_CUDA, "walk lists: count pass failed");
+        int badH = 0;
+        CK(cudaMemcpyAsync(&badH, bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaStreamSynchronize(c->stream));
+        bool fits = false;
+        if (newLists && !badH) {
+            c->tileListEntries = total;
+            int rc = fits_half(c, 8.0 * double(total), fits);
+            if (rc) return rc;
+            if (fits) {
+                CKA(c->tileCnt.alloc(8));
+                CKA(c->tileTerm.alloc(size_t(std::max<int64_t>(total, 1))));
+                CKA(c->tileMask.alloc(size_t(std::max<int64_t>(total, 1))));
+                CK(cudaMemsetAsync(c->tileCnt.p, 0, 8 * sizeof(unsigned long long), c->stream));
+                launch_tile_record(tree_dev(c), tf, vol_dev(c), rec, k, tile_dev(c), c->tileOffs.p, c->tileTerm.p,
+                                   c->tileMask.p, c->tileCnt.p, c->stream);
+                rc = check_launch(c, "walk lists");
+                if (rc) return rc;
+            }
+            c->tileListState = fits ? 1 : -1;
+        }
+        if (!off && !badH && c->tileListState > 0) {
+            const size_t steps = size_t(std::max<int64_t>(c->tileListEntries / 16, 1));
+            if (c->tileListState == 1) {
+                int rc = fits_half(c, 256.0 * sizeof(uint4) * double(steps), fits);
+                if (rc) return rc;
+                if (fits) {
+                    CKA(c->tileDig.alloc(192 * steps));
+                    CKA(c->tileDig3.alloc(64 * steps));
+                    c->tileListState = 2;
+                }
+            }
+            if (c->tileListState == 2) {
+                lists.offs = c->tileOffs.p;
+                lists.term = c->tileTerm.p;
+                lists.mask = c->tileMask.p;
+                launch_tile_build(vol_dev(c), rec, k, tile_dev(c), lists, c->nUnique, c->tileDig.p, c->tileDig3.p,
+                                  c->stream);
+                int rc = check_launch(c, "weight digits");
+                if (rc) return rc;
+            }
+        }
+        c->tileErrTol = c->opt.errTol;
+        c->tileLdefFact = c->opt.LdefFact;
+        c->tileAlphaToB = k.law.alphaToBexp;
+        c->tileState = badH ? -1 : 1;
+    }
+    use = c->tileState == 1;
+    lists = TileLists{};
+    if (use && !off && c->tileListState > 0) {
+        lists.offs = c->tileOffs.p;
+        lists.term = c->tileTerm.p;
+        lists.mask = c->tileMask.p;
+        lists.counters = c->tileCnt.p;
+        if (c->tileListState == 2) {
+            lists.dig = c->tileDig.p;
+            lists.dig3 = c->tileDig3.p;
+        }
+    }
+    return IDW_OK;
+}
+
+// A tile walk over the motions (ptMB, nodeMB).
+static int run_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalConsts &k, const TileLists &lists,
+                    const double *ptMB, const double *nodeMB, const WalkOut &o) {
+    launch_tile_motions(tree_dev(c), c->nUnique, ptMB, nodeMB, c->tileWord.p, c->tileMot.p, c->refDB.p, c->stream);
+    CK(cudaEventRecord(c->ev0, c->stream));
+    launch_tile_walk(tree_dev(c), tf, vol_dev(c), rec, k, tile_dev(c), lists, c->refDB.p, c->tileSums.p, o, c->stream);
+    return IDW_OK;
+}
+
 // Before the warped grid is overwritten: if an asynchronous read of the
 // current grid may still run, the next grid goes to the other buffer; an
 // older read of that buffer (one warp back) is waited for on the stream.
@@ -890,8 +1066,7 @@ static int prepare_xv_write(Ctx *c) {
 static int run_warp(Ctx *c, double *xvOut, double *denOut) {
     if (!c->haveTree) return fail(c, IDW_ERR_STATE, "setSurfaceDefinition must come first");
     if (int e0 = ensure_den0(c)) return e0;
-    int rc = refresh_nodal(c);
-    if (rc) return rc;
+    int rc;
     EvalConsts k;
     k.law = make_law(c);
     k.errTol = c->opt.errTol;
@@ -910,8 +1085,20 @@ static int run_warp(Ctx *c, double *xvOut, double *denOut) {
     CK(cudaMemsetAsync(c->counters.p, 0, 8 * sizeof(unsigned long long), c->stream));
     CK(cudaEventRecord(c->ev0, c->stream));
     const int exact = c->opt.evalMode == IDW_EVAL_EXACT;
-    if (c->opt.precision == IDW_PREC_MIXED) {
-        const TreeDevF tf = tree_devf(c);
+    const TreeDevF tf = tree_devf(c);
+    WalkRecF rec;
+    rec.hi = c->recHi.p;
+    rec.lo = c->recLo.p;
+    TileLists lists;
+    bool tile = false;
+    rc = ensure_tile(c, tf, rec, k, lists, tile);
+    if (rc) return rc;
+    rc = refresh_nodal(c, !tile);
+    if (rc) return rc;
+    if (tile) {
+        rc = run_tile(c, tf, rec, k, lists, c->ptMB.p, c->nodeMB.p, o);
+        if (rc) return rc;
+    } else if (c->opt.precision == IDW_PREC_MIXED) {
         PointsDevF pf;
         pf.da = c->ptDA.p;
         pf.dl = c->ptDL.p;
@@ -923,9 +1110,6 @@ static int run_warp(Ctx *c, double *xvOut, double *denOut) {
         af.dn = c->nodeDn.p;
         af.ref = c->refDB.p;
         af.rr = c->replayRec.p;
-        WalkRecF rec;
-        rec.hi = c->recHi.p;
-        rec.lo = c->recLo.p;
         int rc2 = ensure_walk_lists(c, tf, rec, k);
         if (rc2) return rc2;
         rc2 = ensure_gate_den(c, tf, pf, af, rec, k, exact);
@@ -952,7 +1136,9 @@ static int read_counters(Ctx *c) {
     c->stats.visited = int64_t(h[2]);
     c->stats.fp64Fallback = int64_t(h[3]);
     c->stats.preciseTerms = int64_t(h[6]);
-    c->stats.walkListEntries = c->listState == 1 ? c->listEntries : (c->listState == -1 ? -1 : 0);
+    // the lists of the walk in use
+    const int ls = c->tileState == 1 ? c->tileListState : c->listState;
+    c->stats.walkListEntries = ls > 0 ? (c->tileState == 1 ? c->tileListEntries : c->listEntries) : (ls == -1 ? -1 : 0);
     if (c->eventsRecorded) {
         float ms = 0.f;
         if (cudaEventElapsedTime(&ms, c->ev0, c->ev1) == cudaSuccess) c->stats.lastKernelMs = ms;
@@ -1073,6 +1259,29 @@ int idw_get_volume_coordinates_cs(void *ctx, double *out, int64_t ndof, int wher
 // and a finalisation per surface.  coords/out are device pointers.
 static constexpr int kBatchWalk = kBatchMax;
 
+// run_warp_batch_mixed by tile walks, one per surface.
+static int run_tile_batch(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalConsts &k, const TileLists &lists,
+                          const double *coordsDev, int nb, double *outDev) {
+    const int n = c->nUnique;
+    const size_t sdof = 3 * size_t(c->nPts), vdof = 3 * size_t(c->nVol);
+    c->nodalValid = false;
+    const SurfaceDev s = surf_dev(c);
+    for (int b = 0; b < nb; ++b) {
+        launch_gather_xu(n, c->xuInd.p, coordsDev + size_t(b) * sdof, c->xu.p, c->stream);
+        launch_nodal(s, c->xu.p, c->ptXA.p, c->normals0.p, c->tmpAi.p, c->isCorner.p, c->opt.useRotations, c->ptMB.p,
+                     c->stream);
+        launch_set_data(tree_dev(c), c->ptMB.p, c->nodeMB.p, setdata_scratch(c), c->stream);
+        WalkOut o;
+        o.xv = outDev + size_t(b) * vdof;
+        o.counters = b == 0 ? c->counters.p : nullptr;
+        int rc = run_tile(c, tf, rec, k, lists, c->ptMB.p, c->nodeMB.p, o);
+        if (rc) return rc;
+    }
+    CK(cudaEventRecord(c->ev1, c->stream));
+    c->eventsRecorded = true;
+    return check_launch(c, "batch walk");
+}
+
 // tangent = 1: coordsDev holds surface tangents dXs; the walk then uses the
 // tangent nodal properties (Md + I, bd) at the current surface and writes
 // dXv = num / den (warpDerivFwd for nb directions), gated by tangentGate.
@@ -1080,6 +1289,21 @@ static int run_warp_batch_mixed(Ctx *c, const double *coordsDev, int nb, double 
                                 double tangentGate = 0.0) {
     const int n = c->nUnique, nn = c->nNodes;
     const size_t sdof = 3 * size_t(c->nPts), vdof = 3 * size_t(c->nVol);
+    {
+        EvalConsts k{};
+        k.law = make_law(c);
+        k.errTol = c->opt.errTol;
+        k.sym = c->sym;
+        const TreeDevF tf = tree_devf(c);
+        WalkRecF rec;
+        rec.hi = c->recHi.p;
+        rec.lo = c->recLo.p;
+        TileLists lists;
+        bool tile = false;
+        int rc = tangent ? IDW_OK : ensure_tile(c, tf, rec, k, lists, tile);
+        if (rc) return rc;
+        if (tile) return run_tile_batch(c, tf, rec, k, lists, coordsDev, nb, outDev);
+    }
     if (c->batchCap < nb) {
         const size_t B = kBatchWalk;
         CKA(c->bXu.alloc(B * 3 * n));
@@ -1523,7 +1747,7 @@ static int run_deriv(Ctx *c, const double *dxvDev, int nSeeds, int64_t seedStrid
     }
     if (int e0 = ensure_den0(c)) return e0;
     if (!c->haveWarp) return fail(c, IDW_ERR_STATE, "warpMesh must be called before warpDeriv");
-    int rc = refresh_nodal(c);
+    int rc = refresh_nodal(c, 0);  // the reverse walks read no motions
     if (rc) return rc;
     EvalConsts k;
     k.law = make_law(c);
@@ -1795,6 +2019,10 @@ int run_deriv_fwd(Ctx *c, const double *xsdDev, double *xvdDev) {
     o.tangent = 1;
     o.denIn = c->den.p;
     CK(cudaMemsetAsync(c->counters.p, 0, 8 * sizeof(unsigned long long), c->stream));
+    const TreeDevF tf = tree_devf(c);
+    WalkRecF rec;
+    rec.hi = c->recHi.p;
+    rec.lo = c->recLo.p;
     if (mixed) {
         // the gate scales with the size of the tangent instead of Ldef
         CK(cudaMemsetAsync(c->counters.p + 7, 0, sizeof(unsigned long long), c->stream));
@@ -1813,7 +2041,6 @@ int run_deriv_fwd(Ctx *c, const double *xsdDev, double *xvdDev) {
                            c->stream);
         launch_replay_records(c->nNodes, c->nodeDC.p, c->nodeDn.p, c->replayRec.p, c->stream);
         c->nodalValid = false;
-        const TreeDevF tf = tree_devf(c);
         PointsDevF pf;
         pf.da = c->ptDA.p;
         pf.dl = c->ptDL.p;
@@ -1825,15 +2052,12 @@ int run_deriv_fwd(Ctx *c, const double *xsdDev, double *xvdDev) {
         af.dn = c->nodeDn.p;
         af.ref = c->refDB.p;
         af.rr = c->replayRec.p;
-        WalkRecF rec;
-        rec.hi = c->recHi.p;
-        rec.lo = c->recLo.p;
-        rec.gden = c->gdenValid ? c->gden.p : nullptr;
-        if (c->listState == 1 && c->listErrTol == c->opt.errTol && !exact) {
-            k.lists.offs = c->walkOffs.p;
-            k.lists.list = c->walkList.p;
-            k.lists.counters = c->walkCnt.p;
-        }
+        // the gated walk's lists and denominators (the tile walks have their own)
+        rc = ensure_walk_lists(c, tf, rec, k);
+        if (rc) return rc;
+        rc = ensure_gate_den(c, tf, pf, af, rec, k, exact);
+        if (rc) return rc;
+        rec.gden = c->gden.p;
         CK(cudaEventRecord(c->ev0, c->stream));
         launch_walk_mixed(tree_dev(c), tf, pf, af, vol_dev(c), rec, k, exact, c->acc.p, o, c->stream);
     } else {
@@ -1979,7 +2203,7 @@ int idw_get_nodal_properties(void *ctx, double *mi, double *bi) {
     if (!c->haveTree) return fail(c, IDW_ERR_STATE, "setSurfaceDefinition must come first");
     CK(cudaSetDevice(c->device));
     if (!c->nodalValid) {
-        int rc = refresh_nodal(c);
+        int rc = refresh_nodal(c, 0);
         if (rc) return rc;
     }
     const int n = c->nUnique;
@@ -2051,7 +2275,7 @@ int idw_warp_deriv_noalloc(void *ctx, const double *dxv, int64_t ndof, double *d
     int rc = noalloc_scratch(c, &scratch);
     if (rc) return rc;
     double *ptAdj = scratch, *nodeAdj = scratch + 12 * size_t(n), *ptRel = nodeAdj + 12 * size_t(nn);
-    rc = refresh_nodal(c);
+    rc = refresh_nodal(c, 0);
     if (rc) return rc;
     EvalConsts k;
     k.law = make_law(c);

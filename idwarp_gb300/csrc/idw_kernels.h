@@ -213,6 +213,49 @@ void launch_walk_record(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v
 void launch_walk_replay(const TreeDevF &tf, const PointsDevF &pf, const NodeAggF &af, const VolumeDev &v,
                         const WalkRecF &rec, const EvalConsts &k, float4 *acc, unsigned long long *counters,
                         cudaStream_t st);
+
+// Tile walks (idw_tile.cu): the terms of a fast walk as matrix products.
+// Lists: per unit (group of 32 volume nodes in tile order, mirror), entries
+// (term, node mask) in whole steps of 16; a term is a point, or nPts + tree
+// node for a cluster.
+struct TileLists {
+    const int64_t *offs = nullptr;  // units + 1 entry offsets
+    const int *term = nullptr;      // null: the walk decides as it goes
+    const unsigned *mask = nullptr;
+    const uint4 *dig = nullptr;     // per step 192: the first three digits of the weights; null: formed as it goes
+    const uint4 *dig3 = nullptr;    // per step 64: the fourth
+    const unsigned long long *counters = nullptr;  // the recording walk's, as WalkLists::counters
+};
+struct TileDev {
+    const int *order;        // tile slot -> walk (Morton) index of a volume node
+    const float *scale;      // per slot: power-of-two weight scale P
+    const float4 *geo;       // per term: (x high, area 2^areaExp high), the low parts
+    const uint4 *mot;        // per term: 8 x 16 bytes, the FP16 digits of its motion (k_tile_mot)
+    const unsigned *colMax;  // largest magnitude of each motion column (float bits)
+    unsigned *counter;       // the walk's next unit (behind colMax: launch_tile_motions clears both)
+    int areaExp;
+};
+// Tile order of the volume nodes (lo, hi: their bounding box).  Returns 0, -1 on
+// a CUDA error, -2 without memory; synchronises st.
+int tile_order(const VolumeDev &v, const double *lo, const double *hi, int *order, cudaStream_t st);
+void launch_tile_geo(const TreeDev &t, int nPts, const dbl4 *xa, int areaExp, float4 *geo, cudaStream_t st);
+// Fills scale, raises *bad when a node has none, fills offs (unless null) and
+// returns the number of entries (-1 on a CUDA error); synchronises st.
+int64_t count_tile_lists(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
+                         const EvalConsts &k, const TileDev &td, int64_t *offs, float *scale, int *bad,
+                         cudaStream_t st);
+void launch_tile_record(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
+                        const EvalConsts &k, const TileDev &td, const int64_t *offs, int *term, unsigned *mask,
+                        unsigned long long *counters, cudaStream_t st);
+void launch_tile_build(const VolumeDev &v, const WalkRecF &rec, const EvalConsts &k, const TileDev &td,
+                       const TileLists &lists, int nPts, uint4 *dig, uint4 *dig3, cudaStream_t st);
+// The current motions (12 per point and tree node) as motion records, and the reference motion.
+void launch_tile_motions(const TreeDev &t, int nPts, const double *ptMB, const double *nodeMB, unsigned *colMax,
+                         uint4 *mot, float *refDB, cudaStream_t st);
+// sums: 2 nLoop nVol float4 of scratch.
+void launch_tile_walk(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
+                      const EvalConsts &k, const TileDev &td, const TileLists &lists, const float *refDB, float4 *sums,
+                      const WalkOut &o, cudaStream_t st);
 // Exact mode as a tiled N-body kernel (idw_exact.cu); launch_walk_mixed uses
 // it for exact = 1.  Fills acc like the walk; no finalisation.
 void launch_exact_mixed(const TreeDevF &tf, const PointsDevF &pf, const NodeAggF &af, const VolumeDev &v,

@@ -87,7 +87,10 @@ typedef struct idw_options {
                            * mixedGate * Ldef0 * den (times 2/nLoop beyond one symmetry
                            * plane) is summed in double-float (S' = the term's motion
                            * less the mean surface motion, den = the node's
-                           * denominator; default 2e-3; 0 = every term) */
+                           * denominator; default 2e-3; 0 = every term).  At the default
+                           * exponents and a gate of 2e-3 or more the fast walk needs no
+                           * such terms: its sums are matrix products of weights in
+                           * double-float (idw_tile.cu) */
     int32_t exactSchedule; /* mixed exact mode: IDW_EXACT_AUTO (default: tiled
                             * kernel when the mesh fills the GPU, else the walk),
                             * IDW_EXACT_TILED or IDW_EXACT_WALK; same sums either way */
@@ -98,7 +101,9 @@ typedef struct idw_options {
                            * walk's open/approximate decisions depend on the set-up state
                            * and errTol only, so they can be recorded once (per warp of 32
                            * volume nodes: the tree nodes where a lane approximates or sums
-                           * a leaf) and replayed by every later warp; same sums either way */
+                           * a leaf) and replayed by every later warp; at the default exponents
+                           * and gate the recorded terms' weights are kept too, when they fit
+                           * (8 bytes per node and term); same sums either way */
     int32_t treeBuild;    /* IDW_TREE_KD (default) or IDW_TREE_MORTON; read by
                            * idw_initialize_warping, as bucketSize */
     int32_t deterministic; /* 0 (default): reverse products (idw_warp_deriv*) land their sums with
@@ -128,7 +133,7 @@ typedef struct idw_stats {
     int64_t warpLeafSlots; /* lane slots of warp-level leaf visits (32 x leaf size); leafPairs / this = lane use */
     int64_t warpNodeSlots; /* lane slots of warp-level interior-node visits (32 per visit) */
     int64_t preciseTerms;  /* mixed mode: cluster terms summed in double-float */
-    int64_t walkListEntries; /* recorded walk decisions (8 bytes each; -1: too large, walks decide) */
+    int64_t walkListEntries; /* recorded list entries of the walk in use (8 bytes each; -1: too large, walks decide) */
     double treeBuildMs;   /* host wall time of the last surface tree build (kd or Morton, with its copies) */
 } idw_stats;
 
