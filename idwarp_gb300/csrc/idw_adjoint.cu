@@ -383,7 +383,9 @@ __global__ void __launch_bounds__(128) k_adjoint_mixed(TreeDev t, TreeDevF tf, P
 //   Bib_i = B_i + sum_q Bq/n_q
 //   Mrel_i = P_i - (Xu0_i - C_L) (x) B_i + sum_q (Pq + (C_q - Xu0_i) (x) Bq)/n_q
 // where q runs over the interior ancestors of point i.  FP64, one thread per
-// (point, seed).
+// (point, seed).  TILE: the layout of the tile adjoint, [r][w, k] with the point
+// moments about the point itself.
+template <bool TILE>
 __global__ void k_adjoint_combine(TreeDev t, const dbl4 *ptXA, int nPts, int nSeeds, const double *ptAcc,
                                   int64_t ptStride, const double *nodeAcc, int64_t nodeStride, double *out) {
     const int64_t tid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -402,23 +404,25 @@ __global__ void k_adjoint_combine(TreeDev t, const dbl4 *ptXA, int nPts, int nSe
         const double dc[3] = {g.x - X[0], g.y - X[1], g.z - X[2]};
 #pragma unroll
         for (int r = 0; r < 3; ++r) {
-            B[r] += a[9 + r] * on;
+            const double w = a[TILE ? 4 * r : 9 + r];
+            B[r] += w * on;
 #pragma unroll
-            for (int k = 0; k < 3; ++k) M[3 * r + k] += (a[3 * r + k] + dc[k] * a[9 + r]) * on;
+            for (int k = 0; k < 3; ++k) M[3 * r + k] += (a[TILE ? 4 * r + 1 + k : 3 * r + k] + dc[k] * w) * on;
         }
         const int4 li = t.info[q + 1];
         q = (i <= li.y) ? q + 1 : li.z;
     }
     // q is now the leaf of point i
     const dbl4 g = t.geom[q];
-    const double dl[3] = {X[0] - g.x, X[1] - g.y, X[2] - g.z};
+    const double dl[3] = {TILE ? 0.0 : X[0] - g.x, TILE ? 0.0 : X[1] - g.y, TILE ? 0.0 : X[2] - g.z};
     const double *p = ptAcc + sd * ptStride + 12 * int64_t(i);
     double *o = out + sd * ptStride + 12 * int64_t(i);
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
-        o[9 + r] = p[9 + r] + B[r];
+        const double w = p[TILE ? 4 * r : 9 + r];
+        o[9 + r] = w + B[r];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) o[3 * r + k] = p[3 * r + k] - dl[k] * p[9 + r] + M[3 * r + k];
+        for (int k = 0; k < 3; ++k) o[3 * r + k] = p[TILE ? 4 * r + 1 + k : 3 * r + k] - dl[k] * w + M[3 * r + k];
     }
 }
 
@@ -467,11 +471,12 @@ void launch_adj_law(const TreeDev &t, const TreeDevF &tf, const PointsDevF &pf, 
 }  // namespace
 
 void launch_adjoint_combine(const TreeDev &t, const dbl4 *ptXA, int nPts, int nSeeds, const double *ptAcc,
-                            const double *nodeAcc, double *ptAdj, cudaStream_t st) {
+                            const double *nodeAcc, double *ptAdj, cudaStream_t st, int tile) {
     const int64_t total = int64_t(nPts) * nSeeds;
     if (total <= 0) return;
-    k_adjoint_combine<<<int((total + 127) / 128), 128, 0, st>>>(t, ptXA, nPts, nSeeds, ptAcc, 12 * int64_t(nPts),
-                                                                nodeAcc, 12 * int64_t(t.nNodes), ptAdj);
+    auto kernel = tile ? k_adjoint_combine<true> : k_adjoint_combine<false>;
+    kernel<<<int((total + 127) / 128), 128, 0, st>>>(t, ptXA, nPts, nSeeds, ptAcc, 12 * int64_t(nPts), nodeAcc,
+                                                     12 * int64_t(t.nNodes), ptAdj);
 }
 
 int launch_adjoint_mixed(const TreeDev &t, const TreeDevF &tf, const PointsDevF &pf, const VolumeDev &v,
@@ -518,8 +523,8 @@ int launch_adjoint_mixed(const TreeDev &t, const TreeDevF &tf, const PointsDevF 
     }
     if (!combine) return 0;
     const int64_t total = int64_t(nPts) * nSeeds;
-    k_adjoint_combine<<<int((total + 127) / 128), 128, 0, st>>>(t, ptXA, nPts, nSeeds, ptAcc, ptStride, nodeAcc,
-                                                                nodeStride, ptAdj);
+    k_adjoint_combine<false><<<int((total + 127) / 128), 128, 0, st>>>(t, ptXA, nPts, nSeeds, ptAcc, ptStride, nodeAcc,
+                                                                       nodeStride, ptAdj);
     return 0;
 }
 

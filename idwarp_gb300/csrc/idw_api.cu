@@ -125,12 +125,14 @@ struct Ctx {
     DevBuf<int> tileOrder;
     DevBuf<float> tileScale;
     DevBuf<float4> tileGeo, tileSums;
-    DevBuf<uint4> tileMot, tileDig, tileDig3;
+    DevBuf<uint4> tileMot, tileDig, tileDig3, tileDig4;
+    DevBuf<double> tileDenInv;
     DevBuf<unsigned> tileWord;  // 12 column maxima, the walk's counter, the bad flag
     DevBuf<int64_t> tileOffs;
     DevBuf<int> tileTerm;
     DevBuf<unsigned> tileMask;
     DevBuf<unsigned long long> tileCnt;
+    int tileFifthState = 0;  // the reverse product's fifth digit and denominators: 1 made, -1 too large, 0 not made
     int tileState = 0, tileListState = 0;  // tileListState: 1 lists, 2 lists and digits, -1 too large, 0 not made
     int64_t tileListEntries = 0;
     double tileErrTol = 0.0, tileLdefFact = 0.0, tileAlphaToB = 0.0;
@@ -954,6 +956,7 @@ static int ensure_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const Ev
             c->tileMask.release();
             c->tileDig.release();
             c->tileDig3.release();
+            c->tileDig4.release();
             CKA(c->tileOffs.alloc(size_t(units) + 1));
         }
         CKA(c->tileGeo.alloc(2 * nTerms));
@@ -1007,6 +1010,7 @@ static int ensure_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const Ev
                 lists.offs = c->tileOffs.p;
                 lists.term = c->tileTerm.p;
                 lists.mask = c->tileMask.p;
+                c->tileFifthState = 0;
                 launch_tile_build(vol_dev(c), rec, k, tile_dev(c), lists, c->nUnique, c->tileDig.p, c->tileDig3.p,
                                   c->stream);
                 int rc = check_launch(c, "weight digits");
@@ -1039,6 +1043,37 @@ static int run_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalC
     launch_tile_motions(tree_dev(c), c->nUnique, ptMB, nodeMB, c->tileWord.p, c->tileMot.p, c->refDB.p, c->stream);
     CK(cudaEventRecord(c->ev0, c->stream));
     launch_tile_walk(tree_dev(c), tf, vol_dev(c), rec, k, tile_dev(c), lists, c->refDB.p, c->tileSums.p, o, c->stream);
+    return IDW_OK;
+}
+
+// The reverse product from the weight digits: what ensure_tile gives, the fifth
+// digit (when it fits) and the reciprocal denominators of the digits' weights,
+// both once per mesh and weight law.
+static int ensure_tile_adjoint(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalConsts &k, TileLists &lists,
+                               bool &use) {
+    int rc = ensure_tile(c, tf, rec, k, lists, use);
+    if (rc) return rc;
+    use = use && lists.dig && c->tileFifthState >= 0;
+    if (use && c->tileFifthState == 0) {
+        const size_t steps = size_t(std::max<int64_t>(c->tileListEntries / 16, 1));
+        bool fits = false;
+        rc = fits_half(c, 64.0 * sizeof(uint4) * double(steps) + 8.0 * double(c->nVol), fits);
+        if (rc) return rc;
+        c->tileFifthState = fits ? 1 : -1;
+        use = fits;
+        if (fits) {
+            CKA(c->tileDig4.alloc(64 * steps));
+            CKA(c->tileDenInv.alloc(size_t(c->nVol)));
+            lists.dig4 = c->tileDig4.p;
+            launch_tile_build(vol_dev(c), rec, k, tile_dev(c), lists, c->nUnique, nullptr, c->tileDig4.p, c->stream);
+            launch_tile_den_inv(c->nVol, c->sym.nLoop, lists, reinterpret_cast<double *>(c->tileSums.p),
+                                c->tileDenInv.p, c->stream);
+            rc = check_launch(c, "fifth digits");
+            if (rc) return rc;
+            CK(cudaEventRecord(c->ev0, c->stream));
+        }
+    }
+    lists.dig4 = c->tileDig4.p;
     return IDW_OK;
 }
 
@@ -1789,8 +1824,13 @@ static int run_deriv(Ctx *c, const double *dxvDev, int nSeeds, int64_t seedStrid
     WalkRecF rec;
     rec.hi = c->recHi.p;
     rec.lo = c->recLo.p;
-    bool precise = false;
-    if (mixed) {
+    bool precise = false, tile = false;
+    TileLists tileLists;
+    if (mixed && !det) {
+        rc = ensure_tile_adjoint(c, tf, rec, k, tileLists, tile);
+        if (rc) return rc;
+    }
+    if (mixed && !tile) {
         rc = ensure_walk_lists(c, tf, rec, k);
         if (rc) return rc;
         precise = c->opt.adjointPrecision == IDW_ADJ_PRECISE && precise_adjoint_supported(k.law);
@@ -1810,7 +1850,10 @@ static int run_deriv(Ctx *c, const double *dxvDev, int nSeeds, int64_t seedStrid
     }
     // the reverse walk: point and cluster moments land in ptAdj / nodeAdj
     auto walk = [&](int) -> int {
-        if (mixed && precise)
+        if (tile)
+            launch_tile_adjoint(vol_dev(c), rec, k, tile_dev(c), tileLists, n, nn, c->tileDenInv.p, dxvDev, nSeeds,
+                                seedStride, ptAdj.p, nodeAdj.p, c->counters.p, c->stream);
+        else if (mixed && precise)
             launch_adjoint_precise(tree_dev(c), tf, pf, vol_dev(c), rec, k, exact, dxvDev, nSeeds, seedStride,
                                    c->denP.p, ptAdj.p, nodeAdj.p, n, c->counters.p, c->stream, det);
         else if (mixed)
@@ -1839,7 +1882,8 @@ static int run_deriv(Ctx *c, const double *dxvDev, int nSeeds, int64_t seedStrid
     }
     if (rc) return rc;
     // the relative moments and the cluster shares (setData_b folded in)
-    if (mixed) launch_adjoint_combine(tree_dev(c), c->ptXA.p, n, nSeeds, ptAdj.p, nodeAdj.p, ptRel.p, c->stream);
+    if (mixed)
+        launch_adjoint_combine(tree_dev(c), c->ptXA.p, n, nSeeds, ptAdj.p, nodeAdj.p, ptRel.p, c->stream, tile);
     CK(cudaEventRecord(c->ev1, c->stream));
     c->eventsRecorded = true;
     rc = check_launch(c, "adjoint walk");

@@ -224,6 +224,7 @@ struct TileLists {
     const unsigned *mask = nullptr;
     const uint4 *dig = nullptr;     // per step 192: the first three digits of the weights; null: formed as it goes
     const uint4 *dig3 = nullptr;    // per step 64: the fourth
+    const uint4 *dig4 = nullptr;    // per step 64: the fifth, which only the reverse product reads
     const unsigned long long *counters = nullptr;  // the recording walk's, as WalkLists::counters
 };
 struct TileDev {
@@ -256,6 +257,17 @@ void launch_tile_motions(const TreeDev &t, int nPts, const double *ptMB, const d
 void launch_tile_walk(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
                       const EvalConsts &k, const TileDev &td, const TileLists &lists, const float *refDB, float4 *sums,
                       const WalkOut &o, cudaStream_t st);
+int tile_sms();
+// Reverse product from the kept digits (idw_tile_adjoint.cu).  denInv: per slot
+// the reciprocal denominator in the digits' units; part: nLoop * nVol doubles of
+// scratch.  ptAdj, nodeAdj: per seed and term 12 sums, [axis][moment 1, x, y, z]
+// about the point or the cluster's centroid.
+void launch_tile_den_inv(int64_t nVol, int nLoop, const TileLists &lists, double *part, double *denInv,
+                         cudaStream_t st);
+void launch_tile_adjoint(const VolumeDev &v, const WalkRecF &rec, const EvalConsts &k, const TileDev &td,
+                         const TileLists &lists, int nPts, int nNodes, const double *denInv, const double *dxv,
+                         int nSeeds, int64_t dxvStride, double *ptAdj, double *nodeAdj, unsigned long long *counters,
+                         cudaStream_t st);
 // Exact mode as a tiled N-body kernel (idw_exact.cu); launch_walk_mixed uses
 // it for exact = 1.  Fills acc like the walk; no finalisation.
 void launch_exact_mixed(const TreeDevF &tf, const PointsDevF &pf, const NodeAggF &af, const VolumeDev &v,
@@ -299,8 +311,10 @@ int launch_adjoint_mixed(const TreeDev &t, const TreeDevF &tf, const PointsDevF 
                          int maxGroup = 16, int combine = 1, int det = 0);
 // Point and cluster moments of a mixed reverse walk -> the relative point
 // adjoints of the reverse nodal properties (setData_b folded in).
+// tile: the accumulators are the tile adjoint's (layout [axis][moment 1, x, y, z],
+// point moments about the points).
 void launch_adjoint_combine(const TreeDev &t, const dbl4 *ptXA, int nPts, int nSeeds, const double *ptAcc,
-                            const double *nodeAcc, double *ptAdj, cudaStream_t st);
+                            const double *nodeAcc, double *ptAdj, cudaStream_t st, int tile = 0);
 // Precise (double-float) mixed reverse walk and its denominator walk
 // (idw_adjoint_precise.cu); integer exponents only.
 bool precise_adjoint_supported(const WeightLaw &wl);

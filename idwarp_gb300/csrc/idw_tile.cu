@@ -231,44 +231,9 @@ __device__ __forceinline__ void unit_rows(TileRows *rows, const VolumeDev &v, co
     __syncwarp();
 }
 
-// Work distribution of the persistent kernels: units are taken from a global
-// counter in chunks of consecutive ones, shared by the warps of a block (their
-// terms overlap, so the block's L1 serves them together).  state holds the
-// block's chunk as (end << 32 | next).  A warp that finds it empty takes the
-// next chunk for the block; if another warp published one meanwhile, it keeps
-// what was left of that to itself.  Nothing waits.
-struct UnitQueue {
-    unsigned long long *state;
-    unsigned *counter;
-    unsigned total, chunk, p, pe;
-    __device__ __forceinline__ bool next(unsigned &unit) {
-        unsigned u = 0xffffffffu;
-        if ((threadIdx.x & 31) == 0) {
-            if (p < pe) {
-                u = p++;
-            } else {
-                const unsigned long long s = atomicAdd(state, 1ull);
-                if (unsigned(s) < unsigned(s >> 32)) {
-                    u = unsigned(s);
-                } else {
-                    const unsigned c = atomicAdd(counter, chunk);
-                    if (c < total) {
-                        u = c;
-                        const unsigned e = min(c + chunk, total);
-                        const unsigned long long o =
-                            atomicExch(state, (static_cast<unsigned long long>(e) << 32) | (c + 1));
-                        p = unsigned(o);
-                        pe = unsigned(o >> 32);
-                    }
-                }
-            }
-        }
-        unit = __shfl_sync(kFull, u, 0);
-        return unit != 0xffffffffu;
-    }
-};
-
-// The digits of every list entry's weights.
+// The digits of every list entry's weights: the first four, or FIFTH the fifth
+// (into dig3).
+template <bool FIFTH>
 __global__ void __launch_bounds__(128)
     k_tile_build(VolumeDev v, WalkRecF rec, MixedParams mp, TileDev td, TileLists lists, TileLaw law, int nPts,
                  unsigned nUnits, uint4 *dig, uint4 *dig3) {
@@ -286,14 +251,16 @@ __global__ void __launch_bounds__(128)
             st.mask[lane] = lists.mask[e + lane];
         }
         __syncwarp();
-        stage_weights(st, td.geo, nPts, rows[warp], law);
+        stage_weights<FIFTH>(st, td.geo, nPts, rows[warp], law);
         __syncwarp();
         const int64_t step = e / kTileTerms;
         const uint4 *src = &st.dig[0][0][0];
+        if constexpr (!FIFTH) {
 #pragma unroll
-        for (int c = 0; c < 6; ++c) dig[192 * step + 32 * c + lane] = src[32 * c + lane];
+            for (int c = 0; c < 6; ++c) dig[192 * step + 32 * c + lane] = src[32 * c + lane];
+        }
 #pragma unroll
-        for (int c = 0; c < 2; ++c) dig3[64 * step + 32 * c + lane] = src[192 + 32 * c + lane];
+        for (int c = 0; c < 2; ++c) dig3[64 * step + 32 * c + lane] = src[(FIFTH ? 0 : 192) + 32 * c + lane];
         __syncwarp();
     }
 }
@@ -601,6 +568,8 @@ TileLaw make_tile_law(const EvalConsts &k) {
     return law;
 }
 
+}  // namespace
+
 int tile_sms() {
     static int cached[16] = {0};
     int dev = 0;
@@ -609,8 +578,6 @@ int tile_sms() {
     if (n == 0 && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n = 1;
     return n;
 }
-
-}  // namespace
 
 int tile_order(const VolumeDev &v, const double *lo, const double *hi, int *order, cudaStream_t st) {
     if (v.nVol <= 0) return 0;
@@ -690,9 +657,9 @@ void launch_tile_build(const VolumeDev &v, const WalkRecF &rec, const EvalConsts
                        const TileLists &lists, int nPts, uint4 *dig, uint4 *dig3, cudaStream_t st) {
     const MixedParams mp = make_mixed_params(k);
     const int64_t units = walk_list_warps(v.nVol) * mp.nLoop;
-    if (units > 0)
-        k_tile_build<<<blocks(32 * units, 128), 128, 0, st>>>(v, rec, mp, td, lists, make_tile_law(k), nPts,
-                                                              unsigned(units), dig, dig3);
+    if (units <= 0) return;
+    (dig ? k_tile_build<false> : k_tile_build<true>)<<<blocks(32 * units, 128), 128, 0, st>>>(
+        v, rec, mp, td, lists, make_tile_law(k), nPts, unsigned(units), dig, dig3);
 }
 
 template <int SRC, int ND>

@@ -19,14 +19,14 @@ constexpr int kTileTerms = 16;  // list entries per step
 
 // d += a b, FP16 operands, FP32 accumulators.
 __device__ __forceinline__ void mma_f16(float (&d)[4], const uint4 a, unsigned b0, unsigned b1) {
-    asm volatile(
+    asm(
         "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
 }
 // d = a b.
 __device__ __forceinline__ void mma_f16_first(float (&d)[4], const uint4 a, unsigned b0, unsigned b1) {
-    asm volatile(
+    asm(
         "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
         : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
         : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1), "f"(0.f));
@@ -112,27 +112,45 @@ __device__ __forceinline__ float2 tile_mask(float2 w, unsigned mg, int m) {
 // and B in the high one, at a row pair: s[.][0] row g, s[.][1] row g + 8.  A
 // node's weights are scaled so that its denominator lies in [2^13, 2^14); the
 // digits lie on the grids of 8, 2^-8 and 2^-19, and the last carries 2^22 times
-// what is left, rounded (44 bits of the denominator in all).
+// what is left, rounded (44 bits of the denominator in all).  FIFTH: s[0] is
+// 2^22 times what those four leave (for the reverse product, where a term's own
+// size counts and not the denominator's), the others are not set.
+template <bool FIFTH>
 __device__ __forceinline__ void tile_digits(float2 wa, float2 la, float2 wb, float2 lb, unsigned (&s)[4][2]) {
+    float2 ra = dup2(0.f), rb = dup2(0.f);
     const float grid[3] = {1.5f * 67108864.0f, 1.5f * 32768.0f, 1.5f * 16.0f};
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const float2 M = dup2(grid[d]);
         const float2 a = sub2(add2(wa, M), M), b = sub2(add2(wb, M), M);
-        s[d][0] = pack_f16(a.x, b.x);
-        s[d][1] = pack_f16(a.y, b.y);
+        if constexpr (!FIFTH) {
+            s[d][0] = pack_f16(a.x, b.x);
+            s[d][1] = pack_f16(a.y, b.y);
+        }
         wa = sub2(wa, a);
         wb = sub2(wb, b);
         if (d == 1) {
             // the rest of w is below 2^-9 and exact; the low parts join it
-            wa = add2(wa, la);
-            wb = add2(wb, lb);
+            if constexpr (FIFTH) {
+                two_sum2(wa, la, wa, ra);
+                two_sum2(wb, lb, wb, rb);
+            } else {
+                wa = add2(wa, la);
+                wb = add2(wb, lb);
+            }
         }
     }
-    wa = mul2(wa, dup2(4194304.0f));
-    wb = mul2(wb, dup2(4194304.0f));
-    s[3][0] = pack_f16(wa.x, wb.x);
-    s[3][1] = pack_f16(wa.y, wb.y);
+    const float2 S = dup2(4194304.0f);
+    wa = mul2(wa, S);
+    wb = mul2(wb, S);
+    if constexpr (FIFTH) {
+        const float2 a = make_float2(__half2float(__float2half_rn(wa.x)), __half2float(__float2half_rn(wa.y)));
+        const float2 b = make_float2(__half2float(__float2half_rn(wb.x)), __half2float(__float2half_rn(wb.y)));
+        wa = fma2(ra, S, sub2(wa, a));
+        wb = fma2(rb, S, sub2(wb, b));
+    }
+    s[FIFTH ? 0 : 3][0] = pack_f16(wa.x, wb.x);
+    s[FIFTH ? 0 : 3][1] = pack_f16(wa.y, wb.y);
 }
 
 // One step's data in shared memory, a stage per warp.  dig: digit d of tile m as
@@ -160,6 +178,43 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// Work distribution of the persistent kernels: units are taken from a global
+// counter in chunks of consecutive ones, shared by the warps of a block (their
+// terms overlap, so the block's L1 serves them together).  state holds the
+// block's chunk as (end << 32 | next).  A warp that finds it empty takes the
+// next chunk for the block; if another warp published one meanwhile, it keeps
+// what was left of that to itself.  Nothing waits.
+struct UnitQueue {
+    unsigned long long *state;
+    unsigned *counter;
+    unsigned total, chunk, p, pe;
+    __device__ __forceinline__ bool next(unsigned &unit) {
+        unsigned u = 0xffffffffu;
+        if ((threadIdx.x & 31) == 0) {
+            if (p < pe) {
+                u = p++;
+            } else {
+                const unsigned long long s = atomicAdd(state, 1ull);
+                if (unsigned(s) < unsigned(s >> 32)) {
+                    u = unsigned(s);
+                } else {
+                    const unsigned c = atomicAdd(counter, chunk);
+                    if (c < total) {
+                        u = c;
+                        const unsigned e = min(c + chunk, total);
+                        const unsigned long long o =
+                            atomicExch(state, (static_cast<unsigned long long>(e) << 32) | (c + 1));
+                        p = unsigned(o);
+                        pe = unsigned(o >> 32);
+                    }
+                }
+            }
+        }
+        unit = __shfl_sync(kFull, u, 0);
+        return unit != 0xffffffffu;
+    }
+};
+
 // The terms whose motion records a lane copies into a stage (one 16-byte chunk
 // of each of four).
 struct StageIds {
@@ -181,7 +236,9 @@ struct TileRows {
     float2 h[3], l[3], P;
 };
 
-// The digits of a step's weights into st.dig, from its terms and masks.
+// The four digits of a step's weights into st.dig, or the fifth into st.dig[0],
+// from its terms and masks.
+template <bool FIFTH = false>
 __device__ __forceinline__ void stage_weights(TileStage &st, const float4 *geo, int nPts, const TileRows *rows,
                                               const TileLaw law) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -209,9 +266,9 @@ __device__ __forceinline__ void stage_weights(TileStage &st, const float4 *geo, 
         wb = tile_mask(wb, mb, m);
         lb = tile_mask(lb, mb, m);
         unsigned s[4][2];
-        tile_digits(wa, la, wb, lb, s);
+        tile_digits<FIFTH>(wa, la, wb, lb, s);
 #pragma unroll
-        for (int d = 0; d < 4; ++d)
+        for (int d = 0; d < (FIFTH ? 1 : 4); ++d)
             reinterpret_cast<uint2 *>(&st.dig[d][m][lane])[p] = make_uint2(s[d][0], s[d][1]);
     }
 }
