@@ -64,8 +64,30 @@ __device__ __forceinline__ float ipowf(float x, int n) {
     return r;
 }
 
+// 1 / sqrt(q), FP64, to an ulp: Householder's third-order step (e the residual
+// 1 - q y^2 of the FP32 reciprocal square root y, |e| < 2^-21: y (1 + e/2 + 3/8
+// e^2)).  Five FP64 operations, the conversions being moves of bits, where a
+// square root and a division take some 18; an FP64 instruction holds this GPU's
+// pipe for 16 cycles (the denominator estimate of the 2M-node wing 111 -> 59 ms,
+// the error tables 9.8 -> 5.1, the FP64 walk of the 95k-node sphere 7.04 -> 5.30;
+// all three fill that pipe).  q outside FP32's normal range goes the long way.
+__device__ __forceinline__ double inv_sqrt64(double q) {
+    const unsigned hi = unsigned(__double2hiint(q)) - 0x38000000u;  // exponent to FP32's bias
+    if (hi - 0x00200000u >= 0x0fb00000u) return 1.0 / sqrt(q);
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float(__funnelshift_l(__double2loint(q), hi, 3))));
+    const unsigned b = __float_as_uint(y);
+    const double y0 = __hiloint2double(int((b >> 3) + 0x38000000u), int(b << 29));
+    const double e = fma(-q, y0 * y0, 1.0);  // the square is exact
+    return fma(y0 * e, fma(e, 0.375, 0.5), y0);
+}
+
 // (L/d)^a + alpha^b (L/d)^b for a given LdefoDist = L/d, FP64.
 __device__ __forceinline__ double law64(const WeightLaw &w, double LoD) {
+    if (w.isInt && w.ia == 3 && w.ib == 5) {
+        const double s = LoD * LoD;
+        return (s * LoD) * fma(w.alphaToBexp, s, 1.0);
+    }
     if (w.isInt) {
         double ta = ipow(LoD, w.ia);
         double tb = ta * ipow(LoD, w.ib - w.ia);

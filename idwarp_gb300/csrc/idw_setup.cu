@@ -83,8 +83,7 @@ __global__ void k_err_partial(TreeDev t, const dbl4 *ptXA, WeightLaw law, const 
             for (int k = 0; k < m; ++k) {
                 dbl4 x = sx[k];
                 double r0 = pt[0] - x.x, r1 = pt[1] - x.y, r2 = pt[2] - x.z;
-                double dist = sqrt(r0 * r0 + r1 * r1 + r2 * r2);
-                acc += x.w * law64(law, law.Ldef / dist);
+                acc += x.w * law64(law, law.Ldef * inv_sqrt64(r0 * r0 + r1 * r1 + r2 * r2));
             }
         }
     }
@@ -104,8 +103,7 @@ __global__ void k_err_final(TreeDev t, WeightLaw law, const int *nodeItem0, cons
         double pt[3];
         sphere_point(g, tid, pt);
         double r0 = pt[0] - g.x, r1 = pt[1] - g.y, r2 = pt[2] - g.z;
-        double dist = sqrt(r0 * r0 + r1 * r1 + r2 * r2);
-        double dApprox = t.ai[q] * law64(law, law.Ldef / dist);
+        double dApprox = t.ai[q] * law64(law, law.Ldef * inv_sqrt64(r0 * r0 + r1 * r1 + r2 * r2));
         double d = dExact - dApprox;
         sq[tid] = d * d;
     }
@@ -155,8 +153,7 @@ __global__ void k_den0(TreeDev t, const NodeRecF *rf, const dbl4 *ptXA, VolumeDe
                     for (int i = inf.x; i <= inf.y; ++i) {
                         dbl4 x = ptXA[i];
                         double r0 = r[0] - x.x, r1 = r[1] - x.y, r2 = r[2] - x.z;
-                        double LoD = law.Ldef / sqrt(r0 * r0 + r1 * r1 + r2 * r2 + 1e-16);
-                        acc += x.w * law64(law, LoD);
+                        acc += x.w * law64(law, law.Ldef * inv_sqrt64(r0 * r0 + r1 * r1 + (r2 * r2 + 1e-16)));
                     }
                 }
                 node = inf.z;
@@ -176,9 +173,9 @@ __global__ void k_den0(TreeDev t, const NodeRecF *rf, const dbl4 *ptXA, VolumeDe
                     if (dec != 0) {
                         const dbl4 g = t.geom[node];
                         double r0 = r[0] - g.x, r1 = r[1] - g.y, r2 = r[2] - g.z;
-                        double dist = sqrt(r0 * r0 + r1 * r1 + r2 * r2 + 1e-16);
-                        if (dec == 1 || dist * g.w > 5.0) {
-                            acc += t.ai[node] * law64(law, law.Ldef / dist);
+                        const double d2 = r0 * r0 + r1 * r1 + r2 * r2 + 1e-16;
+                        if (dec == 1 || sqrt(d2) * g.w > 5.0) {
+                            acc += t.ai[node] * law64(law, law.Ldef * inv_sqrt64(d2));
                             skip = inf.z;
                         } else {
                             open = true;

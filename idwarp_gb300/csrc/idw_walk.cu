@@ -57,8 +57,7 @@ __device__ __forceinline__ void load12(const double *src, double *d) {
 __device__ __forceinline__ void pair64(const EvalConsts &k, const dbl4 &x, const double *mb, const double *r,
                                        int tangent, double *num, double &den) {
     double r0 = r[0] - x.x, r1 = r[1] - x.y, r2 = r[2] - x.z;
-    double LoD = k.law.Ldef / sqrt(r0 * r0 + r1 * r1 + r2 * r2 + 1e-15);
-    double W = x.w * law64(k.law, LoD);
+    double W = x.w * law64(k.law, k.law.Ldef * inv_sqrt64(r0 * r0 + r1 * r1 + r2 * r2 + 1e-15));
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         double S = mb[3 * a] * r[0] + mb[3 * a + 1] * r[1] + mb[3 * a + 2] * r[2] + mb[9 + a];
@@ -219,8 +218,7 @@ __global__ void __launch_bounds__(128) k_walk_adj64(TreeDev t, PointsDev p, Volu
                         if (active) {
                             dbl4 x = ldg4(p.xa + i);
                             double r0 = r[0] - x.x, r1 = r[1] - x.y, r2 = r[2] - x.z;
-                            double dist = sqrt(r0 * r0 + r1 * r1 + r2 * r2 + 1e-15);
-                            W = x.w * law64(k.law, k.law.Ldef / dist);
+                            W = x.w * law64(k.law, k.law.Ldef * inv_sqrt64(r0 * r0 + r1 * r1 + r2 * r2 + 1e-15));
                         }
 #pragma unroll
                         for (int s = 0; s < NS; ++s) {
