@@ -21,8 +21,10 @@ constexpr int kTile = 256;  // surface points per shared-memory pass
 constexpr int kThreads = 128;
 
 // Volume nodes carried by each thread: four on large meshes (more reuse of
-// each staged point; 168 registers, three blocks per SM), two otherwise.
-constexpr int kBlocksPerSmNV4 = 3;
+// each staged point; 168 registers, three blocks per SM), two otherwise (128
+// registers, four blocks per SM: 96 registers and five blocks wait longer for
+// each pair's chain, 14.1 against 12.8 ms on the 245k-node wing).
+constexpr int kBlocksPerSmNV4 = 3, kBlocksPerSmNV2 = 4;
 
 int sm_count() {
     static int cached[16] = {0};
@@ -170,9 +172,9 @@ __global__ void __launch_bounds__(kThreads) k_exact_mixed(TreeDevF tf, PointsDev
 constexpr int kTile2 = 128;  // surface points per shared-memory pass (static shared memory)
 
 template <int NV>
-__global__ void __launch_bounds__(kThreads) k_exact_mixed2(TreeDevF tf, PointsDevF pf, NodeAggF af, VolumeDev v,
-                                                           WalkRecF rec, MixedParams mp, Law32<0> law, float4 *acc,
-                                                           unsigned long long *counters) {
+__global__ void __launch_bounds__(kThreads, NV == 2 ? kBlocksPerSmNV2 : kBlocksPerSmNV4)
+    k_exact_mixed2(TreeDevF tf, PointsDevF pf, NodeAggF af, VolumeDev v, WalkRecF rec, MixedParams mp, Law32<0> law,
+                   float4 *acc, unsigned long long *counters) {
     constexpr int NP = NV / 2;  // node pairs per thread
     const int nPts = tf.nPts;
     // per point: (dx, dx, dy, dy), (dz, dz, A, A), (lx, lx, ly, ly), (lz, lz, 0, 0), then D', u' in pairs
@@ -533,12 +535,23 @@ __global__ void __launch_bounds__(kThreads) k_exact_adjoint(TreeDevF tf, PointsD
 
 inline int blocks_for(int64_t n, int per) { return int((n + per - 1) / per); }
 
+}  // namespace
+
+bool exact_tiled_fills(int64_t nVol) {
+    return blocks_for(nVol, kThreads * 4) >= 2 * sm_count() * kBlocksPerSmNV4;
+}
+
+namespace {
+
 template <int KIND>
 void launch_kind(const TreeDevF &tf, const PointsDevF &pf, const NodeAggF &af, const VolumeDev &v,
                  const WalkRecF &rec, const MixedParams &mp, const Law32<KIND> &law, float4 *acc,
                  unsigned long long *counters, cudaStream_t st) {
     if constexpr (KIND == 0) {
-        if (blocks_for(v.nVol, kThreads * 4) >= sm_count() * kBlocksPerSmNV4)
+        // four nodes a thread from two full waves of its blocks on; below, the
+        // last wave is the emptier one (245k nodes, 1.05 waves: 14.7 against 12.8 ms
+        // with two nodes; 466k nodes, 2.0 waves: 20.2 against 21.3 ms)
+        if (exact_tiled_fills(v.nVol))
             k_exact_mixed2<4><<<blocks_for(v.nVol, kThreads * 4), kThreads, 0, st>>>(tf, pf, af, v, rec, mp, law, acc,
                                                                                     counters);
         else
@@ -584,9 +597,6 @@ void launch_exact_adjoint(const TreeDevF &tf, const PointsDevF &pf, const Volume
     }
 }
 
-bool exact_tiled_fills(int64_t nVol) {
-    return blocks_for(nVol, kThreads * 4) >= 2 * sm_count() * kBlocksPerSmNV4;
-}
 
 void launch_exact_mixed(const TreeDevF &tf, const PointsDevF &pf, const NodeAggF &af, const VolumeDev &v,
                         const WalkRecF &rec, const MixedParams &mp, const WeightLaw &wl, float4 *acc,

@@ -280,7 +280,8 @@ void launch_exact_adjoint(const TreeDevF &tf, const PointsDevF &pf, const Volume
                           const MixedParams &mp, const WeightLaw &wl, const double *dxv, const double *den,
                           double *ptAdj, unsigned long long *counters, cudaStream_t st, int det = 0);
 // True when the tiled exact kernel has volume nodes for at least two full
-// waves of the device (below that the walk's finer grain is faster).
+// waves of the device (below that the walk's finer grain is faster for the
+// reverse product, for batches and for exponents without the packed form).
 bool exact_tiled_fills(int64_t nVol);
 // Per node (Morton order): the scaled denominator of the last mixed walk (acc).
 void launch_gate_den(int64_t nVol, const float4 *acc, float *gden, cudaStream_t st);

@@ -91,7 +91,8 @@ typedef struct idw_options {
                            * exponents and a gate of 2e-3 or more the fast walk needs no
                            * such terms: its sums are matrix products of weights in
                            * double-float (idw_tile.cu) */
-    int32_t exactSchedule; /* mixed exact mode: IDW_EXACT_AUTO (default: tiled
+    int32_t exactSchedule; /* mixed exact mode: IDW_EXACT_AUTO (default: tiled at
+                            * the exponents (3, 5), at others the tiled
                             * kernel when the mesh fills the GPU, else the walk),
                             * IDW_EXACT_TILED or IDW_EXACT_WALK; same sums either way */
     int32_t adjointPrecision; /* mixed warpDeriv: IDW_ADJ_PRECISE (default) or
