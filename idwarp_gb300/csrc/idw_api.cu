@@ -70,8 +70,6 @@ struct Ctx {
     DevBuf<int4> info;
     DevBuf<dbl4> geom;
     DevBuf<double> nodeErr, nodeAi, nodeMB, nodeSum;
-    DevBuf<int> parent;
-    DevBuf<unsigned> nodeFlags;
     bool haveTree = false, haveWarp = false, nodalValid = false;
     bool den0Valid = false;  // denominator estimate and walk records (computed at the first walk, or loaded)
     // FP32 companion arrays of the mixed-precision walk
@@ -247,15 +245,7 @@ TreeDev tree_dev(Ctx *c) {
     t.geom = c->geom.p;
     t.err = c->nodeErr.p;
     t.ai = c->nodeAi.p;
-    t.parent = c->parent.p;
     return t;
-}
-
-SetDataScratch setdata_scratch(Ctx *c) {
-    SetDataScratch sc;
-    sc.sum = c->nodeSum.p;
-    sc.flags = c->nodeFlags.p;
-    return sc;
 }
 
 SurfaceDev surf_dev(Ctx *c) {
@@ -316,7 +306,7 @@ int refresh_nodal(Ctx *c, int gated) {
     launch_gather_xu(c->nUnique, c->xuInd.p, c->xs.p, c->xu.p, c->stream);
     launch_nodal(s, c->xu.p, c->ptXA.p, c->normals0.p, c->tmpAi.p, c->isCorner.p, c->opt.useRotations, c->ptMB.p,
                  c->stream);
-    launch_set_data(tree_dev(c), c->ptMB.p, c->nodeMB.p, setdata_scratch(c), c->stream);
+    launch_set_data(tree_dev(c), c->nUnique, c->ptMB.p, c->nodeMB.p, c->nodeSum.p, c->stream);
     if (gated && c->opt.precision == IDW_PREC_MIXED) {
         launch_mixed_nodal(c->nUnique, tree_dev(c), c->nodeMB.p, c->ptXA.p, c->ptMB.p, c->ptDM.p, c->ptDMl.p,
                            c->stream);
@@ -642,9 +632,7 @@ int idw_initialize_warping(void *ctx, const double *pts, int32_t npts, const dou
     CKA(c->nodeErr.alloc(kNerr * size_t(nn)));
     CKA(c->nodeAi.alloc(nn));
     CKA(c->nodeMB.alloc(12 * size_t(nn)));
-    CKA(c->nodeSum.alloc(12 * size_t(nn)));
-    CKA(c->nodeFlags.alloc(size_t(nn)));
-    CKA(c->parent.alloc(size_t(nn)));
+    CKA(c->nodeSum.alloc(size_t(set_data_scratch(n))));
     CKA(c->nodeAdj.alloc(12 * size_t(nn)));
     CKA(c->nodeRec.alloc(nn));
     CKA(c->nodeDC.alloc(12 * size_t(nn)));
@@ -679,7 +667,6 @@ int idw_initialize_warping(void *ctx, const double *pts, int32_t npts, const dou
     CKA(c->leafList.alloc(leaves.size()));
     if (!leaves.empty())
         CK(cudaMemcpyAsync(c->leafList.p, leaves.data(), sizeof(int4) * leaves.size(), cudaMemcpyHostToDevice, st));
-    launch_tree_parents(tree_dev(c), c->parent.p, st);
     // initial nodal properties: normals0, Ai, corners (kd_tree.F90:1547-1578)
     SurfaceDev s = surf_dev(c);
     launch_gather_xu(n, c->xuInd.p, c->xs.p, c->xu.p, st);
@@ -1240,7 +1227,7 @@ int idw_warp_mesh_cs(void *ctx) {
     CKA(c->xvIm.alloc(3 * size_t(c->nVol)));
     launch_nodal_cs(surf_dev(c), c->xuInd.p, c->xsC.p, c->xuC.p, c->ptXA.p, c->normals0.p, c->tmpAi.p,
                     c->isCorner.p, c->opt.useRotations, c->ptMBim.p, c->stream);
-    launch_set_data(tree_dev(c), c->ptMBim.p, c->nodeMBim.p, setdata_scratch(c), c->stream);
+    launch_set_data(tree_dev(c), c->nUnique, c->ptMBim.p, c->nodeMBim.p, c->nodeSum.p, c->stream);
     rc = check_launch(c, "complex nodal properties");
     if (rc) return rc;
     EvalConsts k;
@@ -1305,7 +1292,7 @@ static int run_tile_batch(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const
         launch_gather_xu(n, c->xuInd.p, coordsDev + size_t(b) * sdof, c->xu.p, c->stream);
         launch_nodal(s, c->xu.p, c->ptXA.p, c->normals0.p, c->tmpAi.p, c->isCorner.p, c->opt.useRotations, c->ptMB.p,
                      c->stream);
-        launch_set_data(tree_dev(c), c->ptMB.p, c->nodeMB.p, setdata_scratch(c), c->stream);
+        launch_set_data(tree_dev(c), c->nUnique, c->ptMB.p, c->nodeMB.p, c->nodeSum.p, c->stream);
         WalkOut o;
         o.xv = outDev + size_t(b) * vdof;
         o.counters = b == 0 ? c->counters.p : nullptr;
@@ -1371,7 +1358,7 @@ static int run_warp_batch_mixed(Ctx *c, const double *coordsDev, int nb, double 
         else
             launch_nodal(s, xu, c->ptXA.p, c->normals0.p, c->tmpAi.p, c->isCorner.p, c->opt.useRotations, mb,
                          c->stream);
-        launch_set_data(tree_dev(c), mb, nmb, setdata_scratch(c), c->stream);
+        launch_set_data(tree_dev(c), c->nUnique, mb, nmb, c->nodeSum.p, c->stream);
         if (tiledExact) {
             launch_mixed_nodal(n, tree_dev(c), nmb, c->ptXA.p, mb, c->bPtDM.p + size_t(b) * 12 * n,
                                c->bPtDMl.p + size_t(b) * 12 * n, c->stream);
@@ -2047,7 +2034,7 @@ int run_deriv_fwd(Ctx *c, const double *xsdDev, double *xvdDev) {
     // for the mixed walk, whose motions are relative to the identity
     launch_nodal_d(surf_dev(c), c->xu.p, xud.p, c->ptXA.p, c->normals0.p, c->tmpAi.p, c->isCorner.p,
                    c->opt.useRotations, mixed ? 1 : 0, ptMBd.p, c->stream);
-    launch_set_data(tree_dev(c), ptMBd.p, nodeMBd.p, setdata_scratch(c), c->stream);
+    launch_set_data(tree_dev(c), c->nUnique, ptMBd.p, nodeMBd.p, c->nodeSum.p, c->stream);
     int rc = check_launch(c, "tangent nodal properties");
     if (rc) return rc;
     EvalConsts k;

@@ -26,13 +26,6 @@ struct TreeDev {
     const dbl4 *geom;  // X, oradius
     const double *err;    // 12 per node
     const double *ai;     // per node
-    const int *parent = nullptr;  // per node: parent index, -1 at the root
-};
-
-// Scratch of the bottom-up cluster sums: 12 doubles and one arrival counter per node.
-struct SetDataScratch {
-    double *sum;
-    unsigned *flags;
 };
 
 // Everything the mixed walks read at a tree node, packed in one 128-byte
@@ -141,8 +134,9 @@ void launch_corners(const SurfaceDev &s, const double *Xu, const double *normals
                     int *isCorner, cudaStream_t st);
 void launch_nodal(const SurfaceDev &s, const double *Xu, const dbl4 *xa, const double *normals0,
                   const double *Ai, const int *isCorner, int useRotations, double *ptMB, cudaStream_t st);
-void launch_set_data(const TreeDev &t, const double *ptMB, double *nodeMB, const SetDataScratch &sc, cudaStream_t st);
-void launch_tree_parents(const TreeDev &t, int *parent, cudaStream_t st);
+// Cluster means; sums: set_data_scratch(nPts) doubles of scratch.
+int64_t set_data_scratch(int nPts);
+void launch_set_data(const TreeDev &t, int nPts, const double *ptMB, double *nodeMB, double *sums, cudaStream_t st);
 void launch_set_data_b(const TreeDev &t, const double *nodeAdj, double *ptAdj, int nPts, cudaStream_t st);
 // faceProps = 0 reuses the face areas and normals of the previous call (same surface)
 void launch_nodal_b(const SurfaceDev &s, const double *Xu, const dbl4 *xa, const double *normals0,

@@ -258,55 +258,94 @@ __global__ void k_nodal(SurfaceDev s, const double *Xu, const dbl4 *xa, const do
 }
 
 // setData: unweighted mean of the 12 node values over each interior node's
-// range (kd_tree.F90:595-617), bottom-up: a leaf sums its own points, and the
-// second child to finish adds the two child sums into the parent and carries
-// on towards the root (the first one stops).  Every point is read once.
-__global__ void k_set_data(TreeDev t, const double *ptMB, double *nodeMB, double *sum, unsigned *flags) {
-    const int q0 = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q0 >= t.nNodes) return;
-    const int4 inf = t.info[q0];
-    if (!inf.w) return;
-    double acc[12];
-#pragma unroll
-    for (int c = 0; c < 12; ++c) acc[c] = 0.0;
-    for (int i = inf.x; i <= inf.y; ++i) {
-        const double2 *p = reinterpret_cast<const double2 *>(ptMB + 12 * i);
-#pragma unroll
-        for (int c = 0; c < 6; ++c) {
-            const double2 v = __ldg(p + c);
-            acc[2 * c] += v.x;
-            acc[2 * c + 1] += v.y;
-        }
+// range (kd_tree.F90:595-617).  A node's points are contiguous, so its sum is
+// the sums of the whole chunks of kMeanChunk points inside its range and the
+// points beside them: no node waits for another.  (Bottom-up, the second child
+// to finish adding into its parent, the climb of one thread through 13 levels of
+// fences and atomics took 113 us on a 40k-point surface and 62 us on 700 points,
+// whatever the bandwidth; these two kernels take 37 and 21 us under the same
+// profiler, and 63 us less of a 7k-node warp's 182.)
+constexpr int kMeanChunk = 128;
+
+// Sums of every chunk: column threadIdx % 12, ten points at a time.
+__global__ void __launch_bounds__(128) k_chunk_sums(int nPts, const double *ptMB, double *sums) {
+    __shared__ double part[120];
+    const int c = threadIdx.x % 12, r = threadIdx.x / 12;
+    const int64_t i0 = int64_t(blockIdx.x) * kMeanChunk;
+    const int n = int(min(int64_t(kMeanChunk), nPts - i0));
+    double acc = 0.0;
+    if (r < 10) {
+        const double *p = ptMB + 12 * i0 + c;
+#pragma unroll 13
+        for (int i = r; i < n; i += 10) acc += __ldg(p + 12 * i);
+        part[threadIdx.x] = acc;
     }
-#pragma unroll
-    for (int c = 0; c < 12; ++c) sum[12 * q0 + c] = acc[c];
-    int q = q0;
-    while (true) {
-        const int p = t.parent[q];
-        if (p < 0) break;
-        __threadfence();
-        if (atomicAdd(flags + p, 1u) == 0u) break;  // the sibling is not done yet
-        const int a = p + 1, b = t.info[a].z;
-        const int4 pi = t.info[p];
-        const double cnt = double(pi.y - pi.x + 1);
-#pragma unroll
-        for (int c = 0; c < 12; ++c) {
-            const double s = __ldcg(sum + 12 * a + c) + __ldcg(sum + 12 * b + c);
-            sum[12 * p + c] = s;
-            nodeMB[12 * p + c] = s / cnt;
-        }
-        q = p;
+    __syncthreads();
+    if (threadIdx.x < 12) {
+        for (int k = 1; k < 10; ++k) acc += part[12 * k + c];
+        sums[12 * int64_t(blockIdx.x) + c] = acc;
     }
 }
 
-__global__ void k_tree_parents(TreeDev t, int *parent) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+// Partial sum of columns 2 c, 2 c + 1 of node range [x, y] over every `step`th of
+// the points before the first whole chunk, the whole chunks, and the points after
+// the last.
+__device__ __forceinline__ double2 range_sum(const double *ptMB, const double *sums, int x, int y, int c, int r,
+                                             int step) {
+    const int k0 = (x + kMeanChunk - 1) / kMeanChunk, k1 = (y + 1) / kMeanChunk;
+    const int head = k0 < k1 ? k0 * kMeanChunk : y + 1, tail = k0 < k1 ? k1 * kMeanChunk : y + 1;
+    const double2 *p = reinterpret_cast<const double2 *>(ptMB) + c, *s = reinterpret_cast<const double2 *>(sums) + c;
+    double2 a = make_double2(0.0, 0.0);
+    auto add = [&](const double2 v) {
+        a.x += v.x;
+        a.y += v.y;
+    };
+#pragma unroll 8
+    for (int i = x + r; i < head; i += step) add(__ldg(p + 6 * int64_t(i)));
+#pragma unroll 8
+    for (int k = k0 + r; k < k1; k += step) add(__ldg(s + 6 * int64_t(k)));
+#pragma unroll 8
+    for (int i = tail + r; i <= y; i += step) add(__ldg(p + 6 * int64_t(i)));
+    return a;
+}
+
+// The means of four nodes a block: a warp each (30 lanes, five items at a time),
+// or the block together (21 at a time) for a node of more than kMeanWide points.
+// The four lie apart in preorder, where the wide nodes follow one another.
+constexpr int kMeanWide = 128;
+__global__ void __launch_bounds__(128) k_node_means(TreeDev t, const double *ptMB, const double *sums, double *nodeMB) {
+    __shared__ double2 part[126];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int j = 0; j < 4; ++j) {
+        const int q = blockIdx.x + j * gridDim.x;
+        if (q >= t.nNodes) break;
+        const int4 inf = t.info[q];
+        if (inf.w || inf.y - inf.x < kMeanWide) continue;  // the same for the whole block
+        const int r = threadIdx.x / 6, c = threadIdx.x - 6 * r;
+        if (r < 21) part[threadIdx.x] = range_sum(ptMB, sums, inf.x, inf.y, c, r, 21);
+        __syncthreads();
+        if (threadIdx.x < 12) {
+            const double *v = reinterpret_cast<const double *>(part) + threadIdx.x;
+            double a = v[0];
+            for (int k = 1; k < 21; ++k) a += v[12 * k];
+            nodeMB[12 * int64_t(q) + threadIdx.x] = a / double(inf.y - inf.x + 1);
+        }
+        __syncthreads();
+    }
+    const int q = blockIdx.x + warp * gridDim.x;
     if (q >= t.nNodes) return;
-    if (q == 0) parent[0] = -1;
     const int4 inf = t.info[q];
-    if (inf.w) return;
-    parent[q + 1] = q;
-    parent[t.info[q + 1].z] = q;
+    if (inf.w || inf.y - inf.x >= kMeanWide) return;
+    const int r = lane / 6, c = lane - 6 * r;
+    double2 a = make_double2(0.0, 0.0);
+    if (r < 5) a = range_sum(ptMB, sums, inf.x, inf.y, c, r, 5);
+    // lane k < 12: column k over the five rows
+    double sum = 0.0;
+    for (int k = 0; k < 30; k += 6) {
+        const double x = __shfl_sync(kFull, a.x, ((lane >> 1) + k) & 31), y = __shfl_sync(kFull, a.y, ((lane >> 1) + k) & 31);
+        sum += lane & 1 ? y : x;
+    }
+    if (lane < 12) nodeMB[12 * int64_t(q) + lane] = sum / double(inf.y - inf.x + 1);
 }
 
 // setData_b: push the cluster adjoints down to the member points
@@ -584,13 +623,11 @@ void launch_nodal(const SurfaceDev &s, const double *Xu, const dbl4 *xa, const d
     if (useRotations && s.nFaces > 0) k_face_props<<<blocks(s.nFaces, 128), 128, 0, st>>>(s, Xu);
     k_nodal<<<blocks(s.n, 128), 128, 0, st>>>(s, Xu, xa, normals0, Ai, isCorner, useRotations, ptMB);
 }
-void launch_set_data(const TreeDev &t, const double *ptMB, double *nodeMB, const SetDataScratch &sc, cudaStream_t st) {
-    if (t.nNodes <= 0) return;
-    cudaMemsetAsync(sc.flags, 0, sizeof(unsigned) * size_t(t.nNodes), st);
-    k_set_data<<<blocks(t.nNodes, 128), 128, 0, st>>>(t, ptMB, nodeMB, sc.sum, sc.flags);
-}
-void launch_tree_parents(const TreeDev &t, int *parent, cudaStream_t st) {
-    if (t.nNodes > 0) k_tree_parents<<<blocks(t.nNodes, 128), 128, 0, st>>>(t, parent);
+int64_t set_data_scratch(int nPts) { return 12 * ((int64_t(nPts) + kMeanChunk - 1) / kMeanChunk); }
+void launch_set_data(const TreeDev &t, int nPts, const double *ptMB, double *nodeMB, double *sums, cudaStream_t st) {
+    if (t.nNodes <= 1) return;  // a lone leaf has no interior node
+    k_chunk_sums<<<blocks(nPts, kMeanChunk), 128, 0, st>>>(nPts, ptMB, sums);
+    k_node_means<<<blocks(t.nNodes, 4), 128, 0, st>>>(t, ptMB, sums, nodeMB);
 }
 void launch_set_data_b(const TreeDev &t, const double *nodeAdj, double *ptAdj, int nPts, cudaStream_t st) {
     if (nPts > 0) k_set_data_b<<<blocks(nPts, 128), 128, 0, st>>>(t, nodeAdj, ptAdj, nPts);
