@@ -638,7 +638,7 @@ int idw_initialize_warping(void *ctx, const double *pts, int32_t npts, const dou
     CKA(c->nodeDC.alloc(12 * size_t(nn)));
     CKA(c->nodeDCl.alloc(12 * size_t(nn)));
     CKA(c->nodeDn.alloc(nn));
-    CKA(c->refDB.alloc(24));
+    CKA(c->refDB.alloc(48));
     CKA(c->ptDA.alloc(n));
     CKA(c->ptDL.alloc(n));
     CKA(c->ptDM.alloc(12 * size_t(n)));
@@ -948,7 +948,7 @@ static int ensure_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const Ev
         }
         CKA(c->tileGeo.alloc(2 * nTerms));
         CKA(c->tileMot.alloc(8 * nTerms));
-        CKA(c->tileWord.alloc(14));
+        CKA(c->tileWord.alloc(2 * kTileWords));
         CKA(c->tileScale.alloc(size_t(c->nVol)));
         CKA(c->tileSums.alloc(2 * size_t(c->sym.nLoop) * size_t(c->nVol)));
         CKA(c->tileOrder.alloc(size_t(c->nVol)));
@@ -1281,23 +1281,43 @@ int idw_get_volume_coordinates_cs(void *ctx, double *out, int64_t ndof, int wher
 // and a finalisation per surface.  coords/out are device pointers.
 static constexpr int kBatchWalk = kBatchMax;
 
-// run_warp_batch_mixed by tile walks, one per surface.
+// run_warp_batch_mixed by tile walks, two surfaces each where the weight digits
+// stream from memory and the scratch for two is to be had.
 static int run_tile_batch(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalConsts &k, const TileLists &lists,
                           const double *coordsDev, int nb, double *outDev) {
     const int n = c->nUnique;
     const size_t sdof = 3 * size_t(c->nPts), vdof = 3 * size_t(c->nVol);
     c->nodalValid = false;
     const SurfaceDev s = surf_dev(c);
-    for (int b = 0; b < nb; ++b) {
-        launch_gather_xu(n, c->xuInd.p, coordsDev + size_t(b) * sdof, c->xu.p, c->stream);
-        launch_nodal(s, c->xu.p, c->ptXA.p, c->normals0.p, c->tmpAi.p, c->isCorner.p, c->opt.useRotations, c->ptMB.p,
-                     c->stream);
-        launch_set_data(tree_dev(c), c->nUnique, c->ptMB.p, c->nodeMB.p, c->nodeSum.p, c->stream);
-        WalkOut o;
-        o.xv = outDev + size_t(b) * vdof;
-        o.counters = b == 0 ? c->counters.p : nullptr;
-        int rc = run_tile(c, tf, rec, k, lists, c->ptMB.p, c->nodeMB.p, o);
+    const size_t nTerms = size_t(n) + size_t(c->nNodes);
+    int per = nb > 1 ? tile_batch(vol_dev(c), c->sym.nLoop, lists) : 1;
+    if (per > 1) {
+        bool fits = false;
+        const size_t sums = 2 * size_t(c->sym.nLoop) * size_t(c->nVol);
+        int rc = fits_half(c, double(sizeof(float4)) * per * double(sums + 8 * nTerms), fits);
         if (rc) return rc;
+        if (!fits && (c->tileSums.n < per * sums || c->tileMot.n < 8 * per * nTerms)) per = 1;
+        if (per > 1) {
+            CKA(c->tileSums.alloc(per * sums));
+            CKA(c->tileMot.alloc(8 * per * nTerms));
+        }
+    }
+    CK(cudaEventRecord(c->ev0, c->stream));
+    for (int b0 = 0; b0 < nb; b0 += per) {
+        const int m = std::min(per, nb - b0);
+        for (int b = 0; b < m; ++b) {
+            launch_gather_xu(n, c->xuInd.p, coordsDev + size_t(b0 + b) * sdof, c->xu.p, c->stream);
+            launch_nodal(s, c->xu.p, c->ptXA.p, c->normals0.p, c->tmpAi.p, c->isCorner.p, c->opt.useRotations,
+                         c->ptMB.p, c->stream);
+            launch_set_data(tree_dev(c), n, c->ptMB.p, c->nodeMB.p, c->nodeSum.p, c->stream);
+            launch_tile_motions(tree_dev(c), n, c->ptMB.p, c->nodeMB.p, c->tileWord.p + kTileWords * b,
+                                c->tileMot.p + 8 * nTerms * b, c->refDB.p + 24 * b, c->stream);
+        }
+        WalkOut o;
+        o.xv = outDev + size_t(b0) * vdof;
+        o.counters = b0 == 0 ? c->counters.p : nullptr;
+        launch_tile_walk(tree_dev(c), tf, vol_dev(c), rec, k, tile_dev(c), lists, c->refDB.p, c->tileSums.p, o,
+                         c->stream, m);
     }
     CK(cudaEventRecord(c->ev1, c->stream));
     c->eventsRecorded = true;

@@ -221,6 +221,7 @@ struct TileLists {
     const uint4 *dig4 = nullptr;    // per step 64: the fifth, which only the reverse product reads
     const unsigned long long *counters = nullptr;  // the recording walk's, as WalkLists::counters
 };
+constexpr int kTileWords = 16;  // per surface of a batch: 12 column maxima (and the walk's counter, a flag)
 struct TileDev {
     const int *order;        // tile slot -> walk (Morton) index of a volume node
     const float *scale;      // per slot: power-of-two weight scale P
@@ -250,7 +251,10 @@ void launch_tile_motions(const TreeDev &t, int nPts, const double *ptMB, const d
 // sums: 2 nLoop nVol float4 of scratch.
 void launch_tile_walk(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
                       const EvalConsts &k, const TileDev &td, const TileLists &lists, const float *refDB, float4 *sums,
-                      const WalkOut &o, cudaStream_t st);
+                      const WalkOut &o, cudaStream_t st, int nb = 1);
+// Surfaces that one tile walk takes (launch_tile_walk's nb): 2 where the digits
+// stream from memory.
+int tile_batch(const VolumeDev &v, int nLoop, const TileLists &lists);
 int tile_sms();
 // Reverse product from the kept digits (idw_tile_adjoint.cu).  denInv: per slot
 // the reciprocal denominator in the digits' units; part: nLoop * nVol doubles of

@@ -32,7 +32,6 @@ namespace {
 
 constexpr int kScaleExp = 13;   // node denominators are scaled to [2^13, 2^14)
 constexpr int kMotExp = 14;     // motions are scaled to at most 2^14
-constexpr int kTileWarps = 12;  // warps of a block: one block per SM
 constexpr int64_t kFourDigits = int64_t(1) << 17;  // node images up to which a warp uses four digits
 
 inline int blocks(int64_t n, int b) { return int((n + b - 1) / b); }
@@ -368,45 +367,65 @@ __global__ void k_tile_mot(TreeDev t, int nPts, const double *ptMB, const double
 
 enum { kStream = 0, kLists = 1, kDecide = 2 };
 
-// Shared memory of a stage: a streamed one holds the digits in use.
-constexpr size_t tile_stage_bytes(int src, int nd) {
-    return sizeof(TileStage) - (src == kStream && nd < 4 ? sizeof(uint4) * 64 : 0);
+// Warps of a block at nb surfaces (one block per SM): 16 at 128 registers, where
+// a walk of one surface waits for its copies (245k-node wing 243 -> 236 us against
+// 12 warps at 144 registers, 8M nodes 6.05 -> 5.94 ms; a third stage for 12 warps
+// is worth 0.13 ms there).  Two surfaces share a step's digits at 12 warps: 2.3 ms
+// a pair on the 2M-node wing, twice 1.33 alone; ten warps with three stages take
+// 3.2 ms.  The forms that make the weights as they go need more registers.
+constexpr int tile_warps(int src, int nb) { return src == kStream && nb == 1 ? 16 : 12; }
+// Shared memory of a stage with nb surfaces' motions: a streamed one holds the
+// digits in use.
+constexpr size_t tile_stage_bytes(int src, int nd, int nb) {
+    return nb * sizeof(uint4) * 8 * kTileTerms + sizeof(TileStage) -
+           (src == kStream && nd < 4 ? sizeof(uint4) * 64 : 0);
 }
 
 // The sums of one unit per warp: numerators about the reference motion and
-// denominator of each node, as pairs (high, low), into out.
+// denominator of each node, as pairs (high, low), into out, for NB surfaces
+// (td.mot, td.colMax and out in a row).
 // SRC: the digits streamed from memory (the next step's copied while one is
 // computed), formed from the lists, or formed from the decisions as they are
 // taken.
-template <int SRC, int ND>
-__global__ void __launch_bounds__(32 * kTileWarps, 1)
+template <int SRC, int ND, int NB>
+__global__ void __launch_bounds__(32 * tile_warps(SRC, NB), 1)
     k_tile_walk(TreeDev t, TreeDevF tf, VolumeDev v, WalkRecF rec, MixedParams mp, TileDev td, TileLists lists,
                 TileLaw law, unsigned nUnits, unsigned chunk, float4 *out, unsigned long long *counters) {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ unsigned long long qstate;
-    __shared__ TileRows rowsAll[SRC == kStream ? 1 : kTileWarps][16];
+    __shared__ TileRows rowsAll[SRC == kStream ? 1 : tile_warps(SRC, NB)][16];
     if (threadIdx.x == 0) qstate = 0ull;
     __syncthreads();
     const int lane = threadIdx.x & 31, g = lane >> 2, a = lane & 3;
-    constexpr size_t stageBytes = tile_stage_bytes(SRC, ND);
-    unsigned char *mine = smraw + (SRC == kStream ? 2 : 1) * stageBytes * (threadIdx.x >> 5);
-    auto stage = [&](int s) -> TileStage & { return *reinterpret_cast<TileStage *>(mine + stageBytes * (s & 1)); };
+    constexpr size_t stageBytes = tile_stage_bytes(SRC, ND, NB);
+    constexpr int NS = SRC == kStream ? 2 : 1;  // stages
+    unsigned char *mine = smraw + NS * stageBytes * (threadIdx.x >> 5);
+    const int64_t nTerms = tf.nPts + t.nNodes;
+    auto motions = [&](int s) { return reinterpret_cast<uint4 *>(mine + stageBytes * s); };
+    auto stage = [&](int s) -> TileStage & {
+        return *reinterpret_cast<TileStage *>(motions(s) + 8 * kTileTerms * NB);
+    };
+    auto fetch_motions = [&](int s, const StageIds &ids) {
+#pragma unroll
+        for (int b = 0; b < NB; ++b) stage_motions(motions(s) + 8 * kTileTerms * b, ids, td.mot + 8 * nTerms * b);
+    };
     UnitQueue queue = {&qstate, td.counter, nUnits, chunk, 0u, 0u};
     unsigned unit;
     while (queue.next(unit)) {
         const int64_t group = unit / unsigned(mp.nLoop);
         const int kk = int(unit - unsigned(group) * unsigned(mp.nLoop));
-        TileAcc<ND> acc;
-        tile_zero(acc);
+        TileAcc<ND> acc[NB];
+#pragma unroll
+        for (int b = 0; b < NB; ++b) tile_zero(acc[b]);
         if constexpr (SRC == kStream) {
             const int64_t e0 = lists.offs[unit];
             const int n = int((lists.offs[unit + 1] - e0) / kTileTerms);
             const int *term = lists.term + e0;
             const uint4 *dig = lists.dig + 192 * (e0 / kTileTerms), *dig3 = lists.dig3 + 64 * (e0 / kTileTerms);
             StageIds ids;
-            auto issue = [&](int s) {
-                TileStage &st = stage(s);
-                uint4 *dst = &st.dig[0][0][0];
+            // step s into stage b
+            auto issue = [&](int s, int b) {
+                uint4 *dst = &stage(b).dig[0][0][0];
 #pragma unroll
                 for (int c = 0; c < 6; ++c) cp_async16(dst + 32 * c + lane, dig + 192 * int64_t(s) + 32 * c + lane);
                 if constexpr (ND > 3) {
@@ -414,24 +433,24 @@ __global__ void __launch_bounds__(32 * kTileWarps, 1)
                     for (int c = 0; c < 2; ++c)
                         cp_async16(dst + 192 + 32 * c + lane, dig3 + 64 * int64_t(s) + 32 * c + lane);
                 }
-                stage_motions(st, ids, td.mot);
+                fetch_motions(b, ids);
+                if (s + 1 < n) ids = stage_ids(term + kTileTerms * (s + 1));
             };
-            if (n > 0) {
-                ids = stage_ids(term);
-                issue(0);
-                if (n > 1) ids = stage_ids(term + kTileTerms);
-            }
-            cp_async_commit();
-            for (int s = 0; s < n; ++s) {
-                if (s + 1 < n) {
-                    issue(s + 1);
-                    if (s + 2 < n) ids = stage_ids(term + kTileTerms * (s + 2));
-                }
+            if (n > 0) ids = stage_ids(term);
+#pragma unroll
+            for (int s = 0; s < NS - 1; ++s) {
+                if (s < n) issue(s, s);
                 cp_async_commit();
-                cp_async_wait<1>();
+            }
+            int b = 0;
+            for (int s = 0; s < n; ++s) {
+                if (s + NS - 1 < n) issue(s + NS - 1, b == 0 ? NS - 1 : b - 1);
+                cp_async_commit();
+                cp_async_wait<NS - 1>();
                 __syncwarp();
-                tile_step(stage(s), acc);
+                tile_step(stage(b), motions(b), acc);
                 __syncwarp();
+                b = b == NS - 1 ? 0 : b + 1;
             }
             cp_async_wait<0>();
         } else {
@@ -440,12 +459,12 @@ __global__ void __launch_bounds__(32 * kTileWarps, 1)
             unit_rows(rows, v, rec, td, group, kk);
             auto step = [&]() {
                 __syncwarp();
-                stage_motions(st, stage_ids(st.term), td.mot);
+                fetch_motions(0, stage_ids(st.term));
                 cp_async_commit();
                 stage_weights(st, td.geo, tf.nPts, rows, law);
                 cp_async_wait<0>();
                 __syncwarp();
-                tile_step(st, acc);
+                tile_step(st, motions(0), acc);
                 __syncwarp();
             };
             if constexpr (SRC == kLists) {
@@ -482,45 +501,49 @@ __global__ void __launch_bounds__(32 * kTileWarps, 1)
         }
         // component a of the numerator: D'_a . (r - O) + e_a; lane column 3: the denominator
         const float4 oh = ldgf4(td.geo + 2 * int64_t(tf.nPts)), ol = ldgf4(td.geo + 2 * int64_t(tf.nPts) + 1);
-        float cs[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) cs[k] = a < 3 ? pow2f(-column_exp(__ldg(td.colMax + 4 * a + k))) : 0.125f;
-        float *o = reinterpret_cast<float *>(out);
+        for (int b = 0; b < NB; ++b) {
+            float cs[4];
 #pragma unroll
-        for (int m = 0; m < 2; ++m)
+            for (int k = 0; k < 4; ++k)
+                cs[k] = a < 3 ? pow2f(-column_exp(__ldg(td.colMax + kTileWords * b + 4 * a + k))) : 0.125f;
+            float *o = reinterpret_cast<float *>(out + 2 * int64_t(mp.nLoop) * v.nVol * b);
 #pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                const int64_t slot = group * 32 + g + 16 * m + 8 * r;
-                if (slot >= v.nVol) continue;
-                dfl M[4];
+            for (int m = 0; m < 2; ++m)
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    // columns in the order of the motion records: D'_a0, D'_a1 | D'_a2, e_a
-                    const int n = k >> 1, j = 2 * r + (k & 1);
-                    const float2 a1 = acc.a1[m][n][r];
-                    float s, e;
-                    two_sum(acc.a0[m][n][j], k & 1 ? a1.y : a1.x, s, e);
-                    float low = e + acc.a2[m][n][j];
-                    if constexpr (ND > 3) low = fmaf(acc.a3[m][n][j], 1.0f / 4194304.0f, low);
-                    M[k] = df_norm(s * cs[k], low * cs[k]);
+                for (int r = 0; r < 2; ++r) {
+                    const int64_t slot = group * 32 + g + 16 * m + 8 * r;
+                    if (slot >= v.nVol) continue;
+                    dfl M[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        // columns in the order of the motion records: D'_a0, D'_a1 | D'_a2, e_a
+                        const int n = k >> 1, j = 2 * r + (k & 1);
+                        const float2 a1 = acc[b].a1[m][n][r];
+                        float s, e;
+                        two_sum(acc[b].a0[m][n][j], k & 1 ? a1.y : a1.x, s, e);
+                        float low = e + acc[b].a2[m][n][j];
+                        if constexpr (ND > 3) low = fmaf(acc[b].a3[m][n][j], 1.0f / 4194304.0f, low);
+                        M[k] = df_norm(s * cs[k], low * cs[k]);
+                    }
+                    const int64_t gid = kk * v.nVol + td.order[slot];
+                    const float4 hi = rec.hi[gid], lo = rec.lo[gid];
+                    const float h[3] = {hi.x, hi.y, hi.z}, l[3] = {lo.x, lo.y, lo.z};
+                    const float oh3[3] = {oh.x, oh.y, oh.z}, ol3[3] = {ol.x, ol.y, ol.z};
+                    dfl s = M[3];
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) {
+                        dfl x;
+                        two_diff(h[k], oh3[k], x.h, x.l);
+                        x.l += l[k] - ol3[k];
+                        s = df_add(s, df_mul(M[k], df_norm(x.h, x.l)));
+                    }
+                    if (a == 3) s = M[0];
+                    float *p = o + 8 * (kk * v.nVol + slot);
+                    p[a] = s.h;
+                    p[4 + a] = s.l;
                 }
-                const int64_t gid = kk * v.nVol + td.order[slot];
-                const float4 hi = rec.hi[gid], lo = rec.lo[gid];
-                const float h[3] = {hi.x, hi.y, hi.z}, l[3] = {lo.x, lo.y, lo.z};
-                const float oh3[3] = {oh.x, oh.y, oh.z}, ol3[3] = {ol.x, ol.y, ol.z};
-                dfl s = M[3];
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    dfl x;
-                    two_diff(h[k], oh3[k], x.h, x.l);
-                    x.l += l[k] - ol3[k];
-                    s = df_add(s, df_mul(M[k], df_norm(x.h, x.l)));
-                }
-                if (a == 3) s = M[0];
-                float *p = o + 8 * (kk * v.nVol + slot);
-                p[a] = s.h;
-                p[4 + a] = s.l;
-            }
+        }
     }
 }
 
@@ -610,6 +633,10 @@ void launch_tile_motions(const TreeDev &t, int nPts, const double *ptMB, const d
     k_tile_mot<<<blocks(n, 256), 256, 0, st>>>(t, nPts, ptMB, nodeMB, colMax, mot, refDB);
 }
 
+int tile_batch(const VolumeDev &v, int nLoop, const TileLists &lists) {
+    return lists.dig && v.nVol * nLoop > kFourDigits ? 2 : 1;
+}
+
 int64_t count_tile_lists(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
                          const EvalConsts &k, const TileDev &td, int64_t *offs, float *scale, int *bad,
                          cudaStream_t st) {
@@ -662,45 +689,53 @@ void launch_tile_build(const VolumeDev &v, const WalkRecF &rec, const EvalConsts
         v, rec, mp, td, lists, make_tile_law(k), nPts, unsigned(units), dig, dig3);
 }
 
-template <int SRC, int ND>
-static void walk_src(int nb, const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
+template <int SRC, int ND, int NB>
+static void walk_src(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
                      const MixedParams &mp, const TileDev &td, const TileLists &lists, const TileLaw &law,
-                     unsigned nUnits, unsigned chunk, float4 *sums, unsigned long long *counters, cudaStream_t st) {
-    const size_t smem = kTileWarps * (SRC == kStream ? 2 : 1) * tile_stage_bytes(SRC, ND);
-    cudaFuncSetAttribute(k_tile_walk<SRC, ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    k_tile_walk<SRC, ND><<<nb, 32 * kTileWarps, smem, st>>>(t, tf, v, rec, mp, td, lists, law, nUnits, chunk, sums,
+                     unsigned nUnits, float4 *sums, unsigned long long *counters, cudaStream_t st) {
+    constexpr int warps = tile_warps(SRC, NB);
+    const int sms = tile_sms(), grid = int(min(int64_t(sms), (int64_t(nUnits) + warps - 1) / warps));
+    const unsigned chunk = unsigned(max(int64_t(1), min(int64_t(32), int64_t(nUnits) / (4 * sms * warps))));
+    const size_t smem = warps * (SRC == kStream ? 2 : 1) * tile_stage_bytes(SRC, ND, NB);
+    cudaFuncSetAttribute(k_tile_walk<SRC, ND, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    k_tile_walk<SRC, ND, NB><<<grid, 32 * warps, smem, st>>>(t, tf, v, rec, mp, td, lists, law, nUnits, chunk, sums,
                                                         counters);
 }
 
 void launch_tile_walk(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
                       const EvalConsts &k, const TileDev &td, const TileLists &lists, const float *refDB, float4 *sums,
-                      const WalkOut &o, cudaStream_t st) {
+                      const WalkOut &o, cudaStream_t st, int nb) {
     if (v.nVol <= 0) return;
     const MixedParams mp = make_mixed_params(k);
     const TileLaw law = make_tile_law(k);
     const unsigned nUnits = unsigned(walk_list_warps(v.nVol) * mp.nLoop);
-    const int sms = tile_sms(), nb = int(min(int64_t(sms), (int64_t(nUnits) + kTileWarps - 1) / kTileWarps));
-    const unsigned chunk = unsigned(max(int64_t(1), min(int64_t(32), int64_t(nUnits) / (4 * sms * kTileWarps))));
     if (lists.term) launch_add_walk_counters(o.counters, lists.counters, st);
     // Four digits for small meshes, where they stay in cache; three stream a
     // quarter less.
+    const bool four = v.nVol * mp.nLoop <= kFourDigits;
     const int src = lists.dig ? kStream : (lists.term ? kLists : kDecide);
-    auto go = [&](auto srcC, auto ndC) {
-        walk_src<decltype(srcC)::value, decltype(ndC)::value>(nb, t, tf, v, rec, mp, td, lists, law, nUnits, chunk, sums,
-                                                              o.counters, st);
+    auto go = [&](auto srcC, auto ndC, auto nbC) {
+        walk_src<decltype(srcC)::value, decltype(ndC)::value, decltype(nbC)::value>(
+            t, tf, v, rec, mp, td, lists, law, nUnits, sums, o.counters, st);
     };
+    using One = std::integral_constant<int, 1>;
     auto goSrc = [&](auto ndC) {
-        if (src == kStream) go(std::integral_constant<int, kStream>(), ndC);
-        else if (src == kLists) go(std::integral_constant<int, kLists>(), ndC);
-        else go(std::integral_constant<int, kDecide>(), ndC);
+        if (src == kStream) go(std::integral_constant<int, kStream>(), ndC, One());
+        else if (src == kLists) go(std::integral_constant<int, kLists>(), ndC, One());
+        else go(std::integral_constant<int, kDecide>(), ndC, One());
     };
-    if (v.nVol * mp.nLoop <= kFourDigits) goSrc(std::integral_constant<int, 4>());
+    if (nb == 2)
+        go(std::integral_constant<int, kStream>(), std::integral_constant<int, 3>(), std::integral_constant<int, 2>());
+    else if (four) goSrc(std::integral_constant<int, 4>());
     else goSrc(std::integral_constant<int, 3>());
-    NodeAggF af{};
-    af.ref = refDB;
     const double L = k.law.Ldef;
-    k_tile_finalize<<<blocks(v.nVol, 128), 128, 0, st>>>(v, rec, af, mp, td, sums, ldexp(L * L * L, -td.areaExp),
-                                                         o.xv, o.den);
+    for (int b = 0; b < nb; ++b) {
+        NodeAggF af{};
+        af.ref = refDB + 24 * b;
+        k_tile_finalize<<<blocks(v.nVol, 128), 128, 0, st>>>(v, rec, af, mp, td, sums + 2 * mp.nLoop * v.nVol * b,
+                                                             ldexp(L * L * L, -td.areaExp),
+                                                             o.xv ? o.xv + 3 * v.nVol * b : nullptr, o.den);
+    }
 }
 
 }  // namespace idw

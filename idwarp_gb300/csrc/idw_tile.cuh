@@ -154,11 +154,11 @@ __device__ __forceinline__ void tile_digits(float2 wa, float2 la, float2 wb, flo
 }
 
 // One step's data in shared memory, a stage per warp.  dig: digit d of tile m as
-// the lanes' fragment registers.  mot: the terms' motion records, chunk g of
-// term k at 8 k + (g ^ 2 (k / 4)), so that the fragment-order reads (lane
-// (g, t): terms 4t .. 4t+3) meet no bank conflict.
+// the lanes' fragment registers.  The terms' motion records lie in front of it,
+// kTileTerms x 8 chunks of each surface, chunk g of term k at 8 k + (g ^ 2 (k /
+// 4)), so that the fragment-order reads (lane (g, t): terms 4t .. 4t+3) meet no
+// bank conflict.
 struct TileStage {
-    uint4 mot[8 * kTileTerms];
     int term[kTileTerms];
     unsigned mask[kTileTerms];
     uint4 dig[4][2][32];
@@ -224,11 +224,11 @@ __device__ __forceinline__ StageIds stage_ids(const int *term) {
     const int r = (threadIdx.x & 31) >> 3;
     return {{term[r], term[4 + r], term[8 + r], term[12 + r]}};
 }
-__device__ __forceinline__ void stage_motions(TileStage &st, const StageIds &s, const uint4 *mot) {
+__device__ __forceinline__ void stage_motions(uint4 *dst, const StageIds &s, const uint4 *mot) {
     const int lane = threadIdx.x & 31, g = lane & 7;
 #pragma unroll
     for (int c = 0; c < 4; ++c)
-        cp_async16_l1(&st.mot[8 * (4 * c + (lane >> 3)) + (g ^ (2 * c))], mot + 8 * int64_t(s.t[c]) + g);
+        cp_async16_l1(&dst[8 * (4 * c + (lane >> 3)) + (g ^ (2 * c))], mot + 8 * int64_t(s.t[c]) + g);
 }
 
 // The volume nodes of a lane: row pair (g + 16 m, g + 16 m + 8) of tile m.
@@ -298,53 +298,66 @@ __device__ __forceinline__ void tile_zero(TileAcc<ND> &acc) {
         }
 }
 
-// One step of the forward sums with ND digits of the weights and the motions.
-template <int ND>
-__device__ __forceinline__ void tile_step(const TileStage &st, TileAcc<ND> &acc) {
+// One step of the forward sums with ND digits of the weights and of NB surfaces'
+// motions (mot: one array of the step's records each).
+template <int ND, int NB>
+__device__ __forceinline__ void tile_step(const TileStage &st, const uint4 *mot, TileAcc<ND> (&accs)[NB]) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    uint4 q[4];
+    // motion digits of the lane's terms: [surface][8-column tile][digit][fragment register]
+    unsigned B[NB][2][ND][2];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) q[j] = st.mot[8 * (4 * t + j) + (g ^ (2 * t))];
-#pragma unroll
-    for (int n = 0; n < 2; ++n) {
-        // motion digits of the lane's terms: [digit][fragment register]
-        unsigned B[ND][2];
+    for (int b = 0; b < NB; ++b)
 #pragma unroll
         for (int p = 0; p < 2; ++p) {
-            const uint4 x = q[2 * p], y = q[2 * p + 1];
-            B[0][p] = n ? __byte_perm(x.z, y.z, 0x5410) : __byte_perm(x.x, y.x, 0x5410);
-            B[1][p] = n ? __byte_perm(x.z, y.z, 0x7632) : __byte_perm(x.x, y.x, 0x7632);
-            B[2][p] = n ? __byte_perm(x.w, y.w, 0x5410) : __byte_perm(x.y, y.y, 0x5410);
-            if constexpr (ND > 3) B[3][p] = n ? __byte_perm(x.w, y.w, 0x7632) : __byte_perm(x.y, y.y, 0x7632);
-        }
-#pragma unroll
-        for (int m = 0; m < 2; ++m) {
-            const uint4 A0 = st.dig[0][m][lane], A1 = st.dig[1][m][lane], A2 = st.dig[2][m][lane];
-            mma_f16(acc.a0[m][n], A0, B[0][0], B[0][1]);
-            // one digit down: exact in a step (the tensor core truncates its
-            // sums, which over a list would be a bias), added by two-sums whose
-            // errors join the rest
-            float d[4];
-            mma_f16_first(d, A0, B[1][0], B[1][1]);
-            mma_f16(d, A1, B[0][0], B[0][1]);
-            mma_f16(acc.a2[m][n], A1, B[1][0], B[1][1]);
-            mma_f16(acc.a2[m][n], A0, B[2][0], B[2][1]);
-            mma_f16(acc.a2[m][n], A2, B[0][0], B[0][1]);
+            const uint4 *q = mot + 8 * kTileTerms * b + 8 * (4 * t + 2 * p) + (g ^ (2 * t));
+            const uint4 x = q[0], y = q[8];
+            B[b][0][0][p] = __byte_perm(x.x, y.x, 0x5410);
+            B[b][0][1][p] = __byte_perm(x.x, y.x, 0x7632);
+            B[b][0][2][p] = __byte_perm(x.y, y.y, 0x5410);
+            B[b][1][0][p] = __byte_perm(x.z, y.z, 0x5410);
+            B[b][1][1][p] = __byte_perm(x.z, y.z, 0x7632);
+            B[b][1][2][p] = __byte_perm(x.w, y.w, 0x5410);
             if constexpr (ND > 3) {
-                mma_f16(acc.a2[m][n], A1, B[2][0], B[2][1]);
-                mma_f16(acc.a2[m][n], A2, B[1][0], B[1][1]);
-                mma_f16(acc.a3[m][n], A0, B[3][0], B[3][1]);
-                mma_f16(acc.a3[m][n], st.dig[3][m][lane], B[0][0], B[0][1]);
-            }
-#pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                float2 s, e;
-                two_sum2(acc.a1[m][n][r], make_float2(d[2 * r], d[2 * r + 1]), s, e);
-                acc.a1[m][n][r] = s;
-                acc.a2[m][n][2 * r] += e.x;
-                acc.a2[m][n][2 * r + 1] += e.y;
+                B[b][0][3][p] = __byte_perm(x.y, y.y, 0x7632);
+                B[b][1][3][p] = __byte_perm(x.w, y.w, 0x7632);
             }
         }
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+        const uint4 A0 = st.dig[0][m][lane], A1 = st.dig[1][m][lane], A2 = st.dig[2][m][lane];
+        uint4 A3 = make_uint4(0u, 0u, 0u, 0u);
+        if constexpr (ND > 3) A3 = st.dig[3][m][lane];
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                TileAcc<ND> &acc = accs[b];
+                const unsigned(&C)[ND][2] = B[b][n];
+                mma_f16(acc.a0[m][n], A0, C[0][0], C[0][1]);
+                // one digit down: exact in a step (the tensor core truncates its
+                // sums, which over a list would be a bias), added by two-sums whose
+                // errors join the rest
+                float d[4];
+                mma_f16_first(d, A0, C[1][0], C[1][1]);
+                mma_f16(d, A1, C[0][0], C[0][1]);
+                mma_f16(acc.a2[m][n], A1, C[1][0], C[1][1]);
+                mma_f16(acc.a2[m][n], A0, C[2][0], C[2][1]);
+                mma_f16(acc.a2[m][n], A2, C[0][0], C[0][1]);
+                if constexpr (ND > 3) {
+                    mma_f16(acc.a2[m][n], A1, C[2][0], C[2][1]);
+                    mma_f16(acc.a2[m][n], A2, C[1][0], C[1][1]);
+                    mma_f16(acc.a3[m][n], A0, C[3][0], C[3][1]);
+                    mma_f16(acc.a3[m][n], A3, C[0][0], C[0][1]);
+                }
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    float2 s, e;
+                    two_sum2(acc.a1[m][n][r], make_float2(d[2 * r], d[2 * r + 1]), s, e);
+                    acc.a1[m][n][r] = s;
+                    acc.a2[m][n][2 * r] += e.x;
+                    acc.a2[m][n][2 * r + 1] += e.y;
+                }
+            }
     }
 }
 

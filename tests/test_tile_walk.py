@@ -80,3 +80,17 @@ def test_law_change_rebuilds_the_weights(built_lib):
     f.setSurfaceCoordinates(m["xs"])
     f.warpMesh()
     assert np.abs(g.getWarpGrid() - f.getWarpGrid()).max() < 1e-9 * f.getStats()["Ldef0"]
+
+
+@pytest.mark.parametrize("count", [2, 3, 5])
+def test_batch_pairs_equal_single_warps(built_lib, count):
+    """Above 2^17 node images a batch takes two surfaces a walk: the same bits."""
+    m = S.wing_shell(121, 41, 16)
+    g = build_gpu(m, {"errTol": 1e-3}, precision="mixed")
+    xs = np.stack([np.asarray(m["pts"]) * (1.0 + 0.01 * i) for i in range(count)])
+    assert g.nVol * 2 > 2**17
+    out = np.asarray(g.warpMeshBatch(xs)).reshape(count, -1)
+    for x, a in zip(xs, out):
+        g.setSurfaceCoordinates(x)
+        g.warpMesh()
+        np.testing.assert_array_equal(a, np.asarray(g.getWarpGrid()).reshape(-1))
