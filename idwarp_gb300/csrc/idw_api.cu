@@ -127,8 +127,13 @@ struct Ctx {
     DevBuf<double> tileDenInv;
     DevBuf<unsigned> tileWord;  // 12 column maxima, the walk's counter, the bad flag
     DevBuf<int64_t> tileOffs;
-    DevBuf<int> tileTerm;
-    DevBuf<unsigned> tileMask;
+    DevBuf<int> tileTerm, tileCTerm;
+    DevBuf<unsigned> tileMask, tileCMask;
+    DevBuf<uint4> tileCDig, tileCDig3;  // scratch of one run of groups where no digits are kept
+    struct TileRun {
+        TileRange list, dig;
+    };
+    std::vector<TileRun> tileChunks;  // the runs
     DevBuf<unsigned long long> tileCnt;
     int tileFifthState = 0;  // the reverse product's fifth digit and denominators: 1 made, -1 too large, 0 not made
     int tileState = 0, tileListState = 0;  // tileListState: 1 lists, 2 lists and digits, -1 too large, 0 not made
@@ -922,6 +927,60 @@ static int fits_half(Ctx *c, double bytes, bool &yes) {
     return IDW_OK;
 }
 
+// Every group of the mesh.
+static TileRange tile_all(const Ctx *c) {
+    TileRange r;
+    r.group1 = walk_list_warps(c->nVol);
+    return r;
+}
+
+// Without kept digits a walk makes them a run of groups at a time, and the lists
+// for a longer run before that unless they are kept: list runs of at most
+// kListSteps steps (128 bytes each) in digit runs of at most kDigitSteps (4 kB
+// each), or one group.  Recorded, made and walked apart, at full occupancy each:
+// formed within the walk they took 12.1 instead of 7.9 ms on the 2M-node wing with
+// the lists off.  A short list run still takes one warp's traversal (0.4 ms).
+constexpr int64_t kListSteps = int64_t(1) << 22, kDigitSteps = int64_t(1) << 19;
+
+static int ensure_tile_chunks(Ctx *c) {
+    if (!c->tileChunks.empty()) return IDW_OK;
+    const int64_t groups = walk_list_warps(c->nVol), nl = c->sym.nLoop;
+    std::vector<int64_t> offs(size_t(groups * nl) + 1);
+    CK(cudaMemcpyAsync(offs.data(), c->tileOffs.p, sizeof(int64_t) * offs.size(), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    int64_t widest = 1;
+    for (int64_t g = 0; g < groups; ++g) widest = std::max(widest, (offs[(g + 1) * nl] - offs[g * nl]) / 16);
+    // a run of groups from g on, at most cap steps and up to group end
+    auto run = [&](int64_t g, int64_t end, int64_t cap) {
+        TileRange r;
+        r.group0 = g;
+        r.entry0 = offs[g * nl];
+        while (g < end && offs[(g + 1) * nl] - r.entry0 <= 16 * cap) ++g;
+        r.group1 = g;
+        return r;
+    };
+    int64_t listCap = std::max(widest, std::min(kListSteps, offs.back() / 16));
+    int64_t digCap = std::max(widest, std::min(kDigitSteps, offs.back() / 16));
+    while (c->tileCTerm.alloc(16 * size_t(listCap)) != cudaSuccess ||
+           c->tileCMask.alloc(16 * size_t(listCap)) != cudaSuccess ||
+           c->tileCDig.alloc(192 * size_t(digCap)) != cudaSuccess ||
+           c->tileCDig3.alloc(64 * size_t(digCap)) != cudaSuccess) {
+        (void)cudaGetLastError();
+        if (listCap == widest && digCap == widest) return fail(c, IDW_ERR_NOMEM, "no room for the walk's scratch");
+        listCap = std::max(widest, listCap / 2);
+        digCap = std::max(widest, digCap / 2);
+    }
+    for (int64_t g = 0; g < groups;) {
+        const TileRange l = run(g, groups, listCap);
+        for (g = l.group0; g < l.group1;) {
+            const TileRange d = run(g, l.group1, digCap);
+            c->tileChunks.push_back({l, d});
+            g = d.group1;
+        }
+    }
+    return IDW_OK;
+}
+
 // What a tile walk needs besides the motions: node order, term geometry, node
 // scales, and (unless off) the lists and the weight digits, each when it fits.
 // use = false when the walk does not apply or some node has no scale.
@@ -938,14 +997,15 @@ static int ensure_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const Ev
         const int64_t units = walk_list_warps(c->nVol) * c->sym.nLoop;
         const bool newLists = !off && c->tileListState == 0;
         c->tileState = 0;
+        c->tileChunks.clear();
         if (newLists) {
             c->tileTerm.release();
             c->tileMask.release();
             c->tileDig.release();
             c->tileDig3.release();
             c->tileDig4.release();
-            CKA(c->tileOffs.alloc(size_t(units) + 1));
         }
+        CKA(c->tileOffs.alloc(size_t(units) + 1));
         CKA(c->tileGeo.alloc(2 * nTerms));
         CKA(c->tileMot.alloc(8 * nTerms));
         CKA(c->tileWord.alloc(2 * kTileWords));
@@ -959,15 +1019,16 @@ static int ensure_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const Ev
         }
         launch_tile_geo(tree_dev(c), c->nUnique, c->ptXA.p, c->areaExp, c->tileGeo.p, c->stream);
         int *bad = reinterpret_cast<int *>(c->tileWord.p + 13);
-        const int64_t total = count_tile_lists(tree_dev(c), tf, vol_dev(c), rec, k, tile_dev(c),
-                                               newLists ? c->tileOffs.p : nullptr, c->tileScale.p, bad, c->stream);
+        const int64_t total = count_tile_lists(tree_dev(c), tf, vol_dev(c), rec, k, tile_dev(c), c->tileOffs.p,
+                                               reinterpret_cast<float *>(c->tileSums.p), c->tileScale.p, bad,
+                                               c->stream);
         if (total < 0) return fail(c, IDW_ERR_CUDA, "walk lists: count pass failed");
         int badH = 0;
         CK(cudaMemcpyAsync(&badH, bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
         bool fits = false;
+        c->tileListEntries = total;
         if (newLists && !badH) {
-            c->tileListEntries = total;
             int rc = fits_half(c, 8.0 * double(total), fits);
             if (rc) return rc;
             if (fits) {
@@ -975,8 +1036,8 @@ static int ensure_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const Ev
                 CKA(c->tileTerm.alloc(size_t(std::max<int64_t>(total, 1))));
                 CKA(c->tileMask.alloc(size_t(std::max<int64_t>(total, 1))));
                 CK(cudaMemsetAsync(c->tileCnt.p, 0, 8 * sizeof(unsigned long long), c->stream));
-                launch_tile_record(tree_dev(c), tf, vol_dev(c), rec, k, tile_dev(c), c->tileOffs.p, c->tileTerm.p,
-                                   c->tileMask.p, c->tileCnt.p, c->stream);
+                launch_tile_record(tree_dev(c), tf, vol_dev(c), rec, k, tile_dev(c), tile_all(c), c->tileOffs.p,
+                                   c->tileTerm.p, c->tileMask.p, c->tileCnt.p, c->stream);
                 rc = check_launch(c, "walk lists");
                 if (rc) return rc;
             }
@@ -998,8 +1059,8 @@ static int ensure_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const Ev
                 lists.term = c->tileTerm.p;
                 lists.mask = c->tileMask.p;
                 c->tileFifthState = 0;
-                launch_tile_build(vol_dev(c), rec, k, tile_dev(c), lists, c->nUnique, c->tileDig.p, c->tileDig3.p,
-                                  c->stream);
+                launch_tile_build(vol_dev(c), rec, k, tile_dev(c), lists, tile_all(c), 0, c->nUnique, c->tileDig.p,
+                                  c->tileDig3.p, c->stream);
                 int rc = check_launch(c, "weight digits");
                 if (rc) return rc;
             }
@@ -1011,8 +1072,8 @@ static int ensure_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const Ev
     }
     use = c->tileState == 1;
     lists = TileLists{};
+    lists.offs = c->tileOffs.p;
     if (use && !off && c->tileListState > 0) {
-        lists.offs = c->tileOffs.p;
         lists.term = c->tileTerm.p;
         lists.mask = c->tileMask.p;
         lists.counters = c->tileCnt.p;
@@ -1021,16 +1082,39 @@ static int ensure_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const Ev
             lists.dig3 = c->tileDig3.p;
         }
     }
-    return IDW_OK;
+    return use && !lists.dig ? ensure_tile_chunks(c) : IDW_OK;
 }
 
-// A tile walk over the motions (ptMB, nodeMB).
+// The tile walk of nb surfaces whose motion records are laid out, and their grids.
 static int run_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalConsts &k, const TileLists &lists,
-                    const double *ptMB, const double *nodeMB, const WalkOut &o) {
-    launch_tile_motions(tree_dev(c), c->nUnique, ptMB, nodeMB, c->tileWord.p, c->tileMot.p, c->refDB.p, c->stream);
-    CK(cudaEventRecord(c->ev0, c->stream));
-    launch_tile_walk(tree_dev(c), tf, vol_dev(c), rec, k, tile_dev(c), lists, c->refDB.p, c->tileSums.p, o, c->stream);
-    return IDW_OK;
+                    const WalkOut &o, int nb) {
+    const TreeDev t = tree_dev(c);
+    const VolumeDev v = vol_dev(c);
+    const TileDev td = tile_dev(c);
+    if (lists.counters && o.counters) launch_add_walk_counters(o.counters, lists.counters, c->stream);
+    if (lists.dig) {
+        launch_tile_walk(t, tf, v, rec, k, td, lists, tile_all(c), c->tileSums.p, c->stream, nb);
+    } else {
+        for (const Ctx::TileRun &r : c->tileChunks) {
+            TileLists l = lists;
+            int64_t first = r.dig.entry0;  // where the run's lists begin
+            if (!lists.term) {
+                l.term = c->tileCTerm.p;
+                l.mask = c->tileCMask.p;
+                first -= r.list.entry0;
+                if (first == 0)
+                    launch_tile_record(t, tf, v, rec, k, td, r.list, lists.offs, c->tileCTerm.p, c->tileCMask.p,
+                                       o.counters, c->stream);
+            }
+            launch_tile_build(v, rec, k, td, l, r.dig, first, c->nUnique, c->tileCDig.p, c->tileCDig3.p, c->stream);
+            l.term += first;
+            l.dig = c->tileCDig.p;
+            l.dig3 = c->tileCDig3.p;
+            launch_tile_walk(t, tf, v, rec, k, td, l, r.dig, c->tileSums.p, c->stream, nb);
+        }
+    }
+    launch_tile_finalize(v, rec, k, td, c->refDB.p, c->tileSums.p, o, c->stream, nb);
+    return check_launch(c, "tile walk");
 }
 
 // The reverse product from the weight digits: what ensure_tile gives, the fifth
@@ -1052,7 +1136,8 @@ static int ensure_tile_adjoint(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, 
             CKA(c->tileDig4.alloc(64 * steps));
             CKA(c->tileDenInv.alloc(size_t(c->nVol)));
             lists.dig4 = c->tileDig4.p;
-            launch_tile_build(vol_dev(c), rec, k, tile_dev(c), lists, c->nUnique, nullptr, c->tileDig4.p, c->stream);
+            launch_tile_build(vol_dev(c), rec, k, tile_dev(c), lists, tile_all(c), 0, c->nUnique, nullptr,
+                              c->tileDig4.p, c->stream);
             launch_tile_den_inv(c->nVol, c->sym.nLoop, lists, reinterpret_cast<double *>(c->tileSums.p),
                                 c->tileDenInv.p, c->stream);
             rc = check_launch(c, "fifth digits");
@@ -1118,7 +1203,10 @@ static int run_warp(Ctx *c, double *xvOut, double *denOut) {
     rc = refresh_nodal(c, !tile);
     if (rc) return rc;
     if (tile) {
-        rc = run_tile(c, tf, rec, k, lists, c->ptMB.p, c->nodeMB.p, o);
+        launch_tile_motions(tree_dev(c), c->nUnique, c->ptMB.p, c->nodeMB.p, c->tileWord.p, c->tileMot.p, c->refDB.p,
+                            c->stream);
+        CK(cudaEventRecord(c->ev0, c->stream));
+        rc = run_tile(c, tf, rec, k, lists, o, 1);
         if (rc) return rc;
     } else if (c->opt.precision == IDW_PREC_MIXED) {
         PointsDevF pf;
@@ -1290,7 +1378,7 @@ static int run_tile_batch(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const
     c->nodalValid = false;
     const SurfaceDev s = surf_dev(c);
     const size_t nTerms = size_t(n) + size_t(c->nNodes);
-    int per = nb > 1 ? tile_batch(vol_dev(c), c->sym.nLoop, lists) : 1;
+    int per = nb > 1 ? tile_batch(vol_dev(c), c->sym.nLoop) : 1;
     if (per > 1) {
         bool fits = false;
         const size_t sums = 2 * size_t(c->sym.nLoop) * size_t(c->nVol);
@@ -1316,8 +1404,8 @@ static int run_tile_batch(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const
         WalkOut o;
         o.xv = outDev + size_t(b0) * vdof;
         o.counters = b0 == 0 ? c->counters.p : nullptr;
-        launch_tile_walk(tree_dev(c), tf, vol_dev(c), rec, k, tile_dev(c), lists, c->refDB.p, c->tileSums.p, o,
-                         c->stream, m);
+        int rc = run_tile(c, tf, rec, k, lists, o, m);
+        if (rc) return rc;
     }
     CK(cudaEventRecord(c->ev1, c->stream));
     c->eventsRecorded = true;

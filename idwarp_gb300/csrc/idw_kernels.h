@@ -214,9 +214,9 @@ void launch_walk_replay(const TreeDevF &tf, const PointsDevF &pf, const NodeAggF
 // node for a cluster.
 struct TileLists {
     const int64_t *offs = nullptr;  // units + 1 entry offsets
-    const int *term = nullptr;      // null: the walk decides as it goes
+    const int *term = nullptr;      // null: not kept
     const unsigned *mask = nullptr;
-    const uint4 *dig = nullptr;     // per step 192: the first three digits of the weights; null: formed as it goes
+    const uint4 *dig = nullptr;     // per step 192: the first three digits of the weights; null: not kept
     const uint4 *dig3 = nullptr;    // per step 64: the fourth
     const uint4 *dig4 = nullptr;    // per step 64: the fifth, which only the reverse product reads
     const unsigned long long *counters = nullptr;  // the recording walk's, as WalkLists::counters
@@ -235,26 +235,36 @@ struct TileDev {
 // a CUDA error, -2 without memory; synchronises st.
 int tile_order(const VolumeDev &v, const double *lo, const double *hi, int *order, cudaStream_t st);
 void launch_tile_geo(const TreeDev &t, int nPts, const dbl4 *xa, int areaExp, float4 *geo, cudaStream_t st);
-// Fills scale, raises *bad when a node has none, fills offs (unless null) and
-// returns the number of entries (-1 on a CUDA error); synchronises st.
+// Fills scale, raises *bad when a node has none, fills offs and returns the number
+// of entries (-1 on a CUDA error); part: nLoop nVol floats of scratch.  Synchronises st.
 int64_t count_tile_lists(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
-                         const EvalConsts &k, const TileDev &td, int64_t *offs, float *scale, int *bad,
+                         const EvalConsts &k, const TileDev &td, int64_t *offs, float *part, float *scale, int *bad,
                          cudaStream_t st);
+// A run of groups; entry0 is the list entry that lies first in the arrays given.
+struct TileRange {
+    int64_t group0 = 0, group1 = 0, entry0 = 0;
+};
 void launch_tile_record(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
-                        const EvalConsts &k, const TileDev &td, const int64_t *offs, int *term, unsigned *mask,
-                        unsigned long long *counters, cudaStream_t st);
+                        const EvalConsts &k, const TileDev &td, const TileRange &range, const int64_t *offs, int *term,
+                        unsigned *mask, unsigned long long *counters, cudaStream_t st);
+// The digits of the range's entries (dig null: the fifth, into dig3); its lists lie
+// from entry listEntry0 of lists.term and lists.mask.
 void launch_tile_build(const VolumeDev &v, const WalkRecF &rec, const EvalConsts &k, const TileDev &td,
-                       const TileLists &lists, int nPts, uint4 *dig, uint4 *dig3, cudaStream_t st);
+                       const TileLists &lists, const TileRange &range, int64_t listEntry0, int nPts, uint4 *dig,
+                       uint4 *dig3, cudaStream_t st);
 // The current motions (12 per point and tree node) as motion records, and the reference motion.
 void launch_tile_motions(const TreeDev &t, int nPts, const double *ptMB, const double *nodeMB, unsigned *colMax,
                          uint4 *mot, float *refDB, cudaStream_t st);
-// sums: 2 nLoop nVol float4 of scratch.
+// The range's sums of nb surfaces (sums: 2 nLoop nVol float4 each), then their grids
+// (o.xv in a row) and denominators.
 void launch_tile_walk(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
-                      const EvalConsts &k, const TileDev &td, const TileLists &lists, const float *refDB, float4 *sums,
-                      const WalkOut &o, cudaStream_t st, int nb = 1);
+                      const EvalConsts &k, const TileDev &td, const TileLists &lists, const TileRange &range,
+                      float4 *sums, cudaStream_t st, int nb = 1);
+void launch_tile_finalize(const VolumeDev &v, const WalkRecF &rec, const EvalConsts &k, const TileDev &td,
+                          const float *refDB, const float4 *sums, const WalkOut &o, cudaStream_t st, int nb = 1);
 // Surfaces that one tile walk takes (launch_tile_walk's nb): 2 where the digits
 // stream from memory.
-int tile_batch(const VolumeDev &v, int nLoop, const TileLists &lists);
+int tile_batch(const VolumeDev &v, int nLoop);
 int tile_sms();
 // Reverse product from the kept digits (idw_tile_adjoint.cu).  denInv: per slot
 // the reciprocal denominator in the digits' units; part: nLoop * nVol doubles of

@@ -16,8 +16,8 @@
 //
 // The terms are those of the reference's decisions (decide32 + resolve64, as
 // k_walk_record), recorded once per den0, errTol and law.  Without room for the
-// digits a walk forms them as it goes, from the lists or (walkLists off) from
-// the decisions as it takes them; every form gives the same bits.
+// digits or (walkLists off) the lists a walk makes them for a run of groups at a
+// time; every form gives the same bits.
 #include <climits>
 #include <type_traits>
 
@@ -138,73 +138,79 @@ __device__ __forceinline__ void decide_group(const TreeDev &t, const TreeDevF &t
     }
 }
 
-// List lengths (whole steps) of every unit into counts, and each node's weight
-// scale: its FP32 denominator over all mirrors, under a first guess from the
-// estimate (den0 2^(5s) ~ 1), and from it the power of two that brings the
-// denominator to [2^13, 2^14).  A node whose denominator is not a positive
-// normal number, or whose scale leaves the range, raises bad (the gated walk
-// then serves the mesh).
-__global__ void __launch_bounds__(128, 8)
-    k_tile_count(TreeDev t, TreeDevF tf, VolumeDev v, WalkRecF rec, MixedParams mp, TileDev td, TileLaw law,
-                 int lawExp, int64_t nGroups, int64_t *counts, float *scale, int *bad) {
-    const int64_t slot = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    const int64_t group = slot >> 5;
-    if (group >= nGroups) return;  // whole warps only
-    const int lane = threadIdx.x & 31;
-    const int64_t gid = td.order[min(slot, v.nVol - 1)];
-    const int first = max(-110, min(110, 5 * __float_as_int(rec.lo[gid].w) + lawExp));
-    const float P = pow2f(first);
-    float den = 0.f;
-    MixedCounters cnt;
-    for (int kk = 0; kk < mp.nLoop; ++kk) {
-        const float4 rhi = rec.hi[kk * v.nVol + gid], rlo = rec.lo[kk * v.nVol + gid];
-        int n = 0;
-        decide_group(t, tf, v, rec, mp, td, slot, kk, cnt, nullptr, [&](int term, unsigned m) {
-            ++n;
-            if ((m >> lane) & 1u) {
-                const float4 c = ldgf4(td.geo + 2 * int64_t(term)), d = ldgf4(td.geo + 2 * int64_t(term) + 1);
-                const float dx = (rhi.x - c.x) + (rlo.x - d.x), dy = (rhi.y - c.y) + (rlo.y - d.y),
-                            dz = (rhi.z - c.z) + (rlo.z - d.z);
-                const float y = rsqrt_normal(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, term < tf.nPts ? 1e-15f : 0.f))));
-                const float y2 = y * y;
-                den = fmaf(c.w * (y2 * (y * P)), fmaf(law.kh, y2, 1.0f), den);
-            }
-        });
-        if (lane == 0 && counts)
-            counts[group * mp.nLoop + kk] = int64_t(n + kTileTerms - 1) / kTileTerms * kTileTerms;
-    }
-    if (slot < v.nVol) {
-        const int ex = int((__float_as_uint(den) >> 23) & 0xffu);
-        const int k = kScaleExp - (ex - 127) + first;
-        const bool ok = den > 0.f && ex > 0 && ex < 255 && k >= -118 && k <= 118;
-        if (!ok) *bad = 1;
-        scale[slot] = ok ? pow2f(k) : 1.0f;
-    }
+// First guess of a node's weight scale (log2), from the estimate: den0 2^(5s) ~ 1.
+__device__ __forceinline__ int first_scale(const WalkRecF &rec, int64_t gid, int lawExp) {
+    return max(-110, min(110, 5 * __float_as_int(rec.lo[gid].w) + lawExp));
 }
 
-// The lists' entries at offs, padded with empty ones.
+// List lengths (whole steps) of every unit, a warp each, into counts, and the
+// unit's share of its nodes' FP32 denominators under the first guess into part
+// (nLoop x nVol).
 __global__ void __launch_bounds__(128, 8)
-    k_tile_record(TreeDev t, TreeDevF tf, VolumeDev v, WalkRecF rec, MixedParams mp, TileDev td, int64_t nGroups,
-                  const int64_t *offs, int *term, unsigned *mask, unsigned long long *counters) {
-    const int64_t slot = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    const int64_t group = slot >> 5;
+    k_tile_count(TreeDev t, TreeDevF tf, VolumeDev v, WalkRecF rec, MixedParams mp, TileDev td, TileLaw law,
+                 int lawExp, int64_t nGroups, int64_t *counts, float *part) {
+    const int64_t unit = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const int64_t group = unit / mp.nLoop;
     if (group >= nGroups) return;  // whole warps only
-    const int lane = threadIdx.x & 31;
+    const int kk = int(unit - group * mp.nLoop), lane = threadIdx.x & 31;
+    const int64_t slot = 32 * group + lane, gid = td.order[min(slot, v.nVol - 1)];
+    const float P = pow2f(first_scale(rec, gid, lawExp));
+    float den = 0.f;
     MixedCounters cnt;
-    for (int kk = 0; kk < mp.nLoop; ++kk) {
-        int64_t pos = offs[group * mp.nLoop + kk];
-        const int64_t end = offs[group * mp.nLoop + kk + 1];
-        decide_group(t, tf, v, rec, mp, td, slot, kk, cnt, counters, [&](int i, unsigned m) {
-            if (lane == 0) {
-                term[pos] = i;
-                mask[pos] = m;
-            }
-            ++pos;
-        });
-        if (pos + lane < end) {
-            term[pos + lane] = 0;
-            mask[pos + lane] = 0u;
+    const float4 rhi = rec.hi[kk * v.nVol + gid], rlo = rec.lo[kk * v.nVol + gid];
+    int n = 0;
+    decide_group(t, tf, v, rec, mp, td, slot, kk, cnt, nullptr, [&](int term, unsigned m) {
+        ++n;
+        if ((m >> lane) & 1u) {
+            const float4 c = ldgf4(td.geo + 2 * int64_t(term)), d = ldgf4(td.geo + 2 * int64_t(term) + 1);
+            const float dx = (rhi.x - c.x) + (rlo.x - d.x), dy = (rhi.y - c.y) + (rlo.y - d.y),
+                        dz = (rhi.z - c.z) + (rlo.z - d.z);
+            const float y = rsqrt_normal(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, term < tf.nPts ? 1e-15f : 0.f))));
+            const float y2 = y * y;
+            den = fmaf(c.w * (y2 * (y * P)), fmaf(law.kh, y2, 1.0f), den);
         }
+    });
+    if (lane == 0) counts[unit] = int64_t(n + kTileTerms - 1) / kTileTerms * kTileTerms;
+    if (slot < v.nVol) part[kk * v.nVol + slot] = den;
+}
+
+// Each node's weight scale: the power of two that brings its denominator to
+// [2^13, 2^14).  A node whose denominator is not a positive normal number, or
+// whose scale leaves the range, raises bad (the gated walk then serves the mesh).
+__global__ void k_tile_scale(VolumeDev v, WalkRecF rec, TileDev td, int nLoop, int lawExp, const float *part,
+                             float *scale, int *bad) {
+    const int64_t slot = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (slot >= v.nVol) return;
+    float den = 0.f;
+    for (int kk = 0; kk < nLoop; ++kk) den += part[kk * v.nVol + slot];
+    const int ex = int((__float_as_uint(den) >> 23) & 0xffu);
+    const int k = kScaleExp - (ex - 127) + first_scale(rec, td.order[slot], lawExp);
+    const bool ok = den > 0.f && ex > 0 && ex < 255 && k >= -118 && k <= 118;
+    if (!ok) *bad = 1;
+    scale[slot] = ok ? pow2f(k) : 1.0f;
+}
+
+// The lists' entries at offs, padded with empty ones; a warp per unit.
+__global__ void __launch_bounds__(128, 8)
+    k_tile_record(TreeDev t, TreeDevF tf, VolumeDev v, WalkRecF rec, MixedParams mp, TileDev td, TileRange range,
+                  const int64_t *offs, int *term, unsigned *mask, unsigned long long *counters) {
+    const int64_t unit = range.group0 * mp.nLoop + ((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
+    const int64_t group = unit / mp.nLoop;
+    if (group >= range.group1) return;  // whole warps only
+    const int kk = int(unit - group * mp.nLoop), lane = threadIdx.x & 31;
+    MixedCounters cnt;
+    int64_t pos = offs[unit] - range.entry0;
+    const int64_t end = offs[unit + 1] - range.entry0;
+    decide_group(t, tf, v, rec, mp, td, 32 * group + lane, kk, cnt, counters, [&](int i, unsigned m) {
+        if (lane == 0) {
+            term[pos] = i;
+            mask[pos] = m;
+        }
+        ++pos;
+    });
+    if (pos + lane < end) {
+        term[pos + lane] = 0;
+        mask[pos + lane] = 0u;
     }
     cnt.flush(counters);
 }
@@ -235,19 +241,19 @@ __device__ __forceinline__ void unit_rows(TileRows *rows, const VolumeDev &v, co
 template <bool FIFTH>
 __global__ void __launch_bounds__(128)
     k_tile_build(VolumeDev v, WalkRecF rec, MixedParams mp, TileDev td, TileLists lists, TileLaw law, int nPts,
-                 unsigned nUnits, uint4 *dig, uint4 *dig3) {
+                 TileRange range, int64_t listEntry0, uint4 *dig, uint4 *dig3) {
     __shared__ __align__(16) TileStage stage[4];
     __shared__ TileRows rows[4][16];
-    const unsigned unit = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (unit >= nUnits) return;  // whole warps only
+    const int64_t unit = range.group0 * mp.nLoop + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (unit >= range.group1 * mp.nLoop) return;  // whole warps only
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     TileStage &st = stage[warp];
     unit_rows(rows[warp], v, rec, td, unit / mp.nLoop, int(unit % mp.nLoop));
-    const int64_t e1 = lists.offs[unit + 1];
-    for (int64_t e = lists.offs[unit]; e < e1; e += kTileTerms) {
+    const int64_t e1 = lists.offs[unit + 1] - range.entry0;
+    for (int64_t e = lists.offs[unit] - range.entry0; e < e1; e += kTileTerms) {
         if (lane < kTileTerms) {
-            st.term[lane] = lists.term[e + lane];
-            st.mask[lane] = lists.mask[e + lane];
+            st.term[lane] = lists.term[listEntry0 + e + lane];
+            st.mask[lane] = lists.mask[listEntry0 + e + lane];
         }
         __syncwarp();
         stage_weights<FIFTH>(st, td.geo, nPts, rows[warp], law);
@@ -365,140 +371,75 @@ __global__ void k_tile_mot(TreeDev t, int nPts, const double *ptMB, const double
 
 // ---- the walk ----
 
-enum { kStream = 0, kLists = 1, kDecide = 2 };
-
 // Warps of a block at nb surfaces (one block per SM): 16 at 128 registers, where
 // a walk of one surface waits for its copies (245k-node wing 243 -> 236 us against
 // 12 warps at 144 registers, 8M nodes 6.05 -> 5.94 ms; a third stage for 12 warps
 // is worth 0.13 ms there).  Two surfaces share a step's digits at 12 warps: 2.3 ms
 // a pair on the 2M-node wing, twice 1.33 alone; ten warps with three stages take
-// 3.2 ms.  The forms that make the weights as they go need more registers.
-constexpr int tile_warps(int src, int nb) { return src == kStream && nb == 1 ? 16 : 12; }
-// Shared memory of a stage with nb surfaces' motions: a streamed one holds the
-// digits in use.
-constexpr size_t tile_stage_bytes(int src, int nd, int nb) {
-    return nb * sizeof(uint4) * 8 * kTileTerms + sizeof(TileStage) -
-           (src == kStream && nd < 4 ? sizeof(uint4) * 64 : 0);
-}
+// 3.2 ms.
+constexpr int tile_warps(int nb) { return nb == 1 ? 16 : 12; }
+// Shared memory of a stage with nd digits and nb surfaces' motions.
+constexpr size_t tile_stage_bytes(int nd, int nb) { return sizeof(uint4) * (8 * kTileTerms * nb + 64 * nd); }
 
 // The sums of one unit per warp: numerators about the reference motion and
 // denominator of each node, as pairs (high, low), into out, for NB surfaces
-// (td.mot, td.colMax and out in a row).
-// SRC: the digits streamed from memory (the next step's copied while one is
-// computed), formed from the lists, or formed from the decisions as they are
-// taken.
-template <int SRC, int ND, int NB>
-__global__ void __launch_bounds__(32 * tile_warps(SRC, NB), 1)
+// (td.mot, td.colMax and out in a row).  The weight digits stream from memory,
+// the next step's copied while one is computed.
+template <int ND, int NB>
+__global__ void __launch_bounds__(32 * tile_warps(NB), 1)
     k_tile_walk(TreeDev t, TreeDevF tf, VolumeDev v, WalkRecF rec, MixedParams mp, TileDev td, TileLists lists,
-                TileLaw law, unsigned nUnits, unsigned chunk, float4 *out, unsigned long long *counters) {
+                TileRange range, unsigned chunk, float4 *out) {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ unsigned long long qstate;
-    __shared__ TileRows rowsAll[SRC == kStream ? 1 : tile_warps(SRC, NB)][16];
     if (threadIdx.x == 0) qstate = 0ull;
     __syncthreads();
     const int lane = threadIdx.x & 31, g = lane >> 2, a = lane & 3;
-    constexpr size_t stageBytes = tile_stage_bytes(SRC, ND, NB);
-    constexpr int NS = SRC == kStream ? 2 : 1;  // stages
-    unsigned char *mine = smraw + NS * stageBytes * (threadIdx.x >> 5);
+    constexpr size_t stageBytes = tile_stage_bytes(ND, NB);
+    unsigned char *mine = smraw + 2 * stageBytes * (threadIdx.x >> 5);
     const int64_t nTerms = tf.nPts + t.nNodes;
-    auto motions = [&](int s) { return reinterpret_cast<uint4 *>(mine + stageBytes * s); };
-    auto stage = [&](int s) -> TileStage & {
-        return *reinterpret_cast<TileStage *>(motions(s) + 8 * kTileTerms * NB);
-    };
-    auto fetch_motions = [&](int s, const StageIds &ids) {
-#pragma unroll
-        for (int b = 0; b < NB; ++b) stage_motions(motions(s) + 8 * kTileTerms * b, ids, td.mot + 8 * nTerms * b);
-    };
-    UnitQueue queue = {&qstate, td.counter, nUnits, chunk, 0u, 0u};
-    unsigned unit;
-    while (queue.next(unit)) {
-        const int64_t group = unit / unsigned(mp.nLoop);
-        const int kk = int(unit - unsigned(group) * unsigned(mp.nLoop));
+    auto motions = [&](int s) { return reinterpret_cast<uint4 *>(mine + stageBytes * (s & 1)); };
+    auto digits = [&](int s) { return motions(s) + 8 * kTileTerms * NB; };
+    UnitQueue queue = {&qstate, td.counter, unsigned((range.group1 - range.group0) * mp.nLoop), chunk, 0u, 0u};
+    unsigned idx;
+    while (queue.next(idx)) {
+        const int64_t group = range.group0 + idx / unsigned(mp.nLoop);
+        const int kk = int(idx % unsigned(mp.nLoop));
+        const int64_t unit = group * mp.nLoop + kk;
         TileAcc<ND> acc[NB];
 #pragma unroll
         for (int b = 0; b < NB; ++b) tile_zero(acc[b]);
-        if constexpr (SRC == kStream) {
-            const int64_t e0 = lists.offs[unit];
-            const int n = int((lists.offs[unit + 1] - e0) / kTileTerms);
-            const int *term = lists.term + e0;
-            const uint4 *dig = lists.dig + 192 * (e0 / kTileTerms), *dig3 = lists.dig3 + 64 * (e0 / kTileTerms);
-            StageIds ids;
-            // step s into stage b
-            auto issue = [&](int s, int b) {
-                uint4 *dst = &stage(b).dig[0][0][0];
+        const int64_t e0 = lists.offs[unit] - range.entry0;
+        const int n = int((lists.offs[unit + 1] - range.entry0 - e0) / kTileTerms);
+        const int *term = lists.term + e0;
+        const uint4 *dig = lists.dig + 192 * (e0 / kTileTerms), *dig3 = lists.dig3 + 64 * (e0 / kTileTerms);
+        StageIds ids;
+        auto issue = [&](int s) {
+            uint4 *dst = digits(s);
 #pragma unroll
-                for (int c = 0; c < 6; ++c) cp_async16(dst + 32 * c + lane, dig + 192 * int64_t(s) + 32 * c + lane);
-                if constexpr (ND > 3) {
+            for (int c = 0; c < 6; ++c) cp_async16(dst + 32 * c + lane, dig + 192 * int64_t(s) + 32 * c + lane);
+            if constexpr (ND > 3) {
 #pragma unroll
-                    for (int c = 0; c < 2; ++c)
-                        cp_async16(dst + 192 + 32 * c + lane, dig3 + 64 * int64_t(s) + 32 * c + lane);
-                }
-                fetch_motions(b, ids);
-                if (s + 1 < n) ids = stage_ids(term + kTileTerms * (s + 1));
-            };
-            if (n > 0) ids = stage_ids(term);
+                for (int c = 0; c < 2; ++c)
+                    cp_async16(dst + 192 + 32 * c + lane, dig3 + 64 * int64_t(s) + 32 * c + lane);
+            }
 #pragma unroll
-            for (int s = 0; s < NS - 1; ++s) {
-                if (s < n) issue(s, s);
-                cp_async_commit();
-            }
-            int b = 0;
-            for (int s = 0; s < n; ++s) {
-                if (s + NS - 1 < n) issue(s + NS - 1, b == 0 ? NS - 1 : b - 1);
-                cp_async_commit();
-                cp_async_wait<NS - 1>();
-                __syncwarp();
-                tile_step(stage(b), motions(b), acc);
-                __syncwarp();
-                b = b == NS - 1 ? 0 : b + 1;
-            }
-            cp_async_wait<0>();
-        } else {
-            TileStage &st = stage(0);
-            TileRows *rows = rowsAll[threadIdx.x >> 5];
-            unit_rows(rows, v, rec, td, group, kk);
-            auto step = [&]() {
-                __syncwarp();
-                fetch_motions(0, stage_ids(st.term));
-                cp_async_commit();
-                stage_weights(st, td.geo, tf.nPts, rows, law);
-                cp_async_wait<0>();
-                __syncwarp();
-                tile_step(st, motions(0), acc);
-                __syncwarp();
-            };
-            if constexpr (SRC == kLists) {
-                const int64_t e1 = lists.offs[unit + 1];
-                for (int64_t e = lists.offs[unit]; e < e1; e += kTileTerms) {
-                    if (lane < kTileTerms) {
-                        st.term[lane] = lists.term[e + lane];
-                        st.mask[lane] = lists.mask[e + lane];
-                    }
-                    step();
-                }
-            } else {
-                MixedCounters cnt;
-                int n = 0;
-                decide_group(t, tf, v, rec, mp, td, group * 32 + lane, kk, cnt, counters, [&](int i, unsigned m) {
-                    if (lane == 0) {
-                        st.term[n] = i;
-                        st.mask[n] = m;
-                    }
-                    if (++n == kTileTerms) {
-                        step();
-                        n = 0;
-                    }
-                });
-                if (n) {
-                    if (lane >= n && lane < kTileTerms) {
-                        st.term[lane] = 0;
-                        st.mask[lane] = 0u;
-                    }
-                    step();
-                }
-                cnt.flush(counters);
-            }
+            for (int b = 0; b < NB; ++b) stage_motions(motions(s) + 8 * kTileTerms * b, ids, td.mot + 8 * nTerms * b);
+            if (s + 1 < n) ids = stage_ids(term + kTileTerms * (s + 1));
+        };
+        if (n > 0) {
+            ids = stage_ids(term);
+            issue(0);
         }
+        cp_async_commit();
+        for (int s = 0; s < n; ++s) {
+            if (s + 1 < n) issue(s + 1);
+            cp_async_commit();
+            cp_async_wait<1>();
+            __syncwarp();
+            tile_step(digits(s), motions(s), acc);
+            __syncwarp();
+        }
+        cp_async_wait<0>();
         // component a of the numerator: D'_a . (r - O) + e_a; lane column 3: the denominator
         const float4 oh = ldgf4(td.geo + 2 * int64_t(tf.nPts)), ol = ldgf4(td.geo + 2 * int64_t(tf.nPts) + 1);
 #pragma unroll
@@ -628,17 +569,15 @@ void launch_tile_geo(const TreeDev &t, int nPts, const dbl4 *xa, int areaExp, fl
 void launch_tile_motions(const TreeDev &t, int nPts, const double *ptMB, const double *nodeMB, unsigned *colMax,
                          uint4 *mot, float *refDB, cudaStream_t st) {
     const int64_t n = 8 * (int64_t(nPts) + t.nNodes);
-    cudaMemsetAsync(colMax, 0, 13 * sizeof(unsigned), st);  // and the walk's unit counter behind them
+    cudaMemsetAsync(colMax, 0, 12 * sizeof(unsigned), st);
     k_tile_max<<<blocks(n, 256), 256, 0, st>>>(t, nPts, ptMB, nodeMB, colMax);
     k_tile_mot<<<blocks(n, 256), 256, 0, st>>>(t, nPts, ptMB, nodeMB, colMax, mot, refDB);
 }
 
-int tile_batch(const VolumeDev &v, int nLoop, const TileLists &lists) {
-    return lists.dig && v.nVol * nLoop > kFourDigits ? 2 : 1;
-}
+int tile_batch(const VolumeDev &v, int nLoop) { return v.nVol * nLoop > kFourDigits ? 2 : 1; }
 
 int64_t count_tile_lists(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
-                         const EvalConsts &k, const TileDev &td, int64_t *offs, float *scale, int *bad,
+                         const EvalConsts &k, const TileDev &td, int64_t *offs, float *part, float *scale, int *bad,
                          cudaStream_t st) {
     const MixedParams mp = make_mixed_params(k);
     const int64_t nGroups = walk_list_warps(v.nVol);
@@ -651,21 +590,19 @@ int64_t count_tile_lists(const TreeDev &t, const TreeDevF &tf, const VolumeDev &
     void *tmp = nullptr;
     size_t tmpBytes = 0;
     int64_t total = 0;
-    bool ok = true;
-    if (offs) ok = cudaMalloc(&counts, sizeof(int64_t) * (n + 1)) == cudaSuccess;
-    if (ok && offs) ok = cudaMemsetAsync(counts + n, 0, sizeof(int64_t), st) == cudaSuccess;
+    bool ok = cudaMalloc(&counts, sizeof(int64_t) * (n + 1)) == cudaSuccess;
+    if (ok) ok = cudaMemsetAsync(counts + n, 0, sizeof(int64_t), st) == cudaSuccess;
     if (ok) ok = cudaMemsetAsync(bad, 0, sizeof(int), st) == cudaSuccess;
     if (ok) {
-        k_tile_count<<<blocks(v.nVol, 128), 128, 0, st>>>(t, tf, v, rec, mp, td, make_tile_law(k), lawExp, nGroups,
-                                                          counts, scale, bad);
+        k_tile_count<<<blocks(32 * n, 128), 128, 0, st>>>(t, tf, v, rec, mp, td, make_tile_law(k), lawExp, nGroups,
+                                                          counts, part);
+        k_tile_scale<<<blocks(v.nVol, 128), 128, 0, st>>>(v, rec, td, mp.nLoop, lawExp, part, scale, bad);
         ok = cudaGetLastError() == cudaSuccess;
     }
-    if (offs) {
-        if (ok) ok = cub::DeviceScan::ExclusiveSum(nullptr, tmpBytes, counts, offs, int(n + 1), st) == cudaSuccess;
-        if (ok) ok = cudaMalloc(&tmp, tmpBytes) == cudaSuccess;
-        if (ok) ok = cub::DeviceScan::ExclusiveSum(tmp, tmpBytes, counts, offs, int(n + 1), st) == cudaSuccess;
-        if (ok) ok = cudaMemcpyAsync(&total, offs + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st) == cudaSuccess;
-    }
+    if (ok) ok = cub::DeviceScan::ExclusiveSum(nullptr, tmpBytes, counts, offs, int(n + 1), st) == cudaSuccess;
+    if (ok) ok = cudaMalloc(&tmp, tmpBytes) == cudaSuccess;
+    if (ok) ok = cub::DeviceScan::ExclusiveSum(tmp, tmpBytes, counts, offs, int(n + 1), st) == cudaSuccess;
+    if (ok) ok = cudaMemcpyAsync(&total, offs + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st) == cudaSuccess;
     if (cudaStreamSynchronize(st) != cudaSuccess) ok = false;
     if (tmp) cudaFree(tmp);
     if (counts) cudaFree(counts);
@@ -673,61 +610,53 @@ int64_t count_tile_lists(const TreeDev &t, const TreeDevF &tf, const VolumeDev &
 }
 
 void launch_tile_record(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
-                        const EvalConsts &k, const TileDev &td, const int64_t *offs, int *term, unsigned *mask,
-                        unsigned long long *counters, cudaStream_t st) {
-    if (v.nVol <= 0) return;
-    k_tile_record<<<blocks(v.nVol, 128), 128, 0, st>>>(t, tf, v, rec, make_mixed_params(k), td,
-                                                       walk_list_warps(v.nVol), offs, term, mask, counters);
+                        const EvalConsts &k, const TileDev &td, const TileRange &range, const int64_t *offs, int *term,
+                        unsigned *mask, unsigned long long *counters, cudaStream_t st) {
+    const MixedParams mp = make_mixed_params(k);
+    const int64_t units = (range.group1 - range.group0) * mp.nLoop;
+    if (units > 0)
+        k_tile_record<<<blocks(32 * units, 128), 128, 0, st>>>(t, tf, v, rec, mp, td, range, offs, term, mask,
+                                                               counters);
 }
 
 void launch_tile_build(const VolumeDev &v, const WalkRecF &rec, const EvalConsts &k, const TileDev &td,
-                       const TileLists &lists, int nPts, uint4 *dig, uint4 *dig3, cudaStream_t st) {
+                       const TileLists &lists, const TileRange &range, int64_t listEntry0, int nPts, uint4 *dig,
+                       uint4 *dig3, cudaStream_t st) {
     const MixedParams mp = make_mixed_params(k);
-    const int64_t units = walk_list_warps(v.nVol) * mp.nLoop;
+    const int64_t units = (range.group1 - range.group0) * mp.nLoop;
     if (units <= 0) return;
     (dig ? k_tile_build<false> : k_tile_build<true>)<<<blocks(32 * units, 128), 128, 0, st>>>(
-        v, rec, mp, td, lists, make_tile_law(k), nPts, unsigned(units), dig, dig3);
+        v, rec, mp, td, lists, make_tile_law(k), nPts, range, listEntry0, dig, dig3);
 }
 
-template <int SRC, int ND, int NB>
-static void walk_src(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
-                     const MixedParams &mp, const TileDev &td, const TileLists &lists, const TileLaw &law,
-                     unsigned nUnits, float4 *sums, unsigned long long *counters, cudaStream_t st) {
-    constexpr int warps = tile_warps(SRC, NB);
-    const int sms = tile_sms(), grid = int(min(int64_t(sms), (int64_t(nUnits) + warps - 1) / warps));
-    const unsigned chunk = unsigned(max(int64_t(1), min(int64_t(32), int64_t(nUnits) / (4 * sms * warps))));
-    const size_t smem = warps * (SRC == kStream ? 2 : 1) * tile_stage_bytes(SRC, ND, NB);
-    cudaFuncSetAttribute(k_tile_walk<SRC, ND, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    k_tile_walk<SRC, ND, NB><<<grid, 32 * warps, smem, st>>>(t, tf, v, rec, mp, td, lists, law, nUnits, chunk, sums,
-                                                        counters);
+template <int ND, int NB>
+static void walk_digits(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
+                        const MixedParams &mp, const TileDev &td, const TileLists &lists, const TileRange &range,
+                        float4 *sums, cudaStream_t st) {
+    constexpr int warps = tile_warps(NB);
+    const int64_t units = (range.group1 - range.group0) * mp.nLoop;
+    const int sms = tile_sms(), grid = int(min(int64_t(sms), (units + warps - 1) / warps));
+    const unsigned chunk = unsigned(max(int64_t(1), min(int64_t(32), units / (4 * sms * warps))));
+    const size_t smem = warps * 2 * tile_stage_bytes(ND, NB);
+    cudaMemsetAsync(td.counter, 0, sizeof(unsigned), st);
+    cudaFuncSetAttribute(k_tile_walk<ND, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    k_tile_walk<ND, NB><<<grid, 32 * warps, smem, st>>>(t, tf, v, rec, mp, td, lists, range, chunk, sums);
 }
 
 void launch_tile_walk(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
-                      const EvalConsts &k, const TileDev &td, const TileLists &lists, const float *refDB, float4 *sums,
-                      const WalkOut &o, cudaStream_t st, int nb) {
+                      const EvalConsts &k, const TileDev &td, const TileLists &lists, const TileRange &range,
+                      float4 *sums, cudaStream_t st, int nb) {
+    if (range.group1 <= range.group0) return;
+    const MixedParams mp = make_mixed_params(k);
+    if (nb == 2) walk_digits<3, 2>(t, tf, v, rec, mp, td, lists, range, sums, st);
+    else if (v.nVol * mp.nLoop <= kFourDigits) walk_digits<4, 1>(t, tf, v, rec, mp, td, lists, range, sums, st);
+    else walk_digits<3, 1>(t, tf, v, rec, mp, td, lists, range, sums, st);
+}
+
+void launch_tile_finalize(const VolumeDev &v, const WalkRecF &rec, const EvalConsts &k, const TileDev &td,
+                          const float *refDB, const float4 *sums, const WalkOut &o, cudaStream_t st, int nb) {
     if (v.nVol <= 0) return;
     const MixedParams mp = make_mixed_params(k);
-    const TileLaw law = make_tile_law(k);
-    const unsigned nUnits = unsigned(walk_list_warps(v.nVol) * mp.nLoop);
-    if (lists.term) launch_add_walk_counters(o.counters, lists.counters, st);
-    // Four digits for small meshes, where they stay in cache; three stream a
-    // quarter less.
-    const bool four = v.nVol * mp.nLoop <= kFourDigits;
-    const int src = lists.dig ? kStream : (lists.term ? kLists : kDecide);
-    auto go = [&](auto srcC, auto ndC, auto nbC) {
-        walk_src<decltype(srcC)::value, decltype(ndC)::value, decltype(nbC)::value>(
-            t, tf, v, rec, mp, td, lists, law, nUnits, sums, o.counters, st);
-    };
-    using One = std::integral_constant<int, 1>;
-    auto goSrc = [&](auto ndC) {
-        if (src == kStream) go(std::integral_constant<int, kStream>(), ndC, One());
-        else if (src == kLists) go(std::integral_constant<int, kLists>(), ndC, One());
-        else go(std::integral_constant<int, kDecide>(), ndC, One());
-    };
-    if (nb == 2)
-        go(std::integral_constant<int, kStream>(), std::integral_constant<int, 3>(), std::integral_constant<int, 2>());
-    else if (four) goSrc(std::integral_constant<int, 4>());
-    else goSrc(std::integral_constant<int, 3>());
     const double L = k.law.Ldef;
     for (int b = 0; b < nb; ++b) {
         NodeAggF af{};

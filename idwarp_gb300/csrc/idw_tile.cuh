@@ -153,11 +153,8 @@ __device__ __forceinline__ void tile_digits(float2 wa, float2 la, float2 wb, flo
     s[FIFTH ? 0 : 3][1] = pack_f16(wa.y, wb.y);
 }
 
-// One step's data in shared memory, a stage per warp.  dig: digit d of tile m as
-// the lanes' fragment registers.  The terms' motion records lie in front of it,
-// kTileTerms x 8 chunks of each surface, chunk g of term k at 8 k + (g ^ 2 (k /
-// 4)), so that the fragment-order reads (lane (g, t): terms 4t .. 4t+3) meet no
-// bank conflict.
+// One step's weights being made, per warp.  dig: digit d of tile m as the lanes'
+// fragment registers.
 struct TileStage {
     int term[kTileTerms];
     unsigned mask[kTileTerms];
@@ -224,6 +221,8 @@ __device__ __forceinline__ StageIds stage_ids(const int *term) {
     const int r = (threadIdx.x & 31) >> 3;
     return {{term[r], term[4 + r], term[8 + r], term[12 + r]}};
 }
+// Chunk g of term k lies at 8 k + (g ^ 2 (k / 4)), so that the fragment-order reads
+// (lane (g, t): terms 4t .. 4t+3) meet no bank conflict.
 __device__ __forceinline__ void stage_motions(uint4 *dst, const StageIds &s, const uint4 *mot) {
     const int lane = threadIdx.x & 31, g = lane & 7;
 #pragma unroll
@@ -299,40 +298,36 @@ __device__ __forceinline__ void tile_zero(TileAcc<ND> &acc) {
 }
 
 // One step of the forward sums with ND digits of the weights and of NB surfaces'
-// motions (mot: one array of the step's records each).
+// motions (dig: digit d of 16-node tile m as the lanes' fragment registers at 64 d
+// + 32 m; mot: each surface's records of the step).
 template <int ND, int NB>
-__device__ __forceinline__ void tile_step(const TileStage &st, const uint4 *mot, TileAcc<ND> (&accs)[NB]) {
+__device__ __forceinline__ void tile_step(const uint4 *dig, const uint4 *mot, TileAcc<ND> (&accs)[NB]) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    // motion digits of the lane's terms: [surface][8-column tile][digit][fragment register]
-    unsigned B[NB][2][ND][2];
 #pragma unroll
-    for (int b = 0; b < NB; ++b)
-#pragma unroll
-        for (int p = 0; p < 2; ++p) {
-            const uint4 *q = mot + 8 * kTileTerms * b + 8 * (4 * t + 2 * p) + (g ^ (2 * t));
-            const uint4 x = q[0], y = q[8];
-            B[b][0][0][p] = __byte_perm(x.x, y.x, 0x5410);
-            B[b][0][1][p] = __byte_perm(x.x, y.x, 0x7632);
-            B[b][0][2][p] = __byte_perm(x.y, y.y, 0x5410);
-            B[b][1][0][p] = __byte_perm(x.z, y.z, 0x5410);
-            B[b][1][1][p] = __byte_perm(x.z, y.z, 0x7632);
-            B[b][1][2][p] = __byte_perm(x.w, y.w, 0x5410);
-            if constexpr (ND > 3) {
-                B[b][0][3][p] = __byte_perm(x.y, y.y, 0x7632);
-                B[b][1][3][p] = __byte_perm(x.w, y.w, 0x7632);
-            }
-        }
-#pragma unroll
-    for (int m = 0; m < 2; ++m) {
-        const uint4 A0 = st.dig[0][m][lane], A1 = st.dig[1][m][lane], A2 = st.dig[2][m][lane];
-        uint4 A3 = make_uint4(0u, 0u, 0u, 0u);
-        if constexpr (ND > 3) A3 = st.dig[3][m][lane];
+    for (int n = 0; n < 2; ++n) {
+        // motion digits of the lane's terms: [surface][digit][fragment register]
+        unsigned B[NB][ND][2];
 #pragma unroll
         for (int b = 0; b < NB; ++b)
 #pragma unroll
-            for (int n = 0; n < 2; ++n) {
+            for (int p = 0; p < 2; ++p) {
+                const uint2 *q =
+                    reinterpret_cast<const uint2 *>(mot + 8 * kTileTerms * b + 8 * (4 * t + 2 * p) + (g ^ (2 * t))) + n;
+                const uint2 x = q[0], y = q[16];
+                B[b][0][p] = __byte_perm(x.x, y.x, 0x5410);
+                B[b][1][p] = __byte_perm(x.x, y.x, 0x7632);
+                B[b][2][p] = __byte_perm(x.y, y.y, 0x5410);
+                if constexpr (ND > 3) B[b][3][p] = __byte_perm(x.y, y.y, 0x7632);
+            }
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+            const uint4 A0 = dig[32 * m + lane], A1 = dig[64 + 32 * m + lane], A2 = dig[128 + 32 * m + lane];
+            uint4 A3 = make_uint4(0u, 0u, 0u, 0u);
+            if constexpr (ND > 3) A3 = dig[192 + 32 * m + lane];
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
                 TileAcc<ND> &acc = accs[b];
-                const unsigned(&C)[ND][2] = B[b][n];
+                const unsigned(&C)[ND][2] = B[b];
                 mma_f16(acc.a0[m][n], A0, C[0][0], C[0][1]);
                 // one digit down: exact in a step (the tensor core truncates its
                 // sums, which over a list would be a bias), added by two-sums whose
@@ -358,6 +353,7 @@ __device__ __forceinline__ void tile_step(const TileStage &st, const uint4 *mot,
                     acc.a2[m][n][2 * r + 1] += e.y;
                 }
             }
+        }
     }
 }
 

@@ -94,3 +94,18 @@ def test_batch_pairs_equal_single_warps(built_lib, count):
         g.setSurfaceCoordinates(x)
         g.warpMesh()
         np.testing.assert_array_equal(a, np.asarray(g.getWarpGrid()).reshape(-1))
+
+
+def test_runs_of_groups_equal_kept_digits(built_lib):
+    """With the lists off a mesh of more than 2^17 steps is walked in several runs: the same bits."""
+    m = S.wing_shell(201, 61, 20)
+    out = []
+    for lists in ("auto", "off"):
+        g = build_gpu(m, {"errTol": 1e-4, "walkLists": lists}, precision="mixed")
+        g.setSurfaceCoordinates(np.asarray(m["pts"]) * 1.01)
+        g.warpMesh()
+        s = g.getStats()
+        out.append((g.getWarpGrid(), g.getDenominator(), s["leafPairs"], s["approx"], s["visited"], s["walkListEntries"]))
+    assert out[0][5] > 16 * 2**17 and out[1][5] == 0
+    for a, b in zip(out[0][:5], out[1][:5]):
+        np.testing.assert_array_equal(a, b)
