@@ -129,7 +129,8 @@ struct Ctx {
     DevBuf<int64_t> tileOffs;
     DevBuf<int> tileTerm, tileCTerm;
     DevBuf<unsigned> tileMask, tileCMask;
-    DevBuf<uint4> tileCDig, tileCDig3;  // scratch of one run of groups where no digits are kept
+    DevBuf<unsigned> tileMot5;
+    DevBuf<uint4> tileCDig, tileCDig3, tileCDig4;  // scratch of one run of groups where no digits are kept
     struct TileRun {
         TileRange list, dig;
     };
@@ -913,6 +914,7 @@ static TileDev tile_dev(Ctx *c) {
     td.scale = c->tileScale.p;
     td.geo = c->tileGeo.p;
     td.mot = c->tileMot.p;
+    td.mot5 = c->tileMot5.p;
     td.colMax = c->tileWord.p;
     td.counter = c->tileWord.p + 12;
     td.areaExp = c->areaExp;
@@ -1107,9 +1109,13 @@ static int run_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalC
                                        o.counters, c->stream);
             }
             launch_tile_build(v, rec, k, td, l, r.dig, first, c->nUnique, c->tileCDig.p, c->tileCDig3.p, c->stream);
-            l.term += first;
             l.dig = c->tileCDig.p;
             l.dig3 = c->tileCDig3.p;
+            if (o.tangent) {
+                launch_tile_build(v, rec, k, td, l, r.dig, first, c->nUnique, nullptr, c->tileCDig4.p, c->stream);
+                l.dig4 = c->tileCDig4.p;
+            }
+            l.term += first;
             launch_tile_walk(t, tf, v, rec, k, td, l, r.dig, c->tileSums.p, c->stream, nb);
         }
     }
@@ -1117,21 +1123,15 @@ static int run_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalC
     return check_launch(c, "tile walk");
 }
 
-// The reverse product from the weight digits: what ensure_tile gives, the fifth
-// digit (when it fits) and the reciprocal denominators of the digits' weights,
-// both once per mesh and weight law.
-static int ensure_tile_adjoint(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalConsts &k, TileLists &lists,
-                               bool &use) {
-    int rc = ensure_tile(c, tf, rec, k, lists, use);
-    if (rc) return rc;
-    use = use && lists.dig && c->tileFifthState >= 0;
-    if (use && c->tileFifthState == 0) {
+// The kept digits' fifth and the reciprocal denominators of the digits' weights,
+// both once per mesh and weight law; have = false when they do not fit.
+static int ensure_tile_fifth(Ctx *c, const WalkRecF &rec, const EvalConsts &k, TileLists &lists, bool &have) {
+    if (c->tileFifthState == 0) {
         const size_t steps = size_t(std::max<int64_t>(c->tileListEntries / 16, 1));
         bool fits = false;
-        rc = fits_half(c, 64.0 * sizeof(uint4) * double(steps) + 8.0 * double(c->nVol), fits);
+        int rc = fits_half(c, 64.0 * sizeof(uint4) * double(steps) + 8.0 * double(c->nVol), fits);
         if (rc) return rc;
         c->tileFifthState = fits ? 1 : -1;
-        use = fits;
         if (fits) {
             CKA(c->tileDig4.alloc(64 * steps));
             CKA(c->tileDenInv.alloc(size_t(c->nVol)));
@@ -1145,8 +1145,48 @@ static int ensure_tile_adjoint(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, 
             CK(cudaEventRecord(c->ev0, c->stream));
         }
     }
-    lists.dig4 = c->tileDig4.p;
+    have = c->tileFifthState > 0;
+    lists.dig4 = have ? c->tileDig4.p : nullptr;
     return IDW_OK;
+}
+
+// The reverse product from the weight digits: where they are kept.
+static int ensure_tile_adjoint(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalConsts &k, TileLists &lists,
+                               bool &use) {
+    int rc = ensure_tile(c, tf, rec, k, lists, use);
+    if (rc) return rc;
+    use = use && lists.dig;
+    return use ? ensure_tile_fifth(c, rec, k, lists, use) : IDW_OK;
+}
+
+// A tangent's walk: five digits of the weights, kept or made in runs, and the
+// scratch of its motions' fifth.
+static int ensure_tile_tangent(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalConsts &k, TileLists &lists,
+                               bool &use) {
+    int rc = ensure_tile(c, tf, rec, k, lists, use);
+    if (rc || !use) return rc;
+    if (lists.dig) {
+        bool have = false;
+        rc = ensure_tile_fifth(c, rec, k, lists, have);
+        if (rc) return rc;
+        if (!have) {
+            lists.dig = lists.dig3 = nullptr;
+            rc = ensure_tile_chunks(c);
+            if (rc) return rc;
+        }
+    }
+    if (!lists.dig) CKA(c->tileCDig4.alloc(c->tileCDig3.n));
+    CKA(c->tileMot5.alloc(8 * (size_t(c->nUnique) + size_t(c->nNodes))));
+    return IDW_OK;
+}
+
+// One tangent (motions Md, bd of the direction) by a tile walk.
+static int run_tile_tangent(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalConsts &k,
+                            const TileLists &lists, const double *ptMBd, const double *nodeMBd, const WalkOut &o) {
+    launch_tile_motions(tree_dev(c), c->nUnique, ptMBd, nodeMBd, c->tileWord.p, c->tileMot.p, c->tileMot5.p,
+                        c->refDB.p, c->stream);
+    c->nodalValid = false;
+    return run_tile(c, tf, rec, k, lists, o, 1);
 }
 
 // Before the warped grid is overwritten: if an asynchronous read of the
@@ -1203,8 +1243,8 @@ static int run_warp(Ctx *c, double *xvOut, double *denOut) {
     rc = refresh_nodal(c, !tile);
     if (rc) return rc;
     if (tile) {
-        launch_tile_motions(tree_dev(c), c->nUnique, c->ptMB.p, c->nodeMB.p, c->tileWord.p, c->tileMot.p, c->refDB.p,
-                            c->stream);
+        launch_tile_motions(tree_dev(c), c->nUnique, c->ptMB.p, c->nodeMB.p, c->tileWord.p, c->tileMot.p, nullptr,
+                            c->refDB.p, c->stream);
         CK(cudaEventRecord(c->ev0, c->stream));
         rc = run_tile(c, tf, rec, k, lists, o, 1);
         if (rc) return rc;
@@ -1399,7 +1439,7 @@ static int run_tile_batch(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const
                          c->ptMB.p, c->stream);
             launch_set_data(tree_dev(c), n, c->ptMB.p, c->nodeMB.p, c->nodeSum.p, c->stream);
             launch_tile_motions(tree_dev(c), n, c->ptMB.p, c->nodeMB.p, c->tileWord.p + kTileWords * b,
-                                c->tileMot.p + 8 * nTerms * b, c->refDB.p + 24 * b, c->stream);
+                                c->tileMot.p + 8 * nTerms * b, nullptr, c->refDB.p + 24 * b, c->stream);
         }
         WalkOut o;
         o.xv = outDev + size_t(b0) * vdof;
@@ -1410,6 +1450,30 @@ static int run_tile_batch(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const
     CK(cudaEventRecord(c->ev1, c->stream));
     c->eventsRecorded = true;
     return check_launch(c, "batch walk");
+}
+
+// nb tangents (surface tangents in coordsDev) at the current surface, a walk each.
+static int run_tile_tangents(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalConsts &k,
+                             const TileLists &lists, const double *coordsDev, int nb, double *outDev) {
+    const int n = c->nUnique;
+    CKA(c->bXu.alloc(3 * size_t(n)));
+    launch_gather_xu(n, c->xuInd.p, c->xs.p, c->xu.p, c->stream);
+    CK(cudaEventRecord(c->ev0, c->stream));
+    for (int b = 0; b < nb; ++b) {
+        launch_gather_xu(n, c->xuInd.p, coordsDev + size_t(b) * 3 * size_t(c->nPts), c->bXu.p, c->stream);
+        launch_nodal_d(surf_dev(c), c->xu.p, c->bXu.p, c->ptXA.p, c->normals0.p, c->tmpAi.p, c->isCorner.p,
+                       c->opt.useRotations, 0, c->ptMB.p, c->stream);
+        launch_set_data(tree_dev(c), n, c->ptMB.p, c->nodeMB.p, c->nodeSum.p, c->stream);
+        WalkOut o;
+        o.xv = outDev + size_t(b) * 3 * size_t(c->nVol);
+        o.tangent = 1;
+        o.counters = b == 0 ? c->counters.p : nullptr;
+        int rc = run_tile_tangent(c, tf, rec, k, lists, c->ptMB.p, c->nodeMB.p, o);
+        if (rc) return rc;
+    }
+    CK(cudaEventRecord(c->ev1, c->stream));
+    c->eventsRecorded = true;
+    return check_launch(c, "tangent walks");
 }
 
 // tangent = 1: coordsDev holds surface tangents dXs; the walk then uses the
@@ -1430,8 +1494,9 @@ static int run_warp_batch_mixed(Ctx *c, const double *coordsDev, int nb, double 
         rec.lo = c->recLo.p;
         TileLists lists;
         bool tile = false;
-        int rc = tangent ? IDW_OK : ensure_tile(c, tf, rec, k, lists, tile);
+        int rc = tangent ? ensure_tile_tangent(c, tf, rec, k, lists, tile) : ensure_tile(c, tf, rec, k, lists, tile);
         if (rc) return rc;
+        if (tile && tangent) return run_tile_tangents(c, tf, rec, k, lists, coordsDev, nb, outDev);
         if (tile) return run_tile_batch(c, tf, rec, k, lists, coordsDev, nb, outDev);
     }
     if (c->batchCap < nb) {
@@ -2138,13 +2203,6 @@ int run_deriv_fwd(Ctx *c, const double *xsdDev, double *xvdDev) {
     // Xu, Xud = Xs, Xsd at the first caller occurrence of each unique point
     launch_gather_xu(n, c->xuInd.p, c->xs.p, c->xu.p, c->stream);
     launch_gather_xu(n, c->xuInd.p, xsdDev, xud.p, c->stream);
-    // (Md, bd) for the FP64 walk in tangent mode (S = Md r + bd); (Md + I, bd)
-    // for the mixed walk, whose motions are relative to the identity
-    launch_nodal_d(surf_dev(c), c->xu.p, xud.p, c->ptXA.p, c->normals0.p, c->tmpAi.p, c->isCorner.p,
-                   c->opt.useRotations, mixed ? 1 : 0, ptMBd.p, c->stream);
-    launch_set_data(tree_dev(c), c->nUnique, ptMBd.p, nodeMBd.p, c->nodeSum.p, c->stream);
-    int rc = check_launch(c, "tangent nodal properties");
-    if (rc) return rc;
     EvalConsts k;
     k.law = make_law(c);
     k.errTol = c->opt.errTol;
@@ -2162,7 +2220,24 @@ int run_deriv_fwd(Ctx *c, const double *xsdDev, double *xvdDev) {
     WalkRecF rec;
     rec.hi = c->recHi.p;
     rec.lo = c->recLo.p;
+    TileLists tileLists;
+    bool tile = false;
     if (mixed) {
+        int rc = ensure_tile_tangent(c, tf, rec, k, tileLists, tile);
+        if (rc) return rc;
+    }
+    // (Md, bd) for the FP64 and tile walks (S = Md r + bd); (Md + I, bd)
+    // for the gated mixed walk, whose motions are relative to the identity
+    launch_nodal_d(surf_dev(c), c->xu.p, xud.p, c->ptXA.p, c->normals0.p, c->tmpAi.p, c->isCorner.p,
+                   c->opt.useRotations, mixed && !tile ? 1 : 0, ptMBd.p, c->stream);
+    launch_set_data(tree_dev(c), c->nUnique, ptMBd.p, nodeMBd.p, c->nodeSum.p, c->stream);
+    int rc = check_launch(c, "tangent nodal properties");
+    if (rc) return rc;
+    if (tile) {
+        CK(cudaEventRecord(c->ev0, c->stream));
+        rc = run_tile_tangent(c, tf, rec, k, tileLists, ptMBd.p, nodeMBd.p, o);
+        if (rc) return rc;
+    } else if (mixed) {
         // the gate scales with the size of the tangent instead of Ldef
         CK(cudaMemsetAsync(c->counters.p + 7, 0, sizeof(unsigned long long), c->stream));
         const int64_t nd = 3 * int64_t(n);
@@ -2191,7 +2266,6 @@ int run_deriv_fwd(Ctx *c, const double *xsdDev, double *xvdDev) {
         af.dn = c->nodeDn.p;
         af.ref = c->refDB.p;
         af.rr = c->replayRec.p;
-        // the gated walk's lists and denominators (the tile walks have their own)
         rc = ensure_walk_lists(c, tf, rec, k);
         if (rc) return rc;
         rc = ensure_gate_den(c, tf, pf, af, rec, k, exact);

@@ -218,7 +218,7 @@ struct TileLists {
     const unsigned *mask = nullptr;
     const uint4 *dig = nullptr;     // per step 192: the first three digits of the weights; null: not kept
     const uint4 *dig3 = nullptr;    // per step 64: the fourth
-    const uint4 *dig4 = nullptr;    // per step 64: the fifth, which only the reverse product reads
+    const uint4 *dig4 = nullptr;    // per step 64: the fifth, for reverse products and tangents
     const unsigned long long *counters = nullptr;  // the recording walk's, as WalkLists::counters
 };
 constexpr int kTileWords = 16;  // per surface of a batch: 12 column maxima (and the walk's counter, a flag)
@@ -227,6 +227,7 @@ struct TileDev {
     const float *scale;      // per slot: power-of-two weight scale P
     const float4 *geo;       // per term: (x high, area 2^areaExp high), the low parts
     const uint4 *mot;        // per term: 8 x 16 bytes, the FP16 digits of its motion (k_tile_mot)
+    const unsigned *mot5;    // tangents, per term 8 words: its fifth digits
     const unsigned *colMax;  // largest magnitude of each motion column (float bits)
     unsigned *counter;       // the walk's next unit (behind colMax: launch_tile_motions clears both)
     int areaExp;
@@ -252,9 +253,11 @@ void launch_tile_record(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v
 void launch_tile_build(const VolumeDev &v, const WalkRecF &rec, const EvalConsts &k, const TileDev &td,
                        const TileLists &lists, const TileRange &range, int64_t listEntry0, int nPts, uint4 *dig,
                        uint4 *dig3, cudaStream_t st);
-// The current motions (12 per point and tree node) as motion records, and the reference motion.
+// The current motions (12 per point and tree node) as motion records, and the
+// reference motion; with mot5 a tangent's (Md, bd).
 void launch_tile_motions(const TreeDev &t, int nPts, const double *ptMB, const double *nodeMB, unsigned *colMax,
-                         uint4 *mot, float *refDB, cudaStream_t st);
+                         uint4 *mot, unsigned *mot5, float *refDB, cudaStream_t st);
+// With lists.dig4 the motions are a tangent's (td.mot5, nb = 1).
 // The range's sums of nb surfaces (sums: 2 nLoop nVol float4 each), then their grids
 // (o.xv in a row) and denominators.
 void launch_tile_walk(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,

@@ -560,7 +560,25 @@ __device__ void rotation_matrix_d(const double *v1, const double *v2, const doub
         }
 }
 
-__global__ void k_nodal_d(SurfaceDev s, const double *Xu, const double *Xud, const dbl4 *xa, const double *normals0,
+// element_props_d of every face, once per face, into both halves of the face
+// scratch: area and unit normal, then their derivatives.  (Every node going
+// through its faces itself took 142 us on 12k points, this and the nodes XX.)
+__global__ void k_face_props_d(SurfaceDev s, const double *Xu, const double *Xud) {
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= s.nFaces) return;
+    const int f0 = s.facePtr[f], np = s.facePtr[f + 1] - f0;
+    double area, aread, fn[3], fnd[3];
+    element_props_d(Xu, Xud, s.faceConn + f0, np, area, aread, fn, fnd);
+    double *o = s.faceScratch + 4 * int64_t(f), *od = o + 4 * int64_t(s.nFaces);
+    o[0] = area;
+    od[0] = aread;
+    for (int q = 0; q < 3; ++q) {
+        o[1 + q] = fn[q];
+        od[1 + q] = fnd[q];
+    }
+}
+
+__global__ void k_nodal_d(SurfaceDev s, const double *Xud, const dbl4 *xa, const double *normals0,
                           const double *Ai, const int *isCorner, int useRotations, int plusIdentity, double *ptMBd) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= s.n) return;
@@ -572,15 +590,14 @@ __global__ void k_nodal_d(SurfaceDev s, const double *Xu, const double *Xud, con
             double sa = 0.0, sad = 0.0, sn[3] = {0, 0, 0}, snd[3] = {0, 0, 0};
             for (int e = s.n2ePtr[i]; e < s.n2ePtr[i + 1]; ++e) {
                 const int f = s.n2e[e];
-                const int f0 = s.facePtr[f], np = s.facePtr[f + 1] - f0;
-                double area, aread, fn[3], fnd[3];
-                element_props_d(Xu, Xud, s.faceConn + f0, np, area, aread, fn, fnd);
-                const double dA = area / double(np), dAd = aread / double(np);
+                const int np = s.facePtr[f + 1] - s.facePtr[f];
+                const double *fp = s.faceScratch + 4 * int64_t(f), *fpd = fp + 4 * int64_t(s.nFaces);
+                const double dA = fp[0] / double(np), dAd = fpd[0] / double(np);
                 sa += dA;
                 sad += dAd;
                 for (int q = 0; q < 3; ++q) {
-                    sn[q] += dA * fn[q];
-                    snd[q] += dAd * fn[q] + dA * fnd[q];
+                    sn[q] += dA * fp[1 + q];
+                    snd[q] += dAd * fp[1 + q] + dA * fpd[1 + q];
                 }
             }
             double nrm[3], nrmd[3], M[9];
@@ -668,9 +685,9 @@ void launch_nodal_b_faces(const SurfaceDev &s, const double *Xu, int useRotation
 void launch_nodal_d(const SurfaceDev &s, const double *Xu, const double *Xud, const dbl4 *xa, const double *normals0,
                     const double *Ai, const int *isCorner, int useRotations, int plusIdentity, double *ptMBd,
                     cudaStream_t st) {
-    if (s.n > 0)
-        k_nodal_d<<<blocks(s.n, 128), 128, 0, st>>>(s, Xu, Xud, xa, normals0, Ai, isCorner, useRotations,
-                                                    plusIdentity, ptMBd);
+    if (s.n <= 0) return;
+    if (useRotations && s.nFaces > 0) k_face_props_d<<<blocks(s.nFaces, 128), 128, 0, st>>>(s, Xu, Xud);
+    k_nodal_d<<<blocks(s.n, 128), 128, 0, st>>>(s, Xud, xa, normals0, Ai, isCorner, useRotations, plusIdentity, ptMBd);
 }
 void launch_scatter_dxs(int n, const int *xuInd, const double *Xub, double *dXs, cudaStream_t st) {
     if (n > 0) k_scatter_dxs<<<blocks(n, 256), 256, 0, st>>>(n, xuInd, Xub, dXs);

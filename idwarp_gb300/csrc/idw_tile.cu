@@ -274,10 +274,10 @@ __global__ void __launch_bounds__(128)
 
 // Column pair g of a term's motion about the root centroid O: (D'_a0, D'_a2)
 // for g = 2a, (D'_a1, e_a) for g = 2a + 1, with D' = M - I - Dref and
-// e = D' O + b - bref; (8, 0) for g = 6 (8 times the denominator, on the grid
+// e = D' O + b - bref (a tangent's M, ident = 0, has no I); (8, 0) for g = 6 (8 times the denominator, on the grid
 // of the first digits), zero for g = 7.
-__device__ __forceinline__ void motion_pair(const double *mb, const double *root, const dbl4 o, int g, double &u,
-                                            double &w) {
+__device__ __forceinline__ void motion_pair(const double *mb, const double *root, const dbl4 o, int g, int ident,
+                                            double &u, double &w) {
     u = g == 6 ? 8.0 : 0.0;
     w = 0.0;
     if (g >= 6) return;
@@ -285,7 +285,7 @@ __device__ __forceinline__ void motion_pair(const double *mb, const double *root
     double D[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const double id = a == k ? 1.0 : 0.0;
+        const double id = ident && a == k ? 1.0 : 0.0;
         D[k] = mb[3 * a + k] - id - (root ? root[3 * a + k] - id : 0.0);
     }
     if (!(g & 1)) {
@@ -306,7 +306,7 @@ __device__ __forceinline__ int column_exp(unsigned maxBits) {
 
 // Largest magnitude of each column over the terms (float bits; column 4a + k,
 // k = 3 the offset e).  Leaves have no motion of their own: their points do.
-__global__ void k_tile_max(TreeDev t, int nPts, const double *ptMB, const double *nodeMB, unsigned *colMax) {
+__global__ void k_tile_max(TreeDev t, int nPts, const double *ptMB, const double *nodeMB, int ident, unsigned *colMax) {
     __shared__ unsigned sm[12];
     if (threadIdx.x < 12) sm[threadIdx.x] = 0u;
     __syncthreads();
@@ -316,7 +316,7 @@ __global__ void k_tile_max(TreeDev t, int nPts, const double *ptMB, const double
     if (i < nPts + t.nNodes && g < 6 && !(i >= nPts && t.info[i - nPts].w)) {
         const double *root = t.info[0].w ? nullptr : nodeMB;
         double u, w;
-        motion_pair(i < nPts ? ptMB + 12 * i : nodeMB + 12 * (i - nPts), root, t.geom[0], g, u, w);
+        motion_pair(i < nPts ? ptMB + 12 * i : nodeMB + 12 * (i - nPts), root, t.geom[0], g, ident, u, w);
         const int a = g >> 1, odd = g & 1;
         const unsigned fu = __float_as_uint(__double2float_ru(fabs(u))), fw = __float_as_uint(__double2float_ru(fabs(w)));
         if (fu > sm[4 * a + odd]) atomicMax(&sm[4 * a + odd], fu);
@@ -326,47 +326,53 @@ __global__ void k_tile_max(TreeDev t, int nPts, const double *ptMB, const double
     if (threadIdx.x < 12 && sm[threadIdx.x]) atomicMax(colMax + threadIdx.x, sm[threadIdx.x]);
 }
 
-// The four FP16 digits of v 2^e, on the grids of the weights' digits.
-__device__ __forceinline__ void motion_digits(double v, int e, unsigned (&d)[4]) {
+// The five FP16 digits of v 2^e, on the grids of the weights' digits.
+__device__ __forceinline__ void motion_digits(double v, int e, unsigned (&d)[5]) {
     const double s = v * __hiloint2double((1023 + e) << 20, 0);
     const float f = float(s), lo = float(s - double(f));
     const float M[3] = {1.5f * 67108864.0f, 1.5f * 32768.0f, 1.5f * 16.0f};
-    float r = f;
+    float r = f, rest = 0.f;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const float g = __fsub_rn(__fadd_rn(r, M[k]), M[k]);
         d[k] = __half_as_ushort(__float2half_rn(g));
         r = __fsub_rn(r, g);
-        if (k == 1) r = __fadd_rn(r, lo);
+        if (k == 1) two_sum(r, lo, r, rest);
     }
-    d[3] = __half_as_ushort(__float2half_rn(r * 4194304.0f));
+    r *= 4194304.0f;
+    const __half q = __float2half_rn(r);
+    d[3] = __half_as_ushort(q);
+    d[4] = __half_as_ushort(__float2half_rn(fmaf(rest, 4194304.0f, r - __half2float(q))));
 }
 
 // Motion records: per term 8 x 16 bytes, lane row g's digits of its two
 // columns.  Thread 0 also stores the reference motion (Dref 9, bref 3; high
-// parts, then low parts) that the finalisation adds back.
+// parts, then low parts) that the finalisation adds back.  mot5: a tangent's
+// fifth digits, 8 words a term (null: a surface).
 __global__ void k_tile_mot(TreeDev t, int nPts, const double *ptMB, const double *nodeMB, const unsigned *colMax,
-                           uint4 *mot, float *refDB) {
+                           uint4 *mot, unsigned *mot5, float *refDB) {
     const int64_t tid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t i = tid >> 3;
     const int g = int(tid & 7);
     if (i >= nPts + t.nNodes) return;
     const double *root = t.info[0].w ? nullptr : nodeMB;
+    const int ident = mot5 == nullptr;
     if (tid < 12) {
         const int c = int(tid);
-        const double v = root ? root[c] - (c < 9 && c % 4 == 0 ? 1.0 : 0.0) : 0.0;
+        const double v = root ? root[c] - (ident && c < 9 && c % 4 == 0 ? 1.0 : 0.0) : 0.0;
         refDB[c] = float(v);
         refDB[12 + c] = float(v - double(float(v)));
     }
-    unsigned du[4] = {0, 0, 0, 0}, dw[4] = {0, 0, 0, 0};
+    unsigned du[5] = {0, 0, 0, 0, 0}, dw[5] = {0, 0, 0, 0, 0};
     if (!(i >= nPts && t.info[i - nPts].w)) {
         double u, w;
-        motion_pair(i < nPts ? ptMB + 12 * i : nodeMB + 12 * (i - nPts), root, t.geom[0], g, u, w);
+        motion_pair(i < nPts ? ptMB + 12 * i : nodeMB + 12 * (i - nPts), root, t.geom[0], g, ident, u, w);
         const int a = g >> 1, odd = g & 1;
         motion_digits(u, g < 6 ? column_exp(colMax[4 * a + odd]) : 0, du);
         if (g < 6) motion_digits(w, column_exp(colMax[4 * a + 2 + odd]), dw);
     }
     mot[8 * i + g] = make_uint4(du[0] | (du[1] << 16), du[2] | (du[3] << 16), dw[0] | (dw[1] << 16), dw[2] | (dw[3] << 16));
+    if (mot5) mot5[8 * i + g] = du[4] | (dw[4] << 16);
 }
 
 // ---- the walk ----
@@ -377,16 +383,19 @@ __global__ void k_tile_mot(TreeDev t, int nPts, const double *ptMB, const double
 // is worth 0.13 ms there).  Two surfaces share a step's digits at 12 warps: 2.3 ms
 // a pair on the 2M-node wing, twice 1.33 alone; ten warps with three stages take
 // 3.2 ms.
-constexpr int tile_warps(int nb) { return nb == 1 ? 16 : 12; }
-// Shared memory of a stage with nd digits and nb surfaces' motions.
-constexpr size_t tile_stage_bytes(int nd, int nb) { return sizeof(uint4) * (8 * kTileTerms * nb + 64 * nd); }
+constexpr int tile_warps(int nd, int nb) { return nd < 5 && nb == 1 ? 16 : 12; }
+// Shared memory of a stage: nd digits and nb surfaces' motions (a tangent's fifth
+// digits last).
+constexpr size_t tile_stage_bytes(int nd, int nb) {
+    return sizeof(uint4) * ((nd == 5 ? 10 : 8) * kTileTerms * nb + 64 * nd);
+}
 
 // The sums of one unit per warp: numerators about the reference motion and
 // denominator of each node, as pairs (high, low), into out, for NB surfaces
 // (td.mot, td.colMax and out in a row).  The weight digits stream from memory,
 // the next step's copied while one is computed.
 template <int ND, int NB>
-__global__ void __launch_bounds__(32 * tile_warps(NB), 1)
+__global__ void __launch_bounds__(32 * tile_warps(ND, NB), 1)
     k_tile_walk(TreeDev t, TreeDevF tf, VolumeDev v, WalkRecF rec, MixedParams mp, TileDev td, TileLists lists,
                 TileRange range, unsigned chunk, float4 *out) {
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -412,7 +421,9 @@ __global__ void __launch_bounds__(32 * tile_warps(NB), 1)
         const int n = int((lists.offs[unit + 1] - range.entry0 - e0) / kTileTerms);
         const int *term = lists.term + e0;
         const uint4 *dig = lists.dig + 192 * (e0 / kTileTerms), *dig3 = lists.dig3 + 64 * (e0 / kTileTerms);
+        const uint4 *dig4 = ND == 5 ? lists.dig4 + 64 * (e0 / kTileTerms) : nullptr;
         StageIds ids;
+        int id5 = 0;  // a tangent: the term whose fifth digits the lane copies half of
         auto issue = [&](int s) {
             uint4 *dst = digits(s);
 #pragma unroll
@@ -424,9 +435,19 @@ __global__ void __launch_bounds__(32 * tile_warps(NB), 1)
             }
 #pragma unroll
             for (int b = 0; b < NB; ++b) stage_motions(motions(s) + 8 * kTileTerms * b, ids, td.mot + 8 * nTerms * b);
+            if constexpr (ND == 5) {
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+                    cp_async16(dst + 256 + 32 * c + lane, dig4 + 64 * int64_t(s) + 32 * c + lane);
+                const int k = lane >> 1;  // term 4 i + j to row 4 i + (i + j) % 4
+                cp_async16_l1(dst + 320 + 2 * ((k & ~3) + ((k + (k >> 2)) & 3)) + (lane & 1),
+                              reinterpret_cast<const uint4 *>(td.mot5) + 2 * int64_t(id5) + (lane & 1));
+                if (s + 1 < n) id5 = term[kTileTerms * (s + 1) + (lane >> 1)];
+            }
             if (s + 1 < n) ids = stage_ids(term + kTileTerms * (s + 1));
         };
         if (n > 0) {
+            if constexpr (ND == 5) id5 = term[lane >> 1];
             ids = stage_ids(term);
             issue(0);
         }
@@ -436,7 +457,10 @@ __global__ void __launch_bounds__(32 * tile_warps(NB), 1)
             cp_async_commit();
             cp_async_wait<1>();
             __syncwarp();
-            tile_step(digits(s), motions(s), acc);
+            if constexpr (ND == 5)
+                tile_step5(digits(s), motions(s), reinterpret_cast<const unsigned *>(digits(s) + 320), acc[0]);
+            else
+                tile_step(digits(s), motions(s), acc);
             __syncwarp();
         }
         cp_async_wait<0>();
@@ -459,12 +483,8 @@ __global__ void __launch_bounds__(32 * tile_warps(NB), 1)
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
                         // columns in the order of the motion records: D'_a0, D'_a1 | D'_a2, e_a
-                        const int n = k >> 1, j = 2 * r + (k & 1);
-                        const float2 a1 = acc[b].a1[m][n][r];
-                        float s, e;
-                        two_sum(acc[b].a0[m][n][j], k & 1 ? a1.y : a1.x, s, e);
-                        float low = e + acc[b].a2[m][n][j];
-                        if constexpr (ND > 3) low = fmaf(acc[b].a3[m][n][j], 1.0f / 4194304.0f, low);
+                        float s, low;
+                        tile_total(acc[b], m, k >> 1, r, k & 1, s, low);
                         M[k] = df_norm(s * cs[k], low * cs[k]);
                     }
                     const int64_t gid = kk * v.nVol + td.order[slot];
@@ -489,9 +509,9 @@ __global__ void __launch_bounds__(32 * tile_warps(NB), 1)
 }
 
 // The mirrors' sums of each node: reference motion added back, reflected and
-// added (finish_mirror); Xv = Xv0 + num / den and the denominator in the reference's units, den L^3 / (P 2^areaExp).
+// added (finish_mirror); Xv = Xv0 + num / den (a tangent: without Xv0) and the denominator in the reference's units, den L^3 / (P 2^areaExp).
 __global__ void k_tile_finalize(VolumeDev v, WalkRecF rec, NodeAggF af, MixedParams mp, TileDev td, const float4 *sums,
-                                double denUnit, double *xv, double *den) {
+                                double denUnit, int tangent, double *xv, double *den) {
     const int64_t slot = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (slot >= v.nVol) return;
     const int64_t gid = td.order[slot];
@@ -515,7 +535,7 @@ __global__ void k_tile_finalize(VolumeDev v, WalkRecF rec, NodeAggF af, MixedPar
             const dfl n = df_norm(N[a], Nl[a]);
             const float q = n.h * oD;
             const float rem = fmaf(-q, D.l, fmaf(-q, D.h, n.h) + n.l);
-            xv[3 * int64_t(vi) + a] = v.xv0[3 * int64_t(vi) + a] + (double(q) + double(rem * oD));
+            xv[3 * int64_t(vi) + a] = (tangent ? 0.0 : v.xv0[3 * int64_t(vi) + a]) + (double(q) + double(rem * oD));
         }
     }
     if (den) {
@@ -567,11 +587,11 @@ void launch_tile_geo(const TreeDev &t, int nPts, const dbl4 *xa, int areaExp, fl
 }
 
 void launch_tile_motions(const TreeDev &t, int nPts, const double *ptMB, const double *nodeMB, unsigned *colMax,
-                         uint4 *mot, float *refDB, cudaStream_t st) {
+                         uint4 *mot, unsigned *mot5, float *refDB, cudaStream_t st) {
     const int64_t n = 8 * (int64_t(nPts) + t.nNodes);
     cudaMemsetAsync(colMax, 0, 12 * sizeof(unsigned), st);
-    k_tile_max<<<blocks(n, 256), 256, 0, st>>>(t, nPts, ptMB, nodeMB, colMax);
-    k_tile_mot<<<blocks(n, 256), 256, 0, st>>>(t, nPts, ptMB, nodeMB, colMax, mot, refDB);
+    k_tile_max<<<blocks(n, 256), 256, 0, st>>>(t, nPts, ptMB, nodeMB, mot5 == nullptr, colMax);
+    k_tile_mot<<<blocks(n, 256), 256, 0, st>>>(t, nPts, ptMB, nodeMB, colMax, mot, mot5, refDB);
 }
 
 int tile_batch(const VolumeDev &v, int nLoop) { return v.nVol * nLoop > kFourDigits ? 2 : 1; }
@@ -633,7 +653,7 @@ template <int ND, int NB>
 static void walk_digits(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
                         const MixedParams &mp, const TileDev &td, const TileLists &lists, const TileRange &range,
                         float4 *sums, cudaStream_t st) {
-    constexpr int warps = tile_warps(NB);
+    constexpr int warps = tile_warps(ND, NB);
     const int64_t units = (range.group1 - range.group0) * mp.nLoop;
     const int sms = tile_sms(), grid = int(min(int64_t(sms), (units + warps - 1) / warps));
     const unsigned chunk = unsigned(max(int64_t(1), min(int64_t(32), units / (4 * sms * warps))));
@@ -648,7 +668,8 @@ void launch_tile_walk(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, 
                       float4 *sums, cudaStream_t st, int nb) {
     if (range.group1 <= range.group0) return;
     const MixedParams mp = make_mixed_params(k);
-    if (nb == 2) walk_digits<3, 2>(t, tf, v, rec, mp, td, lists, range, sums, st);
+    if (lists.dig4) walk_digits<5, 1>(t, tf, v, rec, mp, td, lists, range, sums, st);
+    else if (nb == 2) walk_digits<3, 2>(t, tf, v, rec, mp, td, lists, range, sums, st);
     else if (v.nVol * mp.nLoop <= kFourDigits) walk_digits<4, 1>(t, tf, v, rec, mp, td, lists, range, sums, st);
     else walk_digits<3, 1>(t, tf, v, rec, mp, td, lists, range, sums, st);
 }
@@ -663,7 +684,7 @@ void launch_tile_finalize(const VolumeDev &v, const WalkRecF &rec, const EvalCon
         af.ref = refDB + 24 * b;
         k_tile_finalize<<<blocks(v.nVol, 128), 128, 0, st>>>(v, rec, af, mp, td, sums + 2 * mp.nLoop * v.nVol * b,
                                                              ldexp(L * L * L, -td.areaExp),
-                                                             o.xv ? o.xv + 3 * v.nVol * b : nullptr, o.den);
+                                                             o.tangent, o.xv ? o.xv + 3 * v.nVol * b : nullptr, o.den);
     }
 }
 

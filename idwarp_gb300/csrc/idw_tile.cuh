@@ -297,6 +297,44 @@ __device__ __forceinline__ void tile_zero(TileAcc<ND> &acc) {
         }
 }
 
+// The sums of a tangent: five digits of both.  A rough surface tangent has
+// gradients D' far above its offsets e, which cancel near the term (D' (r - O) +
+// e), and terms of large motion far from the node, so neither is good enough to
+// the denominator or the largest motion only.
+template <>
+struct TileAcc<5> {
+    float a0[2][2][4], a3[2][2][4], a4[2][2][4];  // leading products; third order and what two-sums leave; 2^22 times the rest
+    float2 a1[2][2][2], a2[2][2][2];              // first and second order, by two-sums
+};
+template <>
+__device__ __forceinline__ void tile_zero<5>(TileAcc<5> &acc) {
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            acc.a1[m][n][0] = acc.a1[m][n][1] = acc.a2[m][n][0] = acc.a2[m][n][1] = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc.a0[m][n][j] = acc.a3[m][n][j] = acc.a4[m][n][j] = 0.f;
+        }
+}
+
+// Total of column pair entry j = 2 r + k (k = 0, 1) of tiles m, n, as high and low.
+template <int ND>
+__device__ __forceinline__ void tile_total(const TileAcc<ND> &acc, int m, int n, int r, int k, float &s, float &low) {
+    const float2 a1 = acc.a1[m][n][r];
+    float e;
+    two_sum(acc.a0[m][n][2 * r + k], k ? a1.y : a1.x, s, e);
+    if constexpr (ND == 5) {
+        const float2 a2 = acc.a2[m][n][r];
+        float e2;
+        two_sum(s, k ? a2.y : a2.x, s, e2);
+        low = e + (e2 + fmaf(acc.a4[m][n][2 * r + k], 1.0f / 4194304.0f, acc.a3[m][n][2 * r + k]));
+    } else {
+        low = e + acc.a2[m][n][2 * r + k];
+        if constexpr (ND > 3) low = fmaf(acc.a3[m][n][2 * r + k], 1.0f / 4194304.0f, low);
+    }
+}
+
 // One step of the forward sums with ND digits of the weights and of NB surfaces'
 // motions (dig: digit d of 16-node tile m as the lanes' fragment registers at 64 d
 // + 32 m; mot: each surface's records of the step).
@@ -352,6 +390,60 @@ __device__ __forceinline__ void tile_step(const uint4 *dig, const uint4 *mot, Ti
                     acc.a2[m][n][2 * r] += e.x;
                     acc.a2[m][n][2 * r + 1] += e.y;
                 }
+            }
+        }
+    }
+}
+
+// One step of a tangent's sums.  mot5: the terms' fifth digits, chunk g of term k =
+// 4 i + j in word 8 (4 i + (i + j) % 4) + g (no bank conflict for lane (g, t)).
+__device__ __forceinline__ void tile_step5(const uint4 *dig, const uint4 *mot, const unsigned *mot5, TileAcc<5> &acc) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+        unsigned C[5][2];
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const uint2 *q = reinterpret_cast<const uint2 *>(mot + 8 * (4 * t + 2 * p) + (g ^ (2 * t))) + n;
+            const uint2 x = q[0], y = q[16];
+            C[0][p] = __byte_perm(x.x, y.x, 0x5410);
+            C[1][p] = __byte_perm(x.x, y.x, 0x7632);
+            C[2][p] = __byte_perm(x.y, y.y, 0x5410);
+            C[3][p] = __byte_perm(x.y, y.y, 0x7632);
+            C[4][p] = __byte_perm(mot5[8 * (4 * t + ((t + 2 * p) & 3)) + g], mot5[8 * (4 * t + ((t + 2 * p + 1) & 3)) + g],
+                                  n ? 0x7632 : 0x5410);
+        }
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+            const uint4 *A = dig + 32 * m + lane;
+            const uint4 A0 = A[0], A1 = A[64], A2 = A[128], A3 = A[192], A4 = A[256];
+            float d[4], f[4];
+            mma_f16_first(d, A0, C[1][0], C[1][1]);
+            mma_f16_first(f, A0, C[2][0], C[2][1]);
+            mma_f16(acc.a3[m][n], A1, C[2][0], C[2][1]);
+            mma_f16(acc.a4[m][n], A0, C[3][0], C[3][1]);
+            mma_f16(d, A1, C[0][0], C[0][1]);
+            mma_f16(f, A1, C[1][0], C[1][1]);
+            mma_f16(acc.a3[m][n], A2, C[1][0], C[1][1]);
+            mma_f16(acc.a4[m][n], A3, C[0][0], C[0][1]);
+            mma_f16(acc.a0[m][n], A0, C[0][0], C[0][1]);
+            mma_f16(f, A2, C[0][0], C[0][1]);
+            mma_f16(acc.a4[m][n], A1, C[3][0], C[3][1]);
+            mma_f16(acc.a3[m][n], A2, C[2][0], C[2][1]);
+            mma_f16(acc.a4[m][n], A3, C[1][0], C[1][1]);
+            mma_f16(acc.a4[m][n], A0, C[4][0], C[4][1]);
+            mma_f16(acc.a4[m][n], A4, C[0][0], C[0][1]);
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                // both orders are exact in a step
+                float2 s, e, h;
+                two_sum2(acc.a1[m][n][r], make_float2(d[2 * r], d[2 * r + 1]), s, e);
+                acc.a1[m][n][r] = s;
+                two_sum2(acc.a2[m][n][r], make_float2(f[2 * r], f[2 * r + 1]), s, h);
+                acc.a2[m][n][r] = s;
+                e = add2(e, h);
+                acc.a3[m][n][2 * r] += e.x;
+                acc.a3[m][n][2 * r + 1] += e.y;
             }
         }
     }
