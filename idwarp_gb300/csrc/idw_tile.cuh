@@ -92,8 +92,11 @@ __device__ __forceinline__ float2 tile_weight(const float4 c, const float4 d, fl
     const float2 t = mul2(v, u);
     // y (1 + r / 2) for y: v u gains v r (5 u - 2) / 2
     const float2 tl = fma2(mul2(v, fma2(dup2(2.5f), u, dup2(-1.0f))), r, fma2(vl, u, fma2(v, ul, fms2(v, u, t))));
-    const float2 w = mul2(dup2(c.w), t);
-    wl = fma2(dup2(c.w), tl, fma2(dup2(d.w), t, fms2(dup2(c.w), t, w)));
+    const float2 w0 = mul2(dup2(c.w), t);
+    const float2 l0 = fma2(dup2(c.w), tl, fma2(dup2(d.w), t, fms2(dup2(c.w), t, w0)));
+    // normalised: the digits take wl to be below an ulp of w (r alone is a few)
+    const float2 w = add2(w0, l0);
+    wl = sub2(l0, sub2(w, w0));
     return w;
 }
 

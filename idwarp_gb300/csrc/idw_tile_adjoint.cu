@@ -18,8 +18,8 @@
 //
 // The double-float walk that this replaces summed the 32 lanes of each term and
 // seed component one after the other (idw_adjoint_precise.cu).  Against it, the
-// 2M-node wing, errTol 1e-4: one seed 13.9 -> 3.5 ms, 16 seeds 105 -> 33 ms, with
-// the same error (4e-14 of the result for the walk alone, wing of 7k nodes).
+// 2M-node wing, errTol 1e-4: one seed 13.9 -> 2.9 ms, 16 seeds 105 -> 36 ms, with
+// the same error (2e-14 to 2e-13 of the result for the walk alone).
 // What bounds it: latency at 16 warps an SM (an instruction issues in 45% of the
 // cycles, tensor pipe 28% busy, L2 atomics 5e10 sectors/s).
 #include <climits>
@@ -33,7 +33,7 @@ namespace {
 
 // Seeds taken together: two, with 16 warps an SM in the shared memory their
 // columns leave, against four with 10 (the 2M-node wing, 16 seeds: 36.4 against
-// 41.5 ms, although the digits are read twice as often) or three with 12 (45 ms).
+// 41.5 ms at one time, although the digits are read twice as often) or three with 12 (45 ms).
 constexpr int kAdjSeeds = 2, kAdjWarps = 16;
 
 // 8 x 8 FP16 tile transposed across the warp.
@@ -238,6 +238,13 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 1)
                 }
             if (st + 1 < n) fetch(st + 1);
             cp_async_commit();
+            // The nodes of a term, unlike the terms of a node, have no bound on their
+            // weights' sum.  Up to 2^16 the products of first weight digits with second
+            // column digits (below 4, on a grid of 2^-5) are exact in their accumulator.
+            float rows[4];
+            mma_f16_first(rows, A[0][0], 0x3c003c00u, 0x3c003c00u);
+            mma_f16(rows, A[0][1], 0x3c003c00u, 0x3c003c00u);
+            const bool heavy = __any_sync(kFull, fmaxf(rows[0], rows[2]) > 65536.0f);
             // the rows' terms: where they land, and O - X on the lane's axis (0 for moment 1)
             const int tA = __ldg(term + kTileTerms * st + 4 * (g >> 1) + (g & 1));
             const int tB = __ldg(term + kTileTerms * st + 4 * (g >> 1) + (g & 1) + 2);
@@ -259,13 +266,12 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 1)
                     mma_f16_first(o4, A[0][0], B[3].x, B[3].y);
                     mma_f16_first(o5, A[1][0], B[3].x, B[3].y);
                     mma_f16_first(o6, A[0][0], B[4].x, B[4].y);
-                    mma_f16_first(o1, A[0][0], B[1].x, B[1].y);
+                    mma_f16_first(o1, A[1][0], B[0].x, B[0].y);
                     mma_f16_first(o0, A[0][0], B[0].x, B[0].y);
                     mma_f16(o2, A[1][0], B[1].x, B[1].y);
                     mma_f16(o3, A[2][0], B[1].x, B[1].y);
                     mma_f16(o4, A[3][0], B[0].x, B[0].y);
                     mma_f16(o5, A[3][0], B[1].x, B[1].y);
-                    mma_f16(o1, A[1][0], B[0].x, B[0].y);
                     mma_f16(o2, A[2][0], B[0].x, B[0].y);
                     mma_f16(o3, A[2][0], B[2].x, B[2].y);
                     mma_f16(o4, A[4][0], B[0].x, B[0].y);
@@ -274,16 +280,34 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 1)
                     mma_f16(o4, A[0][1], B[3].z, B[3].w);
                     mma_f16(o5, A[1][1], B[3].z, B[3].w);
                     mma_f16(o6, A[0][1], B[4].z, B[4].w);
-                    mma_f16(o1, A[0][1], B[1].z, B[1].w);
+                    mma_f16(o1, A[1][1], B[0].z, B[0].w);
                     mma_f16(o0, A[0][1], B[0].z, B[0].w);
                     mma_f16(o2, A[1][1], B[1].z, B[1].w);
                     mma_f16(o3, A[2][1], B[1].z, B[1].w);
                     mma_f16(o4, A[3][1], B[0].z, B[0].w);
                     mma_f16(o5, A[3][1], B[1].z, B[1].w);
-                    mma_f16(o1, A[1][1], B[0].z, B[0].w);
                     mma_f16(o2, A[2][1], B[0].z, B[0].w);
                     mma_f16(o3, A[2][1], B[2].z, B[2].w);
                     mma_f16(o4, A[4][1], B[0].z, B[0].w);
+                    if (!heavy) {
+                        mma_f16(o1, A[0][0], B[1].x, B[1].y);
+                        mma_f16(o1, A[0][1], B[1].z, B[1].w);
+                    } else {
+                        // eight nodes at a time, each sum exact, added with the errors
+                        // of the additions kept in the fourth order
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            float part[4];
+                            mma_f16_first(part, A[0][i >> 1], i & 1 ? 0u : (i & 2 ? B[1].z : B[1].x),
+                                          i & 1 ? (i & 2 ? B[1].w : B[1].y) : 0u);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                float e;
+                                two_sum(o1[j], part[j], o1[j], e);
+                                o3[j] += e;
+                            }
+                        }
+                    }
                 }
                 const float2 rel = *reinterpret_cast<const float2 *>(sm.rel[nt][t]);
                 const int2 off = *reinterpret_cast<const int2 *>(sm.off[nt][t]);
@@ -291,15 +315,19 @@ __global__ void __launch_bounds__(32 * kAdjWarps, 1)
                 float2 H[2], Lo[2];
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
-                    // o0 + o1 + o2 + o3 + 2^-22 (o4 + o5 + o6), components 2 nt and 2 nt + 1 as a pair.
-                    // o0 is a multiple of 64 and o1 below 2^24, o0 + o1 of 2^-5 and o2
-                    // below 2^18: the three-operation sums are exact
-                    const float2 p0 = make_float2(o0[2 * r], o0[2 * r + 1]), p1 = make_float2(o1[2 * r], o1[2 * r + 1]),
-                                 p2 = make_float2(o2[2 * r], o2[2 * r + 1]), p3 = make_float2(o3[2 * r], o3[2 * r + 1]),
-                                 p4 = add2(make_float2(o4[2 * r], o4[2 * r + 1]), add2(make_float2(o5[2 * r], o5[2 * r + 1]), make_float2(o6[2 * r], o6[2 * r + 1])));
-                    const float2 u = add2(p0, p1), ul = sub2(p1, sub2(u, p0));
-                    const float2 w = add2(u, p2), wl = sub2(p2, sub2(w, u));
-                    const float2 low = add2(wl, add2(ul, fma2(p4, dup2(1.0f / 4194304.0f), p3)));
+                    // o0 + o1 + o2 + o3 + 2^-22 (o4 + o5 + o6), components 2 nt and 2 nt + 1 as
+                    // a pair.  o0 is a multiple of 64, o0 + o1 of 2^-5, o1 and o2 are below
+                    // 2^24 of that: the three-operation sums are exact
+                    const auto pair = [&](const float (&o)[4]) { return make_float2(o[2 * r], o[2 * r + 1]); };
+                    float2 w = pair(o0), low = add2(pair(o4), add2(pair(o5), pair(o6)));
+                    low = fma2(low, dup2(1.0f / 4194304.0f), pair(o3));
+                    const auto add = [&](const float2 p) {
+                        const float2 u = add2(w, p);
+                        low = add2(low, sub2(p, sub2(u, w)));
+                        w = u;
+                    };
+                    add(pair(o1));
+                    add(pair(o2));
                     const float2 mh = add2(w, low), ml = sub2(low, sub2(mh, w));
                     // about the term's position: r - X = (r - O) + (O - X)
                     const dfl ox = r ? xB : xA;

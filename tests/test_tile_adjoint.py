@@ -93,3 +93,22 @@ def test_law_change_rebuilds_the_digits(built_lib):
         g.warpDeriv(d, solverVec=False)
         out.append(np.array(g.getdXs()).reshape(-1))
     close(*out)
+
+
+def test_large_low_parts(built_lib):
+    """Nodes whose nearest point carries most of the denominator, layer by layer: the
+    low part of such a weight, left unnormalised, would overflow its third digit."""
+    from idwarp_gb300 import synthetic
+
+    m = synthetic.sphere_ogrid(n=9, layers=53)
+    m = dict(m, xv0=np.asarray(m["xv0"]).reshape(-1, 3)[: 488 * 12])
+    n = m["xv0"].size
+    d = np.random.default_rng(5).standard_normal(n)
+    out = []
+    for precision in ("mixed", "fp64"):
+        g = build_gpu(m, {"errTol": 1e-3}, precision=precision)
+        g.setSurfaceCoordinates(moved(m))
+        g.warpMesh()
+        g.warpDeriv(d, solverVec=False)
+        out.append(np.array(g.getdXs()).reshape(-1))
+    assert np.linalg.norm(out[0] - out[1]) <= 1e-12 * np.linalg.norm(out[1])
