@@ -89,7 +89,7 @@ struct Ctx {
     int adjMaxGroup = 16;        // seeds per adjoint walk
     // warpDeriv accumulators (grown on demand)
     int adjSeeds = 0;
-    DevBuf<double> adjPt, adjNode, adjRel;
+    DevBuf<double> adjPt, adjNode, adjRel, adjXub, adjFace;
     // order-independent landings (option deterministic): per accumulator
     // element an exponent and a 192-bit fixed-point sum
     DevBuf<int> landExpo;
@@ -1929,6 +1929,8 @@ int land_stage(Ctx *c, int nArr, double *const *base, const int64_t *len, F &&st
 
 extern "C" {
 
+constexpr int kNodalSeeds = 1024;  // seeds per launch of the reverse nodal kernels
+
 static int run_deriv(Ctx *c, const double *dxvDev, int nSeeds, int64_t seedStride, double *dxsOut, int where,
                      int64_t dxsStride) {
     if (!c->haveTree) return fail(c, IDW_ERR_STATE, "setSurfaceDefinition must come first");
@@ -1942,8 +1944,9 @@ static int run_deriv(Ctx *c, const double *dxvDev, int nSeeds, int64_t seedStrid
     }
     if (int e0 = ensure_den0(c)) return e0;
     if (!c->haveWarp) return fail(c, IDW_ERR_STATE, "warpMesh must be called before warpDeriv");
-    int rc = refresh_nodal(c, 0);  // the reverse walks read no motions
-    if (rc) return rc;
+    // the reverse product reads the surface, not its motions
+    int rc = IDW_OK;
+    launch_gather_xu(c->nUnique, c->xuInd.p, c->xs.p, c->xu.p, c->stream);
     EvalConsts k;
     k.law = make_law(c);
     k.errTol = c->opt.errTol;
@@ -1964,6 +1967,8 @@ static int run_deriv(Ctx *c, const double *dxvDev, int nSeeds, int64_t seedStrid
         CKA(c->adjPt.alloc(size_t(nSeeds) * 12 * n));
         CKA(c->adjNode.alloc(size_t(nSeeds) * 12 * nn));
         CKA(c->adjRel.alloc(size_t(nSeeds) * 12 * n));
+        CKA(c->adjXub.alloc(size_t(nSeeds) * 3 * n));
+        CKA(c->adjFace.alloc(size_t(nSeeds) * 4 * size_t(std::max(c->nFaces, 1))));
         c->adjSeeds = nSeeds;
     }
     DevView ptAdj{c->adjPt.p}, nodeAdj{c->adjNode.p}, ptRel{c->adjRel.p};
@@ -2050,10 +2055,34 @@ static int run_deriv(Ctx *c, const double *dxvDev, int nSeeds, int64_t seedStrid
     if (rc) return rc;
     SurfaceDev s = surf_dev(c);
     const bool faceLandings = c->opt.useRotations && c->nFaces > 0;
+    if (!det) {
+        // every seed at once (a call per seed took 163 us each on the 2M-node wing's
+        // surface of 40k points, latency most of it)
+        if (!mixed)
+            for (int sd = 0; sd < nSeeds; ++sd)
+                launch_set_data_b(tree_dev(c), nodeAdj.p + size_t(sd) * 12 * nn, ptAdj.p + size_t(sd) * 12 * n, n,
+                                  c->stream);
+        CK(cudaMemsetAsync(c->adjXub.p, 0, sizeof(double) * 3 * size_t(n) * nSeeds, c->stream));
+        for (int s0 = 0; s0 < nSeeds; s0 += kNodalSeeds) {
+            const int m = std::min(kNodalSeeds, nSeeds - s0);
+            launch_nodal_b(s, c->xu.p, c->ptXA.p, c->normals0.p, c->isCorner.p, c->opt.useRotations,
+                           (mixed ? ptRel.p : ptAdj.p) + size_t(s0) * 12 * n, mixed, c->adjXub.p + size_t(s0) * 3 * n,
+                           c->adjFace.p, c->stream, s0 == 0, m);
+            if (where == IDW_DEVICE && nSeeds > 1) {
+                CK(cudaMemset2DAsync(dxsOut + s0 * dxsStride, sizeof(double) * dxsStride, 0,
+                                     sizeof(double) * 3 * c->nPts, m, c->stream));
+                launch_scatter_dxs(n, c->xuInd.p, c->adjXub.p + size_t(s0) * 3 * n, dxsOut + s0 * dxsStride, c->stream,
+                                   m, dxsStride);
+            }
+        }
+        rc = check_launch(c, "reverse nodal properties");
+        if (rc || (where == IDW_DEVICE && nSeeds > 1)) return rc;
+    }
     for (int sd = 0; sd < nSeeds; ++sd) {
         double *pa = (mixed ? ptRel.p : ptAdj.p) + size_t(sd) * 12 * n;
-        if (!mixed) launch_set_data_b(tree_dev(c), nodeAdj.p + size_t(sd) * 12 * nn, pa, n, c->stream);
-        CK(cudaMemsetAsync(c->xub.p, 0, sizeof(double) * 3 * n, c->stream));
+        double *xub = det ? c->xub.p : c->adjXub.p + size_t(sd) * 3 * n;
+        if (det && !mixed) launch_set_data_b(tree_dev(c), nodeAdj.p + size_t(sd) * 12 * nn, pa, n, c->stream);
+        if (det) CK(cudaMemsetAsync(c->xub.p, 0, sizeof(double) * 3 * n, c->stream));
         if (det && faceLandings) {
             // node part: area and normal adjoints land in the faces' scratch
             // (Xub += Bb is the node's own write: from zero in each pass)
@@ -2077,13 +2106,13 @@ static int run_deriv(Ctx *c, const double *dxvDev, int nSeeds, int64_t seedStrid
                 return check_launch(c, "reverse nodal properties");
             });
             if (rc) return rc;
-        } else {
+        } else if (det) {
             launch_nodal_b(s, c->xu.p, c->ptXA.p, c->normals0.p, c->isCorner.p, c->opt.useRotations, pa, mixed,
-                           c->xub.p, c->stream, sd == 0);
+                           c->xub.p, c->faceScratch.p + 4 * size_t(c->nFaces), c->stream, sd == 0);
         }
         double *dst = (where == IDW_DEVICE) ? dxsOut + sd * dxsStride : c->dxs.p;
         CK(cudaMemsetAsync(dst, 0, sizeof(double) * 3 * c->nPts, c->stream));
-        launch_scatter_dxs(n, c->xuInd.p, c->xub.p, dst, c->stream);
+        launch_scatter_dxs(n, c->xuInd.p, xub, dst, c->stream);
         rc = check_launch(c, "reverse nodal properties");
         if (rc) return rc;
         if (where != IDW_DEVICE && dxsOut) {
@@ -2488,8 +2517,7 @@ int idw_warp_deriv_noalloc(void *ctx, const double *dxv, int64_t ndof, double *d
     int rc = noalloc_scratch(c, &scratch);
     if (rc) return rc;
     double *ptAdj = scratch, *nodeAdj = scratch + 12 * size_t(n), *ptRel = nodeAdj + 12 * size_t(nn);
-    rc = refresh_nodal(c, 0);
-    if (rc) return rc;
+    launch_gather_xu(n, c->xuInd.p, c->xs.p, c->xu.p, c->stream);
     EvalConsts k;
     k.law = make_law(c);
     k.errTol = c->opt.errTol;
@@ -2526,7 +2554,7 @@ int idw_warp_deriv_noalloc(void *ctx, const double *dxv, int64_t ndof, double *d
     if (rc) return rc;
     CK(cudaMemsetAsync(c->xub.p, 0, sizeof(double) * 3 * size_t(n), c->stream));
     launch_nodal_b(surf_dev(c), c->xu.p, c->ptXA.p, c->normals0.p, c->isCorner.p, c->opt.useRotations,
-                   mixed ? ptRel : ptAdj, mixed, c->xub.p, c->stream);
+                   mixed ? ptRel : ptAdj, mixed, c->xub.p, c->faceScratch.p + 4 * size_t(c->nFaces), c->stream);
     CK(cudaMemsetAsync(dxs, 0, sizeof(double) * size_t(cdof), c->stream));
     launch_scatter_dxs(n, c->xuInd.p, c->xub.p, dxs, c->stream);
     return check_launch(c, "reverse nodal properties");

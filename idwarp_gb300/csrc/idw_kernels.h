@@ -139,10 +139,13 @@ int64_t set_data_scratch(int nPts);
 void launch_set_data(const TreeDev &t, int nPts, const double *ptMB, double *nodeMB, double *sums, cudaStream_t st);
 void launch_set_data_b(const TreeDev &t, const double *nodeAdj, double *ptAdj, int nPts, cudaStream_t st);
 // faceProps = 0 reuses the face areas and normals of the previous call (same surface)
+// nSeeds point adjoints at once: Xub (3 n each, to be added to) and the scratch
+// faceAdj (4 nFaces each) in a row.
 void launch_nodal_b(const SurfaceDev &s, const double *Xu, const dbl4 *xa, const double *normals0,
                     const int *isCorner, int useRotations, const double *ptAdj, int relative, double *Xub,
-                    cudaStream_t st, int faceProps = 1);
-void launch_scatter_dxs(int n, const int *xuInd, const double *Xub, double *dXs, cudaStream_t st);
+                    double *faceAdj, cudaStream_t st, int faceProps = 1, int nSeeds = 1);
+void launch_scatter_dxs(int n, const int *xuInd, const double *Xub, double *dXs, cudaStream_t st, int nSeeds = 1,
+                        int64_t stride = 0);
 
 // Complex-step nodal properties (idw_complex.cu): Xu from the interleaved
 // complex coordinates xsC, and the imaginary parts of (M + I, b) per node.

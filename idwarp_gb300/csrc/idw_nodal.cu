@@ -384,10 +384,13 @@ __global__ void k_set_data_b(TreeDev t, const double *nodeAdj, double *ptAdj, in
 // element_props_b is linear in those adjoints).
 template <bool DET>
 __global__ void k_nodal_b_nodes(SurfaceDev s, const dbl4 *xa, const double *normals0, const int *isCorner,
-                                int useRotations, const double *ptAdj, int relative, double *Xub) {
+                                int useRotations, const double *ptAdj, int relative, double *Xub, double *faceAdj) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= s.n) return;
-    const double *adj = ptAdj + 12 * i;
+    // one seed per row of blocks
+    Xub += 3 * int64_t(s.n) * blockIdx.y;
+    faceAdj += 4 * int64_t(s.nFaces) * blockIdx.y;
+    const double *adj = ptAdj + 12 * (int64_t(s.n) * blockIdx.y + i);
     double Mb[9];
     double Bb[3] = {adj[9], adj[10], adj[11]};
     Xub[3 * i + 0] += Bb[0];
@@ -409,7 +412,6 @@ __global__ void k_nodal_b_nodes(SurfaceDev s, const dbl4 *xa, const double *norm
     rotation_matrix_b(normals0 + 3 * i, nrm, Mb, nb);
     double snb[3] = {nb[0] / sa, nb[1] / sa, nb[2] / sa};
     double sab = -(sn[0] * nb[0] + sn[1] * nb[1] + sn[2] * nb[2]) / sa / sa;
-    double *faceAdj = s.faceScratch + 4 * int64_t(s.nFaces);
     for (int e = e1 - 1; e >= e0; --e) {
         const int f = s.n2e[e];
         const int np = s.facePtr[f + 1] - s.facePtr[f];
@@ -427,10 +429,11 @@ __global__ void k_nodal_b_nodes(SurfaceDev s, const dbl4 *xa, const double *norm
 // Reverse nodal properties, face part: each face's element adjoint with the
 // summed area and normal adjoints of its nodes, into Xub of its vertices.
 template <bool DET>
-__global__ void k_nodal_b_faces(SurfaceDev s, const double *Xu, double *Xub) {
+__global__ void k_nodal_b_faces(SurfaceDev s, const double *Xu, double *Xub, const double *faceAdj) {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= s.nFaces) return;
-    const double *fa = s.faceScratch + 4 * int64_t(s.nFaces) + 4 * int64_t(f);
+    Xub += 3 * int64_t(s.n) * blockIdx.y;
+    const double *fa = faceAdj + 4 * (int64_t(s.nFaces) * blockIdx.y + f);
     const double areab = fa[0], nb[3] = {fa[1], fa[2], fa[3]};
     if (areab == 0.0 && nb[0] == 0.0 && nb[1] == 0.0 && nb[2] == 0.0) return;
     const int f0 = s.facePtr[f], np = s.facePtr[f + 1] - f0;
@@ -439,9 +442,11 @@ __global__ void k_nodal_b_faces(SurfaceDev s, const double *Xu, double *Xub) {
 
 // dXs[XuInd[i]] = Xub[i]: only the first caller occurrence of a unique point
 // receives the gradient (kd_tree.F90:1155-1159); dXs is pre-zeroed.
-__global__ void k_scatter_dxs(int n, const int *xuInd, const double *Xub, double *dXs) {
+__global__ void k_scatter_dxs(int n, const int *xuInd, const double *Xub, double *dXs, int64_t stride) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    Xub += 3 * int64_t(n) * blockIdx.y;
+    dXs += stride * blockIdx.y;
     int j = xuInd[i];
     dXs[3 * j + 0] = Xub[3 * i + 0];
     dXs[3 * j + 1] = Xub[3 * i + 1];
@@ -651,15 +656,16 @@ void launch_set_data_b(const TreeDev &t, const double *nodeAdj, double *ptAdj, i
 }
 void launch_nodal_b(const SurfaceDev &s, const double *Xu, const dbl4 *xa, const double *normals0,
                     const int *isCorner, int useRotations, const double *ptAdj, int relative, double *Xub,
-                    cudaStream_t st, int faceProps) {
-    if (s.n <= 0) return;
+                    double *faceAdj, cudaStream_t st, int faceProps, int nSeeds) {
+    if (s.n <= 0 || nSeeds <= 0) return;
     if (useRotations && s.nFaces > 0) {
         if (faceProps) k_face_props<<<blocks(s.nFaces, 128), 128, 0, st>>>(s, Xu);
-        cudaMemsetAsync(s.faceScratch + 4 * size_t(s.nFaces), 0, 4 * sizeof(double) * size_t(s.nFaces), st);
+        cudaMemsetAsync(faceAdj, 0, 4 * sizeof(double) * size_t(s.nFaces) * nSeeds, st);
     }
-    k_nodal_b_nodes<false>
-        <<<blocks(s.n, 128), 128, 0, st>>>(s, xa, normals0, isCorner, useRotations, ptAdj, relative, Xub);
-    if (useRotations && s.nFaces > 0) k_nodal_b_faces<false><<<blocks(s.nFaces, 128), 128, 0, st>>>(s, Xu, Xub);
+    k_nodal_b_nodes<false><<<dim3(blocks(s.n, 128), nSeeds), 128, 0, st>>>(s, xa, normals0, isCorner, useRotations,
+                                                                          ptAdj, relative, Xub, faceAdj);
+    if (useRotations && s.nFaces > 0)
+        k_nodal_b_faces<false><<<dim3(blocks(s.nFaces, 128), nSeeds), 128, 0, st>>>(s, Xu, Xub, faceAdj);
 }
 void launch_nodal_b_nodes(const SurfaceDev &s, const double *Xu, const dbl4 *xa, const double *normals0,
                           const int *isCorner, int useRotations, const double *ptAdj, int relative, double *Xub,
@@ -671,16 +677,19 @@ void launch_nodal_b_nodes(const SurfaceDev &s, const double *Xu, const dbl4 *xa,
     }
     if (det)
         k_nodal_b_nodes<true>
-            <<<blocks(s.n, 128), 128, 0, st>>>(s, xa, normals0, isCorner, useRotations, ptAdj, relative, Xub);
+            <<<blocks(s.n, 128), 128, 0, st>>>(s, xa, normals0, isCorner, useRotations, ptAdj, relative, Xub,
+                                               s.faceScratch + 4 * int64_t(s.nFaces));
     else
         k_nodal_b_nodes<false>
-            <<<blocks(s.n, 128), 128, 0, st>>>(s, xa, normals0, isCorner, useRotations, ptAdj, relative, Xub);
+            <<<blocks(s.n, 128), 128, 0, st>>>(s, xa, normals0, isCorner, useRotations, ptAdj, relative, Xub,
+                                               s.faceScratch + 4 * int64_t(s.nFaces));
 }
 void launch_nodal_b_faces(const SurfaceDev &s, const double *Xu, int useRotations, double *Xub, cudaStream_t st,
                           int det) {
     if (!(s.n > 0 && useRotations && s.nFaces > 0)) return;
-    if (det) k_nodal_b_faces<true><<<blocks(s.nFaces, 128), 128, 0, st>>>(s, Xu, Xub);
-    else k_nodal_b_faces<false><<<blocks(s.nFaces, 128), 128, 0, st>>>(s, Xu, Xub);
+    const double *faceAdj = s.faceScratch + 4 * int64_t(s.nFaces);
+    if (det) k_nodal_b_faces<true><<<blocks(s.nFaces, 128), 128, 0, st>>>(s, Xu, Xub, faceAdj);
+    else k_nodal_b_faces<false><<<blocks(s.nFaces, 128), 128, 0, st>>>(s, Xu, Xub, faceAdj);
 }
 void launch_nodal_d(const SurfaceDev &s, const double *Xu, const double *Xud, const dbl4 *xa, const double *normals0,
                     const double *Ai, const int *isCorner, int useRotations, int plusIdentity, double *ptMBd,
@@ -689,8 +698,10 @@ void launch_nodal_d(const SurfaceDev &s, const double *Xu, const double *Xud, co
     if (useRotations && s.nFaces > 0) k_face_props_d<<<blocks(s.nFaces, 128), 128, 0, st>>>(s, Xu, Xud);
     k_nodal_d<<<blocks(s.n, 128), 128, 0, st>>>(s, Xud, xa, normals0, Ai, isCorner, useRotations, plusIdentity, ptMBd);
 }
-void launch_scatter_dxs(int n, const int *xuInd, const double *Xub, double *dXs, cudaStream_t st) {
-    if (n > 0) k_scatter_dxs<<<blocks(n, 256), 256, 0, st>>>(n, xuInd, Xub, dXs);
+void launch_scatter_dxs(int n, const int *xuInd, const double *Xub, double *dXs, cudaStream_t st, int nSeeds,
+                        int64_t stride) {
+    if (n > 0 && nSeeds > 0)
+        k_scatter_dxs<<<dim3(blocks(n, 256), nSeeds), 256, 0, st>>>(n, xuInd, Xub, dXs, stride);
 }
 
 IDW_LAND_SETTER(land_set_nodal)
