@@ -898,7 +898,7 @@ static int ensure_gate_den(Ctx *c, const TreeDevF &tf, const PointsDevF &pf, con
 // The FP32 reverse product (IDW_ADJ_FAST) divides by the gated walk's
 // denominators, so its forward walk stays the gated one, and so do the
 // diagnostics.  Three symmetry planes (8 mirror images) bound the scratch, and
-// kTileMost node images the weight digits (about 2.5 kB each); both limits
+// kTileMost node images the weight digits (2.4 kB each, 3 kB with the fifth); both limits
 // apply with the lists on and off, so the results agree.
 constexpr int64_t kTileMost = int64_t(1) << 25;
 

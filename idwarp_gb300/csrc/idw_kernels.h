@@ -232,7 +232,7 @@ struct TileDev {
     const uint4 *mot;        // per term: 8 x 16 bytes, the FP16 digits of its motion (k_tile_mot)
     const unsigned *mot5;    // tangents, per term 8 words: its fifth digits
     const unsigned *colMax;  // largest magnitude of each motion column (float bits)
-    unsigned *counter;       // the walk's next unit (behind colMax: launch_tile_motions clears both)
+    unsigned *counter;       // the walk's next unit (its launch clears it)
     int areaExp;
 };
 // Tile order of the volume nodes (lo, hi: their bounding box).  Returns 0, -1 on
@@ -260,9 +260,9 @@ void launch_tile_build(const VolumeDev &v, const WalkRecF &rec, const EvalConsts
 // reference motion; with mot5 a tangent's (Md, bd).
 void launch_tile_motions(const TreeDev &t, int nPts, const double *ptMB, const double *nodeMB, unsigned *colMax,
                          uint4 *mot, unsigned *mot5, float *refDB, cudaStream_t st);
-// With lists.dig4 the motions are a tangent's (td.mot5, nb = 1).
 // The range's sums of nb surfaces (sums: 2 nLoop nVol float4 each), then their grids
-// (o.xv in a row) and denominators.
+// (o.xv in a row) and denominators.  With lists.dig4 the motions are a tangent's
+// (td.mot5, nb = 1).
 void launch_tile_walk(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
                       const EvalConsts &k, const TileDev &td, const TileLists &lists, const TileRange &range,
                       float4 *sums, cudaStream_t st, int nb = 1);

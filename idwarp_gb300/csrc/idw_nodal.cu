@@ -263,7 +263,7 @@ __global__ void k_nodal(SurfaceDev s, const double *Xu, const dbl4 *xa, const do
 // points beside them: no node waits for another.  (Bottom-up, the second child
 // to finish adding into its parent, the climb of one thread through 13 levels of
 // fences and atomics took 113 us on a 40k-point surface and 62 us on 700 points,
-// whatever the bandwidth; these two kernels take 37 and 21 us under the same
+// whatever the bandwidth; these two kernels take 37 and 24 us under the same
 // profiler, and 63 us less of a 7k-node warp's 182.)
 constexpr int kMeanChunk = 128;
 
@@ -567,7 +567,7 @@ __device__ void rotation_matrix_d(const double *v1, const double *v2, const doub
 
 // element_props_d of every face, once per face, into both halves of the face
 // scratch: area and unit normal, then their derivatives.  (Every node going
-// through its faces itself took 142 us on 12k points, this and the nodes XX.)
+// through its faces itself took 142 us on 12k points, this and the nodes 63.)
 __global__ void k_face_props_d(SurfaceDev s, const double *Xu, const double *Xud) {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= s.nFaces) return;

@@ -32,7 +32,11 @@ namespace {
 
 constexpr int kScaleExp = 13;   // node denominators are scaled to [2^13, 2^14)
 constexpr int kMotExp = 14;     // motions are scaled to at most 2^14
-constexpr int64_t kFourDigits = int64_t(1) << 17;  // node images up to which a warp uses four digits
+// Node images up to which a warp uses four digits: there they cost little (95k
+// nodes 12 us of a forward and reverse of 490, 7k nodes 2 us) and bring the error
+// from 1e-11 to 1e-14; beyond, a quarter more to stream (245k nodes 234 -> 259 us,
+// 8M 5.9 -> 7.3 ms).
+constexpr int64_t kFourDigits = int64_t(1) << 17;
 
 inline int blocks(int64_t n, int b) { return int((n + b - 1) / b); }
 

@@ -87,8 +87,12 @@ __device__ __forceinline__ float2 tile_weight(const float4 c, const float4 d, fl
     const float2 r = fma2(neg2(ql), y2, fma2(neg2(t0l), y, fma2(neg2(t0), y, one)));
     const float2 yp = mul2(y, P);
     const float2 v = mul2(y2, yp), vl = fma2(y2l, yp, fms2(y2, yp, v));
-    const float2 u = fma2(dup2(law.kh), y2, one);
-    const float2 ul = fma2(dup2(law.kl), y2, fma2(dup2(law.kh), y2l, fma2(dup2(law.kh), y2, sub2(one, u))));
+    // u + ul = 1 + kappa y^2, whichever of the two is larger
+    const float2 ky = mul2(dup2(law.kh), y2);
+    float2 u, ue;
+    two_sum2(ky, one, u, ue);
+    const float2 ul =
+        fma2(dup2(law.kl), y2, fma2(dup2(law.kh), y2l, add2(fms2(dup2(law.kh), y2, ky), ue)));
     const float2 t = mul2(v, u);
     // y (1 + r / 2) for y: v u gains v r (5 u - 2) / 2
     const float2 tl = fma2(mul2(v, fma2(dup2(2.5f), u, dup2(-1.0f))), r, fma2(vl, u, fma2(v, ul, fms2(v, u, t))));

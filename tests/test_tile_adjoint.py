@@ -112,3 +112,16 @@ def test_large_low_parts(built_lib):
         g.warpDeriv(d, solverVec=False)
         out.append(np.array(g.getdXs()).reshape(-1))
     assert np.linalg.norm(out[0] - out[1]) <= 1e-12 * np.linalg.norm(out[1])
+
+
+@pytest.mark.parametrize("first", [1e-3, 1e-5, 1e-7])
+def test_thin_layers(built_lib, first):
+    """First layers far thinner than the surface's spacing: the weight law's second
+    term is up to 1e13 times its first, and the weights of close points still count."""
+    from idwarp_gb300 import synthetic
+
+    m = synthetic.wing_shell(ni=101, nj=9, nk=8, first=first)
+    n = np.asarray(m["xv0"]).size
+    d = np.random.default_rng(6).standard_normal(n)
+    a, b = products(m, d)[0], products(m, d, precision="fp64")[0]
+    assert np.linalg.norm(a - b) <= 1e-12 * np.linalg.norm(b)
