@@ -937,14 +937,14 @@ def main():
                         "step, synchronize at the end; the grid read of step k overlaps the warp of step k + 1",
                 "max_diff_between_step_outputs": e2e_check},
         "clocks": clk,
-        # per step: gather_xu, face_props, nodal, set_data, mixed_nodal,
-        # mixed_nodes, walk, finalize (+ the replay's record refresh and
-        # counter add)
+        # per step: gather_xu, face_props, nodal, chunk_sums, node_means,
+        # tile_max, tile_mot, counter add, tile_walk, tile_finalize (8 for the
+        # gated walks)
         "gpu_launches": (10 if st["walkListEntries"] > 0 else 8) * args.steps,
         "setup_s": setup_s,
         "first_warp_s": first_warp_s,
         "walk_lists": {"entries": st["walkListEntries"], "bytes": 8 * max(0, st["walkListEntries"]),
-                       "note": "decisions recorded by the first warp (first_warp_s) and replayed by every step"},
+                       "note": "decisions and weights recorded by the first warp (first_warp_s) and used by every step"},
         "work": {"leafPairs": st["leafPairs"], "approx": st["approx"], "visited": st["visited"],
                  "fp64Fallback": st["fp64Fallback"]},
     }
@@ -952,19 +952,19 @@ def main():
     flops = 42.0 * (st["leafPairs"] + st["approx"])
     peak = fp32_peak_tflops() if not args.no_extras else None
     achieved = flops / (kernel_ms * 1e-3) / 1e12 if kernel_ms > 0 else None
-    # DRAM traffic of the walk: ncu dram__bytes_read.sum + dram__bytes_write.sum
-    # on the 2M-node wing (2,025,050 volume nodes), scaled by volume nodes: the
-    # per-node records, accumulators and (replay) the warps' decision lists;
-    # the tree stays in L2.  k_walk_mixed: 148.4 + 42.0 MB; k_walk_replay:
-    # 269.3 + 50.4 MB
+    # DRAM traffic of the walk.  The tile walk streams three FP16 digits of 32
+    # weights and a term index per list entry and keeps 64 bytes of sums per
+    # node and mirror; k_walk_mixed: ncu on the 2M-node wing, 148.4 + 42.0 MB
+    # for 2,025,050 nodes, scaled by volume nodes.  The tree stays in L2.
     replay = args.mode == "fast" and st["walkListEntries"] > 0
-    traffic = (157.9 if replay else 94.0) * nvol
-    walk_kernel = "k_exact_mixed" if args.mode == "exact" else ("k_walk_replay" if replay else "k_walk_mixed")
-    out["roofline"] = {"bound": "fp32", "kernel": walk_kernel, "achieved": achieved, "unit": "TFLOP/s",
+    traffic = 196.0 * st["walkListEntries"] + 64.0 * st["nLoop"] * nvol if replay else 94.0 * nvol
+    walk_kernel = "k_exact_mixed" if args.mode == "exact" else ("k_tile_walk" if replay else "k_walk_mixed")
+    out["roofline"] = {"bound": "hbm" if replay else "fp32", "kernel": walk_kernel, "achieved": achieved, "unit": "TFLOP/s",
                        "peak": peak, "peak_source": "measured FFMA probe (idw_probe_ffma) in this run",
                        "frac": (achieved / peak) if (achieved and peak) else None,
                        "flops_per_launch": flops, "kernel_ms": kernel_ms, "traffic": traffic,
-                       "traffic_note": "bytes per launch, ncu on the 2M-node wing scaled by volume nodes",
+                       "traffic_note": "bytes per launch: the tile walk's digits, indices and sums, or ncu on the 2M-node wing "
+                                       "scaled by volume nodes",
                        "hbm": {"achieved_GBs": traffic / (kernel_ms * 1e-3) / 1e9 if kernel_ms > 0 else None,
                                "peak_GBs": _measured_peak("hbm_gbs"), "peak_source": "MEASURED_PEAKS.json"}}
 
