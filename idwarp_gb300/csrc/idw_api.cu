@@ -80,7 +80,6 @@ struct Ctx {
     DevBuf<float4> recHi, recLo, acc;  // per-volume-node walk records and accumulators
     DevBuf<float> gden;                // per node: scaled denominator of a mixed walk (precision gate)
     // per-surface state of the batched mixed walk (grown on demand)
-    int batchCap = 0;
     DevBuf<double> bXs, bXu, bPtMB, bNodeMB;
     DevBuf<float> bPtDM, bPtDMl, bNodeDC, bNodeDCl, bNodeDn, bRef;
     DevBuf<float4> bAcc;
@@ -88,7 +87,6 @@ struct Ctx {
     int batchGroup = kBatchMax;  // surfaces per batched walk
     int adjMaxGroup = 16;        // seeds per adjoint walk
     // warpDeriv accumulators (grown on demand)
-    int adjSeeds = 0;
     DevBuf<double> adjPt, adjNode, adjRel, adjXub, adjFace;
     // order-independent landings (option deterministic): per accumulator
     // element an exponent and a 192-bit fixed-point sum
@@ -1499,7 +1497,7 @@ static int run_warp_batch_mixed(Ctx *c, const double *coordsDev, int nb, double 
         if (tile && tangent) return run_tile_tangents(c, tf, rec, k, lists, coordsDev, nb, outDev);
         if (tile) return run_tile_batch(c, tf, rec, k, lists, coordsDev, nb, outDev);
     }
-    if (c->batchCap < nb) {
+    {
         const size_t B = kBatchWalk;
         CKA(c->bXu.alloc(B * 3 * n));
         CKA(c->bPtMB.alloc(B * 12 * n));
@@ -1511,7 +1509,6 @@ static int run_warp_batch_mixed(Ctx *c, const double *coordsDev, int nb, double 
         CKA(c->bNodeDn.alloc(B * size_t(nn)));
         CKA(c->bRef.alloc(B * 24));
         CKA(c->bAcc.alloc(B * 2 * size_t(c->nVol)));
-        c->batchCap = kBatchWalk;
     }
     SurfaceDev s = surf_dev(c);
     const int exact = c->opt.evalMode == IDW_EVAL_EXACT;
@@ -1960,17 +1957,14 @@ static int run_deriv(Ctx *c, const double *dxvDev, int nSeeds, int64_t seedStrid
     const int n = c->nUnique, nn = c->nNodes;
     const int exact = c->opt.evalMode == IDW_EVAL_EXACT;
     const int mixed = c->opt.precision == IDW_PREC_MIXED;
-    // accumulators owned by the context (grown on demand): a call with device
-    // pointers and a seed count already seen allocates nothing, so it can be
-    // captured in a CUDA graph
-    if (c->adjSeeds < nSeeds) {
-        CKA(c->adjPt.alloc(size_t(nSeeds) * 12 * n));
-        CKA(c->adjNode.alloc(size_t(nSeeds) * 12 * nn));
-        CKA(c->adjRel.alloc(size_t(nSeeds) * 12 * n));
-        CKA(c->adjXub.alloc(size_t(nSeeds) * 3 * n));
-        CKA(c->adjFace.alloc(size_t(nSeeds) * 4 * size_t(std::max(c->nFaces, 1))));
-        c->adjSeeds = nSeeds;
-    }
+    // accumulators owned by the context, grown on demand (a smaller surface may
+    // have come before): a call with device pointers and a seed count already
+    // seen on this surface allocates nothing, so it can be captured in a CUDA graph
+    CKA(c->adjPt.alloc(size_t(nSeeds) * 12 * n));
+    CKA(c->adjNode.alloc(size_t(nSeeds) * 12 * nn));
+    CKA(c->adjRel.alloc(size_t(nSeeds) * 12 * n));
+    CKA(c->adjXub.alloc(size_t(nSeeds) * 3 * n));
+    CKA(c->adjFace.alloc(size_t(std::min(nSeeds, kNodalSeeds)) * 4 * size_t(std::max(c->nFaces, 1))));
     DevView ptAdj{c->adjPt.p}, nodeAdj{c->adjNode.p}, ptRel{c->adjRel.p};
     CK(cudaMemsetAsync(ptAdj.p, 0, sizeof(double) * size_t(nSeeds) * 12 * n, c->stream));
     CK(cudaMemsetAsync(nodeAdj.p, 0, sizeof(double) * size_t(nSeeds) * 12 * nn, c->stream));

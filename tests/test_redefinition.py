@@ -1,0 +1,53 @@
+"""A context whose volume and surface are redefined, larger and smaller, between
+calls: its workspaces follow the sizes, whatever was asked of the first mesh.
+
+Tolerance: grids are the fresh context's bit for bit; reverse products land with
+FP64 atomics, whose order alone differs (1e-12 of the largest entry)."""
+import contextlib
+import io
+
+import numpy as np
+import pytest
+
+from tests.meshes import build_gpu, sphere_small, wing_small
+from idwarp_gb300 import synthetic as S
+
+pytestmark = pytest.mark.gpu
+
+
+def larger():
+    m = S.sphere_ogrid(n=24, layers=10)
+    m["xs"] = S.sphere_perturbation(m["pts"], seed=3)
+    return m
+
+
+def results(g, m):
+    """A batch of three surfaces (one group), and the products of two seeds."""
+    xs = np.stack([m["xs"] * (1.0 + 0.01 * i) for i in range(3)])
+    grids = np.array(g.warpMeshBatch(xs))
+    g.setSurfaceCoordinates(m["xs"])
+    g.warpMesh()
+    seeds = np.random.default_rng(4).standard_normal((2, len(m["xv0"]), 3))
+    return grids, np.array(g.warpDerivBatch(seeds))
+
+
+@pytest.mark.parametrize("opts", [{"precision": "mixed"}, {"precision": "mixed", "adjointPrecision": "fast"},
+                                  {"precision": "mixed", "mixedGate": 1e-3},
+                                  {"precision": "mixed", "evalMode": "exact"},
+                                  {"precision": "mixed", "deterministic": True}, {"precision": "fp64"}])
+def test_workspaces_follow_the_sizes(built_lib, opts):
+    opts = dict(opts)
+    precision = opts.pop("precision")
+    meshes = [dict(m, symmetryPlanes=None) for m in (sphere_small(), larger(), wing_small())]
+    g = None
+    for m in meshes:
+        if g is None:
+            g = build_gpu(m, opts, precision=precision)
+        else:
+            with contextlib.redirect_stdout(io.StringIO()):
+                g.createCommonGrid(m["xv0"])
+                g.setSurfaceDefinition(m["pts"], m["conn"], m["faceSizes"])
+        grids, dxs = results(g, m)
+        want, dwant = results(build_gpu(m, opts, precision=precision), m)
+        np.testing.assert_array_equal(grids, want)
+        assert np.abs(dxs - dwant).max() <= 1e-12 * np.abs(dwant).max()
