@@ -471,12 +471,23 @@ int idw_create_common_grid(void *ctx, const double *volnodes, int64_t nvol, int 
         r.p = nullptr;
     }
     c->xvAlt.release();
-    c->nVol = nvol;
+    // a new volume needs a new initialize (records and estimates are per node),
+    // also when the grid is refused below: the old one is gone by then
+    c->haveVolume = false;
+    c->haveTree = false;
+    c->tileOrderValid = false;
+    c->listState = 0;
+    c->tileListState = c->tileState = 0;
+    c->den0Valid = false;
+    c->haveWarp = false;
+    c->haveDxs = false;
+    c->nVol = 0;
     CKA(c->xv0.alloc(3 * nvol));
     CKA(c->xv.alloc(3 * nvol));
     CKA(c->den0.alloc(nvol));
     CKA(c->den.alloc(nvol));
     CKA(c->perm.alloc(nvol));
+    c->nVol = nvol;
     int rc = copy_in(c, c->xv0.p, volnodes, 3 * size_t(nvol), where);
     if (rc) return rc;
     CK(cudaMemcpyAsync(c->xv.p, c->xv0.p, 3 * nvol * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
@@ -503,14 +514,6 @@ int idw_create_common_grid(void *ctx, const double *volnodes, int64_t nvol, int 
         if (e) return e;
     }
     c->haveVolume = true;
-    c->tileOrderValid = false;
-    // a new volume needs a new initialize (records and estimates are per node)
-    c->haveTree = false;
-    c->listState = 0;
-    c->tileListState = c->tileState = 0;
-    c->den0Valid = false;
-    c->haveWarp = false;
-    c->haveDxs = false;
     c->stats.nVol = nvol;
     return IDW_OK;
 }
@@ -520,6 +523,8 @@ int idw_set_symmetry_planes(void *ctx, const double *pts, const double *normals,
     if (!c) return IDW_ERR_ARG;
     if (n < 0 || n > kMaxSym) return fail(c, IDW_ERR_LIMIT, "at most %d symmetry planes are supported", kMaxSym);
     if (n > 0 && (!pts || !normals)) return fail(c, IDW_ERR_ARG, "null symmetry arrays");
+    // records and lists are per mirror image: another number of images needs a new initialize
+    if (n != c->sym.n) c->haveTree = c->haveWarp = c->haveDxs = false;
     c->sym.n = n;
     c->sym.nLoop = 1 << n;
     for (int j = 0; j < n; ++j)

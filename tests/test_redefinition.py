@@ -51,3 +51,26 @@ def test_workspaces_follow_the_sizes(built_lib, opts):
         want, dwant = results(build_gpu(m, opts, precision=precision), m)
         np.testing.assert_array_equal(grids, want)
         assert np.abs(dxs - dwant).max() <= 1e-12 * np.abs(dwant).max()
+
+
+def test_other_planes_need_a_new_surface_definition(built_lib):
+    from idwarp_gb300 import _lib
+
+    g = build_gpu(sphere_small(), precision="mixed")
+    p, nrm = np.zeros((1, 3)), np.array([[0.0, 1.0, 0.0]])
+    assert g.lib.idw_set_symmetry_planes(g.ctx, _lib.dptr(p), _lib.dptr(nrm), 1) == 0
+    assert g.lib.idw_warp_mesh(g.ctx) == _lib.IDW_ERR_STATE
+
+
+def test_a_refused_grid_needs_a_new_one(built_lib):
+    from idwarp_gb300 import _lib
+
+    m = sphere_small()
+    g = build_gpu(m, precision="mixed")
+    x = np.full((2 * len(m["xv0"]), 3), np.nan)
+    assert g.lib.idw_create_common_grid(g.ctx, _lib.dptr(x), len(x), _lib.IDW_HOST) == _lib.IDW_ERR_NONFINITE
+    assert g.lib.idw_warp_mesh(g.ctx) == _lib.IDW_ERR_STATE
+    with contextlib.redirect_stdout(io.StringIO()):
+        g.createCommonGrid(m["xv0"])
+        g.setSurfaceDefinition(m["pts"], m["conn"], m["faceSizes"])
+    assert g.lib.idw_warp_mesh(g.ctx) == 0
