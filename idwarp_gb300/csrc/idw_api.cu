@@ -120,8 +120,8 @@ struct Ctx {
     bool tileOrderValid = false;
     DevBuf<int> tileOrder;
     DevBuf<float> tileScale;
-    DevBuf<float4> tileGeo, tileSums;
-    DevBuf<uint4> tileMot, tileDig, tileDig3, tileDig4;
+    DevBuf<float4> tileGeo, tileSums, bTileSums;
+    DevBuf<uint4> tileMot, bTileMot, tileDig, tileDig3, tileDig4;
     DevBuf<double> tileDenInv;
     DevBuf<unsigned> tileWord;  // 12 column maxima, the walk's counter, the bad flag
     DevBuf<int64_t> tileOffs;
@@ -1090,15 +1090,15 @@ static int ensure_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const Ev
     return use && !lists.dig ? ensure_tile_chunks(c) : IDW_OK;
 }
 
-// The tile walk of nb surfaces whose motion records are laid out, and their grids.
+// The tile walk of nb surfaces whose motion records are laid out in td, and their
+// grids; sums: 2 nLoop nVol each.
 static int run_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalConsts &k, const TileLists &lists,
-                    const WalkOut &o, int nb) {
+                    const TileDev &td, float4 *sums, const WalkOut &o, int nb) {
     const TreeDev t = tree_dev(c);
     const VolumeDev v = vol_dev(c);
-    const TileDev td = tile_dev(c);
     if (lists.counters && o.counters) launch_add_walk_counters(o.counters, lists.counters, c->stream);
     if (lists.dig) {
-        launch_tile_walk(t, tf, v, rec, k, td, lists, tile_all(c), c->tileSums.p, c->stream, nb);
+        launch_tile_walk(t, tf, v, rec, k, td, lists, tile_all(c), sums, c->stream, nb);
     } else {
         for (const Ctx::TileRun &r : c->tileChunks) {
             TileLists l = lists;
@@ -1119,10 +1119,10 @@ static int run_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalC
                 l.dig4 = c->tileCDig4.p;
             }
             l.term += first;
-            launch_tile_walk(t, tf, v, rec, k, td, l, r.dig, c->tileSums.p, c->stream, nb);
+            launch_tile_walk(t, tf, v, rec, k, td, l, r.dig, sums, c->stream, nb);
         }
     }
-    launch_tile_finalize(v, rec, k, td, c->refDB.p, c->tileSums.p, o, c->stream, nb);
+    launch_tile_finalize(v, rec, k, td, c->refDB.p, sums, o, c->stream, nb);
     return check_launch(c, "tile walk");
 }
 
@@ -1189,7 +1189,7 @@ static int run_tile_tangent(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, con
     launch_tile_motions(tree_dev(c), c->nUnique, ptMBd, nodeMBd, c->tileWord.p, c->tileMot.p, c->tileMot5.p,
                         c->refDB.p, c->stream);
     c->nodalValid = false;
-    return run_tile(c, tf, rec, k, lists, o, 1);
+    return run_tile(c, tf, rec, k, lists, tile_dev(c), c->tileSums.p, o, 1);
 }
 
 // Before the warped grid is overwritten: if an asynchronous read of the
@@ -1249,7 +1249,7 @@ static int run_warp(Ctx *c, double *xvOut, double *denOut) {
         launch_tile_motions(tree_dev(c), c->nUnique, c->ptMB.p, c->nodeMB.p, c->tileWord.p, c->tileMot.p, nullptr,
                             c->refDB.p, c->stream);
         CK(cudaEventRecord(c->ev0, c->stream));
-        rc = run_tile(c, tf, rec, k, lists, o, 1);
+        rc = run_tile(c, tf, rec, k, lists, tile_dev(c), c->tileSums.p, o, 1);
         if (rc) return rc;
     } else if (c->opt.precision == IDW_PREC_MIXED) {
         PointsDevF pf;
@@ -1413,7 +1413,9 @@ int idw_get_volume_coordinates_cs(void *ctx, double *out, int64_t ndof, int wher
 static constexpr int kBatchWalk = kBatchMax;
 
 // run_warp_batch_mixed by tile walks, two surfaces each where the weight digits
-// stream from memory and the scratch for two is to be had.
+// stream from memory and the scratch for two is to be had.  Two surfaces have
+// motions and sums of their own: a captured graph of idw_warp_mesh keeps the
+// addresses of the single walk's.
 static int run_tile_batch(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalConsts &k, const TileLists &lists,
                           const double *coordsDev, int nb, double *outDev) {
     const int n = c->nUnique;
@@ -1421,17 +1423,25 @@ static int run_tile_batch(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const
     c->nodalValid = false;
     const SurfaceDev s = surf_dev(c);
     const size_t nTerms = size_t(n) + size_t(c->nNodes);
+    const size_t sums = 2 * size_t(c->sym.nLoop) * size_t(c->nVol);
     int per = nb > 1 ? tile_batch(vol_dev(c), c->sym.nLoop) : 1;
-    if (per > 1) {
+    if (per > 1 && (c->bTileSums.n < per * sums || c->bTileMot.n < 8 * per * nTerms)) {
         bool fits = false;
-        const size_t sums = 2 * size_t(c->sym.nLoop) * size_t(c->nVol);
         int rc = fits_half(c, double(sizeof(float4)) * per * double(sums + 8 * nTerms), fits);
         if (rc) return rc;
-        if (!fits && (c->tileSums.n < per * sums || c->tileMot.n < 8 * per * nTerms)) per = 1;
-        if (per > 1) {
-            CKA(c->tileSums.alloc(per * sums));
-            CKA(c->tileMot.alloc(8 * per * nTerms));
+        if (fits) {
+            CKA(c->bTileSums.alloc(per * sums));
+            CKA(c->bTileMot.alloc(8 * per * nTerms));
+        } else {
+            per = 1;
         }
+    }
+    TileDev td = tile_dev(c);
+    float4 *out = c->tileSums.p;
+    uint4 *mot = c->tileMot.p;
+    if (per > 1) {
+        out = c->bTileSums.p;
+        td.mot = mot = c->bTileMot.p;
     }
     CK(cudaEventRecord(c->ev0, c->stream));
     for (int b0 = 0; b0 < nb; b0 += per) {
@@ -1442,12 +1452,12 @@ static int run_tile_batch(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const
                          c->ptMB.p, c->stream);
             launch_set_data(tree_dev(c), n, c->ptMB.p, c->nodeMB.p, c->nodeSum.p, c->stream);
             launch_tile_motions(tree_dev(c), n, c->ptMB.p, c->nodeMB.p, c->tileWord.p + kTileWords * b,
-                                c->tileMot.p + 8 * nTerms * b, nullptr, c->refDB.p + 24 * b, c->stream);
+                                mot + 8 * nTerms * b, nullptr, c->refDB.p + 24 * b, c->stream);
         }
         WalkOut o;
         o.xv = outDev + size_t(b0) * vdof;
         o.counters = b0 == 0 ? c->counters.p : nullptr;
-        int rc = run_tile(c, tf, rec, k, lists, o, m);
+        int rc = run_tile(c, tf, rec, k, lists, td, out, o, m);
         if (rc) return rc;
     }
     CK(cudaEventRecord(c->ev1, c->stream));
@@ -2660,6 +2670,20 @@ int idw_autotune(void *ctx, int32_t nsurfaces, int32_t nseeds, idw_tuning *out) 
     if (rc) return rc;
     c->batchGroup = out->batchGroup;
     CK(cudaStreamSynchronize(c->stream));
+    return IDW_OK;
+}
+
+}  // extern "C"
+
+extern "C" {
+
+int idw_get_internal(void *ctx, const char *name, int64_t *value) {
+    Ctx *c = static_cast<Ctx *>(ctx);
+    if (!c || !name || !value) return IDW_ERR_ARG;
+    const std::string s(name);
+    if (s == "tileSums") *value = int64_t(reinterpret_cast<intptr_t>(c->tileSums.p));
+    else if (s == "tileMot") *value = int64_t(reinterpret_cast<intptr_t>(c->tileMot.p));
+    else return fail(c, IDW_ERR_ARG, "unknown internal value %s", name);
     return IDW_OK;
 }
 
