@@ -136,6 +136,7 @@ struct Ctx {
     DevBuf<unsigned long long> tileCnt;
     int tileFifthState = 0;  // the reverse product's fifth digit and denominators: 1 made, -1 too large, 0 not made
     int tileState = 0, tileListState = 0;  // tileListState: 1 lists, 2 lists and digits, -1 too large, 0 not made
+    bool tileDigits = false;               // tileListState 2: the digits are the current law's
     int64_t tileListEntries = 0;
     double tileErrTol = 0.0, tileLdefFact = 0.0, tileAlphaToB = 0.0;
     // adjoint
@@ -996,8 +997,12 @@ static int ensure_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const Ev
     if (!use) return IDW_OK;
     const bool off = c->opt.walkLists == IDW_WALK_LISTS_OFF;
     if (c->tileErrTol != c->opt.errTol) c->tileState = c->tileListState = 0;
-    if (c->tileLdefFact != c->opt.LdefFact || c->tileAlphaToB != k.law.alphaToBexp) c->tileState = 0;  // the lists stay
-    if (c->tileState == 0 || (c->tileState == 1 && !off && c->tileListState == 0)) {
+    if (c->tileLdefFact != c->opt.LdefFact || c->tileAlphaToB != k.law.alphaToBexp) {
+        c->tileState = 0;  // the lists stay, the digits are another law's (also where off leaves them)
+        c->tileDigits = false;
+    }
+    if (c->tileState == 0 ||
+        (c->tileState == 1 && !off && (c->tileListState == 0 || (c->tileListState == 2 && !c->tileDigits)))) {
         const size_t nTerms = size_t(c->nUnique) + size_t(c->nNodes);
         const int64_t units = walk_list_warps(c->nVol) * c->sym.nLoop;
         const bool newLists = !off && c->tileListState == 0;
@@ -1068,6 +1073,7 @@ static int ensure_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const Ev
                                   c->tileDig3.p, c->stream);
                 int rc = check_launch(c, "weight digits");
                 if (rc) return rc;
+                c->tileDigits = true;
             }
         }
         c->tileErrTol = c->opt.errTol;

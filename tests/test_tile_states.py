@@ -1,0 +1,54 @@
+"""Option changes between calls: what the tile walks keep must follow them, in every
+order.  At the first and the last step the warp, a tangent and a reverse product are
+compared with those of an FP64 context that went through the same options.
+
+Tolerances: those of the walks themselves (warp 1e-9 of Ldef0 below 2^17 node
+images; tangents 5e-10, reverse products 1.5e-11 of the result, as derived in
+their own tests); a stale law is off by its own effect, 1e-3 and more here."""
+import numpy as np
+import pytest
+
+from tests.meshes import build_gpu, wing_small
+
+pytestmark = pytest.mark.gpu
+
+AUTO, OFF = {"walkLists": "auto"}, {"walkLists": "off"}
+SEQUENCES = [
+    [AUTO, {"walkLists": "off", "alpha": 0.6}, AUTO],
+    [AUTO, {"walkLists": "off", "LdefFact": 3.0}, AUTO],
+    [AUTO, {"walkLists": "off", "errTol": 1e-2}, AUTO],
+    [OFF, AUTO, {"walkLists": "off", "alpha": 0.6}, {"walkLists": "off", "alpha": 0.25}, AUTO],
+    [AUTO, {"precision": "fp64", "alpha": 0.6}, {"precision": "mixed"}],
+    [AUTO, {"evalMode": "exact", "alpha": 0.6}, {"evalMode": "fast"}],
+    [AUTO, {"adjointPrecision": "fast", "alpha": 0.6}, {"adjointPrecision": "precise"}],
+    [AUTO, {"mixedGate": 1e-4, "LdefFact": 0.5}, {"mixedGate": 2e-3}],
+]
+
+
+@pytest.mark.parametrize("derivatives", [False, True])  # with them the fifth digits are kept from the first step on
+@pytest.mark.parametrize("steps", SEQUENCES)
+def test_options_in_sequence(built_lib, steps, derivatives):
+    m = wing_small()
+    rng = np.random.default_rng(2)
+    seed, tangent = rng.standard_normal(np.asarray(m["xv0"]).size), rng.standard_normal(np.asarray(m["pts"]).size)
+    g, f = build_gpu(m, precision="mixed"), build_gpu(m, precision="fp64")
+    for mesh in (g, f):
+        mesh.setSurfaceCoordinates(m["xs"])
+    for i, opts in enumerate(steps):
+        out = []
+        for mesh in (g, f):
+            for k, v in opts.items():
+                if not (mesh is f and k == "precision"):
+                    mesh.setOption(k, v)
+            mesh.warpMesh()
+            r = [np.array(mesh.getWarpGrid()).ravel()]
+            if derivatives or i == len(steps) - 1:
+                mesh.warpDeriv(seed, solverVec=False)
+                r += [np.array(mesh.getdXs()).ravel(),
+                      np.array(mesh.warpDerivFwd(tangent, solverVec=False)).ravel()]
+            out.append(r)
+        if g.getOption("precision") == "mixed" and i in (0, len(steps) - 1):
+            a, b = out
+            assert np.abs(a[0] - b[0]).max() < 1e-9 * g.getStats()["Ldef0"]
+            for x, y, tol in zip(a[1:], b[1:], (1.5e-11, 5e-10)):
+                assert np.linalg.norm(x - y) <= tol * np.linalg.norm(y)
