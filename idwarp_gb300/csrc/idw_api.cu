@@ -95,10 +95,10 @@ struct Ctx {
     bool gdenValid = false;
     double gdenLdefFact = 0.0, gdenAlpha = 0.0;
     int gdenMode = -1;
-    // the precise adjoint's denominator (double-float weights), per law and mode
+    // the precise adjoint's denominator (double-float weights), per law, errTol and mode
     DevBuf<double> denP;
     bool denPValid = false;
-    double denPLdefFact = 0.0, denPAlpha = 0.0;
+    double denPLdefFact = 0.0, denPAlpha = 0.0, denPErrTol = 0.0;
     int denPMode = -1;
     DevBuf<float> ptDM, ptDMl, nodeDC, nodeDCl, nodeDn, refDB;
     DevBuf<float4> replayRec;  // NodeAggF::rr: 8 float4 per tree node
@@ -2014,9 +2014,10 @@ static int run_deriv(Ctx *c, const double *dxvDev, int nSeeds, int64_t seedStrid
         rc = ensure_walk_lists(c, tf, rec, k);
         if (rc) return rc;
         precise = c->opt.adjointPrecision == IDW_ADJ_PRECISE && precise_adjoint_supported(k.law);
-        // the precise form's denominator to double-float accuracy: once per weight law and mode
+        // the precise form's denominator to double-float accuracy: once per weight
+        // law, errTol (its terms are the walk's) and mode
         if (precise && !(c->denPValid && c->denPLdefFact == c->opt.LdefFact && c->denPAlpha == c->opt.alpha &&
-                         c->denPMode == c->opt.evalMode)) {
+                         c->denPErrTol == c->opt.errTol && c->denPMode == c->opt.evalMode)) {
             CKA(c->denP.alloc(size_t(c->nVol)));
             launch_precise_denominator(tree_dev(c), tf, pf, vol_dev(c), rec, k, exact, c->denP.p, c->stream);
             rc = check_launch(c, "precise denominator");
@@ -2024,6 +2025,7 @@ static int run_deriv(Ctx *c, const double *dxvDev, int nSeeds, int64_t seedStrid
             c->denPValid = true;
             c->denPLdefFact = c->opt.LdefFact;
             c->denPAlpha = c->opt.alpha;
+            c->denPErrTol = c->opt.errTol;
             c->denPMode = c->opt.evalMode;
             CK(cudaEventRecord(c->ev0, c->stream));
         }

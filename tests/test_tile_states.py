@@ -52,3 +52,21 @@ def test_options_in_sequence(built_lib, steps, derivatives):
             assert np.abs(a[0] - b[0]).max() < 1e-9 * g.getStats()["Ldef0"]
             for x, y, tol in zip(a[1:], b[1:], (1.5e-11, 5e-10)):
                 assert np.linalg.norm(x - y) <= tol * np.linalg.norm(y)
+
+
+@pytest.mark.parametrize("opts", [{"deterministic": True}, {"walkLists": "off"}, {"mixedGate": 1e-3}])
+def test_errtol_change_renews_the_double_float_denominators(built_lib, opts):
+    """Reverse products that sum term by term divide by denominators of their own; their
+    tolerance is 1e-9 of the largest entry (a stale one is off by 4e-3)."""
+    m = wing_small()
+    seed = np.random.default_rng(2).standard_normal(np.asarray(m["xv0"]).size)
+    g, f = build_gpu(m, opts, precision="mixed"), build_gpu(m, precision="fp64")
+    for errTol in (1e-4, 1e-3):
+        out = []
+        for mesh in (g, f):
+            mesh.setOption("errTol", errTol)
+            mesh.setSurfaceCoordinates(m["xs"])
+            mesh.warpMesh()
+            mesh.warpDeriv(seed, solverVec=False)
+            out.append(np.array(mesh.getdXs()).ravel())
+        assert np.abs(out[0] - out[1]).max() <= 1e-9 * np.abs(out[1]).max()
