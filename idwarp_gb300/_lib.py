@@ -125,6 +125,7 @@ _SIGS = {
     "idw_get_surface_state": [_VP, _DP, _DP, _DP, _IP, _IP],
     "idw_get_nodal_properties": [_VP, _DP, _DP],
     "idw_get_internal": [_VP, C.c_char_p, C.POINTER(C.c_int64)],
+    "idw_set_internal": [_VP, C.c_char_p, C.c_int64],
 }
 _VOID = {"idw_default_options"}
 

@@ -113,8 +113,8 @@ struct Ctx {
     int64_t listEntries = 0;
     // tile walks (idw_tile.cu): node order (per volume), term geometry (per
     // surface definition); scales, lists and weight digits, valid for the current
-    // den0, tileErrTol and law (tileState 1; -1 when some node has no scale);
-    // motion records per surface
+    // den0, tileErrTol and law (tileState 1; -1 when some node has no scale or the
+    // memory is not to be had: the gated walks then serve); motion records per surface
     double volLo[3] = {0, 0, 0}, volHi[3] = {0, 0, 0};
     int areaExp = 0;  // scales the largest node area to near one
     bool tileOrderValid = false;
@@ -134,10 +134,15 @@ struct Ctx {
     };
     std::vector<TileRun> tileChunks;  // the runs
     DevBuf<unsigned long long> tileCnt;
-    int tileFifthState = 0;  // the reverse product's fifth digit and denominators: 1 made, -1 too large, 0 not made
-    int tileState = 0, tileListState = 0;  // tileListState: 1 lists, 2 lists and digits, -1 too large, 0 not made
-    bool tileDigits = false;               // tileListState 2: the digits are the current law's
+    int tileRunState = 0;    // the runs' scratch: 1 there, -1 not to be had, 0 not asked for
+    int tileFifthState = 0;  // the kept digits' fifth and the denominators: 1 made, -1 not to be had, 0 not made
+    int tileState = 0;       // scales and offsets: 1 valid, -1 the walk does not serve, 0 not made
+    bool tileKept = false;   // the lists are recorded
+    bool tileDigits = false; // tileKept: the digits are the current law's
     int64_t tileListEntries = 0;
+    // for the tests: allocations that the tile walks may still make (-1: any
+    // number), free bytes that they reckon with (-1: the device's)
+    int64_t tileAllocs = -1, tileFree = -1;
     double tileErrTol = 0.0, tileLdefFact = 0.0, tileAlphaToB = 0.0;
     // adjoint
     DevBuf<double> ptAdj, nodeAdj, xub, dxs;
@@ -323,6 +328,20 @@ int refresh_nodal(Ctx *c, int gated) {
     return check_launch(c, "nodal properties");
 }
 
+// Memory of the tile walks: false where it is not to be had (the walks that need
+// none then serve).
+template <class T>
+bool tile_alloc(Ctx *c, DevBuf<T> &b, size_t n) {
+    if (!(b.p && n <= b.n) && c->tileAllocs >= 0 && c->tileAllocs-- == 0) {
+        c->tileAllocs = 0;
+        b.release();
+        return false;
+    }
+    if (b.alloc(n) == cudaSuccess) return true;
+    (void)cudaGetLastError();
+    return false;
+}
+
 // Walk records of every volume node from the denominator estimate in den0.
 int finish_den0(Ctx *c) {
     launch_walk_records(vol_dev(c), c->sym, c->optInit.bExp, c->recHi.p, c->recLo.p, c->stream);
@@ -331,7 +350,8 @@ int finish_den0(Ctx *c) {
     c->gdenValid = false;
     c->denPValid = false;
     c->listState = 0;
-    c->tileListState = c->tileState = 0;
+    c->tileState = 0;
+    c->tileKept = false;
     c->den0Valid = true;
     return IDW_OK;
 }
@@ -478,7 +498,8 @@ int idw_create_common_grid(void *ctx, const double *volnodes, int64_t nvol, int 
     c->haveTree = false;
     c->tileOrderValid = false;
     c->listState = 0;
-    c->tileListState = c->tileState = 0;
+    c->tileState = 0;
+    c->tileKept = false;
     c->den0Valid = false;
     c->haveWarp = false;
     c->haveDxs = false;
@@ -779,7 +800,8 @@ int idw_initialize_warping(void *ctx, const double *pts, int32_t npts, const dou
     c->gdenValid = false;
     c->denPValid = false;
     c->listState = 0;
-    c->tileListState = c->tileState = 0;
+    c->tileState = 0;
+    c->tileKept = false;
     double maxA = 0.0;
     for (int i = 0; i < n; ++i) maxA = std::max(maxA, std::fabs(ai[i]));
     c->areaExp = maxA > 0.0 && std::isfinite(maxA) ? -std::ilogb(maxA) : 0;
@@ -925,12 +947,44 @@ static TileDev tile_dev(Ctx *c) {
     return td;
 }
 
-// Half of the free device memory holds `bytes` more.
-static int fits_half(Ctx *c, double bytes, bool &yes) {
-    size_t freeB = 0, totalB = 0;
-    CK(cudaMemGetInfo(&freeB, &totalB));
-    yes = bytes <= 0.5 * double(freeB);
+// Half of the free device memory and of `held` bytes to be given back holds `bytes`.
+static int fits_half(Ctx *c, double bytes, bool &yes, double held = 0.0) {
+    size_t freeB = size_t(c->tileFree), totalB = 0;
+    if (c->tileFree < 0) CK(cudaMemGetInfo(&freeB, &totalB));
+    yes = bytes <= 0.5 * (double(freeB) + held);
     return IDW_OK;
+}
+
+// Gives back the kept lists and digits.
+static void drop_tile_kept(Ctx *c) {
+    c->tileKept = c->tileDigits = false;
+    c->tileFifthState = 0;
+    c->tileTerm.release();
+    c->tileMask.release();
+    c->tileDig.release();
+    c->tileDig3.release();
+    c->tileDig4.release();
+    c->tileDenInv.release();
+}
+static void drop_tile_runs(Ctx *c) {
+    c->tileCTerm.release();
+    c->tileCMask.release();
+    c->tileCDig.release();
+    c->tileCDig3.release();
+    c->tileCDig4.release();
+}
+static void drop_tile(Ctx *c) {
+    drop_tile_kept(c);
+    drop_tile_runs(c);
+    c->tileOrderValid = false;
+    c->tileOrder.release();
+    c->tileOffs.release();
+    c->tileGeo.release();
+    c->tileMot.release();
+    c->tileScale.release();
+    c->tileSums.release();
+    c->bTileMot.release();
+    c->bTileSums.release();
 }
 
 // Every group of the mesh.
@@ -940,16 +994,16 @@ static TileRange tile_all(const Ctx *c) {
     return r;
 }
 
-// Without kept digits a walk makes them a run of groups at a time, and the lists
-// for a longer run before that unless they are kept: list runs of at most
-// kListSteps steps (128 bytes each) in digit runs of at most kDigitSteps (4 kB
-// each), or one group.  Recorded, made and walked apart, at full occupancy each:
-// formed within the walk they took 12.1 instead of 7.9 ms on the 2M-node wing with
-// the lists off.  A short list run still takes one warp's traversal (0.4 ms).
+// With the lists off a walk records and makes them a run of groups at a time:
+// list runs of at most kListSteps steps (128 bytes each) in digit runs of at most
+// kDigitSteps (4 kB each), or one group.  Recorded, made and walked apart, at full
+// occupancy each: formed within the walk they took 12.1 instead of 7.9 ms on the
+// 2M-node wing.  A short list run still takes one warp's traversal (0.4 ms).
 constexpr int64_t kListSteps = int64_t(1) << 22, kDigitSteps = int64_t(1) << 19;
 
-static int ensure_tile_chunks(Ctx *c) {
-    if (!c->tileChunks.empty()) return IDW_OK;
+// The runs and their scratch, halved until it is to be had (tileRunState).
+static int ensure_tile_runs(Ctx *c) {
+    if (c->tileRunState) return IDW_OK;
     const int64_t groups = walk_list_warps(c->nVol), nl = c->sym.nLoop;
     std::vector<int64_t> offs(size_t(groups * nl) + 1);
     CK(cudaMemcpyAsync(offs.data(), c->tileOffs.p, sizeof(int64_t) * offs.size(), cudaMemcpyDeviceToHost, c->stream));
@@ -967,15 +1021,17 @@ static int ensure_tile_chunks(Ctx *c) {
     };
     int64_t listCap = std::max(widest, std::min(kListSteps, offs.back() / 16));
     int64_t digCap = std::max(widest, std::min(kDigitSteps, offs.back() / 16));
-    while (c->tileCTerm.alloc(16 * size_t(listCap)) != cudaSuccess ||
-           c->tileCMask.alloc(16 * size_t(listCap)) != cudaSuccess ||
-           c->tileCDig.alloc(192 * size_t(digCap)) != cudaSuccess ||
-           c->tileCDig3.alloc(64 * size_t(digCap)) != cudaSuccess) {
-        (void)cudaGetLastError();
-        if (listCap == widest && digCap == widest) return fail(c, IDW_ERR_NOMEM, "no room for the walk's scratch");
+    while (!(tile_alloc(c, c->tileCTerm, 16 * size_t(listCap)) && tile_alloc(c, c->tileCMask, 16 * size_t(listCap)) &&
+             tile_alloc(c, c->tileCDig, 192 * size_t(digCap)) && tile_alloc(c, c->tileCDig3, 64 * size_t(digCap)))) {
+        drop_tile_runs(c);
+        if (listCap == widest && digCap == widest) {
+            c->tileRunState = -1;
+            return IDW_OK;
+        }
         listCap = std::max(widest, listCap / 2);
         digCap = std::max(widest, digCap / 2);
     }
+    c->tileChunks.clear();
     for (int64_t g = 0; g < groups;) {
         const TileRange l = run(g, groups, listCap);
         for (g = l.group0; g < l.group1;) {
@@ -984,116 +1040,132 @@ static int ensure_tile_chunks(Ctx *c) {
             g = d.group1;
         }
     }
+    c->tileRunState = 1;
     return IDW_OK;
 }
 
+// Scales, offsets and (unless off) lists and weight digits of the current den0,
+// errTol and law: tileState 1, or -1 where the walk does not serve, because some
+// node has no scale or because lists and digits, the fifth ones included, would
+// not fit into half of the free memory.  That holds with the lists off too,
+// where nothing of it is kept: the gated walks are then as they were, and both
+// settings of walkLists give the same bits.
+static int make_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalConsts &k, bool off) {
+    const size_t nTerms = size_t(c->nUnique) + size_t(c->nNodes);
+    const int64_t units = walk_list_warps(c->nVol) * c->sym.nLoop;
+    const bool record = !off && !c->tileKept;
+    c->tileState = 0;
+    c->tileRunState = 0;
+    if (record) drop_tile_kept(c);
+    auto serves = [&](int state) {
+        if (state < 0 && !c->tileKept) drop_tile(c);
+        c->tileErrTol = c->opt.errTol;
+        c->tileLdefFact = c->opt.LdefFact;
+        c->tileAlphaToB = k.law.alphaToBexp;
+        c->tileState = state;
+        return IDW_OK;
+    };
+    if (!(tile_alloc(c, c->tileOffs, size_t(units) + 1) && tile_alloc(c, c->tileGeo, 2 * nTerms) &&
+          tile_alloc(c, c->tileMot, 8 * nTerms) && tile_alloc(c, c->tileWord, 2 * kTileWords) &&
+          tile_alloc(c, c->tileScale, size_t(c->nVol)) &&
+          tile_alloc(c, c->tileSums, 2 * size_t(c->sym.nLoop) * size_t(c->nVol)) &&
+          tile_alloc(c, c->tileOrder, size_t(c->nVol))))
+        return serves(-1);
+    if (!c->tileOrderValid) {
+        const int rc = tile_order(vol_dev(c), c->volLo, c->volHi, c->tileOrder.p, c->stream);
+        if (rc == -2) {
+            (void)cudaGetLastError();
+            return serves(-1);
+        }
+        if (rc) return fail(c, IDW_ERR_CUDA, "node order of the tile walks failed");
+        c->tileOrderValid = true;
+    }
+    launch_tile_geo(tree_dev(c), c->nUnique, c->ptXA.p, c->areaExp, c->tileGeo.p, c->stream);
+    int *bad = reinterpret_cast<int *>(c->tileWord.p + 13);
+    const int64_t total = count_tile_lists(tree_dev(c), tf, vol_dev(c), rec, k, tile_dev(c), c->tileOffs.p,
+                                           reinterpret_cast<float *>(c->tileSums.p), c->tileScale.p, bad, c->stream);
+    if (total == -2) {
+        (void)cudaGetLastError();
+        return serves(-1);
+    }
+    if (total < 0) return fail(c, IDW_ERR_CUDA, "walk lists: count pass failed");
+    int badH = 0;
+    CK(cudaMemcpyAsync(&badH, bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    if (badH) return serves(-1);
+    const size_t entries = size_t(std::max<int64_t>(total, 16)), steps = entries / 16;
+    if (!c->tileKept) {
+        const double need = 8.0 * double(entries) + 320.0 * sizeof(uint4) * double(steps) + 8.0 * double(c->nVol);
+        const double held =
+            8.0 * double(c->tileTerm.n) + sizeof(uint4) * double(c->tileDig.n + c->tileDig3.n + c->tileDig4.n);
+        bool fits = false;
+        int rc = fits_half(c, need, fits, held);
+        if (rc) return rc;
+        if (!fits) return serves(-1);
+    }
+    c->tileListEntries = total;
+    if (record) {
+        if (!(tile_alloc(c, c->tileCnt, 8) && tile_alloc(c, c->tileTerm, entries) &&
+              tile_alloc(c, c->tileMask, entries) && tile_alloc(c, c->tileDig, 192 * steps) &&
+              tile_alloc(c, c->tileDig3, 64 * steps)))
+            return serves(-1);
+        CK(cudaMemsetAsync(c->tileCnt.p, 0, 8 * sizeof(unsigned long long), c->stream));
+        launch_tile_record(tree_dev(c), tf, vol_dev(c), rec, k, tile_dev(c), tile_all(c), c->tileOffs.p, c->tileTerm.p,
+                           c->tileMask.p, c->tileCnt.p, c->stream);
+        int rc = check_launch(c, "walk lists");
+        if (rc) return rc;
+        c->tileKept = true;
+    }
+    if (!off) {
+        TileLists lists;
+        lists.offs = c->tileOffs.p;
+        lists.term = c->tileTerm.p;
+        lists.mask = c->tileMask.p;
+        c->tileFifthState = 0;
+        launch_tile_build(vol_dev(c), rec, k, tile_dev(c), lists, tile_all(c), 0, c->nUnique, c->tileDig.p,
+                          c->tileDig3.p, c->stream);
+        int rc = check_launch(c, "weight digits");
+        if (rc) return rc;
+        c->tileDigits = true;
+    }
+    return serves(1);
+}
+
 // What a tile walk needs besides the motions: node order, term geometry, node
-// scales, and (unless off) the lists and the weight digits, each when it fits.
-// use = false when the walk does not apply or some node has no scale.
+// scales, and the lists and weight digits, or (lists off) the scratch of the runs.
+// use = false when the walk does not apply or does not serve.
 static int ensure_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalConsts &k, TileLists &lists,
                        bool &use) {
     lists = TileLists{};
     use = tile_applies(c, k);
     if (!use) return IDW_OK;
     const bool off = c->opt.walkLists == IDW_WALK_LISTS_OFF;
-    if (c->tileErrTol != c->opt.errTol) c->tileState = c->tileListState = 0;
+    if (c->tileErrTol != c->opt.errTol) {
+        c->tileState = 0;
+        c->tileKept = false;
+    }
     if (c->tileLdefFact != c->opt.LdefFact || c->tileAlphaToB != k.law.alphaToBexp) {
         c->tileState = 0;  // the lists stay, the digits are another law's (also where off leaves them)
         c->tileDigits = false;
     }
-    if (c->tileState == 0 ||
-        (c->tileState == 1 && !off && (c->tileListState == 0 || (c->tileListState == 2 && !c->tileDigits)))) {
-        const size_t nTerms = size_t(c->nUnique) + size_t(c->nNodes);
-        const int64_t units = walk_list_warps(c->nVol) * c->sym.nLoop;
-        const bool newLists = !off && c->tileListState == 0;
-        c->tileState = 0;
-        c->tileChunks.clear();
-        if (newLists) {
-            c->tileTerm.release();
-            c->tileMask.release();
-            c->tileDig.release();
-            c->tileDig3.release();
-            c->tileDig4.release();
-        }
-        CKA(c->tileOffs.alloc(size_t(units) + 1));
-        CKA(c->tileGeo.alloc(2 * nTerms));
-        CKA(c->tileMot.alloc(8 * nTerms));
-        CKA(c->tileWord.alloc(2 * kTileWords));
-        CKA(c->tileScale.alloc(size_t(c->nVol)));
-        CKA(c->tileSums.alloc(2 * size_t(c->sym.nLoop) * size_t(c->nVol)));
-        CKA(c->tileOrder.alloc(size_t(c->nVol)));
-        if (!c->tileOrderValid) {
-            const int rc = tile_order(vol_dev(c), c->volLo, c->volHi, c->tileOrder.p, c->stream);
-            if (rc) return fail(c, rc == -2 ? IDW_ERR_NOMEM : IDW_ERR_CUDA, "node order of the tile walks failed");
-            c->tileOrderValid = true;
-        }
-        launch_tile_geo(tree_dev(c), c->nUnique, c->ptXA.p, c->areaExp, c->tileGeo.p, c->stream);
-        int *bad = reinterpret_cast<int *>(c->tileWord.p + 13);
-        const int64_t total = count_tile_lists(tree_dev(c), tf, vol_dev(c), rec, k, tile_dev(c), c->tileOffs.p,
-                                               reinterpret_cast<float *>(c->tileSums.p), c->tileScale.p, bad,
-                                               c->stream);
-        if (total < 0) return fail(c, IDW_ERR_CUDA, "walk lists: count pass failed");
-        int badH = 0;
-        CK(cudaMemcpyAsync(&badH, bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-        CK(cudaStreamSynchronize(c->stream));
-        bool fits = false;
-        c->tileListEntries = total;
-        if (newLists && !badH) {
-            int rc = fits_half(c, 8.0 * double(total), fits);
-            if (rc) return rc;
-            if (fits) {
-                CKA(c->tileCnt.alloc(8));
-                CKA(c->tileTerm.alloc(size_t(std::max<int64_t>(total, 1))));
-                CKA(c->tileMask.alloc(size_t(std::max<int64_t>(total, 1))));
-                CK(cudaMemsetAsync(c->tileCnt.p, 0, 8 * sizeof(unsigned long long), c->stream));
-                launch_tile_record(tree_dev(c), tf, vol_dev(c), rec, k, tile_dev(c), tile_all(c), c->tileOffs.p,
-                                   c->tileTerm.p, c->tileMask.p, c->tileCnt.p, c->stream);
-                rc = check_launch(c, "walk lists");
-                if (rc) return rc;
-            }
-            c->tileListState = fits ? 1 : -1;
-        }
-        if (!off && !badH && c->tileListState > 0) {
-            const size_t steps = size_t(std::max<int64_t>(c->tileListEntries / 16, 1));
-            if (c->tileListState == 1) {
-                int rc = fits_half(c, 256.0 * sizeof(uint4) * double(steps), fits);
-                if (rc) return rc;
-                if (fits) {
-                    CKA(c->tileDig.alloc(192 * steps));
-                    CKA(c->tileDig3.alloc(64 * steps));
-                    c->tileListState = 2;
-                }
-            }
-            if (c->tileListState == 2) {
-                lists.offs = c->tileOffs.p;
-                lists.term = c->tileTerm.p;
-                lists.mask = c->tileMask.p;
-                c->tileFifthState = 0;
-                launch_tile_build(vol_dev(c), rec, k, tile_dev(c), lists, tile_all(c), 0, c->nUnique, c->tileDig.p,
-                                  c->tileDig3.p, c->stream);
-                int rc = check_launch(c, "weight digits");
-                if (rc) return rc;
-                c->tileDigits = true;
-            }
-        }
-        c->tileErrTol = c->opt.errTol;
-        c->tileLdefFact = c->opt.LdefFact;
-        c->tileAlphaToB = k.law.alphaToBexp;
-        c->tileState = badH ? -1 : 1;
+    if (c->tileState == 0 || (c->tileState == 1 && !off && !(c->tileKept && c->tileDigits))) {
+        int rc = make_tile(c, tf, rec, k, off);
+        if (rc) return rc;
     }
     use = c->tileState == 1;
-    lists = TileLists{};
+    if (!use) return IDW_OK;
     lists.offs = c->tileOffs.p;
-    if (use && !off && c->tileListState > 0) {
-        lists.term = c->tileTerm.p;
-        lists.mask = c->tileMask.p;
-        lists.counters = c->tileCnt.p;
-        if (c->tileListState == 2) {
-            lists.dig = c->tileDig.p;
-            lists.dig3 = c->tileDig3.p;
-        }
+    if (off) {
+        int rc = ensure_tile_runs(c);
+        use = c->tileRunState == 1;
+        return rc;
     }
-    return use && !lists.dig ? ensure_tile_chunks(c) : IDW_OK;
+    lists.term = c->tileTerm.p;
+    lists.mask = c->tileMask.p;
+    lists.counters = c->tileCnt.p;
+    lists.dig = c->tileDig.p;
+    lists.dig3 = c->tileDig3.p;
+    return IDW_OK;
 }
 
 // The tile walk of nb surfaces whose motion records are laid out in td, and their
@@ -1108,15 +1180,12 @@ static int run_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalC
     } else {
         for (const Ctx::TileRun &r : c->tileChunks) {
             TileLists l = lists;
-            int64_t first = r.dig.entry0;  // where the run's lists begin
-            if (!lists.term) {
-                l.term = c->tileCTerm.p;
-                l.mask = c->tileCMask.p;
-                first -= r.list.entry0;
-                if (first == 0)
-                    launch_tile_record(t, tf, v, rec, k, td, r.list, lists.offs, c->tileCTerm.p, c->tileCMask.p,
-                                       o.counters, c->stream);
-            }
+            l.term = c->tileCTerm.p;
+            l.mask = c->tileCMask.p;
+            const int64_t first = r.dig.entry0 - r.list.entry0;  // where the run's lists begin
+            if (first == 0)
+                launch_tile_record(t, tf, v, rec, k, td, r.list, lists.offs, c->tileCTerm.p, c->tileCMask.p, o.counters,
+                                   c->stream);
             launch_tile_build(v, rec, k, td, l, r.dig, first, c->nUnique, c->tileCDig.p, c->tileCDig3.p, c->stream);
             l.dig = c->tileCDig.p;
             l.dig3 = c->tileCDig3.p;
@@ -1133,25 +1202,23 @@ static int run_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalC
 }
 
 // The kept digits' fifth and the reciprocal denominators of the digits' weights,
-// both once per mesh and weight law; have = false when they do not fit.
+// both once per mesh and weight law; have = false where there is no room.
 static int ensure_tile_fifth(Ctx *c, const WalkRecF &rec, const EvalConsts &k, TileLists &lists, bool &have) {
     if (c->tileFifthState == 0) {
         const size_t steps = size_t(std::max<int64_t>(c->tileListEntries / 16, 1));
-        bool fits = false;
-        int rc = fits_half(c, 64.0 * sizeof(uint4) * double(steps) + 8.0 * double(c->nVol), fits);
-        if (rc) return rc;
-        c->tileFifthState = fits ? 1 : -1;
-        if (fits) {
-            CKA(c->tileDig4.alloc(64 * steps));
-            CKA(c->tileDenInv.alloc(size_t(c->nVol)));
+        if (tile_alloc(c, c->tileDig4, 64 * steps) && tile_alloc(c, c->tileDenInv, size_t(c->nVol))) {
             lists.dig4 = c->tileDig4.p;
             launch_tile_build(vol_dev(c), rec, k, tile_dev(c), lists, tile_all(c), 0, c->nUnique, nullptr,
                               c->tileDig4.p, c->stream);
             launch_tile_den_inv(c->nVol, c->sym.nLoop, lists, reinterpret_cast<double *>(c->tileSums.p),
                                 c->tileDenInv.p, c->stream);
-            rc = check_launch(c, "fifth digits");
+            int rc = check_launch(c, "fifth digits");
             if (rc) return rc;
             CK(cudaEventRecord(c->ev0, c->stream));
+            c->tileFifthState = 1;
+        } else {
+            c->tileDig4.release();
+            c->tileFifthState = -1;
         }
     }
     have = c->tileFifthState > 0;
@@ -1175,17 +1242,12 @@ static int ensure_tile_tangent(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, 
     int rc = ensure_tile(c, tf, rec, k, lists, use);
     if (rc || !use) return rc;
     if (lists.dig) {
-        bool have = false;
-        rc = ensure_tile_fifth(c, rec, k, lists, have);
-        if (rc) return rc;
-        if (!have) {
-            lists.dig = lists.dig3 = nullptr;
-            rc = ensure_tile_chunks(c);
-            if (rc) return rc;
-        }
+        rc = ensure_tile_fifth(c, rec, k, lists, use);
+        if (rc || !use) return rc;
+    } else {
+        use = tile_alloc(c, c->tileCDig4, c->tileCDig3.n);
     }
-    if (!lists.dig) CKA(c->tileCDig4.alloc(c->tileCDig3.n));
-    CKA(c->tileMot5.alloc(8 * (size_t(c->nUnique) + size_t(c->nNodes))));
+    use = use && tile_alloc(c, c->tileMot5, 8 * (size_t(c->nUnique) + size_t(c->nNodes)));
     return IDW_OK;
 }
 
@@ -1296,8 +1358,8 @@ static int read_counters(Ctx *c) {
     c->stats.fp64Fallback = int64_t(h[3]);
     c->stats.preciseTerms = int64_t(h[6]);
     // the lists of the walk in use
-    const int ls = c->tileState == 1 ? c->tileListState : c->listState;
-    c->stats.walkListEntries = ls > 0 ? (c->tileState == 1 ? c->tileListEntries : c->listEntries) : (ls == -1 ? -1 : 0);
+    if (c->tileState == 1) c->stats.walkListEntries = c->tileKept ? c->tileListEntries : 0;
+    else c->stats.walkListEntries = c->listState == 1 ? c->listEntries : (c->listState == -1 ? -1 : 0);
     if (c->eventsRecorded) {
         float ms = 0.f;
         if (cudaEventElapsedTime(&ms, c->ev0, c->ev1) == cudaSuccess) c->stats.lastKernelMs = ms;
@@ -1435,12 +1497,7 @@ static int run_tile_batch(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const
         bool fits = false;
         int rc = fits_half(c, double(sizeof(float4)) * per * double(sums + 8 * nTerms), fits);
         if (rc) return rc;
-        if (fits) {
-            CKA(c->bTileSums.alloc(per * sums));
-            CKA(c->bTileMot.alloc(8 * per * nTerms));
-        } else {
-            per = 1;
-        }
+        if (!fits || !tile_alloc(c, c->bTileSums, per * sums) || !tile_alloc(c, c->bTileMot, 8 * per * nTerms)) per = 1;
     }
     TileDev td = tile_dev(c);
     float4 *out = c->tileSums.p;
@@ -2691,6 +2748,18 @@ int idw_get_internal(void *ctx, const char *name, int64_t *value) {
     const std::string s(name);
     if (s == "tileSums") *value = int64_t(reinterpret_cast<intptr_t>(c->tileSums.p));
     else if (s == "tileMot") *value = int64_t(reinterpret_cast<intptr_t>(c->tileMot.p));
+    else if (s == "tileState") *value = c->tileState;
+    else if (s == "tileAllocs") *value = c->tileAllocs;
+    else return fail(c, IDW_ERR_ARG, "unknown internal value %s", name);
+    return IDW_OK;
+}
+
+int idw_set_internal(void *ctx, const char *name, int64_t value) {
+    Ctx *c = static_cast<Ctx *>(ctx);
+    if (!c || !name) return IDW_ERR_ARG;
+    const std::string s(name);
+    if (s == "tileAllocs") c->tileAllocs = value;
+    else if (s == "tileFree") c->tileFree = value;
     else return fail(c, IDW_ERR_ARG, "unknown internal value %s", name);
     return IDW_OK;
 }

@@ -240,7 +240,8 @@ struct TileDev {
 int tile_order(const VolumeDev &v, const double *lo, const double *hi, int *order, cudaStream_t st);
 void launch_tile_geo(const TreeDev &t, int nPts, const dbl4 *xa, int areaExp, float4 *geo, cudaStream_t st);
 // Fills scale, raises *bad when a node has none, fills offs and returns the number
-// of entries (-1 on a CUDA error); part: nLoop nVol floats of scratch.  Synchronises st.
+// of entries (-1 on a CUDA error, -2 without memory); part: nLoop nVol floats of
+// scratch.  Synchronises st.
 int64_t count_tile_lists(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
                          const EvalConsts &k, const TileDev &td, int64_t *offs, float *part, float *scale, int *bad,
                          cudaStream_t st);

@@ -614,8 +614,8 @@ int64_t count_tile_lists(const TreeDev &t, const TreeDevF &tf, const VolumeDev &
     void *tmp = nullptr;
     size_t tmpBytes = 0;
     int64_t total = 0;
-    bool ok = cudaMalloc(&counts, sizeof(int64_t) * (n + 1)) == cudaSuccess;
-    if (ok) ok = cudaMemsetAsync(counts + n, 0, sizeof(int64_t), st) == cudaSuccess;
+    if (cudaMalloc(&counts, sizeof(int64_t) * (n + 1)) != cudaSuccess) return -2;
+    bool room = true, ok = cudaMemsetAsync(counts + n, 0, sizeof(int64_t), st) == cudaSuccess;
     if (ok) ok = cudaMemsetAsync(bad, 0, sizeof(int), st) == cudaSuccess;
     if (ok) {
         k_tile_count<<<blocks(32 * n, 128), 128, 0, st>>>(t, tf, v, rec, mp, td, make_tile_law(k), lawExp, nGroups,
@@ -624,13 +624,13 @@ int64_t count_tile_lists(const TreeDev &t, const TreeDevF &tf, const VolumeDev &
         ok = cudaGetLastError() == cudaSuccess;
     }
     if (ok) ok = cub::DeviceScan::ExclusiveSum(nullptr, tmpBytes, counts, offs, int(n + 1), st) == cudaSuccess;
-    if (ok) ok = cudaMalloc(&tmp, tmpBytes) == cudaSuccess;
+    if (ok) ok = room = cudaMalloc(&tmp, tmpBytes) == cudaSuccess;
     if (ok) ok = cub::DeviceScan::ExclusiveSum(tmp, tmpBytes, counts, offs, int(n + 1), st) == cudaSuccess;
     if (ok) ok = cudaMemcpyAsync(&total, offs + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st) == cudaSuccess;
     if (cudaStreamSynchronize(st) != cudaSuccess) ok = false;
     if (tmp) cudaFree(tmp);
     if (counts) cudaFree(counts);
-    return ok ? total : -1;
+    return ok ? total : (room ? -1 : -2);
 }
 
 void launch_tile_record(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,

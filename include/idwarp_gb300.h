@@ -348,10 +348,11 @@ int idw_autotune(void *ctx, int32_t nsurfaces, int32_t nseeds, idw_tuning *out);
  * the denominator of the mixed walk's roofline.  No reference counterpart. */
 int idw_probe_ffma(void *stream, int device, double *tflops);
 
-/* State of a context that the library's own tests look at (buffer addresses,
- * counts), by name; not part of the interface.  IDW_ERR_ARG for a name that
- * this build does not have. */
+/* State of a context that the library's own tests look at or set (buffer
+ * addresses, states, limits), by name; not part of the interface.  IDW_ERR_ARG
+ * for a name that this build does not have. */
 int idw_get_internal(void *ctx, const char *name, int64_t *value);
+int idw_set_internal(void *ctx, const char *name, int64_t value);
 
 #ifdef __cplusplus
 }
