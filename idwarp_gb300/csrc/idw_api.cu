@@ -120,14 +120,18 @@ struct Ctx {
     bool tileOrderValid = false;
     DevBuf<int> tileOrder;
     DevBuf<float> tileScale;
-    DevBuf<float4> tileGeo, tileSums, bTileSums;
-    DevBuf<uint4> tileMot, bTileMot, tileDig, tileDig3, tileDig4;
+    DevBuf<float4> tileGeo, tileSums;
+    DevBuf<uint4> tileMot, tileDig, tileDig3, tileDig4;
     DevBuf<double> tileDenInv;
     DevBuf<unsigned> tileWord;  // 12 column maxima, the walk's counter, the bad flag
     DevBuf<int64_t> tileOffs;
     DevBuf<int> tileTerm, tileCTerm;
     DevBuf<unsigned> tileMask, tileCMask;
     DevBuf<unsigned> tileMot5;
+    DevBuf<uint4> bTileMot;  // a batch's surfaces with the lists off
+    DevBuf<unsigned> bTileWord;
+    DevBuf<float> bTileRef;
+    DevBuf<float4> bTileSums;
     DevBuf<uint4> tileCDig, tileCDig3, tileCDig4;  // scratch of one run of groups where no digits are kept
     struct TileRun {
         TileRange list, dig;
@@ -669,7 +673,7 @@ int idw_initialize_warping(void *ctx, const double *pts, int32_t npts, const dou
     CKA(c->nodeDC.alloc(12 * size_t(nn)));
     CKA(c->nodeDCl.alloc(12 * size_t(nn)));
     CKA(c->nodeDn.alloc(nn));
-    CKA(c->refDB.alloc(48));
+    CKA(c->refDB.alloc(24));
     CKA(c->ptDA.alloc(n));
     CKA(c->ptDL.alloc(n));
     CKA(c->ptDM.alloc(12 * size_t(n)));
@@ -1066,7 +1070,7 @@ static int make_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const Eval
         return IDW_OK;
     };
     if (!(tile_alloc(c, c->tileOffs, size_t(units) + 1) && tile_alloc(c, c->tileGeo, 2 * nTerms) &&
-          tile_alloc(c, c->tileMot, 8 * nTerms) && tile_alloc(c, c->tileWord, 2 * kTileWords) &&
+          tile_alloc(c, c->tileMot, 8 * nTerms) && tile_alloc(c, c->tileWord, kTileWords) &&
           tile_alloc(c, c->tileScale, size_t(c->nVol)) &&
           tile_alloc(c, c->tileSums, 2 * size_t(c->sym.nLoop) * size_t(c->nVol)) &&
           tile_alloc(c, c->tileOrder, size_t(c->nVol))))
@@ -1168,15 +1172,35 @@ static int ensure_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const Ev
     return IDW_OK;
 }
 
-// The tile walk of nb surfaces whose motion records are laid out in td, and their
-// grids; sums: 2 nLoop nVol each.
+// Surfaces whose motions are laid out in a row (kTileWords words, 24 reference
+// floats and 8 records a term each), with the sums of their walks.
+struct TileSurfaces {
+    uint4 *mot;
+    unsigned *word;
+    float *ref;
+    float4 *sums;
+    int n;
+};
+static TileSurfaces tile_one(Ctx *c) { return {c->tileMot.p, c->tileWord.p, c->refDB.p, c->tileSums.p, 1}; }
+
+// The tile walks of the surfaces, and their grids.  Runs are recorded and made once
+// for all of them.
 static int run_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalConsts &k, const TileLists &lists,
-                    const TileDev &td, float4 *sums, const WalkOut &o, int nb) {
+                    const TileSurfaces &s, const WalkOut &o) {
     const TreeDev t = tree_dev(c);
     const VolumeDev v = vol_dev(c);
+    const TileDev td = tile_dev(c);
+    const int64_t sums = 2 * int64_t(c->sym.nLoop) * c->nVol;
+    auto surface = [&](int b) {
+        TileDev d = td;
+        d.mot = s.mot + 8 * (int64_t(c->nUnique) + c->nNodes) * b;
+        d.colMax = s.word + kTileWords * b;
+        return d;
+    };
     if (lists.counters && o.counters) launch_add_walk_counters(o.counters, lists.counters, c->stream);
     if (lists.dig) {
-        launch_tile_walk(t, tf, v, rec, k, td, lists, tile_all(c), sums, c->stream, nb);
+        for (int b = 0; b < s.n; ++b)
+            launch_tile_walk(t, tf, v, rec, k, surface(b), lists, tile_all(c), s.sums + sums * b, c->stream);
     } else {
         for (const Ctx::TileRun &r : c->tileChunks) {
             TileLists l = lists;
@@ -1194,10 +1218,15 @@ static int run_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalC
                 l.dig4 = c->tileCDig4.p;
             }
             l.term += first;
-            launch_tile_walk(t, tf, v, rec, k, td, l, r.dig, sums, c->stream, nb);
+            for (int b = 0; b < s.n; ++b)
+                launch_tile_walk(t, tf, v, rec, k, surface(b), l, r.dig, s.sums + sums * b, c->stream);
         }
     }
-    launch_tile_finalize(v, rec, k, td, c->refDB.p, sums, o, c->stream, nb);
+    for (int b = 0; b < s.n; ++b) {
+        WalkOut ob = o;
+        if (o.xv) ob.xv = o.xv + 3 * c->nVol * b;
+        launch_tile_finalize(v, rec, k, td, s.ref + 24 * b, s.sums + sums * b, ob, c->stream);
+    }
     return check_launch(c, "tile walk");
 }
 
@@ -1257,7 +1286,7 @@ static int run_tile_tangent(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, con
     launch_tile_motions(tree_dev(c), c->nUnique, ptMBd, nodeMBd, c->tileWord.p, c->tileMot.p, c->tileMot5.p,
                         c->refDB.p, c->stream);
     c->nodalValid = false;
-    return run_tile(c, tf, rec, k, lists, tile_dev(c), c->tileSums.p, o, 1);
+    return run_tile(c, tf, rec, k, lists, tile_one(c), o);
 }
 
 // Before the warped grid is overwritten: if an asynchronous read of the
@@ -1317,7 +1346,7 @@ static int run_warp(Ctx *c, double *xvOut, double *denOut) {
         launch_tile_motions(tree_dev(c), c->nUnique, c->ptMB.p, c->nodeMB.p, c->tileWord.p, c->tileMot.p, nullptr,
                             c->refDB.p, c->stream);
         CK(cudaEventRecord(c->ev0, c->stream));
-        rc = run_tile(c, tf, rec, k, lists, tile_dev(c), c->tileSums.p, o, 1);
+        rc = run_tile(c, tf, rec, k, lists, tile_one(c), o);
         if (rc) return rc;
     } else if (c->opt.precision == IDW_PREC_MIXED) {
         PointsDevF pf;
@@ -1480,47 +1509,33 @@ int idw_get_volume_coordinates_cs(void *ctx, double *out, int64_t ndof, int wher
 // and a finalisation per surface.  coords/out are device pointers.
 static constexpr int kBatchWalk = kBatchMax;
 
-// run_warp_batch_mixed by tile walks, two surfaces each where the weight digits
-// stream from memory and the scratch for two is to be had.  Two surfaces have
-// motions and sums of their own: a captured graph of idw_warp_mesh keeps the
-// addresses of the single walk's.
+// run_warp_batch_mixed by tile walks, a surface each.  With the lists off they share
+// the runs where the scratch is to be had: buffers of their own, as a captured graph
+// of idw_warp_mesh keeps the addresses of the single walk's.
 static int run_tile_batch(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const EvalConsts &k, const TileLists &lists,
                           const double *coordsDev, int nb, double *outDev) {
     const int n = c->nUnique;
-    const size_t sdof = 3 * size_t(c->nPts), vdof = 3 * size_t(c->nVol);
     c->nodalValid = false;
-    const SurfaceDev s = surf_dev(c);
-    const size_t nTerms = size_t(n) + size_t(c->nNodes);
-    const size_t sums = 2 * size_t(c->sym.nLoop) * size_t(c->nVol);
-    int per = nb > 1 ? tile_batch(vol_dev(c), c->sym.nLoop) : 1;
-    if (per > 1 && (c->bTileSums.n < per * sums || c->bTileMot.n < 8 * per * nTerms)) {
-        bool fits = false;
-        int rc = fits_half(c, double(sizeof(float4)) * per * double(sums + 8 * nTerms), fits);
-        if (rc) return rc;
-        if (!fits || !tile_alloc(c, c->bTileSums, per * sums) || !tile_alloc(c, c->bTileMot, 8 * per * nTerms)) per = 1;
-    }
-    TileDev td = tile_dev(c);
-    float4 *out = c->tileSums.p;
-    uint4 *mot = c->tileMot.p;
-    if (per > 1) {
-        out = c->bTileSums.p;
-        td.mot = mot = c->bTileMot.p;
-    }
+    const size_t nTerms = size_t(n) + size_t(c->nNodes), sums = 2 * size_t(c->sym.nLoop) * size_t(c->nVol);
+    TileSurfaces s = tile_one(c);
+    if (!lists.dig && nb > 1 && tile_alloc(c, c->bTileMot, nb * 8 * nTerms) &&
+        tile_alloc(c, c->bTileWord, nb * kTileWords) && tile_alloc(c, c->bTileRef, nb * 24) &&
+        tile_alloc(c, c->bTileSums, nb * sums))
+        s = {c->bTileMot.p, c->bTileWord.p, c->bTileRef.p, c->bTileSums.p, nb};
     CK(cudaEventRecord(c->ev0, c->stream));
-    for (int b0 = 0; b0 < nb; b0 += per) {
-        const int m = std::min(per, nb - b0);
-        for (int b = 0; b < m; ++b) {
-            launch_gather_xu(n, c->xuInd.p, coordsDev + size_t(b0 + b) * sdof, c->xu.p, c->stream);
-            launch_nodal(s, c->xu.p, c->ptXA.p, c->normals0.p, c->tmpAi.p, c->isCorner.p, c->opt.useRotations,
-                         c->ptMB.p, c->stream);
+    for (int b0 = 0; b0 < nb; b0 += s.n) {
+        for (int b = 0; b < s.n; ++b) {
+            launch_gather_xu(n, c->xuInd.p, coordsDev + size_t(b0 + b) * 3 * size_t(c->nPts), c->xu.p, c->stream);
+            launch_nodal(surf_dev(c), c->xu.p, c->ptXA.p, c->normals0.p, c->tmpAi.p, c->isCorner.p,
+                         c->opt.useRotations, c->ptMB.p, c->stream);
             launch_set_data(tree_dev(c), n, c->ptMB.p, c->nodeMB.p, c->nodeSum.p, c->stream);
-            launch_tile_motions(tree_dev(c), n, c->ptMB.p, c->nodeMB.p, c->tileWord.p + kTileWords * b,
-                                mot + 8 * nTerms * b, nullptr, c->refDB.p + 24 * b, c->stream);
+            launch_tile_motions(tree_dev(c), n, c->ptMB.p, c->nodeMB.p, s.word + kTileWords * b, s.mot + 8 * nTerms * b,
+                                nullptr, s.ref + 24 * b, c->stream);
         }
         WalkOut o;
-        o.xv = outDev + size_t(b0) * vdof;
+        o.xv = outDev + size_t(b0) * 3 * size_t(c->nVol);
         o.counters = b0 == 0 ? c->counters.p : nullptr;
-        int rc = run_tile(c, tf, rec, k, lists, td, out, o, m);
+        int rc = run_tile(c, tf, rec, k, lists, s, o);
         if (rc) return rc;
     }
     CK(cudaEventRecord(c->ev1, c->stream));

@@ -224,7 +224,7 @@ struct TileLists {
     const uint4 *dig4 = nullptr;    // per step 64: the fifth, for reverse products and tangents
     const unsigned long long *counters = nullptr;  // the recording walk's, as WalkLists::counters
 };
-constexpr int kTileWords = 16;  // per surface of a batch: 12 column maxima (and the walk's counter, a flag)
+constexpr int kTileWords = 16;  // 12 column maxima, the walk's counter, a flag
 struct TileDev {
     const int *order;        // tile slot -> walk (Morton) index of a volume node
     const float *scale;      // per slot: power-of-two weight scale P
@@ -261,17 +261,13 @@ void launch_tile_build(const VolumeDev &v, const WalkRecF &rec, const EvalConsts
 // reference motion; with mot5 a tangent's (Md, bd).
 void launch_tile_motions(const TreeDev &t, int nPts, const double *ptMB, const double *nodeMB, unsigned *colMax,
                          uint4 *mot, unsigned *mot5, float *refDB, cudaStream_t st);
-// The range's sums of nb surfaces (sums: 2 nLoop nVol float4 each), then their grids
-// (o.xv in a row) and denominators.  With lists.dig4 the motions are a tangent's
-// (td.mot5, nb = 1).
+// The range's sums (2 nLoop nVol float4), then the grid (o.xv) and the
+// denominators.  With lists.dig4 the motions are a tangent's (td.mot5).
 void launch_tile_walk(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
                       const EvalConsts &k, const TileDev &td, const TileLists &lists, const TileRange &range,
-                      float4 *sums, cudaStream_t st, int nb = 1);
+                      float4 *sums, cudaStream_t st);
 void launch_tile_finalize(const VolumeDev &v, const WalkRecF &rec, const EvalConsts &k, const TileDev &td,
-                          const float *refDB, const float4 *sums, const WalkOut &o, cudaStream_t st, int nb = 1);
-// Surfaces that one tile walk takes (launch_tile_walk's nb): 2 where the digits
-// stream from memory.
-int tile_batch(const VolumeDev &v, int nLoop);
+                          const float *refDB, const float4 *sums, const WalkOut &o, cudaStream_t st);
 int tile_sms();
 // Reverse product from the kept digits (idw_tile_adjoint.cu).  denInv: per slot
 // the reciprocal denominator in the digits' units; part: nLoop * nVol doubles of

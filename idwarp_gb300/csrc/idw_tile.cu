@@ -7,17 +7,19 @@
 // r once, at the end) and sum_t w_t e_t: a product of the weights (32 nodes x
 // terms) with the terms' motions (terms x 12) and a column of ones for the
 // denominator.  The weights depend on set-up state and the weight law only, so
-// they are formed once per mesh, in double-float, and kept as FP16 digits in
-// operand layout (8 bytes per node and term); a walk streams the first three
-// digits and multiplies them with the motions' three.  The leading products sum
-// exactly in the FP32 accumulators and the next ones in compensated pairs, so
-// the sums carry about 2^-32 of the denominator and the largest motion; no term
-// needs a second evaluation, however large its weight.
+// they are formed once per mesh, in double-float, and kept as four FP16 digits in
+// operand layout (8 bytes per node and term); a walk streams them and multiplies
+// them with the motions' four.  The leading products sum exactly in the FP32
+// accumulators and the next ones in compensated pairs, so the sums carry about 2^-44
+// of the denominator and the largest motion; no term needs a second evaluation,
+// however large its weight.  Three digits of both are a quarter less to stream
+// (245k-node wing 235 against 258 us, 8M nodes 5.9 against 7.3 ms), but then the nodes
+// beside the surface, which one term carries, and the far field are 1e-10 of the
+// largest motion off where the double-float terms of the gated walk leave 1e-14.
 //
 // The terms are those of the reference's decisions (decide32 + resolve64, as
-// k_walk_record), recorded once per den0, errTol and law.  Without room for the
-// digits or (walkLists off) the lists a walk makes them for a run of groups at a
-// time; every form gives the same bits.
+// k_walk_record), recorded once per den0, errTol and law.  With walkLists off a walk
+// makes lists and digits for a run of groups at a time; both give the same bits.
 #include <climits>
 #include <type_traits>
 
@@ -32,12 +34,6 @@ namespace {
 
 constexpr int kScaleExp = 13;   // node denominators are scaled to [2^13, 2^14)
 constexpr int kMotExp = 14;     // motions are scaled to at most 2^14
-// Node images up to which a warp uses four digits: there they cost little (95k
-// nodes 12 us of a forward and reverse of 490, 7k nodes 2 us) and bring the error
-// from 1e-11 to 1e-14; beyond, a quarter more to stream (245k nodes 234 -> 259 us,
-// 8M 5.9 -> 7.3 ms).
-constexpr int64_t kFourDigits = int64_t(1) << 17;
-
 inline int blocks(int64_t n, int b) { return int((n + b - 1) / b); }
 
 // ---- set-up: node order, term geometry, scales, lists, digits ----
@@ -381,25 +377,22 @@ __global__ void k_tile_mot(TreeDev t, int nPts, const double *ptMB, const double
 
 // ---- the walk ----
 
-// Warps of a block at nb surfaces (one block per SM): 16 at 128 registers, where
-// a walk of one surface waits for its copies (245k-node wing 243 -> 236 us against
-// 12 warps at 144 registers, 8M nodes 6.05 -> 5.94 ms; a third stage for 12 warps
-// is worth 0.13 ms there).  Two surfaces share a step's digits at 12 warps: 2.3 ms
-// a pair on the 2M-node wing, twice 1.33 alone; ten warps with three stages take
-// 3.2 ms.
-constexpr int tile_warps(int nd, int nb) { return nd < 5 && nb == 1 ? 16 : 12; }
-// Shared memory of a stage: nd digits and nb surfaces' motions (a tangent's fifth
-// digits last).
-constexpr size_t tile_stage_bytes(int nd, int nb) {
-    return sizeof(uint4) * ((nd == 5 ? 10 : 8) * kTileTerms * nb + 64 * nd);
-}
+// Warps of a block (one block per SM): 16 at 128 registers, where a walk waits for
+// its copies (three digits, 245k-node wing, 243 -> 236 us against 12 warps at 144
+// registers); a tangent needs 166 registers.  Two surfaces sharing a step's digits,
+// at 12 or 10 warps, spill beside four digits: eight surfaces on the 2M-node wing 17.0
+// and 16.3 ms against 13.9 one at a time.
+constexpr int tile_warps(int nd) { return nd < 5 ? 16 : 12; }
+// Shared memory of a stage: nd digits and the motions (a tangent's fifth digits
+// last).
+constexpr size_t tile_stage_bytes(int nd) { return sizeof(uint4) * ((nd == 5 ? 10 : 8) * kTileTerms + 64 * nd); }
 
 // The sums of one unit per warp: numerators about the reference motion and
-// denominator of each node, as pairs (high, low), into out, for NB surfaces
-// (td.mot, td.colMax and out in a row).  The weight digits stream from memory,
-// the next step's copied while one is computed.
-template <int ND, int NB>
-__global__ void __launch_bounds__(32 * tile_warps(ND, NB), 1)
+// denominator of each node, as pairs (high, low), into out.  The weight digits
+// stream from memory, the next step's copied while one is computed.  ND: 4, or 5
+// for a tangent.
+template <int ND>
+__global__ void __launch_bounds__(32 * tile_warps(ND), 1)
     k_tile_walk(TreeDev t, TreeDevF tf, VolumeDev v, WalkRecF rec, MixedParams mp, TileDev td, TileLists lists,
                 TileRange range, unsigned chunk, float4 *out) {
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -407,20 +400,18 @@ __global__ void __launch_bounds__(32 * tile_warps(ND, NB), 1)
     if (threadIdx.x == 0) qstate = 0ull;
     __syncthreads();
     const int lane = threadIdx.x & 31, g = lane >> 2, a = lane & 3;
-    constexpr size_t stageBytes = tile_stage_bytes(ND, NB);
+    constexpr size_t stageBytes = tile_stage_bytes(ND);
     unsigned char *mine = smraw + 2 * stageBytes * (threadIdx.x >> 5);
-    const int64_t nTerms = tf.nPts + t.nNodes;
     auto motions = [&](int s) { return reinterpret_cast<uint4 *>(mine + stageBytes * (s & 1)); };
-    auto digits = [&](int s) { return motions(s) + 8 * kTileTerms * NB; };
+    auto digits = [&](int s) { return motions(s) + 8 * kTileTerms; };
     UnitQueue queue = {&qstate, td.counter, unsigned((range.group1 - range.group0) * mp.nLoop), chunk, 0u, 0u};
     unsigned idx;
     while (queue.next(idx)) {
         const int64_t group = range.group0 + idx / unsigned(mp.nLoop);
         const int kk = int(idx % unsigned(mp.nLoop));
         const int64_t unit = group * mp.nLoop + kk;
-        TileAcc<ND> acc[NB];
-#pragma unroll
-        for (int b = 0; b < NB; ++b) tile_zero(acc[b]);
+        TileAcc<ND> acc;
+        tile_zero(acc);
         const int64_t e0 = lists.offs[unit] - range.entry0;
         const int n = int((lists.offs[unit + 1] - range.entry0 - e0) / kTileTerms);
         const int *term = lists.term + e0;
@@ -432,13 +423,9 @@ __global__ void __launch_bounds__(32 * tile_warps(ND, NB), 1)
             uint4 *dst = digits(s);
 #pragma unroll
             for (int c = 0; c < 6; ++c) cp_async16(dst + 32 * c + lane, dig + 192 * int64_t(s) + 32 * c + lane);
-            if constexpr (ND > 3) {
 #pragma unroll
-                for (int c = 0; c < 2; ++c)
-                    cp_async16(dst + 192 + 32 * c + lane, dig3 + 64 * int64_t(s) + 32 * c + lane);
-            }
-#pragma unroll
-            for (int b = 0; b < NB; ++b) stage_motions(motions(s) + 8 * kTileTerms * b, ids, td.mot + 8 * nTerms * b);
+            for (int c = 0; c < 2; ++c) cp_async16(dst + 192 + 32 * c + lane, dig3 + 64 * int64_t(s) + 32 * c + lane);
+            stage_motions(motions(s), ids, td.mot);
             if constexpr (ND == 5) {
 #pragma unroll
                 for (int c = 0; c < 2; ++c)
@@ -462,7 +449,7 @@ __global__ void __launch_bounds__(32 * tile_warps(ND, NB), 1)
             cp_async_wait<1>();
             __syncwarp();
             if constexpr (ND == 5)
-                tile_step5(digits(s), motions(s), reinterpret_cast<const unsigned *>(digits(s) + 320), acc[0]);
+                tile_step5(digits(s), motions(s), reinterpret_cast<const unsigned *>(digits(s) + 320), acc);
             else
                 tile_step(digits(s), motions(s), acc);
             __syncwarp();
@@ -470,45 +457,42 @@ __global__ void __launch_bounds__(32 * tile_warps(ND, NB), 1)
         cp_async_wait<0>();
         // component a of the numerator: D'_a . (r - O) + e_a; lane column 3: the denominator
         const float4 oh = ldgf4(td.geo + 2 * int64_t(tf.nPts)), ol = ldgf4(td.geo + 2 * int64_t(tf.nPts) + 1);
+        float cs[4];
 #pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            float cs[4];
+        for (int k = 0; k < 4; ++k)
+            cs[k] = a < 3 ? pow2f(-column_exp(__ldg(td.colMax + 4 * a + k))) : 0.125f;
+        float *o = reinterpret_cast<float *>(out);
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-                cs[k] = a < 3 ? pow2f(-column_exp(__ldg(td.colMax + kTileWords * b + 4 * a + k))) : 0.125f;
-            float *o = reinterpret_cast<float *>(out + 2 * int64_t(mp.nLoop) * v.nVol * b);
+        for (int m = 0; m < 2; ++m)
 #pragma unroll
-            for (int m = 0; m < 2; ++m)
+            for (int r = 0; r < 2; ++r) {
+                const int64_t slot = group * 32 + g + 16 * m + 8 * r;
+                if (slot >= v.nVol) continue;
+                dfl M[4];
 #pragma unroll
-                for (int r = 0; r < 2; ++r) {
-                    const int64_t slot = group * 32 + g + 16 * m + 8 * r;
-                    if (slot >= v.nVol) continue;
-                    dfl M[4];
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        // columns in the order of the motion records: D'_a0, D'_a1 | D'_a2, e_a
-                        float s, low;
-                        tile_total(acc[b], m, k >> 1, r, k & 1, s, low);
-                        M[k] = df_norm(s * cs[k], low * cs[k]);
-                    }
-                    const int64_t gid = kk * v.nVol + td.order[slot];
-                    const float4 hi = rec.hi[gid], lo = rec.lo[gid];
-                    const float h[3] = {hi.x, hi.y, hi.z}, l[3] = {lo.x, lo.y, lo.z};
-                    const float oh3[3] = {oh.x, oh.y, oh.z}, ol3[3] = {ol.x, ol.y, ol.z};
-                    dfl s = M[3];
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) {
-                        dfl x;
-                        two_diff(h[k], oh3[k], x.h, x.l);
-                        x.l += l[k] - ol3[k];
-                        s = df_add(s, df_mul(M[k], df_norm(x.h, x.l)));
-                    }
-                    if (a == 3) s = M[0];
-                    float *p = o + 8 * (kk * v.nVol + slot);
-                    p[a] = s.h;
-                    p[4 + a] = s.l;
+                for (int k = 0; k < 4; ++k) {
+                    // columns in the order of the motion records: D'_a0, D'_a1 | D'_a2, e_a
+                    float s, low;
+                    tile_total(acc, m, k >> 1, r, k & 1, s, low);
+                    M[k] = df_norm(s * cs[k], low * cs[k]);
                 }
-        }
+                const int64_t gid = kk * v.nVol + td.order[slot];
+                const float4 hi = rec.hi[gid], lo = rec.lo[gid];
+                const float h[3] = {hi.x, hi.y, hi.z}, l[3] = {lo.x, lo.y, lo.z};
+                const float oh3[3] = {oh.x, oh.y, oh.z}, ol3[3] = {ol.x, ol.y, ol.z};
+                dfl s = M[3];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    dfl x;
+                    two_diff(h[k], oh3[k], x.h, x.l);
+                    x.l += l[k] - ol3[k];
+                    s = df_add(s, df_mul(M[k], df_norm(x.h, x.l)));
+                }
+                if (a == 3) s = M[0];
+                float *p = o + 8 * (kk * v.nVol + slot);
+                p[a] = s.h;
+                p[4 + a] = s.l;
+            }
     }
 }
 
@@ -598,8 +582,6 @@ void launch_tile_motions(const TreeDev &t, int nPts, const double *ptMB, const d
     k_tile_mot<<<blocks(n, 256), 256, 0, st>>>(t, nPts, ptMB, nodeMB, colMax, mot, mot5, refDB);
 }
 
-int tile_batch(const VolumeDev &v, int nLoop) { return v.nVol * nLoop > kFourDigits ? 2 : 1; }
-
 int64_t count_tile_lists(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
                          const EvalConsts &k, const TileDev &td, int64_t *offs, float *part, float *scale, int *bad,
                          cudaStream_t st) {
@@ -653,43 +635,38 @@ void launch_tile_build(const VolumeDev &v, const WalkRecF &rec, const EvalConsts
         v, rec, mp, td, lists, make_tile_law(k), nPts, range, listEntry0, dig, dig3);
 }
 
-template <int ND, int NB>
+template <int ND>
 static void walk_digits(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
                         const MixedParams &mp, const TileDev &td, const TileLists &lists, const TileRange &range,
                         float4 *sums, cudaStream_t st) {
-    constexpr int warps = tile_warps(ND, NB);
+    constexpr int warps = tile_warps(ND);
     const int64_t units = (range.group1 - range.group0) * mp.nLoop;
     const int sms = tile_sms(), grid = int(min(int64_t(sms), (units + warps - 1) / warps));
     const unsigned chunk = unsigned(max(int64_t(1), min(int64_t(32), units / (4 * sms * warps))));
-    const size_t smem = warps * 2 * tile_stage_bytes(ND, NB);
+    const size_t smem = warps * 2 * tile_stage_bytes(ND);
     cudaMemsetAsync(td.counter, 0, sizeof(unsigned), st);
-    cudaFuncSetAttribute(k_tile_walk<ND, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    k_tile_walk<ND, NB><<<grid, 32 * warps, smem, st>>>(t, tf, v, rec, mp, td, lists, range, chunk, sums);
+    cudaFuncSetAttribute(k_tile_walk<ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    k_tile_walk<ND><<<grid, 32 * warps, smem, st>>>(t, tf, v, rec, mp, td, lists, range, chunk, sums);
 }
 
 void launch_tile_walk(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
                       const EvalConsts &k, const TileDev &td, const TileLists &lists, const TileRange &range,
-                      float4 *sums, cudaStream_t st, int nb) {
+                      float4 *sums, cudaStream_t st) {
     if (range.group1 <= range.group0) return;
     const MixedParams mp = make_mixed_params(k);
-    if (lists.dig4) walk_digits<5, 1>(t, tf, v, rec, mp, td, lists, range, sums, st);
-    else if (nb == 2) walk_digits<3, 2>(t, tf, v, rec, mp, td, lists, range, sums, st);
-    else if (v.nVol * mp.nLoop <= kFourDigits) walk_digits<4, 1>(t, tf, v, rec, mp, td, lists, range, sums, st);
-    else walk_digits<3, 1>(t, tf, v, rec, mp, td, lists, range, sums, st);
+    if (lists.dig4) walk_digits<5>(t, tf, v, rec, mp, td, lists, range, sums, st);
+    else walk_digits<4>(t, tf, v, rec, mp, td, lists, range, sums, st);
 }
 
 void launch_tile_finalize(const VolumeDev &v, const WalkRecF &rec, const EvalConsts &k, const TileDev &td,
-                          const float *refDB, const float4 *sums, const WalkOut &o, cudaStream_t st, int nb) {
+                          const float *refDB, const float4 *sums, const WalkOut &o, cudaStream_t st) {
     if (v.nVol <= 0) return;
     const MixedParams mp = make_mixed_params(k);
     const double L = k.law.Ldef;
-    for (int b = 0; b < nb; ++b) {
-        NodeAggF af{};
-        af.ref = refDB + 24 * b;
-        k_tile_finalize<<<blocks(v.nVol, 128), 128, 0, st>>>(v, rec, af, mp, td, sums + 2 * mp.nLoop * v.nVol * b,
-                                                             ldexp(L * L * L, -td.areaExp),
-                                                             o.tangent, o.xv ? o.xv + 3 * v.nVol * b : nullptr, o.den);
-    }
+    NodeAggF af{};
+    af.ref = refDB;
+    k_tile_finalize<<<blocks(v.nVol, 128), 128, 0, st>>>(v, rec, af, mp, td, sums, ldexp(L * L * L, -td.areaExp),
+                                                         o.tangent, o.xv, o.den);
 }
 
 }  // namespace idw

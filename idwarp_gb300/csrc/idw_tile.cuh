@@ -279,15 +279,13 @@ __device__ __forceinline__ void stage_weights(TileStage &st, const float4 *geo, 
     }
 }
 
-// Accumulators of one unit: per 16-node tile and 8-column tile, the products of
-// the first digits (exact: first digits on grids of 8, below 2^14 in sum), the
-// products one digit down (a compensated pair), and the rest; with four digits
-// also 2^22 times the products with a fourth digit.
+// Accumulators of one unit, four digits: per 16-node tile and 8-column tile, the
+// products of the first digits (exact: first digits on grids of 8, below 2^14 in
+// sum), the products one digit down (a compensated pair), and the rest.
 template <int ND>
 struct TileAcc {
     float a0[2][2][4], a2[2][2][4];
     float2 a1[2][2][2];
-    float a3[ND > 3 ? 2 : 1][ND > 3 ? 2 : 1][4];
 };
 template <int ND>
 __device__ __forceinline__ void tile_zero(TileAcc<ND> &acc) {
@@ -297,10 +295,7 @@ __device__ __forceinline__ void tile_zero(TileAcc<ND> &acc) {
         for (int n = 0; n < 2; ++n) {
             acc.a1[m][n][0] = acc.a1[m][n][1] = make_float2(0.f, 0.f);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                acc.a0[m][n][j] = acc.a2[m][n][j] = 0.f;
-                if (ND > 3) acc.a3[m][n][j] = 0.f;
-            }
+            for (int j = 0; j < 4; ++j) acc.a0[m][n][j] = acc.a2[m][n][j] = 0.f;
         }
 }
 
@@ -338,65 +333,53 @@ __device__ __forceinline__ void tile_total(const TileAcc<ND> &acc, int m, int n,
         low = e + (e2 + fmaf(acc.a4[m][n][2 * r + k], 1.0f / 4194304.0f, acc.a3[m][n][2 * r + k]));
     } else {
         low = e + acc.a2[m][n][2 * r + k];
-        if constexpr (ND > 3) low = fmaf(acc.a3[m][n][2 * r + k], 1.0f / 4194304.0f, low);
     }
 }
 
-// One step of the forward sums with ND digits of the weights and of NB surfaces'
-// motions (dig: digit d of 16-node tile m as the lanes' fragment registers at 64 d
-// + 32 m; mot: each surface's records of the step).
-template <int ND, int NB>
-__device__ __forceinline__ void tile_step(const uint4 *dig, const uint4 *mot, TileAcc<ND> (&accs)[NB]) {
+// One step of the forward sums with four digits of the weights and of the motions
+// (dig: digit d of 16-node tile m as the lanes' fragment registers at 64 d + 32 m;
+// mot: the motion records of the step).
+__device__ __forceinline__ void tile_step(const uint4 *dig, const uint4 *mot, TileAcc<4> &acc) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
-        // motion digits of the lane's terms: [surface][digit][fragment register]
-        unsigned B[NB][ND][2];
+        // motion digits of the lane's terms: [digit][fragment register]
+        unsigned C[4][2];
 #pragma unroll
-        for (int b = 0; b < NB; ++b)
-#pragma unroll
-            for (int p = 0; p < 2; ++p) {
-                const uint2 *q =
-                    reinterpret_cast<const uint2 *>(mot + 8 * kTileTerms * b + 8 * (4 * t + 2 * p) + (g ^ (2 * t))) + n;
-                const uint2 x = q[0], y = q[16];
-                B[b][0][p] = __byte_perm(x.x, y.x, 0x5410);
-                B[b][1][p] = __byte_perm(x.x, y.x, 0x7632);
-                B[b][2][p] = __byte_perm(x.y, y.y, 0x5410);
-                if constexpr (ND > 3) B[b][3][p] = __byte_perm(x.y, y.y, 0x7632);
-            }
+        for (int p = 0; p < 2; ++p) {
+            const uint2 *q = reinterpret_cast<const uint2 *>(mot + 8 * (4 * t + 2 * p) + (g ^ (2 * t))) + n;
+            const uint2 x = q[0], y = q[16];
+            C[0][p] = __byte_perm(x.x, y.x, 0x5410);
+            C[1][p] = __byte_perm(x.x, y.x, 0x7632);
+            C[2][p] = __byte_perm(x.y, y.y, 0x5410);
+            C[3][p] = __byte_perm(x.y, y.y, 0x7632);
+        }
 #pragma unroll
         for (int m = 0; m < 2; ++m) {
-            const uint4 A0 = dig[32 * m + lane], A1 = dig[64 + 32 * m + lane], A2 = dig[128 + 32 * m + lane];
-            uint4 A3 = make_uint4(0u, 0u, 0u, 0u);
-            if constexpr (ND > 3) A3 = dig[192 + 32 * m + lane];
+            const uint4 *A = dig + 32 * m + lane;
+            const uint4 A0 = A[0], A1 = A[64], A2 = A[128], A3 = A[192];
+            // one digit down: exact in a step (the tensor core truncates its sums,
+            // which over a list would be a bias), added by two-sums whose errors
+            // join the rest; f: 2^22 times the products with a fourth digit
+            float d[4], f[4];
+            mma_f16_first(d, A0, C[1][0], C[1][1]);
+            mma_f16_first(f, A0, C[3][0], C[3][1]);
+            mma_f16(acc.a0[m][n], A0, C[0][0], C[0][1]);
+            mma_f16(acc.a2[m][n], A1, C[1][0], C[1][1]);
+            mma_f16(d, A1, C[0][0], C[0][1]);
+            mma_f16(f, A3, C[0][0], C[0][1]);
+            mma_f16(acc.a2[m][n], A0, C[2][0], C[2][1]);
+            mma_f16(acc.a2[m][n], A2, C[0][0], C[0][1]);
+            mma_f16(acc.a2[m][n], A1, C[2][0], C[2][1]);
+            mma_f16(acc.a2[m][n], A2, C[1][0], C[1][1]);
 #pragma unroll
-            for (int b = 0; b < NB; ++b) {
-                TileAcc<ND> &acc = accs[b];
-                const unsigned(&C)[ND][2] = B[b];
-                mma_f16(acc.a0[m][n], A0, C[0][0], C[0][1]);
-                // one digit down: exact in a step (the tensor core truncates its
-                // sums, which over a list would be a bias), added by two-sums whose
-                // errors join the rest
-                float d[4];
-                mma_f16_first(d, A0, C[1][0], C[1][1]);
-                mma_f16(d, A1, C[0][0], C[0][1]);
-                mma_f16(acc.a2[m][n], A1, C[1][0], C[1][1]);
-                mma_f16(acc.a2[m][n], A0, C[2][0], C[2][1]);
-                mma_f16(acc.a2[m][n], A2, C[0][0], C[0][1]);
-                if constexpr (ND > 3) {
-                    mma_f16(acc.a2[m][n], A1, C[2][0], C[2][1]);
-                    mma_f16(acc.a2[m][n], A2, C[1][0], C[1][1]);
-                    mma_f16(acc.a3[m][n], A0, C[3][0], C[3][1]);
-                    mma_f16(acc.a3[m][n], A3, C[0][0], C[0][1]);
-                }
-#pragma unroll
-                for (int r = 0; r < 2; ++r) {
-                    float2 s, e;
-                    two_sum2(acc.a1[m][n][r], make_float2(d[2 * r], d[2 * r + 1]), s, e);
-                    acc.a1[m][n][r] = s;
-                    acc.a2[m][n][2 * r] += e.x;
-                    acc.a2[m][n][2 * r + 1] += e.y;
-                }
+            for (int r = 0; r < 2; ++r) {
+                float2 s, e;
+                two_sum2(acc.a1[m][n][r], make_float2(d[2 * r], d[2 * r + 1]), s, e);
+                acc.a1[m][n][r] = s;
+                e = fma2(make_float2(f[2 * r], f[2 * r + 1]), dup2(1.0f / 4194304.0f), e);
+                acc.a2[m][n][2 * r] += e.x;
+                acc.a2[m][n][2 * r + 1] += e.y;
             }
         }
     }

@@ -48,17 +48,18 @@ def close(a, b, L):
 
 
 @pytest.mark.parametrize("lists,basic", [("auto", 12), ("off", 7)])
-@pytest.mark.parametrize("allowed", range(17))
+@pytest.mark.parametrize("allowed", range(19))
 def test_refused_allocations(built_lib, lists, basic, allowed):
     """The gated walk serves until the tile walk's own memory is there (`basic`
     allocations; off: its runs need four more), the double-float reverse product and
-    the gated tangent until the fifth digits' is."""
+    the gated tangent until the fifth digits' is; with the lists off a batch that
+    cannot have its four buffers goes surface by surface."""
     m = wing_small()
     f, g = build_gpu(m, precision="fp64"), build_gpu(m, {"walkLists": lists}, precision="mixed")
     limit(g, "tileAllocs", allowed)
     close(calls(g, m), calls(f, m), f.getStats()["Ldef0"])
     assert internal(g, "tileState") == (1 if allowed >= basic else -1)
-    assert internal(g, "tileAllocs") == max(0, allowed - (15 if lists == "auto" else 13))
+    assert internal(g, "tileAllocs") == max(0, allowed - (15 if lists == "auto" else 17))
 
 
 def test_refused_allocations_after_an_errtol_change(built_lib):
@@ -90,11 +91,9 @@ def test_digits_beyond_half_of_the_free_memory(built_lib):
 
 
 def test_a_batch_leaves_the_buffers_of_single_warps(built_lib):
-    """A captured graph of a warp holds their addresses.  Above 2^17 node images a
-    batch takes two surfaces a walk."""
+    """A captured graph of a warp holds their addresses."""
     m = S.wing_shell(121, 41, 16)
     g = build_gpu(m, {"errTol": 1e-3}, precision="mixed")
-    assert 2 * g.nVol > 2**17
     g.setSurfaceCoordinates(m["pts"])
     g.warpMesh()
     before = [internal(g, k) for k in ("tileSums", "tileMot")]
