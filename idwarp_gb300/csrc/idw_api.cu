@@ -44,6 +44,9 @@ struct DevBuf {
     }
 };
 
+// Steps of the tile walks' runs (ensure_tile_runs).
+constexpr int64_t kListSteps = int64_t(1) << 22, kDigitSteps = int64_t(1) << 19;
+
 struct Ctx {
     int device = 0;
     idw_options opt{};      // options now in force
@@ -145,8 +148,9 @@ struct Ctx {
     bool tileDigits = false; // tileKept: the digits are the current law's
     int64_t tileListEntries = 0;
     // for the tests: allocations that the tile walks may still make (-1: any
-    // number), free bytes that they reckon with (-1: the device's)
+    // number), free bytes that they reckon with (-1: the device's), lengths of runs
     int64_t tileAllocs = -1, tileFree = -1;
+    int64_t tileListSteps = kListSteps, tileDigitSteps = kDigitSteps;
     double tileErrTol = 0.0, tileLdefFact = 0.0, tileAlphaToB = 0.0;
     // adjoint
     DevBuf<double> ptAdj, nodeAdj, xub, dxs;
@@ -1003,7 +1007,6 @@ static TileRange tile_all(const Ctx *c) {
 // kDigitSteps (4 kB each), or one group.  Recorded, made and walked apart, at full
 // occupancy each: formed within the walk they took 12.1 instead of 7.9 ms on the
 // 2M-node wing.  A short list run still takes one warp's traversal (0.4 ms).
-constexpr int64_t kListSteps = int64_t(1) << 22, kDigitSteps = int64_t(1) << 19;
 
 // The runs and their scratch, halved until it is to be had (tileRunState).
 static int ensure_tile_runs(Ctx *c) {
@@ -1023,8 +1026,8 @@ static int ensure_tile_runs(Ctx *c) {
         r.group1 = g;
         return r;
     };
-    int64_t listCap = std::max(widest, std::min(kListSteps, offs.back() / 16));
-    int64_t digCap = std::max(widest, std::min(kDigitSteps, offs.back() / 16));
+    int64_t listCap = std::max(widest, std::min(c->tileListSteps, offs.back() / 16));
+    int64_t digCap = std::max(widest, std::min(c->tileDigitSteps, offs.back() / 16));
     while (!(tile_alloc(c, c->tileCTerm, 16 * size_t(listCap)) && tile_alloc(c, c->tileCMask, 16 * size_t(listCap)) &&
              tile_alloc(c, c->tileCDig, 192 * size_t(digCap)) && tile_alloc(c, c->tileCDig3, 64 * size_t(digCap)))) {
         drop_tile_runs(c);
@@ -2765,6 +2768,11 @@ int idw_get_internal(void *ctx, const char *name, int64_t *value) {
     else if (s == "tileMot") *value = int64_t(reinterpret_cast<intptr_t>(c->tileMot.p));
     else if (s == "tileState") *value = c->tileState;
     else if (s == "tileAllocs") *value = c->tileAllocs;
+    else if (s == "tileDigitRuns") *value = int64_t(c->tileChunks.size());
+    else if (s == "tileListRuns") {
+        *value = 0;
+        for (const Ctx::TileRun &r : c->tileChunks) *value += r.dig.group0 == r.list.group0;
+    }
     else return fail(c, IDW_ERR_ARG, "unknown internal value %s", name);
     return IDW_OK;
 }
@@ -2775,6 +2783,8 @@ int idw_set_internal(void *ctx, const char *name, int64_t value) {
     const std::string s(name);
     if (s == "tileAllocs") c->tileAllocs = value;
     else if (s == "tileFree") c->tileFree = value;
+    else if (s == "tileListSteps") c->tileListSteps = value;
+    else if (s == "tileDigitSteps") c->tileDigitSteps = value;
     else return fail(c, IDW_ERR_ARG, "unknown internal value %s", name);
     return IDW_OK;
 }
