@@ -929,17 +929,19 @@ static int ensure_gate_den(Ctx *c, const TreeDevF &tf, const PointsDevF &pf, con
 // The tile walks serve the fast mixed walk at the default exponents and the
 // default precision gate (or a looser one: their error is below the gate's).
 // A tighter gate asks for terms in double-float, which the gated walks have.
-// The FP32 reverse product (IDW_ADJ_FAST) divides by the gated walk's
-// denominators, so its forward walk stays the gated one, and so do the
-// diagnostics.  Three symmetry planes (8 mirror images) bound the scratch, and
-// kTileMost node images the weight digits (2.4 kB each, 3 kB with the fifth); both limits
-// apply with the lists on and off, so the results agree.
+// Their digits take every weight to be positive and no larger than its node's
+// denominator: a negative alpha has the gated walks.  So have the FP32 reverse product
+// (IDW_ADJ_FAST) with its forward walk, and the diagnostics.  Three symmetry planes
+// (8 mirror images) bound the scratch, and kTileMost node images the weight digits
+// (2.4 kB each, 3 kB with the fifth); both limits apply with the lists on and off, so
+// the results agree.
 constexpr int64_t kTileMost = int64_t(1) << 25;
 
 static bool tile_applies(const Ctx *c, const EvalConsts &k) {
     return c->opt.precision == IDW_PREC_MIXED && c->opt.evalMode == IDW_EVAL_FAST &&
            c->opt.adjointPrecision == IDW_ADJ_PRECISE && c->opt.mixedGate >= 2e-3 && k.law.isInt && k.law.ia == 3 &&
-           k.law.ib == 5 && !k.slotStats && c->sym.nLoop <= 8 && c->nVol > 0 && c->nVol * c->sym.nLoop <= kTileMost;
+           k.law.ib == 5 && k.law.alphaToBexp >= 0.0 && !k.slotStats && c->sym.nLoop <= 8 && c->nVol > 0 &&
+           c->nVol * c->sym.nLoop <= kTileMost;
 }
 
 static TileDev tile_dev(Ctx *c) {

@@ -70,3 +70,33 @@ def test_errtol_change_renews_the_double_float_denominators(built_lib, opts):
             mesh.warpDeriv(seed, solverVec=False)
             out.append(np.array(mesh.getdXs()).ravel())
         assert np.abs(out[0] - out[1]).max() <= 1e-9 * np.abs(out[1]).max()
+
+
+def test_negative_weights_have_the_gated_walk(built_lib):
+    """alpha < 0: weights of both signs can exceed their node's denominator, which the
+    digits' range does not hold.  Nodes on a line towards the point where the
+    denominator vanishes; the sums are 1e-5 of the weights' sizes off at most (FP32
+    terms).  Digits of such weights are infinite and the quotients not numbers."""
+    m = wing_small()
+    x0, opts = np.asarray(m["xv0"]), {"alpha": -1.0, "errTol": 0.0}  # every point by itself
+
+    def warped(x, precision):
+        g = build_gpu(dict(m, xv0=x), opts, precision=precision)
+        g.setSurfaceCoordinates(m["xs"])
+        g.warpMesh()
+        return np.array(g.getWarpGrid()).reshape(-1, 3), g.getDenominator()
+
+    den = warped(x0, "fp64")[1]
+    start, b = x0[den > 0.0][0], x0[den < 0.0][0]
+    a = start
+    for _ in range(3):
+        line = a + np.linspace(0.0, 1.0, 301)[:, None] * (b - a)
+        den = warped(line, "fp64")[1]
+        k = int(np.argmax(den < 0.0))
+        a, b = line[k - 1], line[k]
+    x = a + np.linspace(0.0, 1.0, 201)[:, None] * (start - a)
+    (got, _), (want, den) = warped(x, "mixed"), warped(x, "fp64")
+    assert den.min() > 0.0 and den.min() < 1e-4 * den.max()
+    assert np.isfinite(got).all()
+    # N / D: an error of D counts with the quotient
+    assert (np.abs(got - want) * den[:, None] <= 1e-5 * den.max() * (1.0 + np.abs(want))).all()
