@@ -58,13 +58,14 @@ struct TileLaw {
 // double-float: w + wl to about 2^-44.  h, l: the nodes' positions, c, d: the
 // term's (high parts and area, low parts and area).  The offset is an exact
 // difference of the high parts plus the low parts, |x|^2 exact squares plus
-// corrections; the residual 1 - q y^2 of the reciprocal square root and the
-// errors of the products are carried to first order.
+// corrections, and the softening eps, which can be larger than all of them, an exact
+// sum; the residual 1 - q y^2 of the reciprocal square root and the errors of the
+// products are carried to first order.
 __device__ __forceinline__ float2 tile_weight(const float4 c, const float4 d, float eps, const float2 *h,
                                               const float2 *l, float2 P, const TileLaw law, float2 &wl) {
     const float2 one = dup2(1.0f);
     const float ch[3] = {c.x, c.y, c.z}, cl[3] = {d.x, d.y, d.z};
-    float2 p[3], low = dup2(eps);
+    float2 p[3], low = dup2(-3.6274936e-9f * eps);  // what FP32 leaves of 1e-15
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         // a + b = (h - ch) + (l - cl), renormalised: b is below an ulp of a
@@ -75,11 +76,12 @@ __device__ __forceinline__ float2 tile_weight(const float4 c, const float4 d, fl
         // (a + b)^2 - a^2 = (2 a + b) b
         low = fma2(fma2(dup2(2.0f), a, b), b, add2(low, fms2(a, a, p[k])));
     }
-    float2 s1, e1, s2, e2;
+    float2 s1, e1, s2, e2, s3, e3;
     two_sum2(p[0], p[1], s1, e1);
     two_sum2(s1, p[2], s2, e2);
-    low = add2(low, add2(e1, e2));
-    const float2 q = add2(s2, low), ql = sub2(low, sub2(q, s2));
+    two_sum2(s2, dup2(eps), s3, e3);
+    low = add2(low, add2(add2(e1, e2), e3));
+    const float2 q = add2(s3, low), ql = sub2(low, sub2(q, s3));
     const float2 y = make_float2(rsqrt_normal(q.x), rsqrt_normal(q.y));
     const float2 y2 = mul2(y, y), y2l = fms2(y, y, y2);
     const float2 t0 = mul2(q, y), t0l = fms2(q, y, t0);
