@@ -505,9 +505,20 @@ __global__ void k_tile_finalize(VolumeDev v, WalkRecF rec, NodeAggF af, MixedPar
     const int64_t gid = td.order[slot];
     float4 S = make_float4(0.f, 0.f, 0.f, 0.f), C = S;
     for (int kk = 0; kk < mp.nLoop; ++kk) {
-        const int64_t at = kk * v.nVol + slot;
-        const float4 h = sums[2 * at], l = sums[2 * at + 1];
         const float4 rhi = rec.hi[kk * v.nVol + gid], rlo = rec.lo[kk * v.nVol + gid];
+        // A node on a plane is its own image there: it has one sum, so that the parts
+        // along the normal cancel and the node stays on the plane to the last bit (the
+        // images' steps, and with them the rounding of their sums, differ).
+        int image = kk;
+        for (int j = 0; j < mp.nSym; ++j) {
+            if (!((image >> j) & 1)) continue;
+            const int64_t other = (image ^ (1 << j)) * v.nVol + gid;
+            const float4 ohi = rec.hi[other], olo = rec.lo[other];
+            if (ohi.x == rhi.x && ohi.y == rhi.y && ohi.z == rhi.z && olo.x == rlo.x && olo.y == rlo.y && olo.z == rlo.z)
+                image ^= 1 << j;
+        }
+        const int64_t at = image * v.nVol + slot;
+        const float4 h = sums[2 * at], l = sums[2 * at + 1];
         const float rh[3] = {rhi.x, rhi.y, rhi.z}, rl[3] = {rlo.x, rlo.y, rlo.z};
         const float sn[3] = {h.x, h.y, h.z}, cn[3] = {l.x, l.y, l.z};
         finish_mirror(af, mp, kk, rh, rl, sn, cn, h.w, l.w, S, C);
