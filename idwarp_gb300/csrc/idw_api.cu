@@ -1065,7 +1065,6 @@ static int make_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const Eval
     const bool record = !off && !c->tileKept;
     c->tileState = 0;
     c->tileRunState = 0;
-    if (record) drop_tile_kept(c);
     auto serves = [&](int state) {
         if (state < 0 && !c->tileKept) drop_tile(c);
         c->tileErrTol = c->opt.errTol;
@@ -1104,9 +1103,15 @@ static int make_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const Eval
     if (badH) return serves(-1);
     const size_t entries = size_t(std::max<int64_t>(total, 16)), steps = entries / 16;
     if (!c->tileKept) {
+        // lists and digits of an earlier recording make room for these, in place where
+        // they are large enough and not twice too large (7 GB take 4 ms to give back)
+        const size_t n = c->tileTerm.n;
+        if (record && (n < entries || n > 2 * entries || c->tileMask.n < entries || c->tileDig.n < 192 * steps ||
+                       c->tileDig3.n < 64 * steps))
+            drop_tile_kept(c);
         const double need = 8.0 * double(entries) + 320.0 * sizeof(uint4) * double(steps) + 8.0 * double(c->nVol);
-        const double held =
-            8.0 * double(c->tileTerm.n) + sizeof(uint4) * double(c->tileDig.n + c->tileDig3.n + c->tileDig4.n);
+        const double held = 8.0 * double(c->tileTerm.n + c->tileDenInv.n) +
+                            sizeof(uint4) * double(c->tileDig.n + c->tileDig3.n + c->tileDig4.n);
         bool fits = false;
         int rc = fits_half(c, need, fits, held);
         if (rc) return rc;

@@ -67,11 +67,12 @@ def test_refused_allocations_after_an_errtol_change(built_lib):
     f, g = build_gpu(m, precision="fp64"), build_gpu(m, precision="mixed")
     calls(g, m)
     limit(g, "tileAllocs", 0)
-    for errTol in (1e-3, 1e-5, 1e-4):
+    # shorter lists go where the longer ones were
+    for errTol, state in ((2e-4, 1), (1e-5, -1), (1e-4, -1)):
         for mesh in (f, g):
             mesh.setOption("errTol", errTol)
         close(calls(g, m), calls(f, m), f.getStats()["Ldef0"])
-        assert internal(g, "tileState") == -1
+        assert internal(g, "tileState") == state
 
 
 def test_digits_beyond_half_of_the_free_memory(built_lib):
