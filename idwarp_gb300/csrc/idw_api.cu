@@ -1076,11 +1076,13 @@ static int make_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const Eval
     if (!(tile_alloc(c, c->tileOffs, size_t(units) + 1) && tile_alloc(c, c->tileGeo, 2 * nTerms) &&
           tile_alloc(c, c->tileMot, 8 * nTerms) && tile_alloc(c, c->tileWord, kTileWords) &&
           tile_alloc(c, c->tileScale, size_t(c->nVol)) &&
-          tile_alloc(c, c->tileSums, 2 * size_t(c->sym.nLoop) * size_t(c->nVol)) &&
+          tile_alloc(c, c->tileSums, std::max(2 * size_t(c->sym.nLoop) * size_t(c->nVol), size_t(1) << 16)) &&
           tile_alloc(c, c->tileOrder, size_t(c->nVol))))
         return serves(-1);
+    // the sums are scratch until the walk; the denominators in front
+    TileScratch scratch{reinterpret_cast<char *>(c->tileSums.p), c->tileSums.n * sizeof(float4)};
     if (!c->tileOrderValid) {
-        const int rc = tile_order(vol_dev(c), c->volLo, c->volHi, c->tileOrder.p, c->stream);
+        const int rc = tile_order(vol_dev(c), c->volLo, c->volHi, c->tileOrder.p, scratch, c->stream);
         if (rc == -2) {
             (void)cudaGetLastError();
             return serves(-1);
@@ -1088,21 +1090,15 @@ static int make_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const Eval
         if (rc) return fail(c, IDW_ERR_CUDA, "node order of the tile walks failed");
         c->tileOrderValid = true;
     }
+    float *part = static_cast<float *>(scratch.take(sizeof(float) * size_t(c->sym.nLoop) * size_t(c->nVol)));
     launch_tile_geo(tree_dev(c), c->nUnique, c->ptXA.p, c->areaExp, c->tileGeo.p, c->stream);
-    int *bad = reinterpret_cast<int *>(c->tileWord.p + 13);
-    const int64_t total = count_tile_lists(tree_dev(c), tf, vol_dev(c), rec, k, tile_dev(c), c->tileOffs.p,
-                                           reinterpret_cast<float *>(c->tileSums.p), c->tileScale.p, bad, c->stream);
-    if (total == -2) {
-        (void)cudaGetLastError();
-        return serves(-1);
-    }
-    if (total < 0) return fail(c, IDW_ERR_CUDA, "walk lists: count pass failed");
-    int badH = 0;
-    CK(cudaMemcpyAsync(&badH, bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    if (badH) return serves(-1);
-    const size_t entries = size_t(std::max<int64_t>(total, 16)), steps = entries / 16;
     if (!c->tileKept) {
+        const int64_t total = count_tile_lists(tree_dev(c), tf, vol_dev(c), rec, k, tile_dev(c), c->tileOffs.p,
+                                               off ? part : nullptr, scratch, c->stream);
+        if (total == -2) return serves(-1);
+        if (total < 0) return fail(c, IDW_ERR_CUDA, "walk lists: count pass failed");
+        c->tileListEntries = total;
+        const size_t entries = size_t(std::max<int64_t>(total, 16)), steps = entries / 16;
         // lists and digits of an earlier recording make room for these, in place where
         // they are large enough and not twice too large (7 GB take 4 ms to give back)
         const size_t n = c->tileTerm.n;
@@ -1116,25 +1112,34 @@ static int make_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const Eval
         int rc = fits_half(c, need, fits, held);
         if (rc) return rc;
         if (!fits) return serves(-1);
+        if (record) {
+            if (!(tile_alloc(c, c->tileCnt, 8) && tile_alloc(c, c->tileTerm, entries) &&
+                  tile_alloc(c, c->tileMask, entries) && tile_alloc(c, c->tileDig, 192 * steps) &&
+                  tile_alloc(c, c->tileDig3, 64 * steps)))
+                return serves(-1);
+            CK(cudaMemsetAsync(c->tileCnt.p, 0, 8 * sizeof(unsigned long long), c->stream));
+            launch_tile_record(tree_dev(c), tf, vol_dev(c), rec, k, tile_dev(c), tile_all(c), c->tileOffs.p,
+                               c->tileTerm.p, c->tileMask.p, c->tileCnt.p, c->stream);
+            rc = check_launch(c, "walk lists");
+            if (rc) return rc;
+            c->tileKept = true;
+        }
     }
-    c->tileListEntries = total;
-    if (record) {
-        if (!(tile_alloc(c, c->tileCnt, 8) && tile_alloc(c, c->tileTerm, entries) &&
-              tile_alloc(c, c->tileMask, entries) && tile_alloc(c, c->tileDig, 192 * steps) &&
-              tile_alloc(c, c->tileDig3, 64 * steps)))
-            return serves(-1);
-        CK(cudaMemsetAsync(c->tileCnt.p, 0, 8 * sizeof(unsigned long long), c->stream));
-        launch_tile_record(tree_dev(c), tf, vol_dev(c), rec, k, tile_dev(c), tile_all(c), c->tileOffs.p, c->tileTerm.p,
-                           c->tileMask.p, c->tileCnt.p, c->stream);
-        int rc = check_launch(c, "walk lists");
-        if (rc) return rc;
-        c->tileKept = true;
-    }
-    if (!off) {
-        TileLists lists;
-        lists.offs = c->tileOffs.p;
+    TileLists lists;
+    lists.offs = c->tileOffs.p;
+    if (c->tileKept) {
         lists.term = c->tileTerm.p;
         lists.mask = c->tileMask.p;
+    }
+    int *bad = reinterpret_cast<int *>(c->tileWord.p + 13), badH = 0;
+    launch_tile_scales(vol_dev(c), rec, k, tile_dev(c), lists, c->nUnique, part, c->tileScale.p, bad, c->stream);
+    CK(cudaMemcpyAsync(&badH, bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    if (badH) {
+        if (record) c->tileKept = false;
+        return serves(-1);
+    }
+    if (!off) {
         c->tileFifthState = 0;
         launch_tile_build(vol_dev(c), rec, k, tile_dev(c), lists, tile_all(c), 0, c->nUnique, c->tileDig.p,
                           c->tileDig3.p, c->stream);

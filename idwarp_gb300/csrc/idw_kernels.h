@@ -235,16 +235,35 @@ struct TileDev {
     unsigned *counter;       // the walk's next unit (its launch clears it)
     int areaExp;
 };
-// Tile order of the volume nodes (lo, hi: their bounding box).  Returns 0, -1 on
-// a CUDA error, -2 without memory; synchronises st.
-int tile_order(const VolumeDev &v, const double *lo, const double *hi, int *order, cudaStream_t st);
+// Device scratch handed out from the front, 256-byte aligned; null when it ends.
+struct TileScratch {
+    char *p = nullptr;
+    size_t left = 0;
+    void *take(size_t bytes) {
+        const size_t n = (bytes + 255) / 256 * 256;
+        if (n > left) return nullptr;
+        void *r = p;
+        p += n;
+        left -= n;
+        return r;
+    }
+};
+// Tile order of the volume nodes (lo, hi: their bounding box); scratch: 20 bytes a
+// node (more saves an allocation).  Returns 0, -1 on a CUDA error, -2 without memory;
+// synchronises st.
+int tile_order(const VolumeDev &v, const double *lo, const double *hi, int *order, TileScratch scratch,
+               cudaStream_t st);
 void launch_tile_geo(const TreeDev &t, int nPts, const dbl4 *xa, int areaExp, float4 *geo, cudaStream_t st);
-// Fills scale, raises *bad when a node has none, fills offs and returns the number
-// of entries (-1 on a CUDA error, -2 without memory); part: nLoop nVol floats of
-// scratch.  Synchronises st.
+// Fills offs and returns the number of entries (-1 on a CUDA error, -2 where the
+// scratch ends), and with part (nLoop nVol floats) the units' FP32 denominators.
+// Synchronises st.
 int64_t count_tile_lists(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
-                         const EvalConsts &k, const TileDev &td, int64_t *offs, float *part, float *scale, int *bad,
+                         const EvalConsts &k, const TileDev &td, int64_t *offs, float *part, TileScratch scratch,
                          cudaStream_t st);
+// Fills scale and raises *bad when a node has none, from the denominators in part
+// (of the lists, if there are any; else those of count_tile_lists).
+void launch_tile_scales(const VolumeDev &v, const WalkRecF &rec, const EvalConsts &k, const TileDev &td,
+                        const TileLists &lists, int nPts, float *part, float *scale, int *bad, cudaStream_t st);
 // A run of groups; entry0 is the list entry that lies first in the arrays given.
 struct TileRange {
     int64_t group0 = 0, group1 = 0, entry0 = 0;
@@ -338,7 +357,7 @@ int launch_adjoint_precise(const TreeDev &t, const TreeDevF &tf, const PointsDev
                            int64_t dxvStride, const double *den, double *ptAcc, double *nodeAcc, int nPts,
                            unsigned long long *counters, cudaStream_t st, int det = 0);
 int sort_morton(int64_t nVol, unsigned long long *codes, int *idx, unsigned long long *codesAlt, int *perm,
-                cudaStream_t st);
+                cudaStream_t st, void *scratch = nullptr, size_t scratchBytes = 0);
 
 // Setters of the landing state (idw_land.cuh), one per translation unit
 // that lands FP64 sums; set all of them on the launching stream.

@@ -552,20 +552,21 @@ void launch_mixed_nodes(const TreeDev &t, const double *nodeMB, const double *pt
 // Sort volume nodes by Morton code (set-up).  perm[k] = common index of the
 // k-th node in Morton order.
 int sort_morton(int64_t nVol, unsigned long long *codes, int *idx, unsigned long long *codesAlt, int *perm,
-                cudaStream_t st) {
+                cudaStream_t st, void *scratch, size_t scratchBytes) {
     // cub takes the item count as int
     if (nVol > INT_MAX) return -1;
     size_t tmp = 0;
     if (cub::DeviceRadixSort::SortPairs(nullptr, tmp, codes, codesAlt, idx, perm, int(nVol), 0, 63, st) !=
         cudaSuccess)
         return -1;
-    void *dTmp = nullptr;
-    if (cudaMalloc(&dTmp, tmp) != cudaSuccess) return -1;
+    void *own = nullptr;
+    if (tmp > scratchBytes && cudaMalloc(&own, tmp) != cudaSuccess) return -2;
     int rc = 0;
-    if (cub::DeviceRadixSort::SortPairs(dTmp, tmp, codes, codesAlt, idx, perm, int(nVol), 0, 63, st) != cudaSuccess)
+    if (cub::DeviceRadixSort::SortPairs(own ? own : scratch, tmp, codes, codesAlt, idx, perm, int(nVol), 0, 63, st) !=
+        cudaSuccess)
         rc = -1;
     if (cudaStreamSynchronize(st) != cudaSuccess) rc = -1;
-    cudaFree(dTmp);
+    if (own) cudaFree(own);
     return rc;
 }
 

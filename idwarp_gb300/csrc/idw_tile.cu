@@ -90,9 +90,9 @@ __global__ void k_tile_geo(TreeDev t, int nPts, const dbl4 *xa, int areaExp, flo
     geo[2 * int64_t(i) + 1] = make_float4(l[0], l[1], l[2], l[3]);
 }
 
-// The traversal of one unit: emit(term, mask) for every point of a leaf that a
-// lane sums and every cluster that a lane approximates, in preorder, with the
-// decisions of k_walk_record.  slot: the lane's walk slot (group 32 + lane).
+// The traversal of one unit: emit(first, n, mask) for the n points of every leaf that
+// a lane sums and (n = 1) every cluster that a lane approximates, in preorder, with
+// the decisions of k_walk_record.  slot: the lane's walk slot (group 32 + lane).
 template <class F>
 __device__ __forceinline__ void decide_group(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v,
                                              const WalkRecF &rec, const MixedParams &mp, const TileDev &td,
@@ -109,8 +109,7 @@ __device__ __forceinline__ void decide_group(const TreeDev &t, const TreeDevF &t
         const bool active = valid && node >= skip;
         if (inf.w) {
             const unsigned m = __ballot_sync(kFull, active);
-            if (m)
-                for (int i = inf.x; i <= inf.y; ++i) emit(i, m);
+            if (m) emit(inf.x, inf.y - inf.x + 1, m);
             if (active) {
                 cnt.leafPairs += inf.y - inf.x + 1;
                 cnt.visited++;
@@ -125,7 +124,7 @@ __device__ __forceinline__ void decide_group(const TreeDev &t, const TreeDevF &t
             }
             dec = resolve64(dec, t, v, g, node, rh, rl, mp.errTol, counters);
             const unsigned m = __ballot_sync(kFull, dec == 1);
-            if (m) emit(tf.nPts + node, m);
+            if (m) emit(tf.nPts + node, 1, m);
             bool open = false;
             if (dec == 1) {
                 skip = inf.z;
@@ -143,9 +142,21 @@ __device__ __forceinline__ int first_scale(const WalkRecF &rec, int64_t gid, int
     return max(-110, min(110, 5 * __float_as_int(rec.lo[gid].w) + lawExp));
 }
 
-// List lengths (whole steps) of every unit, a warp each, into counts, and the
+// One term's part of a node's FP32 denominator under the weight scale P.
+__device__ __forceinline__ float add_den(float den, const float4 *geo, int term, int nPts, const float4 &rhi,
+                                         const float4 &rlo, float P, const TileLaw &law) {
+    const float4 c = ldgf4(geo + 2 * int64_t(term)), d = ldgf4(geo + 2 * int64_t(term) + 1);
+    const float dx = (rhi.x - c.x) + (rlo.x - d.x), dy = (rhi.y - c.y) + (rlo.y - d.y),
+                dz = (rhi.z - c.z) + (rlo.z - d.z);
+    const float y = rsqrt_normal(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, term < nPts ? 1e-15f : 0.f))));
+    const float y2 = y * y;
+    return fmaf(c.w * (y2 * (y * P)), fmaf(law.kh, y2, 1.0f), den);
+}
+
+// List lengths (whole steps) of every unit, a warp each, into counts.  DEN: also the
 // unit's share of its nodes' FP32 denominators under the first guess into part
-// (nLoop x nVol).
+// (nLoop x nVol), as k_tile_part has it from the lists.
+template <bool DEN>
 __global__ void __launch_bounds__(128, 8)
     k_tile_count(TreeDev t, TreeDevF tf, VolumeDev v, WalkRecF rec, MixedParams mp, TileDev td, TileLaw law,
                  int lawExp, int64_t nGroups, int64_t *counts, float *part) {
@@ -154,23 +165,47 @@ __global__ void __launch_bounds__(128, 8)
     if (group >= nGroups) return;  // whole warps only
     const int kk = int(unit - group * mp.nLoop), lane = threadIdx.x & 31;
     const int64_t slot = 32 * group + lane, gid = td.order[min(slot, v.nVol - 1)];
-    const float P = pow2f(first_scale(rec, gid, lawExp));
+    const float P = DEN ? pow2f(first_scale(rec, gid, lawExp)) : 0.f;
     float den = 0.f;
     MixedCounters cnt;
     const float4 rhi = rec.hi[kk * v.nVol + gid], rlo = rec.lo[kk * v.nVol + gid];
     int n = 0;
-    decide_group(t, tf, v, rec, mp, td, slot, kk, cnt, nullptr, [&](int term, unsigned m) {
-        ++n;
-        if ((m >> lane) & 1u) {
-            const float4 c = ldgf4(td.geo + 2 * int64_t(term)), d = ldgf4(td.geo + 2 * int64_t(term) + 1);
-            const float dx = (rhi.x - c.x) + (rlo.x - d.x), dy = (rhi.y - c.y) + (rlo.y - d.y),
-                        dz = (rhi.z - c.z) + (rlo.z - d.z);
-            const float y = rsqrt_normal(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, term < tf.nPts ? 1e-15f : 0.f))));
-            const float y2 = y * y;
-            den = fmaf(c.w * (y2 * (y * P)), fmaf(law.kh, y2, 1.0f), den);
+    decide_group(t, tf, v, rec, mp, td, slot, kk, cnt, nullptr, [&](int first, int k, unsigned m) {
+        n += k;
+        if constexpr (DEN) {
+            if ((m >> lane) & 1u)
+                for (int i = first; i < first + k; ++i) den = add_den(den, td.geo, i, tf.nPts, rhi, rlo, P, law);
         }
     });
     if (lane == 0) counts[unit] = int64_t(n + kTileTerms - 1) / kTileTerms * kTileTerms;
+    if (DEN && slot < v.nVol) part[kk * v.nVol + slot] = den;
+}
+
+// The units' shares of the FP32 denominators from the recorded lists, added in the
+// order of the traversal: a new weight law needs no traversal (8M-node wing, the warp
+// after a new alpha 38.5 -> 29.1 ms), and the first count does without them (2M nodes
+// 3.5 -> 2.25 + 1.1 ms).
+__global__ void __launch_bounds__(128)
+    k_tile_part(VolumeDev v, WalkRecF rec, MixedParams mp, TileDev td, TileLists lists, TileLaw law, int lawExp,
+                int nPts, int64_t nUnits, float *part) {
+    const int64_t unit = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    if (unit >= nUnits) return;  // whole warps only
+    const int64_t group = unit / mp.nLoop;
+    const int kk = int(unit - group * mp.nLoop), lane = threadIdx.x & 31;
+    const int64_t slot = 32 * group + lane, gid = td.order[min(slot, v.nVol - 1)];
+    const float P = pow2f(first_scale(rec, gid, lawExp));
+    const float4 rhi = rec.hi[kk * v.nVol + gid], rlo = rec.lo[kk * v.nVol + gid];
+    float den = 0.f;
+    const int64_t e1 = lists.offs[unit + 1];
+    for (int64_t e = lists.offs[unit]; e < e1; e += kTileTerms) {
+        const int term = lists.term[e + (lane & 15)];
+        const unsigned mask = lists.mask[e + (lane & 15)];
+#pragma unroll 8
+        for (int k = 0; k < kTileTerms; ++k) {
+            const float d = add_den(den, td.geo, __shfl_sync(kFull, term, k), nPts, rhi, rlo, P, law);
+            den = (__shfl_sync(kFull, mask, k) >> lane) & 1u ? d : den;
+        }
+    }
     if (slot < v.nVol) part[kk * v.nVol + slot] = den;
 }
 
@@ -201,12 +236,12 @@ __global__ void __launch_bounds__(128, 8)
     MixedCounters cnt;
     int64_t pos = offs[unit] - range.entry0;
     const int64_t end = offs[unit + 1] - range.entry0;
-    decide_group(t, tf, v, rec, mp, td, 32 * group + lane, kk, cnt, counters, [&](int i, unsigned m) {
-        if (lane == 0) {
-            term[pos] = i;
-            mask[pos] = m;
+    decide_group(t, tf, v, rec, mp, td, 32 * group + lane, kk, cnt, counters, [&](int first, int n, unsigned m) {
+        for (int i = lane; i < n; i += 32) {
+            term[pos + i] = first + i;
+            mask[pos + i] = m;
         }
-        ++pos;
+        pos += n;
     });
     if (pos + lane < end) {
         term[pos + lane] = 0;
@@ -562,23 +597,19 @@ int tile_sms() {
     return n;
 }
 
-int tile_order(const VolumeDev &v, const double *lo, const double *hi, int *order, cudaStream_t st) {
+int tile_order(const VolumeDev &v, const double *lo, const double *hi, int *order, TileScratch scratch,
+               cudaStream_t st) {
     if (v.nVol <= 0) return 0;
     if (v.nVol > INT_MAX) return -1;
     double ext = 0.0;
     for (int k = 0; k < 3; ++k) ext = hi[k] - lo[k] > ext ? hi[k] - lo[k] : ext;
-    unsigned long long *codes = nullptr;
-    int *idx = nullptr;
-    int rc = -2;
-    if (cudaMalloc(&codes, sizeof(*codes) * 2 * size_t(v.nVol)) == cudaSuccess &&
-        cudaMalloc(&idx, sizeof(int) * size_t(v.nVol)) == cudaSuccess) {
-        k_tile_curve<<<blocks(v.nVol, 256), 256, 0, st>>>(v, lo[0], lo[1], lo[2], ext > 0.0 ? 2097151.0 / ext : 0.0,
-                                                          codes, idx);
-        rc = sort_morton(v.nVol, codes, idx, codes + v.nVol, order, st);
-    }
-    if (codes) cudaFree(codes);
-    if (idx) cudaFree(idx);
-    return rc;
+    const size_t n = size_t(v.nVol);
+    auto *codes = static_cast<unsigned long long *>(scratch.take(2 * sizeof(unsigned long long) * n));
+    auto *idx = static_cast<int *>(scratch.take(sizeof(int) * n));
+    if (!codes || !idx) return -2;
+    k_tile_curve<<<blocks(v.nVol, 256), 256, 0, st>>>(v, lo[0], lo[1], lo[2], ext > 0.0 ? 2097151.0 / ext : 0.0, codes,
+                                                      idx);
+    return sort_morton(v.nVol, codes, idx, codes + v.nVol, order, st, scratch.p, scratch.left);
 }
 
 void launch_tile_geo(const TreeDev &t, int nPts, const dbl4 *xa, int areaExp, float4 *geo, cudaStream_t st) {
@@ -593,37 +624,46 @@ void launch_tile_motions(const TreeDev &t, int nPts, const double *ptMB, const d
     k_tile_mot<<<blocks(n, 256), 256, 0, st>>>(t, nPts, ptMB, nodeMB, colMax, mot, mot5, refDB);
 }
 
+// den L^-3 2^areaExp 2^(5s) is near one
+static int law_exp(const EvalConsts &k, const TileDev &td) { return 3 * ilogb(k.law.Ldef) - td.areaExp; }
+
 int64_t count_tile_lists(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
-                         const EvalConsts &k, const TileDev &td, int64_t *offs, float *part, float *scale, int *bad,
+                         const EvalConsts &k, const TileDev &td, int64_t *offs, float *part, TileScratch scratch,
                          cudaStream_t st) {
     const MixedParams mp = make_mixed_params(k);
     const int64_t nGroups = walk_list_warps(v.nVol);
     const int64_t n = nGroups * mp.nLoop;
     if (n <= 0) return 0;
     if (n + 1 > int64_t(INT_MAX)) return -1;
-    // den L^-3 2^areaExp 2^(5s) is near one
-    const int lawExp = 3 * ilogb(k.law.Ldef) - td.areaExp;
-    int64_t *counts = nullptr;
-    void *tmp = nullptr;
     size_t tmpBytes = 0;
     int64_t total = 0;
-    if (cudaMalloc(&counts, sizeof(int64_t) * (n + 1)) != cudaSuccess) return -2;
-    bool room = true, ok = cudaMemsetAsync(counts + n, 0, sizeof(int64_t), st) == cudaSuccess;
-    if (ok) ok = cudaMemsetAsync(bad, 0, sizeof(int), st) == cudaSuccess;
+    auto *counts = static_cast<int64_t *>(scratch.take(sizeof(int64_t) * size_t(n + 1)));
+    if (!counts) return -2;
+    bool ok = cudaMemsetAsync(counts + n, 0, sizeof(int64_t), st) == cudaSuccess;
     if (ok) {
-        k_tile_count<<<blocks(32 * n, 128), 128, 0, st>>>(t, tf, v, rec, mp, td, make_tile_law(k), lawExp, nGroups,
-                                                          counts, part);
-        k_tile_scale<<<blocks(v.nVol, 128), 128, 0, st>>>(v, rec, td, mp.nLoop, lawExp, part, scale, bad);
+        (part ? k_tile_count<true> : k_tile_count<false>)<<<blocks(32 * n, 128), 128, 0, st>>>(
+            t, tf, v, rec, mp, td, make_tile_law(k), law_exp(k, td), nGroups, counts, part);
         ok = cudaGetLastError() == cudaSuccess;
     }
     if (ok) ok = cub::DeviceScan::ExclusiveSum(nullptr, tmpBytes, counts, offs, int(n + 1), st) == cudaSuccess;
-    if (ok) ok = room = cudaMalloc(&tmp, tmpBytes) == cudaSuccess;
+    void *tmp = scratch.take(tmpBytes);
+    if (ok && !tmp) return -2;
     if (ok) ok = cub::DeviceScan::ExclusiveSum(tmp, tmpBytes, counts, offs, int(n + 1), st) == cudaSuccess;
     if (ok) ok = cudaMemcpyAsync(&total, offs + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st) == cudaSuccess;
     if (cudaStreamSynchronize(st) != cudaSuccess) ok = false;
-    if (tmp) cudaFree(tmp);
-    if (counts) cudaFree(counts);
-    return ok ? total : (room ? -1 : -2);
+    return ok ? total : -1;
+}
+
+void launch_tile_scales(const VolumeDev &v, const WalkRecF &rec, const EvalConsts &k, const TileDev &td,
+                        const TileLists &lists, int nPts, float *part, float *scale, int *bad, cudaStream_t st) {
+    if (v.nVol <= 0) return;
+    const MixedParams mp = make_mixed_params(k);
+    const int64_t n = walk_list_warps(v.nVol) * mp.nLoop;
+    cudaMemsetAsync(bad, 0, sizeof(int), st);
+    if (lists.term)
+        k_tile_part<<<blocks(32 * n, 128), 128, 0, st>>>(v, rec, mp, td, lists, make_tile_law(k), law_exp(k, td), nPts, n,
+                                                         part);
+    k_tile_scale<<<blocks(v.nVol, 128), 128, 0, st>>>(v, rec, td, mp.nLoop, law_exp(k, td), part, scale, bad);
 }
 
 void launch_tile_record(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
