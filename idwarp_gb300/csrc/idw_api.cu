@@ -933,15 +933,20 @@ static int ensure_gate_den(Ctx *c, const TreeDevF &tf, const PointsDevF &pf, con
 // denominator: a negative alpha has the gated walks.  So have the FP32 reverse product
 // (IDW_ADJ_FAST) with its forward walk, and the diagnostics.  Three symmetry planes
 // (8 mirror images) bound the scratch, and kTileMost node images the weight digits
-// (2.4 kB each, 3 kB with the fifth); both limits apply with the lists on and off, so
-// the results agree.
-constexpr int64_t kTileMost = int64_t(1) << 25;
+// (2.4 kB each, 3 kB with the fifth), with the lists on and off.
+// With the lists off every walk forms its weights anew, 3.7 ms of double-float
+// arithmetic on 4M images, and from some 2^18 images on the gated walk, which decides
+// and sums in one pass, is ahead: 99k images 0.48 against 0.53 ms (a tangent 0.69, 0.85),
+// 246k 0.63 and 0.63 (0.97, 1.04), 490k 0.93 and 0.81 (1.41, 1.32), 753k 1.32 and 1.05
+// (2.13, 1.81), 4M 4.96 and 3.28 (7.7, 5.4).  The line lies at 2^19, since below it
+// both settings of walkLists keep the same bits for a tenth of a millisecond.
+constexpr int64_t kTileMost = int64_t(1) << 25, kTileOffMost = int64_t(1) << 19;
 
 static bool tile_applies(const Ctx *c, const EvalConsts &k) {
     return c->opt.precision == IDW_PREC_MIXED && c->opt.evalMode == IDW_EVAL_FAST &&
            c->opt.adjointPrecision == IDW_ADJ_PRECISE && c->opt.mixedGate >= 2e-3 && k.law.isInt && k.law.ia == 3 &&
            k.law.ib == 5 && k.law.alphaToBexp >= 0.0 && !k.slotStats && c->sym.nLoop <= 8 && c->nVol > 0 &&
-           c->nVol * c->sym.nLoop <= kTileMost;
+           c->nVol * c->sym.nLoop <= (c->opt.walkLists == IDW_WALK_LISTS_OFF ? kTileOffMost : kTileMost);
 }
 
 static TileDev tile_dev(Ctx *c) {

@@ -103,8 +103,14 @@ typedef struct idw_options {
                            * and errTol only, so they can be recorded once (per warp of 32
                            * volume nodes: the tree nodes where a lane approximates or sums
                            * a leaf) and replayed by every later warp; at the default exponents
-                           * and gate the recorded terms' weights are kept too, when they fit
-                           * (8 bytes per node and term); same sums either way */
+                           * and gate the recorded terms' weights are kept too, as FP16 digits
+                           * (8 bytes per node and term, 10 with what reverse products and
+                           * tangents add), where lists and digits fit into half of the free
+                           * device memory.  Off keeps nothing: up to 2^19 volume node images
+                           * such walks form their digits as they go, with the same sums;
+                           * beyond, every walk decides as it goes in the gated form, as it
+                           * does with the lists on where the digits have no room.  Without
+                           * digits (other exponents, tighter gates) same sums either way */
     int32_t treeBuild;    /* IDW_TREE_KD (default) or IDW_TREE_MORTON; read by
                            * idw_initialize_warping, as bucketSize */
     int32_t deterministic; /* 0 (default): reverse products (idw_warp_deriv*) land their sums with

@@ -100,3 +100,34 @@ def test_negative_weights_have_the_gated_walk(built_lib):
     assert np.isfinite(got).all()
     # N / D: an error of D counts with the quotient
     assert (np.abs(got - want) * den[:, None] <= 1e-5 * den.max() * (1.0 + np.abs(want))).all()
+
+
+@pytest.mark.parametrize("ni,tile", [(201, True), (221, False)])
+def test_lists_off_beyond_half_a_million_images(built_lib, ni, tile):
+    """Up to 2^19 node images the walk from digits made on the way, beyond it the gated
+    walk that decides as it goes (1e-8 of Ldef0; its tangents 1e-6 of the largest entry,
+    its reverse products 1e-9), also after a walk from kept digits."""
+    from idwarp_gb300 import synthetic as S
+
+    m = S.wing_shell(ni, 61, 20)
+    assert (2 * len(m["xv0"]) <= 2**19) == tile
+    xs = S.wing_perturbation(np.asarray(m["pts"]), seed=3)
+    rng = np.random.default_rng(6)
+    seed, d = rng.standard_normal(np.asarray(m["xv0"]).size), rng.standard_normal(np.asarray(m["pts"]).size)
+    g, f = (build_gpu(m, {"errTol": 1e-3}, precision=p) for p in ("mixed", "fp64"))
+
+    def results(mesh):
+        mesh.setSurfaceCoordinates(xs)
+        mesh.warpMesh()
+        r = [np.array(mesh.getWarpGrid()).ravel(), mesh.getStats()["preciseTerms"]]
+        mesh.warpDeriv(seed, solverVec=False)
+        return r + [np.array(mesh.getdXs()).ravel(), np.array(mesh.warpDerivFwd(d, solverVec=False)).ravel()]
+
+    want = results(f)
+    for lists in ("off", "auto", "off"):
+        g.setOption("walkLists", lists)
+        got = results(g)
+        assert (got[1] == 0) == (tile or lists == "auto")
+        assert np.abs(got[0] - want[0]).max() <= 1e-8 * g.getStats()["Ldef0"]
+        for a, b, tol in zip(got[2:], want[2:], (1e-9, 1e-6)):
+            assert np.abs(a - b).max() <= tol * np.abs(b).max()
