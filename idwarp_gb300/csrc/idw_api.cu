@@ -1071,18 +1071,20 @@ static int make_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const Eval
     c->tileState = 0;
     c->tileRunState = 0;
     auto serves = [&](int state) {
-        if (state < 0 && !c->tileKept) drop_tile(c);
+        if (state < 0 && !c->tileKept) {
+            CK(cudaStreamSynchronize(c->stream));  // what is being written is given back
+            drop_tile(c);
+        }
         c->tileErrTol = c->opt.errTol;
         c->tileLdefFact = c->opt.LdefFact;
         c->tileAlphaToB = k.law.alphaToBexp;
         c->tileState = state;
         return IDW_OK;
     };
-    if (!(tile_alloc(c, c->tileOffs, size_t(units) + 1) && tile_alloc(c, c->tileGeo, 2 * nTerms) &&
-          tile_alloc(c, c->tileMot, 8 * nTerms) && tile_alloc(c, c->tileWord, kTileWords) &&
-          tile_alloc(c, c->tileScale, size_t(c->nVol)) &&
-          tile_alloc(c, c->tileSums, std::max(2 * size_t(c->sym.nLoop) * size_t(c->nVol), size_t(1) << 16)) &&
-          tile_alloc(c, c->tileOrder, size_t(c->nVol))))
+    // what a kernel waits for is allocated before it, the rest while it runs: an
+    // allocation takes 40 us and more (615 us for 29 GB) and does not wait for the device
+    if (!(tile_alloc(c, c->tileOrder, size_t(c->nVol)) &&
+          tile_alloc(c, c->tileSums, std::max(2 * size_t(c->sym.nLoop) * size_t(c->nVol), size_t(1) << 16))))
         return serves(-1);
     // the sums are scratch until the walk; the denominators in front
     TileScratch scratch{reinterpret_cast<char *>(c->tileSums.p), c->tileSums.n * sizeof(float4)};
@@ -1095,6 +1097,10 @@ static int make_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const Eval
         if (rc) return fail(c, IDW_ERR_CUDA, "node order of the tile walks failed");
         c->tileOrderValid = true;
     }
+    if (!(tile_alloc(c, c->tileOffs, size_t(units) + 1) && tile_alloc(c, c->tileGeo, 2 * nTerms) &&
+          tile_alloc(c, c->tileMot, 8 * nTerms) && tile_alloc(c, c->tileWord, kTileWords) &&
+          tile_alloc(c, c->tileScale, size_t(c->nVol))))
+        return serves(-1);
     float *part = static_cast<float *>(scratch.take(sizeof(float) * size_t(c->sym.nLoop) * size_t(c->nVol)));
     launch_tile_geo(tree_dev(c), c->nUnique, c->ptXA.p, c->areaExp, c->tileGeo.p, c->stream);
     if (!c->tileKept) {
@@ -1119,14 +1125,14 @@ static int make_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const Eval
         if (!fits) return serves(-1);
         if (record) {
             if (!(tile_alloc(c, c->tileCnt, 8) && tile_alloc(c, c->tileTerm, entries) &&
-                  tile_alloc(c, c->tileMask, entries) && tile_alloc(c, c->tileDig, 192 * steps) &&
-                  tile_alloc(c, c->tileDig3, 64 * steps)))
+                  tile_alloc(c, c->tileMask, entries)))
                 return serves(-1);
             CK(cudaMemsetAsync(c->tileCnt.p, 0, 8 * sizeof(unsigned long long), c->stream));
             launch_tile_record(tree_dev(c), tf, vol_dev(c), rec, k, tile_dev(c), tile_all(c), c->tileOffs.p,
                                c->tileTerm.p, c->tileMask.p, c->tileCnt.p, c->stream);
             rc = check_launch(c, "walk lists");
             if (rc) return rc;
+            if (!(tile_alloc(c, c->tileDig, 192 * steps) && tile_alloc(c, c->tileDig3, 64 * steps))) return serves(-1);
             c->tileKept = true;
         }
     }

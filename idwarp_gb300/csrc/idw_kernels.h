@@ -249,8 +249,8 @@ struct TileScratch {
     }
 };
 // Tile order of the volume nodes (lo, hi: their bounding box); scratch: 20 bytes a
-// node (more saves an allocation).  Returns 0, -1 on a CUDA error, -2 without memory;
-// synchronises st.
+// node (more saves an allocation and a wait for st).  Returns 0, -1 on a CUDA error, -2
+// without memory.
 int tile_order(const VolumeDev &v, const double *lo, const double *hi, int *order, TileScratch scratch,
                cudaStream_t st);
 void launch_tile_geo(const TreeDev &t, int nPts, const dbl4 *xa, int areaExp, float4 *geo, cudaStream_t st);
@@ -356,6 +356,7 @@ int launch_adjoint_precise(const TreeDev &t, const TreeDevF &tf, const PointsDev
                            const WalkRecF &rec, const EvalConsts &k, int exact, const double *dxv, int nSeeds,
                            int64_t dxvStride, const double *den, double *ptAcc, double *nodeAcc, int nPts,
                            unsigned long long *counters, cudaStream_t st, int det = 0);
+// Sorts indices by their codes; waits for st, except with scratch that is large enough.
 int sort_morton(int64_t nVol, unsigned long long *codes, int *idx, unsigned long long *codesAlt, int *perm,
                 cudaStream_t st, void *scratch = nullptr, size_t scratchBytes = 0);
 

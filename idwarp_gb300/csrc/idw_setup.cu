@@ -565,8 +565,10 @@ int sort_morton(int64_t nVol, unsigned long long *codes, int *idx, unsigned long
     if (cub::DeviceRadixSort::SortPairs(own ? own : scratch, tmp, codes, codesAlt, idx, perm, int(nVol), 0, 63, st) !=
         cudaSuccess)
         rc = -1;
-    if (cudaStreamSynchronize(st) != cudaSuccess) rc = -1;
-    if (own) cudaFree(own);
+    if (own || !scratch) {
+        if (cudaStreamSynchronize(st) != cudaSuccess) rc = -1;
+        if (own) cudaFree(own);
+    }
     return rc;
 }
 
