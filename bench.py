@@ -948,25 +948,32 @@ def main():
         "work": {"leafPairs": st["leafPairs"], "approx": st["approx"], "visited": st["visited"],
                  "fp64Fallback": st["fp64Fallback"]},
     }
-    # roofline of the dominant kernel (the mixed walk): FP32-issue bound
+    # roofline of the walk's kernels (the tile walk and its finalisation): bytes against
+    # the measured copy rate for the tile walk, FP32 operations against the FFMA probe
+    # for the others; the other figure beside it
     flops = 42.0 * (st["leafPairs"] + st["approx"])
     peak = fp32_peak_tflops() if not args.no_extras else None
-    achieved = flops / (kernel_ms * 1e-3) / 1e12 if kernel_ms > 0 else None
-    # DRAM traffic of the walk.  The tile walk streams three FP16 digits of 32
+    kernel_s = kernel_ms * 1e-3 if kernel_ms > 0 else None
+    # DRAM traffic of the walk.  The tile walk streams four FP16 digits of 32
     # weights and a term index per list entry and keeps 64 bytes of sums per
     # node and mirror; k_walk_mixed: ncu on the 2M-node wing, 148.4 + 42.0 MB
     # for 2,025,050 nodes, scaled by volume nodes.  The tree stays in L2.
-    replay = args.mode == "fast" and st["walkListEntries"] > 0
-    traffic = 196.0 * st["walkListEntries"] + 64.0 * st["nLoop"] * nvol if replay else 94.0 * nvol
-    walk_kernel = "k_exact_mixed" if args.mode == "exact" else ("k_tile_walk" if replay else "k_walk_mixed")
-    out["roofline"] = {"bound": "hbm" if replay else "fp32", "kernel": walk_kernel, "achieved": achieved, "unit": "TFLOP/s",
-                       "peak": peak, "peak_source": "measured FFMA probe (idw_probe_ffma) in this run",
-                       "frac": (achieved / peak) if (achieved and peak) else None,
+    tile = args.mode == "fast" and st["walkListEntries"] > 0
+    traffic = 260.0 * st["walkListEntries"] + 64.0 * st["nLoop"] * nvol if tile else 94.0 * nvol
+
+    def rate(amount, most, unit, source):
+        a = amount / kernel_s if kernel_s else None
+        return {"achieved": a, "unit": unit, "peak": most, "peak_source": source,
+                "frac": a / most if a and most else None}
+
+    hbm = rate(traffic / 1e9, _measured_peak("hbm_gbs"), "GB/s", "MEASURED_PEAKS.json")
+    fp32 = rate(flops / 1e12, peak, "TFLOP/s", "measured FFMA probe (idw_probe_ffma) in this run")
+    out["roofline"] = {"bound": "hbm" if tile else "fp32",
+                       "kernel": "k_exact_mixed" if args.mode == "exact" else ("k_tile_walk" if tile else "k_walk_mixed"),
+                       **(hbm if tile else fp32), "fp32" if tile else "hbm": fp32 if tile else hbm,
                        "flops_per_launch": flops, "kernel_ms": kernel_ms, "traffic": traffic,
                        "traffic_note": "bytes per launch: the tile walk's digits, indices and sums, or ncu on the 2M-node wing "
-                                       "scaled by volume nodes",
-                       "hbm": {"achieved_GBs": traffic / (kernel_ms * 1e-3) / 1e9 if kernel_ms > 0 else None,
-                               "peak_GBs": _measured_peak("hbm_gbs"), "peak_source": "MEASURED_PEAKS.json"}}
+                                       "scaled by volume nodes"}
 
     if args.mode == "exact":
         args.no_extras = args.no_cpu_baseline = True
