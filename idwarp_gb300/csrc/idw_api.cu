@@ -930,10 +930,13 @@ static int ensure_gate_den(Ctx *c, const TreeDevF &tf, const PointsDevF &pf, con
 // default precision gate (or a looser one: their error is below the gate's).
 // A tighter gate asks for terms in double-float, which the gated walks have.
 // Their digits take every weight to be positive and no larger than its node's
-// denominator: a negative alpha has the gated walks.  So have the FP32 reverse product
-// (IDW_ADJ_FAST) with its forward walk, and the diagnostics.  Three symmetry planes
-// (8 mirror images) bound the scratch, and kTileMost node images the weight digits
-// (2.4 kB each, 3 kB with the fifth), with the lists on and off.
+// denominator: a negative alpha has the gated walks.  So has the FP32 reverse product
+// (IDW_ADJ_FAST) with its forward walk: it replays their lists, and such a context keeps
+// those alone (60 bytes a node instead of 4.3 kB; which walk's denominators divide its
+// sums makes no difference, 2.2e-7 from FP64 with each on a 7k-node wing).  So have the
+// diagnostics.  Three symmetry planes (8 mirror images) bound the scratch, and kTileMost
+// node images the weight digits (2.1 kB each, 2.6 kB with the fifth, on the 8M-node wing
+// at errTol 1e-4), with the lists on and off.
 // With the lists off every walk forms its weights anew, 3.7 ms of double-float
 // arithmetic on 4M images, and from some 2^18 images on the gated walk, which decides
 // and sums in one pass, is ahead: 99k images 0.48 against 0.53 ms (a tangent 0.69, 0.85),
