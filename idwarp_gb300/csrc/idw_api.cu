@@ -163,6 +163,7 @@ struct Ctx {
     // solver ordering
     DevBuf<int> solverInd;
     int64_t nSolver = -1;
+    int32_t solverMax = -1;  // largest of them
     // asynchronous reads of the warped grid (idw_get_volume_coordinates_async):
     // a copy stream, the grid's second buffer, and per buffer the event that
     // ends its last read (a warp writes the other buffer while a read of the
@@ -511,6 +512,7 @@ int idw_create_common_grid(void *ctx, const double *volnodes, int64_t nvol, int 
     c->den0Valid = false;
     c->haveWarp = false;
     c->haveDxs = false;
+    if (c->solverMax >= 3 * nvol) c->nSolver = -1;  // solver indices of a larger grid
     c->nVol = 0;
     CKA(c->xv0.alloc(3 * nvol));
     CKA(c->xv.alloc(3 * nvol));
@@ -2304,6 +2306,7 @@ int idw_set_external_mesh_indices(void *ctx, const int32_t *ind, int64_t ndof_so
         CK(cudaMemcpyAsync(c->solverInd.p, ind, sizeof(int) * ndof_solver, cudaMemcpyHostToDevice, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     c->nSolver = ndof_solver;
+    c->solverMax = ndof_solver > 0 ? *std::max_element(ind, ind + ndof_solver) : -1;
     return IDW_OK;
 }
 

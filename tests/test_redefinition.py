@@ -74,3 +74,24 @@ def test_a_refused_grid_needs_a_new_one(built_lib):
         g.createCommonGrid(m["xv0"])
         g.setSurfaceDefinition(m["pts"], m["conn"], m["faceSizes"])
     assert g.lib.idw_warp_mesh(g.ctx) == 0
+
+
+def test_solver_indices_of_a_larger_grid(built_lib):
+    """A smaller grid ends the indices that would reach past it; the others stay."""
+    import ctypes as C
+
+    from idwarp_gb300 import _lib
+
+    m = sphere_small()
+    g = build_gpu(m, precision="mixed")
+    n = len(m["xv0"])
+    for last, state in ((3 * n - 1, _lib.IDW_ERR_STATE), (n, 0)):
+        with contextlib.redirect_stdout(io.StringIO()):
+            g.createCommonGrid(m["xv0"])
+        ind = np.array([0, last], dtype=np.int32)
+        assert g.lib.idw_set_external_mesh_indices(g.ctx, ind.ctypes.data_as(C.POINTER(C.c_int32)), 2) == 0
+        with contextlib.redirect_stdout(io.StringIO()):
+            g.createCommonGrid(m["xv0"][: n // 2])
+        w, s = np.arange(3.0 * (n // 2)), np.zeros(2)
+        assert g.lib.idw_warp_to_solver_grid(g.ctx, _lib.dptr(w), w.size, _lib.dptr(s), 2, _lib.IDW_HOST) == state
+        assert s.tolist() == ([0.0, float(n)] if state == 0 else [0.0, 0.0])
