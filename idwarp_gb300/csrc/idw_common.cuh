@@ -68,9 +68,9 @@ __device__ __forceinline__ float ipowf(float x, int n) {
 // 1 - q y^2 of the FP32 reciprocal square root y, |e| < 2^-21: y (1 + e/2 + 3/8
 // e^2)).  Five FP64 operations, the conversions being moves of bits, where a
 // square root and a division take some 18; an FP64 instruction holds this GPU's
-// pipe for 16 cycles (the denominator estimate of the 2M-node wing 111 -> 59 ms,
-// the error tables 9.8 -> 5.1, the FP64 walk of the 95k-node sphere 7.04 -> 5.30;
-// all three fill that pipe).  q outside FP32's normal range goes the long way.
+// pipe for 16 cycles (the error tables of the 2M-node wing 9.8 -> 5.1 ms, the FP64
+// walk of the 95k-node sphere 7.04 -> 5.30; both fill that pipe).  q outside FP32's
+// normal range goes the long way.
 __device__ __forceinline__ double inv_sqrt64(double q) {
     const unsigned hi = unsigned(__double2hiint(q)) - 0x38000000u;  // exponent to FP32's bias
     if (hi - 0x00200000u >= 0x0fb00000u) return 1.0 / sqrt(q);
@@ -80,6 +80,21 @@ __device__ __forceinline__ double inv_sqrt64(double q) {
     const double y0 = __hiloint2double(int((b >> 3) + 0x38000000u), int(b << 29));
     const double e = fma(-q, y0 * y0, 1.0);  // the square is exact
     return fma(y0 * e, fma(e, 0.375, 0.5), y0);
+}
+
+// L / sqrt(q), the root and the quotient rounded as the two operations are: each
+// approximation from y = 1 / sqrt(q) corrected by its residual, which an FMA gives
+// exactly (P. Markstein, IBM J. Res. Dev. 34, 1990).  A corrected value is within 2^-104
+// before its rounding, so one in 2^50 may fall on the other side.  11 FP64 operations.
+// L within 1e-60 and 1e60.
+__device__ __forceinline__ double div_sqrt64(double L, double q) {
+    const unsigned hi = unsigned(__double2hiint(q)) - 0x38000000u;
+    if (hi - 0x00200000u >= 0x0fb00000u) return L / sqrt(q);
+    const double y = inv_sqrt64(q);
+    const double s0 = q * y;
+    const double s = fma(fma(-s0, s0, q), __hiloint2double(__double2hiint(y) - 0x100000, __double2loint(y)), s0);
+    const double l0 = L * y;
+    return fma(fma(-l0, s, L), y, l0);
 }
 
 // (L/d)^a + alpha^b (L/d)^b for a given LdefoDist = L/d, FP64.

@@ -135,18 +135,19 @@ __global__ void k_den0(TreeDev t, const NodeRecF *rf, const dbl4 *ptXA, VolumeDe
     const int vi = !valid ? 0 : (stride > 0 ? int(gid * stride) : v.perm[gid]);
     double x0[3] = {v.xv0[3 * vi], v.xv0[3 * vi + 1], v.xv0[3 * vi + 2]};
     double acc = 0.0;
-    // at the exponents (3, 5) a term is L^3 A y^3 (1 + kappa y^2), y = 1/d, and L^3
-    // waits for the end: one operation fewer of 17 a pair (59.1 -> 55.5 ms, 2M
-    // nodes)
-    const bool law35 = law.isInt && law.ia == 3 && law.ib == 5 && law.Ldef > 1e-60 && law.Ldef < 1e60;
-    const double kappa = law.alphaToBexp * law.Ldef * law.Ldef;
+    // A restart file keeps these sums, and its check refuses them when the estimate is
+    // 1e-15 below: the last bits of sums of thousands of terms, so every term has the
+    // bits of A ((L/d)^3 + alpha^5 (L/d)^5) with a rounded root and quotient.  (Terms
+    // L^3 A y^3 (1 + kappa y^2) from a reciprocal square root take 16 instead of 23 FP64
+    // operations a pair, and moved the sums of the 8M-node wing by up to 2.5e-14.)
+    const bool law35 = law.isInt && law.ia == 3 && law.ib == 5, usual = law.Ldef > 1e-60 && law.Ldef < 1e60;
     auto add = [&](double A, double d2) {
-        const double y = inv_sqrt64(d2);
+        const double LoD = usual ? div_sqrt64(law.Ldef, d2) : law.Ldef / sqrt(d2);
         if (law35) {
-            const double y2 = y * y;
-            acc = fma(A, (y2 * y) * fma(kappa, y2, 1.0), acc);
+            const double s = LoD * LoD, ta = LoD * s;
+            acc = fma(A, fma(law.alphaToBexp, ta * s, ta), acc);
         } else {
-            acc += A * law64(law, law.Ldef * y);
+            acc += A * law64(law, LoD);
         }
     };
     for (int kk = 0; kk < sym.nLoop; ++kk) {
@@ -167,7 +168,7 @@ __global__ void k_den0(TreeDev t, const NodeRecF *rf, const dbl4 *ptXA, VolumeDe
                     for (int i = inf.x; i <= inf.y; ++i) {
                         dbl4 x = ptXA[i];
                         double r0 = r[0] - x.x, r1 = r[1] - x.y, r2 = r[2] - x.z;
-                        add(x.w, r0 * r0 + r1 * r1 + (r2 * r2 + 1e-16));
+                        add(x.w, r0 * r0 + r1 * r1 + r2 * r2 + 1e-16);
                     }
                 }
                 node = inf.z;
@@ -202,7 +203,6 @@ __global__ void k_den0(TreeDev t, const NodeRecF *rf, const dbl4 *ptXA, VolumeDe
             }
         }
     }
-    if (law35) acc *= law.Ldef * law.Ldef * law.Ldef;
     if (valid) out[stride > 0 ? gid : int64_t(vi)] = acc;
 }
 
