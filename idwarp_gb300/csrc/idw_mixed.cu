@@ -231,7 +231,10 @@ void launch_walk_mixed(const TreeDev &t, const TreeDevF &tf, const PointsDevF &p
         // every pair: the tiled kernel, with the walk's arithmetic.  Its packed
         // form at the default exponents is ahead of the walk from the smallest
         // meshes on (1.5k nodes 0.22 against 0.26 ms, 30k 1.85 against 2.22, 245k
-        // 12.8 against 24.1); the others need full waves
+        // 12.8 against 24.1), but for meshes of half a wave with few surface points
+        // whose motions leave a third of the pairs to double-float (95k-node sphere, 1946
+        // points, 2.61 against 2.28; 0.47 against 0.78 where none is left), which sizes do
+        // not tell.  The others need full waves
         launch_exact_mixed(tf, pf, af, v, rec, mp, k.law, acc, o.counters, st);
     } else if (!exact && k.lists.list && !mp.slotStats) {
         // recorded decisions: the walk's terms without the walk's decisions;
