@@ -934,7 +934,7 @@ static int ensure_gate_den(Ctx *c, const TreeDevF &tf, const PointsDevF &pf, con
 // Their digits take every weight to be positive and no larger than its node's
 // denominator: a negative alpha has the gated walks.  So has the FP32 reverse product
 // (IDW_ADJ_FAST) with its forward walk: it replays their lists, and such a context keeps
-// those alone (60 bytes a node instead of 4.3 kB; which walk's denominators divide its
+// those alone (60 bytes a node instead of 4.4 kB; which walk's denominators divide its
 // sums makes no difference, 2.2e-7 from FP64 with each on a 7k-node wing).  So have the
 // diagnostics.  Three symmetry planes (8 mirror images) bound the scratch, and kTileMost
 // node images the weight digits (2.1 kB each, 2.6 kB with the fifth, on the 8M-node wing
@@ -967,11 +967,11 @@ static TileDev tile_dev(Ctx *c) {
     return td;
 }
 
-// Half of the free device memory and of `held` bytes to be given back holds `bytes`.
-static int fits_half(Ctx *c, double bytes, bool &yes, double held = 0.0) {
+// Half of the free device memory and of `held` bytes to be given back.
+static int half_free(Ctx *c, double held, double &half) {
     size_t freeB = size_t(c->tileFree), totalB = 0;
     if (c->tileFree < 0) CK(cudaMemGetInfo(&freeB, &totalB));
-    yes = bytes <= 0.5 * (double(freeB) + held);
+    half = 0.5 * (double(freeB) + held);
     return IDW_OK;
 }
 
@@ -1109,29 +1109,32 @@ static int make_tile(Ctx *c, const TreeDevF &tf, const WalkRecF &rec, const Eval
     float *part = static_cast<float *>(scratch.take(sizeof(float) * size_t(c->sym.nLoop) * size_t(c->nVol)));
     launch_tile_geo(tree_dev(c), c->nUnique, c->ptXA.p, c->areaExp, c->tileGeo.p, c->stream);
     if (!c->tileKept) {
-        const int64_t total = count_tile_lists(tree_dev(c), tf, vol_dev(c), rec, k, tile_dev(c), c->tileOffs.p,
-                                               off ? part : nullptr, scratch, c->stream);
-        if (total == -2) return serves(-1);
-        if (total < 0) return fail(c, IDW_ERR_CUDA, "walk lists: count pass failed");
-        c->tileListEntries = total;
-        const size_t entries = size_t(std::max<int64_t>(total, 16)), steps = entries / 16;
-        // lists and digits of an earlier recording make room for these, in place where
-        // they are large enough and not twice too large (7 GB take 4 ms to give back)
-        const size_t n = c->tileTerm.n;
-        if (record && (n < entries || n > 2 * entries || c->tileMask.n < entries || c->tileDig.n < 192 * steps ||
-                       c->tileDig3.n < 64 * steps))
-            drop_tile_kept(c);
-        const double need = 8.0 * double(entries) + 320.0 * sizeof(uint4) * double(steps) + 8.0 * double(c->nVol);
         const double held = 8.0 * double(c->tileTerm.n + c->tileDenInv.n) +
                             sizeof(uint4) * double(c->tileDig.n + c->tileDig3.n + c->tileDig4.n);
-        bool fits = false;
-        int rc = fits_half(c, need, fits, held);
+        double half = 0.0;
+        int rc = IDW_OK;
+        bool room = true;
+        const int64_t total = count_tile_lists(
+            tree_dev(c), tf, vol_dev(c), rec, k, tile_dev(c), c->tileOffs.p, off ? part : nullptr, scratch, c->stream, [&] {
+                rc = half_free(c, held, half);
+                // the first lists' memory before their length is known: 16 entries a node
+                // image hold most meshes' (4 to 16), and are a twentieth of the digits at 8
+                const size_t guess = 16 * std::max<size_t>(size_t(c->sym.nLoop) * size_t(c->nVol), 1);
+                room = !record ||
+                       (tile_alloc(c, c->tileCnt, 8) && (c->tileTerm.p || tile_alloc(c, c->tileTerm, guess)) &&
+                        (c->tileMask.p || tile_alloc(c, c->tileMask, guess)));
+            });
         if (rc) return rc;
-        if (!fits) return serves(-1);
+        if (total == -2 || (total >= 0 && !room)) return serves(-1);
+        if (total < 0) return fail(c, IDW_ERR_CUDA, "walk lists: count pass failed");
+        c->tileListEntries = total;
+        const size_t entries = size_t(std::max<int64_t>(total, 16)), steps = entries / 16, n = c->tileDig.n;
+        // lists and digits of an earlier recording make room for these, in place where
+        // they are large enough and not twice too large (7 GB take 4 ms to give back)
+        if (record && n && (n < 192 * steps || n > 2 * 192 * steps || c->tileDig3.n < 64 * steps)) drop_tile_kept(c);
+        if (8.0 * double(entries) + 320.0 * sizeof(uint4) * double(steps) + 8.0 * double(c->nVol) > half) return serves(-1);
         if (record) {
-            if (!(tile_alloc(c, c->tileCnt, 8) && tile_alloc(c, c->tileTerm, entries) &&
-                  tile_alloc(c, c->tileMask, entries)))
-                return serves(-1);
+            if (!(tile_alloc(c, c->tileTerm, entries) && tile_alloc(c, c->tileMask, entries))) return serves(-1);
             CK(cudaMemsetAsync(c->tileCnt.p, 0, 8 * sizeof(unsigned long long), c->stream));
             launch_tile_record(tree_dev(c), tf, vol_dev(c), rec, k, tile_dev(c), tile_all(c), c->tileOffs.p,
                                c->tileTerm.p, c->tileMask.p, c->tileCnt.p, c->stream);

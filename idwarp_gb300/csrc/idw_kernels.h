@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <functional>
+
 #include "idw_common.cuh"
 
 namespace idw {
@@ -256,10 +258,10 @@ int tile_order(const VolumeDev &v, const double *lo, const double *hi, int *orde
 void launch_tile_geo(const TreeDev &t, int nPts, const dbl4 *xa, int areaExp, float4 *geo, cudaStream_t st);
 // Fills offs and returns the number of entries (-1 on a CUDA error, -2 where the
 // scratch ends), and with part (nLoop nVol floats) the units' FP32 denominators.
-// Synchronises st.
+// Calls meanwhile while the kernel runs; synchronises st.
 int64_t count_tile_lists(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
                          const EvalConsts &k, const TileDev &td, int64_t *offs, float *part, TileScratch scratch,
-                         cudaStream_t st);
+                         cudaStream_t st, const std::function<void()> &meanwhile);
 // Fills scale and raises *bad when a node has none, from the denominators in part
 // (of the lists, if there are any; else those of count_tile_lists).
 void launch_tile_scales(const VolumeDev &v, const WalkRecF &rec, const EvalConsts &k, const TileDev &td,

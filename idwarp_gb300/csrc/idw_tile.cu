@@ -629,7 +629,7 @@ static int law_exp(const EvalConsts &k, const TileDev &td) { return 3 * ilogb(k.
 
 int64_t count_tile_lists(const TreeDev &t, const TreeDevF &tf, const VolumeDev &v, const WalkRecF &rec,
                          const EvalConsts &k, const TileDev &td, int64_t *offs, float *part, TileScratch scratch,
-                         cudaStream_t st) {
+                         cudaStream_t st, const std::function<void()> &meanwhile) {
     const MixedParams mp = make_mixed_params(k);
     const int64_t nGroups = walk_list_warps(v.nVol);
     const int64_t n = nGroups * mp.nLoop;
@@ -649,6 +649,7 @@ int64_t count_tile_lists(const TreeDev &t, const TreeDevF &tf, const VolumeDev &
     void *tmp = scratch.take(tmpBytes);
     if (ok && !tmp) return -2;
     if (ok) ok = cub::DeviceScan::ExclusiveSum(tmp, tmpBytes, counts, offs, int(n + 1), st) == cudaSuccess;
+    meanwhile();
     if (ok) ok = cudaMemcpyAsync(&total, offs + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st) == cudaSuccess;
     if (cudaStreamSynchronize(st) != cudaSuccess) ok = false;
     return ok ? total : -1;
